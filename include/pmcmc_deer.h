@@ -273,8 +273,8 @@ int pmcmc_slice_result(pmcmc_handle* h, const void* xbar0, void* S_out, void* lo
 
 /* ---- diagonal affine scan ----------------------------------------------------
  * Replaces DEERScan.solve_affine_scan_diag! (src/DEER/DEERScan.jl:102-173):
- * S[:,t] = A[:,t] .* S[:,t-1] + B[:,t], S[:,0-1] = s0.  Single-pass
- * decoupled-lookback scan.  S may not alias A or B (DEERScan.jl:124-125). */
+ * S[:,t] = A[:,t] .* S[:,t-1] + B[:,t], S[:,0-1] = s0.  One
+ * cooperative launch (a few for long scans).  S may not alias A or B (DEERScan.jl:124-125). */
 int pmcmc_affine_scan_diag(pmcmc_handle* h, int32_t dtype, int64_t D, int64_t T, const void* A,
                            const void* B, const void* s0, void* S, int32_t mem);
 
@@ -285,11 +285,11 @@ int pmcmc_affine_scan_diag(pmcmc_handle* h, int32_t dtype, int64_t D, int64_t T,
  * memory budget, or a latency-critical loop that cannot take an allocation's
  * implicit synchronisation): the same scan as pmcmc_affine_scan_diag, with A,
  * B, s0 and S device pointers on the current device and no handle.  The
- * look-back scratch is a static device array of PMCMC_NOALLOC_SCRATCH_BYTES
+ * scan's scratch is a static device array of PMCMC_NOALLOC_SCRATCH_BYTES
  * (4 MiB) that every GPU loading the library holds until the process exits;
  * no cudaMalloc, cudaFree or allocating library routine is called.  A size
- * whose scratch exceeds the array returns PMCMC_ERR_NOMEM (the scratch needed
- * is about 3 * sizeof(element) * D * ceil(T / tile) bytes, tile <= 64 columns).
+ * whose scratch exceeds the array returns PMCMC_ERR_NOMEM (counted
+ * as about 3 * sizeof(element) * D * ceil(T / tile) bytes, tile <= 64 columns).
  * The first call on a device looks up the array's device address; make that
  * first call before any stream capture.  The array takes its device memory
  * when the library's device code is loaded on a device: under lazy module

@@ -67,7 +67,6 @@ struct pmcmc_handle {
   size_t ws_bytes = 0;
   unsigned char* scan_ws = nullptr;
   size_t scan_ws_bytes = 0;
-  uint32_t scan_epoch = 0;
   cudaGraphExec_t gexec = nullptr;
   cudaGraphConditionalHandle cond = 0;
   GraphKey gkey;
@@ -2226,14 +2225,8 @@ int pmcmc_affine_scan_diag(pmcmc_handle* h, int32_t dtype, int64_t D, int64_t T,
     return fail(h, PMCMC_ERR_UNSUPPORTED, "dimension %lld too large for the scan kernel",
                 (long long)D);
   DeviceGuard guard(h->device);
-  const int TT = scan_tile_cols(D, T);
-  const int64_t nt = (T + TT - 1) / TT;
-  // scratch: counter[2] | flags[nt] | agg_a | agg_b | incl | (host I/O staging)
-  const size_t o_flags = 64;
-  const size_t o_agg_a = (o_flags + 4 * static_cast<size_t>(nt) + 255) & ~size_t(255);
-  const size_t o_agg_b = o_agg_a + ((es * nt * D + 255) & ~size_t(255));
-  const size_t o_incl = o_agg_b + ((es * nt * D + 255) & ~size_t(255));
-  const size_t o_io = o_incl + ((es * nt * D + 255) & ~size_t(255));
+  // scratch of the scan | host I/O staging
+  const size_t o_io = (scan_scratch_bytes(f64, D, T) + 255) & ~size_t(255);
   const size_t need = o_io + (mem == PMCMC_MEM_HOST ? 3 * es * D * T + es * D + 256 : 0);
   if (need > h->scan_ws_bytes) {
     CK(cudaStreamSynchronize(h->stream));
@@ -2244,16 +2237,9 @@ int pmcmc_affine_scan_diag(pmcmc_handle* h, int32_t dtype, int64_t D, int64_t T,
       cudaGetLastError();
       return fail(h, PMCMC_ERR_NOMEM, "scan scratch allocation failed");
     }
-    CK(cudaMemsetAsync(h->scan_ws, 0, need, h->stream));
     h->scan_ws_bytes = need;
   }
   unsigned char* base = h->scan_ws;
-  ScanScratch scr;
-  scr.counter = reinterpret_cast<uint32_t*>(base);
-  scr.flags = reinterpret_cast<uint32_t*>(base + o_flags);
-  scr.agg_a = base + o_agg_a;
-  scr.agg_b = base + o_agg_b;
-  scr.incl = base + o_incl;
   const void *dA = A, *dB = B, *ds0 = s0;
   void* dS = S;
   if (mem == PMCMC_MEM_HOST) {
@@ -2266,15 +2252,10 @@ int pmcmc_affine_scan_diag(pmcmc_handle* h, int32_t dtype, int64_t D, int64_t T,
     CK(cudaMemcpyAsync(const_cast<void*>(dB), B, es * D * T, cudaMemcpyHostToDevice, h->stream));
     CK(cudaMemcpyAsync(const_cast<void*>(ds0), s0, es * D, cudaMemcpyHostToDevice, h->stream));
   }
-  h->scan_epoch = (h->scan_epoch + 1) & 0x3fffffffu;
-  if (h->scan_epoch == 0) h->scan_epoch = 1;
-  CK(launch_affine_scan(h->stream, f64, D, T, dA, dB, ds0, dS, scr, h->scan_epoch));
+  CK(launch_affine_scan(h->stream, f64, D, T, dA, dB, ds0, dS, base));
   if (mem == PMCMC_MEM_HOST)
     CK(cudaMemcpyAsync(S, dS, es * D * T, cudaMemcpyDeviceToHost, h->stream));
-  uint32_t flags[2] = {0, 0};
-  CK(cudaMemcpyAsync(flags, scr.counter, sizeof flags, cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
-  if (flags[1]) return fail(h, PMCMC_ERR_TIMEOUT, "scan look-back wait exceeded its bound");
   return PMCMC_OK;
 }
 
@@ -2545,18 +2526,11 @@ int pmcmc_deer_adjoint(pmcmc_handle* h, const pmcmc_target* tg, const pmcmc_deer
       std::min<int64_t>((T * (Dp / 4) + 255) / 256, int64_t(h->num_sms) * 8));
   void* init_args[] = {&h->d_params, &h->d_state};
   CK(cudaLaunchKernel(k.init, dim3(init_grid), dim3(256), init_args, 0, h->stream));
-  h->scan_epoch = (h->scan_epoch + 1) & 0x3fffffffu;
-  if (h->scan_epoch == 0) h->scan_epoch = 1;
   double* out = reinterpret_cast<double*>(ws + L.aout);
   CK(full_adjoint(h->stream, h->d_params, h->d_full, F, D, Dp, T, tg->kind, h->num_sms,
-                  objective, reinterpret_cast<const float*>(ws + L.S0), out, ws + L.ascr,
-                  h->scan_epoch));
-  uint32_t flags[2] = {0, 0};
+                  objective, reinterpret_cast<const float*>(ws + L.S0), out, ws + L.ascr));
   CK(cudaMemcpyAsync(grad, out, sizeof(double) * (1 + D), cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaMemcpyAsync(flags, ws + L.ascr, sizeof flags, cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
-  if (flags[1])
-    return fail(h, PMCMC_ERR_TIMEOUT, "adjoint scan look-back wait exceeded its bound");
   return PMCMC_OK;
 }
 
@@ -2582,33 +2556,10 @@ int slice_copy_out(pmcmc_handle* h, void* dst, const void* src, size_t bytes, in
   return PMCMC_OK;
 }
 
-ScanScratch slice_scratch(pmcmc_handle* h) {
-  SliceState& sl = h->slice;
-  unsigned char* w = h->ws + sl.scr;
-  const int64_t Dp = sl.P.Dp, W = sl.P.T;
-  const int TT = scan_tile_cols(Dp, W);
-  const int64_t nt = (W + TT - 1) / TT;
-  auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
-  ScanScratch scr;
-  scr.counter = reinterpret_cast<uint32_t*>(w);
-  size_t off = 256;
-  scr.flags = reinterpret_cast<uint32_t*>(w + off);
-  off += al(4 * static_cast<size_t>(nt));
-  scr.agg_a = w + off;
-  off += al(sl.es * nt * Dp);
-  scr.agg_b = w + off;
-  off += al(sl.es * nt * Dp);
-  scr.incl = w + off;
-  return scr;
-}
-
 int slice_scan(pmcmc_handle* h, const void* B, const void* s0, void* out) {
   SliceState& sl = h->slice;
-  ScanScratch scr = slice_scratch(h);
-  h->scan_epoch = (h->scan_epoch + 1) & 0x3fffffffu;
-  if (h->scan_epoch == 0) h->scan_epoch = 1;
-  CK(launch_affine_scan(h->stream, sl.es == 8, sl.P.Dp, sl.P.T, h->ws + sl.A, B, s0, out, scr,
-                        h->scan_epoch));
+  CK(launch_affine_scan(h->stream, sl.es == 8, sl.P.Dp, sl.P.T, h->ws + sl.A, B, s0, out,
+                        h->ws + sl.scr));
   return PMCMC_OK;
 }
 
@@ -2655,7 +2606,7 @@ int pmcmc_slice_begin(pmcmc_handle* h, const pmcmc_target* tg, const pmcmc_deer_
   sl.xi = take(4 * W * Dp);
   sl.logu = take(8 * static_cast<size_t>(W));
   sl.red = take(4 * sizeof(unsigned long long));
-  sl.scr = take(scan_scratch_bytes(es == 8, Dp, W) + 1024);
+  sl.scr = take(scan_scratch_bytes(es == 8, Dp, W));
   sl.out_S = take(es * W * D);
   sl.out_lp = take(es * W);
   sl.out_acc = take(static_cast<size_t>(W));
@@ -2751,10 +2702,7 @@ int pmcmc_slice_local(pmcmc_handle* h, const void* xbar0, void* agg, int32_t mem
   if (rc) return rc;
   rc = slice_copy_out(h, out, ws + sl.Sloc + es * (W - 1) * Dp, es * D, mem);
   if (rc) return rc;
-  uint32_t flags[2] = {0, 0};
-  CK(cudaMemcpyAsync(flags, ws + sl.scr, sizeof flags, cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
-  if (flags[1]) return fail(h, PMCMC_ERR_TIMEOUT, "slice scan look-back wait exceeded its bound");
   return PMCMC_OK;
 }
 
@@ -2781,11 +2729,8 @@ int pmcmc_slice_finish(pmcmc_handle* h, const void* carry_in, void* last_out, do
     if (rc) return rc;
   }
   unsigned long long hr[3] = {0, 0, 0};
-  uint32_t flags[2] = {0, 0};
   CK(cudaMemcpyAsync(hr, r, sizeof hr, cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaMemcpyAsync(flags, ws + sl.scr, sizeof flags, cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
-  if (flags[1]) return fail(h, PMCMC_ERR_TIMEOUT, "slice scan look-back wait exceeded its bound");
   std::memcpy(&red[0], &hr[0], 8);
   std::memcpy(&red[1], &hr[1], 8);
   sl.cur ^= 1;

@@ -63,20 +63,12 @@ cudaError_t launch_mala_chains(cudaStream_t s, bool f64, int tk, const DevParams
 cudaError_t launch_tape(cudaStream_t s, int64_t D, int64_t T, uint64_t seed, uint64_t block,
                         float* Xi, float* u);
 
-// Standalone diagonal affine scan (scan_diag.cu).  Scratch: flags[ntiles],
-// agg_a/agg_b/incl[ntiles * Dp] of the element type, counter[1].
-struct ScanScratch {
-  uint32_t* flags;
-  void* agg_a;
-  void* agg_b;
-  void* incl;
-  uint32_t* counter;
-};
+// Standalone diagonal affine scan (tape_scan.cu); `scratch` holds
+// scan_scratch_bytes and needs no clearing.
 int scan_tile_cols(int64_t D, int64_t T);
 size_t scan_scratch_bytes(bool f64, int64_t D, int64_t T);
 cudaError_t launch_affine_scan(cudaStream_t s, bool f64, int64_t D, int64_t T, const void* A,
-                               const void* B, const void* s0, void* S, const ScanScratch& scr,
-                               uint32_t epoch);
+                               const void* B, const void* s0, void* S, void* scratch);
 
 // Plain path (tape_scan.cu): the reference's Hillis-Steele doubling scan
 // (DEERScan.jl:102-173) as one launch per level over buffers of T x Dp

@@ -950,17 +950,14 @@ cudaError_t full_sweep(cudaStream_t s, const FullPlan& fp, const DevParams* Pg, 
   return cudaSuccess;
 }
 
-// scratch: counter (256 B) | zero vector | flags | agg_a | agg_b | incl
+// scratch: zero vector | the scan's
 size_t full_adjoint_scratch_bytes(int64_t Dp, int64_t T) {
-  const int TT = scan_tile_cols(Dp, T);
-  const int64_t nt = (T + TT - 1) / TT;
-  return 256 + al256(4 * Dp) + al256(4 * static_cast<size_t>(nt)) + 3 * al256(4 * nt * Dp);
+  return al256(4 * Dp) + al256(scan_scratch_bytes(false, Dp, T));
 }
 
 cudaError_t full_adjoint(cudaStream_t s, const DevParams* Pg, const FullArgs* Fg,
                          const FullArgs& Fh, int64_t D, int64_t Dp, int64_t T, int tkind,
-                         int num_sms, int objective, const float* S, double* out, void* scratch,
-                         uint32_t epoch) {
+                         int num_sms, int objective, const float* S, double* out, void* scratch) {
   const bool dense = tkind == kDenseGauss;
   cudaError_t e = cudaMemsetAsync(out, 0, sizeof(double) * (1 + D), s);
   if (e == cudaSuccess) e = cudaMemsetAsync(Fh.direct, 0, sizeof(double), s);
@@ -983,25 +980,10 @@ cudaError_t full_adjoint(cudaStream_t s, const DevParams* Pg, const FullArgs* Fg
   if (e != cudaSuccess) return e;
   // reverse scan in reversed time: Lrev_tau = Arev_tau * Lrev_{tau-1} + Brev_tau, Lrev_{-1} = 0
   unsigned char* w = static_cast<unsigned char*>(scratch);
-  const int TT = scan_tile_cols(Dp, T);
-  const int64_t ntl = (T + TT - 1) / TT;
-  ScanScratch scr;
-  scr.counter = reinterpret_cast<uint32_t*>(w);
-  size_t off = 256;
-  float* zero = reinterpret_cast<float*>(w + off);
-  off += al256(4 * Dp);
-  scr.flags = reinterpret_cast<uint32_t*>(w + off);
-  off += al256(4 * static_cast<size_t>(ntl));
-  scr.agg_a = w + off;
-  off += al256(4 * ntl * Dp);
-  scr.agg_b = w + off;
-  off += al256(4 * ntl * Dp);
-  scr.incl = w + off;
+  float* zero = reinterpret_cast<float*>(w);
   e = cudaMemsetAsync(zero, 0, sizeof(float) * Dp, s);
-  // the workspace may hold other data where the flags live: clear them (epoch 0 is never used)
-  if (e == cudaSuccess) e = cudaMemsetAsync(scr.flags, 0, 4 * static_cast<size_t>(ntl), s);
   if (e != cudaSuccess) return e;
-  e = launch_affine_scan(s, false, Dp, T, Arev, Brev, zero, Fh.lam_adj, scr, epoch);
+  e = launch_affine_scan(s, false, Dp, T, Arev, Brev, zero, Fh.lam_adj, w + al256(4 * Dp));
   if (e != cudaSuccess) return e;
   e = cudaMemcpyAsync(out, Fh.direct, sizeof(double), cudaMemcpyDeviceToDevice, s);
   if (e != cudaSuccess) return e;

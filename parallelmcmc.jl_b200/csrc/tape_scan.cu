@@ -1,4 +1,5 @@
 // tape_scan.cu -- tape materialisation and the standalone diagonal affine scan.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -8,7 +9,20 @@
 #include "deer_device.cuh"
 #include "deer_launch.h"
 
+namespace cg = cooperative_groups;
+
 namespace pmcmc {
+
+namespace {
+constexpr int kScanWindow = 2048;  // most columns composed before a state is applied
+
+struct ScanPlan {
+  int nchunks, L;       // chunks of L columns
+  int nblk_d, blk_d;    // blocks of blk_d coordinates
+  int nsub, Ls;         // runs of Ls columns inside a chunk
+  int group, threads;   // chunks composed at a time; threads a CTA
+};
+}  // namespace
 
 // Tape block of (seed, block): Xi (D x T, column-major) and u (T)
 // (counterpart of _make_mala_tape_block, interface.jl:334-358).
@@ -40,84 +54,175 @@ cudaError_t launch_tape(cudaStream_t s, int64_t D, int64_t T, uint64_t seed, uin
 
 // ---------------------------------------------------------------------------
 // S[:,t] = A[:,t] .* S[:,t-1] + B[:,t] (solve_affine_scan_diag!, DEERScan.jl:102-173)
-// as one pass: each CTA stages a tile of TT columns, scans it in shared memory,
-// and obtains the state entering the tile by decoupled look-back.  HBM traffic
-// is one read of A and B and one write of S.
+// in one cooperative launch.  The columns are cut into chunks, one a CTA (and a
+// block of up to 256 coordinates); inside it `nsub` runs of consecutive columns a
+// coordinate, one a thread:
+//   1. every thread composes its run, 64 bytes of A and of B in flight; the runs'
+//      maps are composed in shared memory into the chunk's;
+//   2. after a grid barrier, one warp a coordinate carries the state over the
+//      chunks: each lane composes `group` chunks, the lanes' maps are applied to
+//      the state in turn, and each lane replays its group;
+//   3. after a second barrier every thread replays the recurrence over its run.
+// Bound: HBM, one read of A and B and one write of S; phase 3's second read of A
+// and B comes from L2, which a launch's columns fit (scan_plan).  The look-back over
+// 64-column tiles that this replaces was a serial chain of T / 2048 hops: 471 us at
+// D = 100, T = 65536 in FP32 (78.6 MB), against 29 us here (2.7 TB/s; the floor is
+// 12 us, phase 2 and the barriers take 9).
+// States are carried by composition over at most 2048 columns at a time, as the
+// look-back did, so a coordinate that stays at zero under growing maps stays at
+// zero.  A cooperative launch's CTAs are co-resident, so the barriers end.
 // ---------------------------------------------------------------------------
+// CTAs an SM and chunks a lane composes at a time, without spills: a spilled value in
+// phase 2 is read from L2 each time, because the CTAs that already wait at the barrier
+// invalidate the SM's L1 with every poll (17 us of a 28 us scan at D = 64, T = 2048)
+constexpr int kScanCtas = 3;
 template <typename Real>
-__global__ void __launch_bounds__(kThreads)
-    affine_scan_kernel(int64_t D, int64_t T, int TT, const Real* __restrict__ A,
-                       const Real* __restrict__ B, const Real* __restrict__ s0,
-                       Real* __restrict__ S, ScanScratch scr, uint32_t epoch) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ int s_tile, s_err, s_jstar;
+constexpr int kScanLoads = 64 / sizeof(Real);  // columns of loads in flight a thread
+template <typename Real>
+constexpr int kScanGroup = sizeof(Real) == 4 ? 8 : 4;
+
+template <typename Real>
+__global__ void __launch_bounds__(kThreads, kScanCtas)
+    affine_scan_kernel(int64_t D, int64_t T, ScanPlan pl, const Real* __restrict__ A,
+                       const Real* __restrict__ B, const Real* s0, Real* __restrict__ S,
+                       Real* __restrict__ agg_a, Real* __restrict__ agg_b,
+                       Real* __restrict__ carry) {
+  __shared__ Real s_a[kThreads], s_b[kThreads];
+  cg::grid_group grid = cg::this_grid();
+  constexpr int kScanUnroll = kScanLoads<Real>;
   const int tid = threadIdx.x;
-  if (tid == 0) {
-    s_tile = static_cast<int>(atomicAdd(scr.counter, 1u));
-    s_err = 0;
-  }
-  __syncthreads();
-  const int tile = s_tile;
+  const int nch = pl.nchunks;
+  const int db = static_cast<int>(blockIdx.x) % pl.nblk_d;
+  const int ch = static_cast<int>(blockIdx.x) / pl.nblk_d;
+  const int sub = tid / pl.blk_d, dl = tid - sub * pl.blk_d;
+  const int64_t d = static_cast<int64_t>(db) * pl.blk_d + dl;
+  const bool active = sub < pl.nsub && d < D;
+  const int64_t c0 = static_cast<int64_t>(ch) * pl.L, c1 = imin64(T, c0 + pl.L);
+  const int64_t u0 = imin64(c1, c0 + static_cast<int64_t>(sub) * pl.Ls);
+  const int64_t u1 = imin64(c1, u0 + pl.Ls);
+  // columns past the run load the identity map, which changes nothing
   const int Di = static_cast<int>(D);
-  const int64_t t0 = static_cast<int64_t>(tile) * TT;
-  const int ncols = static_cast<int>(imin64(TT, T - t0));
-  Real* As = reinterpret_cast<Real*>(smem_raw);
-  Real* Bs = As + static_cast<size_t>(TT) * Di;
-  Real* carry = Bs + static_cast<size_t>(TT) * Di;
-  const int64_t base = t0 * D, n = static_cast<int64_t>(ncols) * D;
-  for (int64_t i = tid; i < n; i += kThreads) {
-    As[i] = A[base + i];
-    Bs[i] = B[base + i];
+  auto load = [&](const Real* pa, const Real* pb, int n, Real (&va)[kScanUnroll],
+                   Real (&vb)[kScanUnroll]) {
+#pragma unroll
+    for (int k = 0; k < kScanUnroll; ++k) {
+      va[k] = k < n ? pa[k * Di] : Real(1);
+      vb[k] = k < n ? pb[k * Di] : Real(0);
+    }
+  };
+  Real a = 1, b = 0;
+  if (active) {
+    const Real *pa = A + u0 * D + d, *pb = B + u0 * D + d;
+    for (int n = static_cast<int>(u1 - u0); n > 0;
+         n -= kScanUnroll, pa += kScanUnroll * Di, pb += kScanUnroll * Di) {
+      Real va[kScanUnroll], vb[kScanUnroll];
+      load(pa, pb, n, va, vb);
+#pragma unroll
+      for (int k = 0; k < kScanUnroll; ++k)
+        if (k < n) {
+          b = va[k] * b + vb[k];
+          a = va[k] * a;
+        }
+    }
   }
+  s_a[tid] = a;
+  s_b[tid] = b;
   __syncthreads();
-  tile_scan_inplace<Real>(As, Bs, ncols, Di, Di);
-  __syncthreads();
-  Real* agg_a = static_cast<Real*>(scr.agg_a);
-  Real* agg_b = static_cast<Real*>(scr.agg_b);
-  Real* incl = static_cast<Real*>(scr.incl);
-  const size_t last = static_cast<size_t>(ncols - 1) * Di;
-  if (tile == 0) {
-    for (int d = tid; d < Di; d += kThreads) {
-      carry[d] = s0[d];
-      incl[d] = As[last + d] * s0[d] + Bs[last + d];
+  // the maps of the chunk's earlier runs, composed
+  Real ea = 1, eb = 0;
+  if (active) {
+    for (int j = 0; j < sub; ++j) {
+      const Real aj = s_a[j * pl.blk_d + dl], bj = s_b[j * pl.blk_d + dl];
+      eb = aj * eb + bj;
+      ea = aj * ea;
     }
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) st_release(scr.flags, (epoch << 2) | kFlagIncl);
-  } else {
-    for (int d = tid; d < Di; d += kThreads) {
-      agg_a[static_cast<size_t>(tile) * Di + d] = As[last + d];
-      agg_b[static_cast<size_t>(tile) * Di + d] = Bs[last + d];
+    if (sub == pl.nsub - 1) {
+      agg_a[ch * D + d] = a * ea;
+      agg_b[ch * D + d] = a * eb + b;
     }
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) st_release(scr.flags + tile, (epoch << 2) | kFlagAgg);
-    if ((tid >> 5) == 0) {
-      int err = 0;
-      const int js = lookback_fixed(tile, epoch, scr.flags, &err);
-      if (tid == 0) {
-        s_jstar = js;
-        if (err) s_err = 1;
+  }
+  grid.sync();
+  {
+    const int lane = tid & 31, nw = static_cast<int>(blockDim.x) >> 5;
+    constexpr int kG = kScanGroup<Real>;
+    for (int64_t dd = static_cast<int64_t>(tid >> 5) * gridDim.x + blockIdx.x; dd < D;
+         dd += static_cast<int64_t>(nw) * gridDim.x) {
+      Real st = s0[dd];
+      for (int base = 0; base < nch; base += 32 * pl.group) {
+        const int j0 = base + lane * pl.group;
+        Real ra[kG], rb[kG];
+        Real ga = 1, gb = 0;
+#pragma unroll
+        for (int k = 0; k < kG; ++k) {
+          const bool in = k < pl.group && j0 + k < nch;
+          ra[k] = in ? __ldcg(agg_a + (j0 + k) * D + dd) : Real(1);
+          rb[k] = in ? __ldcg(agg_b + (j0 + k) * D + dd) : Real(0);
+        }
+#pragma unroll
+        for (int k = 0; k < kG; ++k)
+          if (k < pl.group && j0 + k < nch) {
+            gb = ra[k] * gb + rb[k];
+            ga = ra[k] * ga;
+          }
+        __syncwarp();
+        s_a[tid] = ga;  // (the runs' maps were last read before the barrier)
+        s_b[tid] = gb;
+        __syncwarp();
+        Real mine = st;  // state entering this lane's group
+        const int w0 = tid - lane;
+#pragma unroll 8
+        for (int l = 0; l < 32; ++l) {  // identity maps past the last group
+          const Real al = s_a[w0 + l], bl = s_b[w0 + l];
+          st = al * st + bl;
+          if (l < lane) mine = st;
+        }
+#pragma unroll
+        for (int k = 0; k < kG; ++k)
+          if (k < pl.group && j0 + k < nch) {
+            carry[dd * nch + j0 + k] = mine;
+            mine = ra[k] * mine + rb[k];
+          }
       }
     }
-    __syncthreads();
-    const int js = s_jstar;
-    for (int d = tid; d < Di; d += kThreads) {
-      const Real c = js >= 0 ? lookback_compose<Real>(tile, js, d, Di, agg_a, agg_b, incl)
-                             : Real(0);
-      carry[d] = c;
-      incl[static_cast<size_t>(tile) * Di + d] = As[last + d] * c + Bs[last + d];
+  }
+  grid.sync();
+  if (active && u0 < u1) {
+    Real st = __ldcg(carry + d * nch + ch);
+    if (sub > 0) st = ea * st + eb;
+    const Real *pa = A + u0 * D + d, *pb = B + u0 * D + d;
+    Real* ps = S + u0 * D + d;
+    for (int n = static_cast<int>(u1 - u0); n > 0; n -= kScanUnroll, pa += kScanUnroll * Di,
+             pb += kScanUnroll * Di, ps += kScanUnroll * Di) {
+      Real va[kScanUnroll], vb[kScanUnroll];
+      load(pa, pb, n, va, vb);
+#pragma unroll
+      for (int k = 0; k < kScanUnroll; ++k)
+        if (k < n) {
+          st = va[k] * st + vb[k];
+          ps[k * Di] = st;
+        }
     }
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) st_release(scr.flags + tile, (epoch << 2) | kFlagIncl);
   }
-  __syncthreads();
-  for (int64_t i = tid; i < n; i += kThreads) {
-    const int d = static_cast<int>(i % D);
-    S[base + i] = As[i] * carry[d] + Bs[i];
-  }
-  if (tid == 0 && s_err) atomicExch(scr.counter + 1, 1u);  // timeout flag
+}
+
+// Split of a scan over T columns (a launch's share of them) and D coordinates.
+// Up to 3 CTAs an SM, 96 KB of loads in flight an SM; chunks of
+// min_cols columns at least (scan_tile_cols of the whole scan), so that the chunks
+// fit the scratch.
+static ScanPlan scan_plan(int64_t D, int64_t T, int max_ctas, int min_cols,
+                          int max_group) {
+  ScanPlan p{};
+  p.nblk_d = static_cast<int>((D + kThreads - 1) / kThreads);
+  p.blk_d = static_cast<int>((D + p.nblk_d - 1) / p.nblk_d);
+  const int64_t most = imax64(1, max_ctas / p.nblk_d);
+  p.L = static_cast<int>(imax64((T + most - 1) / most, min_cols));
+  p.nchunks = static_cast<int>((T + p.L - 1) / p.L);
+  p.nsub = static_cast<int>(imin64(imin64(kThreads / p.blk_d, 16), p.L));
+  p.Ls = (p.L + p.nsub - 1) / p.nsub;
+  p.nsub = (p.L + p.Ls - 1) / p.Ls;
+  p.threads = (p.nsub * p.blk_d + 31) / 32 * 32;
+  p.group = static_cast<int>(imax64(1, imin64(max_group, kScanWindow / p.L)));
+  return p;
 }
 
 cudaError_t raise_smem_limit(const void* fn, size_t bytes) {
@@ -136,8 +241,8 @@ cudaError_t raise_smem_limit(const void* fn, size_t bytes) {
 }
 
 int scan_tile_cols(int64_t D, int64_t T) {
-  // Largest power of two <= 64 whose tile (A, B, carry) fits 96 KB, reduced
-  // while that leaves fewer than ~2 tiles per SM.
+  // Fewest columns a chunk of the scan has, which sizes its scratch: a power of
+  // two in 8 .. 64 (fewer for D > 768) that leaves about 2 chunks per SM.
   int TT = 64;
   while (TT > 1 && static_cast<int64_t>(2 * TT + 1) * D * 8 > 96 * 1024) TT >>= 1;
   while (TT > 8 && (T + TT - 1) / TT < 296) TT >>= 1;
@@ -147,34 +252,49 @@ int scan_tile_cols(int64_t D, int64_t T) {
 size_t scan_scratch_bytes(bool f64, int64_t D, int64_t T) {
   const int TT = scan_tile_cols(D, T);
   const int64_t nt = (T + TT - 1) / TT;
-  const size_t es = f64 ? 8 : 4;
-  return 256 + 4 * static_cast<size_t>(nt) + 3 * es * static_cast<size_t>(nt * D) + 64;
+  return 3 * (f64 ? 8 : 4) * static_cast<size_t>(nt * D);
+}
+
+template <typename Real>
+static cudaError_t scan_launches(cudaStream_t s, int64_t D, int64_t T, const Real* A,
+                                 const Real* B, const Real* s0, Real* S, Real* scratch) {
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
+  const void* fn = reinterpret_cast<const void*>(affine_scan_kernel<Real>);
+  const int max_ctas = kScanCtas * sms;  // co-resident by the launch bounds
+  const int64_t nblk_d = (D + kThreads - 1) / kThreads;
+  if (nblk_d > max_ctas) return cudaErrorInvalidValue;
+  // Columns of a launch: chunks within the composition window, and A and B of
+  // the launch inside L2 for phase 3's read (about 64 MB of its 126).
+  const int64_t by_window = (max_ctas / nblk_d) * (kScanWindow / 8);
+  const int64_t by_l2 = (int64_t(64) << 20) / (2 * static_cast<int64_t>(sizeof(Real)) * D);
+  const int64_t seg = imin64(by_window, imax64(by_l2, 4096));
+  const int64_t nseg = (T + seg - 1) / seg, Tseg = (T + nseg - 1) / nseg;
+  for (int64_t t0 = 0; t0 < T; t0 += Tseg) {
+    int64_t Tn = imin64(Tseg, T - t0), Dn = D;
+    ScanPlan pl = scan_plan(D, Tn, max_ctas, scan_tile_cols(D, T), kScanGroup<Real>);
+    const Real *An = A + t0 * D, *Bn = B + t0 * D, *sn = t0 ? S + (t0 - 1) * D : s0;
+    Real *Sn = S + t0 * D, *aa = scratch, *ab = aa + static_cast<size_t>(pl.nchunks) * D,
+         *ca = ab + static_cast<size_t>(pl.nchunks) * D;
+    void* args[] = {&Dn, &Tn, &pl, &An, &Bn, &sn, &Sn, &aa, &ab, &ca};
+    e = cudaLaunchCooperativeKernel(fn, dim3(pl.nchunks * pl.nblk_d), dim3(pl.threads), args, 0,
+                                    s);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaGetLastError();
 }
 
 cudaError_t launch_affine_scan(cudaStream_t s, bool f64, int64_t D, int64_t T, const void* A,
-                               const void* B, const void* s0, void* S, const ScanScratch& scr,
-                               uint32_t epoch) {
+                               const void* B, const void* s0, void* S, void* scratch) {
   if (T == 0 || D == 0) return cudaSuccess;
-  const int TT = scan_tile_cols(D, T);
-  const int ntiles = static_cast<int>((T + TT - 1) / TT);
-  const size_t es = f64 ? 8 : 4;
-  const size_t smem = es * (2 * static_cast<size_t>(TT) + 1) * D;
-  cudaError_t e = cudaMemsetAsync(scr.counter, 0, 2 * sizeof(uint32_t), s);
-  if (e != cudaSuccess) return e;
-  if (f64) {
-    if (smem > 0)
-      raise_smem_limit(reinterpret_cast<const void*>(affine_scan_kernel<double>), smem);
-    affine_scan_kernel<double><<<ntiles, kThreads, smem, s>>>(
-        D, T, TT, static_cast<const double*>(A), static_cast<const double*>(B),
-        static_cast<const double*>(s0), static_cast<double*>(S), scr, epoch);
-  } else {
-    if (smem > 0)
-      raise_smem_limit(reinterpret_cast<const void*>(affine_scan_kernel<float>), smem);
-    affine_scan_kernel<float><<<ntiles, kThreads, smem, s>>>(
-        D, T, TT, static_cast<const float*>(A), static_cast<const float*>(B),
-        static_cast<const float*>(s0), static_cast<float*>(S), scr, epoch);
-  }
-  return cudaGetLastError();
+  return f64 ? scan_launches(s, D, T, static_cast<const double*>(A), static_cast<const double*>(B),
+                             static_cast<const double*>(s0), static_cast<double*>(S),
+                             static_cast<double*>(scratch))
+             : scan_launches(s, D, T, static_cast<const float*>(A), static_cast<const float*>(B),
+                             static_cast<const float*>(s0), static_cast<float*>(S),
+                             static_cast<float*>(scratch));
 }
 
 // ---------------------------------------------------------------------------
