@@ -27,8 +27,8 @@
 // [Rh | S | Rl].
 //
 // Roles: warps 0-15 run the epilogue (warps w, w+4, w+8, w+12 share TMEM lane
-// quarter w % 4 and take 8 columns each); lane 0 of warp 16 issues TMA loads
-// and MMAs and warp 16 owns the TMEM allocation.
+// quarter w % 4 and take 8 columns each); warp 16 issues TMA loads and MMAs
+// (one elected lane) and owns the TMEM allocation.
 // Every mbarrier wait is bounded; on timeout the kernel records an error,
 // drains its own MMAs and frees TMEM before returning.
 #include <cuda.h>
@@ -161,6 +161,22 @@ __device__ __forceinline__ void fence_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+// One lane of the warp (the same on every call): the issuer of the warp's TMA loads
+// and MMAs.  The warp runs the issue loop together and only the instructions
+// themselves are predicated, so descriptors and addresses stay in uniform
+// registers; a loop inside a lane-0 branch moves every operand there for each
+// MMA, 97 cycles an MMA whatever its size, against the 40 - 56 that these
+// widths take (M = 128: N = 96 in 56, N = 32 in 40).  At N = 10000, D = 256,
+// T = 65536 a pass went from 4.99 to 4.12 ms, the wide one (N = 5000, D = 400,
+// T = 8192) from 1.26 to 0.91 ms.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(p));
+  return p != 0;
+}
+
 // 32 consecutive FP32 TMEM columns of this warp's 32 lanes (one per thread).
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
   uint32_t r[32];
@@ -286,7 +302,6 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
   uint64_t* bar_g = bars + 7;  // [2] GEMM2 half h done (X boxes of half h free; R free after the last)
   uint64_t* bar_z = bars + 9;  // teardown drain
   __shared__ uint32_t s_tmem;
-  __shared__ int s_abort;
   __shared__ double s_red[kEpi][BT / kParts];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -303,7 +318,6 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
     mbar_init(bar_g, 1);
     mbar_init(bar_g + 1, 1);
     mbar_init(bar_z, 1);
-    s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kProd) tmem_alloc(&s_tmem, kTmemCols);
@@ -317,12 +331,18 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
   const uint32_t tG = tmem + 128;
 
   if (warp == kProd) {
-    if (lane == 0) {
-      bool ok = true;
-      const uint32_t i1_all = idesc_f16(128, 3 * BT, false, false);
-      const uint32_t i1_v = idesc_f16(128, BT, false, false);
-      const uint32_t i2_all = idesc_f16(128, 3 * BT, true, true);
-      const uint32_t i2_v = idesc_f16(128, BT, true, true);
+    bool ok = true;
+    const bool el = elect_one();
+    const uint32_t i1_all = idesc_f16(128, 3 * BT, false, false);
+    const uint32_t i1_v = idesc_f16(128, BT, false, false);
+    const uint32_t i2_all = idesc_f16(128, 3 * BT, true, true);
+    const uint32_t i2_v = idesc_f16(128, BT, true, true);
+    // descriptors of the first box; a step adds its byte offset / 16
+    const uint64_t xh1 = sdesc(su32(sXh), 16, 1024, 2), xl1 = sdesc(su32(sXl), 16, 1024, 2);
+    const uint64_t b1 = sdesc(su32(sB), 16, 1024, 2);
+    const uint64_t xh2 = sdesc(su32(sXh), kBoxX, 1024, 2), xl2 = sdesc(su32(sXl), kBoxX, 1024, 2);
+    const uint64_t r2 = sdesc(su32(sR), kRAtom, 1024, 2);
+    if (el) {
       mbar_expect_tx(bar_b, nkb * kBoxB);
       for (int kb = 0; kb < nkb; ++kb) {
         unsigned char* b = sB + kb * kBoxB;
@@ -332,65 +352,72 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
         tma_2d(b + BT * 128, has_tangent ? &tmBt : &tmBh, kb * 64, static_cast<int>(t0), bar_b);
         tma_2d(b + 2 * BT * 128, &tmBl, kb * 64, static_cast<int>(t0), bar_b);
       }
-      ok = mbar_wait(bar_b, 0, err);
-      auto load_x = [&](int nb, int kb) {
+    }
+    __syncwarp();
+    ok = mbar_wait(bar_b, 0, err);
+    auto load_x = [&](int nb, int kb) {
+      if (el) {
         mbar_expect_tx(bar_x + kb, 2 * kBoxX);
         tma_2d(sXh + kb * kBoxX, &tmXh, kb * 64, nb * BN, bar_x + kb);
         tma_2d(sXl + kb * kBoxX, &tmXl, kb * 64, nb * BN, bar_x + kb);
-      };
-      if (ok)
-        for (int kb = 0; kb < nkb; ++kb) load_x(0, kb);
-      for (int nb = 0; nb < nblocks && ok; ++nb) {
-        // GEMM1: L = Xh [Bh | Bt | Bl] + Xl Bh, box by box as X arrives
-        for (int kb = 0; kb < nkb; ++kb) {
-          if (!(ok = mbar_wait(bar_x + kb, nb & 1, err))) break;
-          tc_fence_after();
+      }
+      __syncwarp();
+    };
+    if (ok)
+      for (int kb = 0; kb < nkb; ++kb) load_x(0, kb);
+    for (int nb = 0; nb < nblocks && ok; ++nb) {
+      // GEMM1: L = Xh [Bh | Bt | Bl] + Xl Bh, box by box as X arrives
+      for (int kb = 0; kb < nkb; ++kb) {
+        if (!(ok = mbar_wait(bar_x + kb, nb & 1, err))) break;
+        tc_fence_after();
+        if (el) {
 #pragma unroll
           for (int ks = 0; ks < 4; ++ks) {
-            const uint64_t ah = sdesc(su32(sXh + kb * kBoxX) + ks * 32, 16, 1024, 2);
-            const uint64_t al = sdesc(su32(sXl + kb * kBoxX) + ks * 32, 16, 1024, 2);
-            const uint64_t bb = sdesc(su32(sB + kb * kBoxB) + ks * 32, 16, 1024, 2);
-            mma_f16(tL, ah, bb, i1_all, (kb | ks) != 0);
-            mma_f16(tL, al, bb, i1_v, 1);
+            const uint32_t ox = (kb * kBoxX + ks * 32) >> 4, ob = (kb * kBoxB + ks * 32) >> 4;
+            mma_f16(tL, xh1 + ox, b1 + ob, i1_all, (kb | ks) != 0);
+            mma_f16(tL, xl1 + ox, b1 + ob, i1_v, 1);
           }
         }
-        if (!ok) break;
-        mma_commit(bar_l);
-        if (!(ok = mbar_wait(bar_r, nb & 1, err))) break;
-        tc_fence_after();
-        // GEMM2: G_h += Xh^T [Rh | S | Rl] + Xl^T Rh  (A MN-major, B MN-major)
-        for (int h = 0; h < nh; ++h) {
+        __syncwarp();
+      }
+      if (!ok) break;
+      if (el) mma_commit(bar_l);
+      __syncwarp();
+      if (!(ok = mbar_wait(bar_r, nb & 1, err))) break;
+      tc_fence_after();
+      // GEMM2: G_h += Xh^T [Rh | S | Rl] + Xl^T Rh  (A MN-major, B MN-major)
+      for (int h = 0; h < nh; ++h) {
+        if (el) {
           if (has_g) {
 #pragma unroll
             for (int kn = 0; kn < BN / 16; ++kn) {
-              const uint64_t ah = sdesc(su32(sXh + 2 * h * kBoxX) + kn * 2048, kBoxX, 1024, 2);
-              const uint64_t al = sdesc(su32(sXl + 2 * h * kBoxX) + kn * 2048, kBoxX, 1024, 2);
-              const uint64_t br = sdesc(su32(sR) + kn * 2048, kRAtom, 1024, 2);
+              const uint32_t ox = (2 * h * kBoxX + kn * 2048) >> 4, orr = (kn * 2048) >> 4;
               // every row block starts G afresh: the epilogue has added the
               // previous block's G into its registers before it wrote R
-              const uint32_t acc = kn > 0 ? 1u : 0u;
-              mma_f16(tG + 128 * h, ah, br, i2_all, acc);
-              mma_f16(tG + 128 * h, al, br, i2_v, 1);
+              mma_f16(tG + 128 * h, xh2 + ox, r2 + orr, i2_all, kn > 0 ? 1u : 0u);
+              mma_f16(tG + 128 * h, xl2 + ox, r2 + orr, i2_v, 1);
             }
           }
           mma_commit(bar_g + h);
         }
-        // the next block's X, half h as soon as GEMM2's half h has read it
-        if (nb + 1 < nblocks)
-          for (int h = 0; h < nh; ++h) {
-            if (!(ok = mbar_wait(bar_g + h, nb & 1, err))) break;
-            load_x(nb + 1, 2 * h);
-            load_x(nb + 1, 2 * h + 1);
-          }
+        __syncwarp();
       }
-      if (!ok) {
-        s_abort = 1;
-        atomicExch(err, 1);
-      }
-      // drain every MMA this thread issued before TMEM is released
-      mma_commit(bar_z);
-      if (!mbar_wait(bar_z, 0, err)) atomicExch(err, 1);
+      // the next block's X, half h as soon as GEMM2's half h has read it
+      if (nb + 1 < nblocks)
+        for (int h = 0; h < nh; ++h) {
+          if (!(ok = mbar_wait(bar_g + h, nb & 1, err))) break;
+          load_x(nb + 1, 2 * h);
+          load_x(nb + 1, 2 * h + 1);
+        }
     }
+    ok = __all_sync(0xffffffffu, ok);
+    if (el) {
+      if (!ok) atomicExch(err, 1);
+      // drain every MMA this warp issued before TMEM is released
+      mma_commit(bar_z);
+    }
+    __syncwarp();
+    if (!mbar_wait(bar_z, 0, err) && el) atomicExch(err, 1);
     __syncwarp();
   } else {
     // ---- epilogue: thread = TMEM lane = data row; warp part = column block ----
@@ -691,8 +718,13 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
   auto tG = [&](int q) { return tmem + 64u * static_cast<uint32_t>(q + 1); };
 
   if (warp == kProd) {
-    if (lane == 0) {
+    {
       bool ok = true;
+      const bool el = elect_one();
+      const uint64_t xh1 = sdesc(su32(sXh), 16, 1024, 2), xl1 = sdesc(su32(sXl), 16, 1024, 2);
+      const uint64_t b1 = sdesc(su32(sB), 16, 1024, 2), r2 = sdesc(su32(sR), kRAtom, 1024, 2);
+      const uint64_t xh2 = sdesc(su32(sXh), kBoxX, 1024, 2),
+                     xl2 = sdesc(su32(sXl), kBoxX, 1024, 2);
       uint32_t xph = 0, fph = 0;  // phase bit of each slot's two barriers
       const uint32_t i1_all = idesc_f16(128, 3 * BTW, false, false);
       const uint32_t i1_v = idesc_f16(128, BTW, false, false);
@@ -709,42 +741,53 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
         return r;
       };
       auto load_box = [&](int s, int box, int nb) {
-        mbar_expect_tx(bar_x + s, 2 * kBoxX);
-        tma_2d(sXh + s * kBoxX, &tmXh, box * 64, nb * BN, bar_x + s);
-        tma_2d(sXl + s * kBoxX, &tmXl, box * 64, nb * BN, bar_x + s);
+        if (el) {
+          mbar_expect_tx(bar_x + s, 2 * kBoxX);
+          tma_2d(sXh + s * kBoxX, &tmXh, box * 64, nb * BN, bar_x + s);
+          tma_2d(sXl + s * kBoxX, &tmXl, box * 64, nb * BN, bar_x + s);
+        }
+        __syncwarp();
       };
       // GEMM1 over the box in slot s: L += Xh [Bh | Bt | Bl] + Xl Bh
       auto gemm1 = [&](int s, int box) {
+        if (el) {
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks) {
-          const uint64_t ah = sdesc(su32(sXh + s * kBoxX) + ks * 32, 16, 1024, 2);
-          const uint64_t al = sdesc(su32(sXl + s * kBoxX) + ks * 32, 16, 1024, 2);
-          const uint64_t bb = sdesc(su32(sB + box * kBoxBW) + ks * 32, 16, 1024, 2);
-          mma_f16(tL, ah, bb, i1_all, (box | ks) != 0);
-          mma_f16(tL, al, bb, i1_v, 1);
+          for (int ks = 0; ks < 4; ++ks) {
+            const uint32_t ox = (s * kBoxX + ks * 32) >> 4, ob = (box * kBoxBW + ks * 32) >> 4;
+            mma_f16(tL, xh1 + ox, b1 + ob, i1_all, (box | ks) != 0);
+            mma_f16(tL, xl1 + ox, b1 + ob, i1_v, 1);
+          }
         }
+        __syncwarp();
       };
       // GEMM2 for d quarter q from the boxes in slots 2p, 2p + 1
       auto gemm2 = [&](int q, int p, int nb) {
         if (!has_g) return;
+        if (el) {
 #pragma unroll
-        for (int kn = 0; kn < BN / 16; ++kn) {
-          const uint64_t ah = sdesc(su32(sXh + 2 * p * kBoxX) + kn * 2048, kBoxX, 1024, 2);
-          const uint64_t al = sdesc(su32(sXl + 2 * p * kBoxX) + kn * 2048, kBoxX, 1024, 2);
-          const uint64_t br = sdesc(su32(sR) + kn * 2048, kRAtom, 1024, 2);
-          // every row block starts G afresh (the epilogue adds the blocks up)
-          const uint32_t acc = kn > 0 ? 1u : 0u;
-          mma_f16(tG(q), ah, br, i2_all, acc);
-          mma_f16(tG(q), al, br, i2_v, 1);
+          for (int kn = 0; kn < BN / 16; ++kn) {
+            const uint32_t ox = (2 * p * kBoxX + kn * 2048) >> 4, orr = (kn * 2048) >> 4;
+            // every row block starts G afresh (the epilogue adds the blocks up)
+            mma_f16(tG(q), xh2 + ox, r2 + orr, i2_all, kn > 0 ? 1u : 0u);
+            mma_f16(tG(q), xl2 + ox, r2 + orr, i2_v, 1);
+          }
         }
+        __syncwarp();
       };
-      mbar_expect_tx(bar_b, kNkbW * kBoxBW);
-      for (int kb = 0; kb < kNkbW; ++kb) {
-        unsigned char* b = sB + kb * kBoxBW;
-        tma_2d(b, &tmBh, kb * 64, static_cast<int>(t0), bar_b);
-        tma_2d(b + BTW * 128, has_tangent ? &tmBt : &tmBh, kb * 64, static_cast<int>(t0), bar_b);
-        tma_2d(b + 2 * BTW * 128, &tmBl, kb * 64, static_cast<int>(t0), bar_b);
+      auto commit = [&](uint64_t* bar) {
+        if (el) mma_commit(bar);
+        __syncwarp();
+      };
+      if (el) {
+        mbar_expect_tx(bar_b, kNkbW * kBoxBW);
+        for (int kb = 0; kb < kNkbW; ++kb) {
+          unsigned char* b = sB + kb * kBoxBW;
+          tma_2d(b, &tmBh, kb * 64, static_cast<int>(t0), bar_b);
+          tma_2d(b + BTW * 128, has_tangent ? &tmBt : &tmBh, kb * 64, static_cast<int>(t0), bar_b);
+          tma_2d(b + 2 * BTW * 128, &tmBl, kb * 64, static_cast<int>(t0), bar_b);
+        }
       }
+      __syncwarp();
       ok = mbar_wait(bar_b, 0, err);
       if (ok)
         for (int s = 0; s < kSlots; ++s) load_box(s, s, 0);
@@ -754,7 +797,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
           if (!(ok = wait_x(s))) break;
           tc_fence_after();
           gemm1(s, s);
-          mma_commit(bar_f + s);
+          commit(bar_f + s);
         }
         // boxes 4-7 into the slots as they free, then their GEMM1
         for (int s = 0; s < kSlots && ok; ++s) {
@@ -767,14 +810,14 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
           gemm1(s, kSlots + s);
         }
         if (!ok) break;
-        mma_commit(bar_l);
+        commit(bar_l);
         if (!(ok = mbar_wait(bar_r, nb & 1, err))) break;
         tc_fence_after();
         // GEMM2, quarters 2 and 3 from the resident boxes 4-7
         for (int p = 0; p < 2; ++p) {
           gemm2(2 + p, p, nb);
-          mma_commit(bar_f + 2 * p);
-          mma_commit(bar_f + 2 * p + 1);
+          commit(bar_f + 2 * p);
+          commit(bar_f + 2 * p + 1);
         }
         // boxes 0-3 again, then quarters 0 and 1
         for (int s = 0; s < kSlots && ok; ++s) {
@@ -785,11 +828,11 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
           if (!(ok = wait_x(2 * p)) || !(ok = wait_x(2 * p + 1))) break;
           tc_fence_after();
           gemm2(p, p, nb);
-          mma_commit(bar_f + 2 * p);
-          mma_commit(bar_f + 2 * p + 1);
+          commit(bar_f + 2 * p);
+          commit(bar_f + 2 * p + 1);
         }
         if (!ok) break;
-        mma_commit(bar_g);
+        commit(bar_g);
         // the next block's boxes 0-3
         if (nb + 1 < nblocks)
           for (int s = 0; s < kSlots && ok; ++s) {
@@ -797,10 +840,14 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
             load_box(s, s, nb + 1);
           }
       }
-      if (!ok) atomicExch(err, 1);
-      // drain every MMA this thread issued before TMEM is released
-      mma_commit(bar_z);
-      if (!mbar_wait(bar_z, 0, err)) atomicExch(err, 1);
+      ok = __all_sync(0xffffffffu, ok);
+      if (el) {
+        if (!ok) atomicExch(err, 1);
+        // drain every MMA this warp issued before TMEM is released
+        mma_commit(bar_z);
+      }
+      __syncwarp();
+      if (!mbar_wait(bar_z, 0, err) && el) atomicExch(err, 1);
     }
     __syncwarp();
   } else {
