@@ -386,7 +386,7 @@ struct SolveLayout {
 SolveLayout layout(int64_t D, int64_t Dp, int64_t T, int ntiles, size_t es, bool plain,
                    int64_t N = 0, int64_t Tc = 0, size_t tc_bytes = 0,
                    const FullPlan* fp = nullptr, bool adjoint = false,
-                   bool dual_out = false, size_t tie_bytes = 0) {
+                   bool dual_out = false, size_t tie_bytes = 0, int tc_split = 1) {
   SolveLayout L{};
   size_t off = 0;
   auto take = [&](size_t bytes) {
@@ -438,7 +438,7 @@ SolveLayout layout(int64_t D, int64_t Dp, int64_t T, int ntiles, size_t es, bool
   }
   if (tc_bytes) {
     L.tcws = take(tc_bytes);
-    L.Gtc = take(4 * Dp * 2 * static_cast<size_t>(T));
+    L.Gtc = take(4 * Dp * 2 * static_cast<size_t>(T) * tc_split);
   }
   if (fp || adjoint) L.facc = take(static_cast<size_t>(T));
   if (fp) {
@@ -739,7 +739,7 @@ int run_logistic(pmcmc_handle* h, const pmcmc_target* tg, const SweepKernels& k,
   const TieBufs tb = lg_tie_carve(ws + L.tie, tg->lg, P.T, tie_kmax(P.T));
   P.la_ref = refine ? la_ref : nullptr;
   P.lg_acc = ws + L.lg_acc;
-  P.tc_err = use_tc ? lg_tc_err_word(ws + L.tcws, tg->lg, P.T) : nullptr;
+  P.tc_err = use_tc ? lg_tc_err_word(ws + L.tcws) : nullptr;
   const void* k_acc = k.eval;  // the probe accumulation kernel of the logistic target
   CK(cudaMemcpyAsync(h->d_params, &P, sizeof(DevParams), cudaMemcpyHostToDevice, h->stream));
   if (smem_sweep > 0)
@@ -752,7 +752,7 @@ int run_logistic(pmcmc_handle* h, const pmcmc_target* tg, const SweepKernels& k,
   int zero = 0;
   void* sweep_args[] = {&h->d_params, &h->d_state, &none, &zero};
   void *Bb = ws + L.Bb, *Lb = ws + L.Lb, *Gb = ws + L.Gb;
-  int* tc_err = use_tc ? lg_tc_err_word(ws + L.tcws, tg->lg, P.T) : nullptr;
+  int* tc_err = use_tc ? lg_tc_err_word(ws + L.tcws) : nullptr;
   if (use_tc) CK(cudaMemsetAsync(tc_err, 0, sizeof(int), h->stream));
   auto pass_impl = [&](int mode, double* lp, int probe) -> int {
     if (use_tc) {
@@ -761,7 +761,8 @@ int run_logistic(pmcmc_handle* h, const pmcmc_target* tg, const SweepKernels& k,
                      probe))
         return 1;
       if (mode != 2 && lg_mid(h->stream, false, h->d_params, h->d_state, mode + 1, 0,
-                              static_cast<int>(P.T), probe, P.Dp, G) != cudaSuccess)
+                              static_cast<int>(P.T), probe, P.Dp, G,
+                              lg_tc_split(tg->lg, P.T)) != cudaSuccess)
         return 1;
       return 0;
     }
@@ -1309,7 +1310,8 @@ int solve_core(pmcmc_handle* h, const pmcmc_target* tg, const pmcmc_deer_params*
   const SolveLayout L = layout(D, Dp, T, ntiles, es, plain, logistic ? tg->N : 0, Tc,
                                use_tc ? lg_tc_ws_bytes(tg->lg, T) : 0, full ? &fplan : nullptr,
                                false, pipe,
-                               logistic ? lg_tie_ws_bytes(tg->lg, T, tie_kmax(T)) : 0);
+                               logistic ? lg_tie_ws_bytes(tg->lg, T, tie_kmax(T)) : 0,
+                               use_tc ? lg_tc_split(tg->lg, T) : 1);
   rc = ensure_ws(h, L.total);
   if (rc) return rc;
   if (defer) {

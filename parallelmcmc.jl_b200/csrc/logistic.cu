@@ -152,7 +152,8 @@ __global__ void lg_epilogue_kernel(const Real* __restrict__ ylab, int64_t N, int
 //   stage 6 -> dla += H_x u                              in lg[4].
 template <typename Real>
 __global__ void lg_mid_kernel(const DevParams* __restrict__ Pg, const DevState* __restrict__ st,
-                              int stage, int64_t t0, int Tc, int probe, const Real* __restrict__ G) {
+                              int stage, int64_t t0, int Tc, int probe, const Real* __restrict__ G,
+                              int nsplit) {
   const DevParams& P = *Pg;
   const int64_t Dp = P.Dp, D = P.D;
   const int64_t nq = Dp / 4;
@@ -170,8 +171,19 @@ __global__ void lg_mid_kernel(const DevParams* __restrict__ Pg, const DevState* 
     const int64_t q = i % nq;
     const int64_t t = t0 + j;
     if (t >= P.T) continue;
-    const Real* gv = G + static_cast<int64_t>(j) * Dp + 4 * q;
-    const Real* gt = G + static_cast<int64_t>(Tc + j) * Dp + 4 * q;
+    Real gv[4], gt[4];
+    {
+      const Real* pv = G + static_cast<int64_t>(j) * Dp + 4 * q;
+      const Real* pt = G + static_cast<int64_t>(Tc + j) * Dp + 4 * q;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) gv[e] = pv[e], gt[e] = pt[e];
+      for (int p = 1; p < nsplit; ++p) {  // the pass's parts, in order
+        pv += 2 * static_cast<int64_t>(Tc) * Dp;
+        pt += 2 * static_cast<int64_t>(Tc) * Dp;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) gv[e] += pv[e], gt[e] += pt[e];
+      }
+    }
     const size_t o = static_cast<size_t>(t) * Dp + 4 * q;
     if (stage == 1) {
       float xi[4];
@@ -299,14 +311,14 @@ cudaError_t lg_epilogue(cudaStream_t s, bool f64, const void* ylab, int64_t N, i
 }
 
 cudaError_t lg_mid(cudaStream_t s, bool f64, const DevParams* dP, const DevState* dS, int stage,
-                   int64_t t0, int Tc, int probe, int64_t Dp, const void* G) {
+                   int64_t t0, int Tc, int probe, int64_t Dp, const void* G, int nsplit) {
   const int g = grid_for(static_cast<int64_t>(Tc) * (Dp / 4));
   if (f64)
     lg_mid_kernel<double><<<g, 256, 0, s>>>(dP, dS, stage, t0, Tc, probe,
-                                            static_cast<const double*>(G));
+                                            static_cast<const double*>(G), nsplit);
   else
     lg_mid_kernel<float><<<g, 256, 0, s>>>(dP, dS, stage, t0, Tc, probe,
-                                           static_cast<const float*>(G));
+                                           static_cast<const float*>(G), nsplit);
   return cudaGetLastError();
 }
 

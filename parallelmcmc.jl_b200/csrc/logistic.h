@@ -36,18 +36,20 @@ int lg_plain_pass(cudaStream_t s, cublasHandle_t cb, const LogisticDev& X, bool 
                   int64_t Dp, void* Bbuf, void* Lbuf, void* Gbuf, int64_t Tc, int probe);
 
 cudaError_t lg_mid(cudaStream_t s, bool f64, const DevParams* dP, const DevState* dS, int stage,
-                   int64_t t0, int Tc, int probe, int64_t Dp, const void* G);
+                   int64_t t0, int Tc, int probe, int64_t Dp, const void* G, int nsplit = 1);
 // X2 = X .* X in the state's precision (once; the caller serialises first uses).
 cudaError_t lg_make_square(cudaStream_t s, LogisticDev& X, bool f64);
 
 // Tensor-core pass (logistic_tc.cu): mode 0/1/2 as in lg_plain_pass; writes G
-// (Dp x 2T FP32, value block then tangent block) and lp.  ws holds the FP16
+// (lg_tc_split parts of Dp x 2T FP32, value block then tangent block, that lg_mid
+// adds) and lp.  ws holds the FP16
 // operand arrays and an error word (lg_tc_ws_bytes).
 bool lg_tc_supported(const LogisticDev& X);
 size_t lg_tc_ws_bytes(const LogisticDev& X, int64_t T);
 int lg_tc_pass(cudaStream_t s, const LogisticDev& X, const DevParams* dP, const DevState* dS,
                double* lp, int mode, int64_t T, void* ws, float* G, int probe);
-int* lg_tc_err_word(void* ws, const LogisticDev& X, int64_t T);
+int* lg_tc_err_word(void* ws);
+int lg_tc_split(const LogisticDev& X, int64_t T);  // parts of G that a pass writes
 // One bounded mbarrier wait that nothing completes (bound check); err[0] = 1
 // when it gave up.
 cudaError_t lg_tc_mbar_bound(cudaStream_t s, int* err);

@@ -1,34 +1,26 @@
 // logistic_tc.cu -- one logistic-regression pass on the 5th-generation tensor
 // cores (tcgen05 + TMEM + TMA), fused GEMM -> epilogue -> GEMM.
 //
-// For a tile of BT trajectory columns (value columns v_t = x_bar_t or y_t, and
+// For a tile of trajectory columns (value columns v_t = x_bar_t or y_t, and
 // the matching tangent columns z_t or w_t) and all N data rows:
-//   GEMM1  L[n, t] = sum_d X[n, d] B[d, t]                     (M = 128 rows of X)
+//   GEMM1  L[n, t] = sum_d X[n, d] B[d, t]
 //   epilogue (per row n, per column t): p = sigmoid(L), r = y_n - p,
 //          s = p (1 - p) L_tangent, loglik = y_n L - softplus(L)  (bayes_logreg.jl:118-154)
-//   GEMM2  G[d, t] += sum_n X[n, d] R[n, t],  R = [r | s]       (M = 128 values of d)
-// The N x 2T intermediate never leaves the SM: L lives in TMEM, R in shared
-// memory.  G starts afresh in TMEM at every 128-row block and the epilogue
-// threads add the blocks' partial sums in registers (round-to-nearest FP32):
+//   GEMM2  G[d, t] += sum_n X[n, d] R[n, t],  R = [r | s]
+// The N x 2T intermediate never leaves the SM, and the same shared-memory X tile
+// serves both GEMMs.  G starts afresh in TMEM after every 128 rows and the epilogue
+// threads add the partial sums in registers (round-to-nearest FP32):
 // one TMEM accumulation chain over all N rows left the N = 10000 gradient about
 // 10x less accurate than an FP32 SGEMM, enough to move the chain by 1.5e-5.
-// The same shared-memory X tile is GEMM1's K-major A operand and GEMM2's
-// MN-major A operand.
 //
 // Precision: X, the value columns and r are carried as FP16 hi + lo pairs
 // (about 22 significant bits); each value-column product is
 // hi*hi + hi*lo + lo*hi with FP32 accumulation.  Tangent columns (only used
 // for the Jacobian estimate) and s use a single FP16 term.
 //
-// The MMAs are bound by shared-memory reads of the X operand at these widths,
-// so each k step issues two: Xh [Bh | Bt | Bl] (N = 96, the hi*lo product in
-// accumulator columns of its own, added in the epilogue) and Xl Bh (N = 32,
-// accumulated onto the hi*hi columns).  GEMM2 is arranged the same way with
-// [Rh | S | Rl].
-//
-// Roles: warps 0-15 run the epilogue (warps w, w+4, w+8, w+12 share TMEM lane
-// quarter w % 4 and take 8 columns each); warp 16 issues TMA loads and MMAs
-// (one elected lane) and owns the TMEM allocation.
+// Two kernels: logistic_pass_kernel for D <= 256 and logistic_pass_tc_wide_kernel
+// above.  Warps 0-15 run the epilogue (warps w, w+4, w+8, w+12 share TMEM lane
+// quarter w % 4); one elected lane of warp 16 issues the MMAs.
 // Every mbarrier wait is bounded; on timeout the kernel records an error,
 // drains its own MMAs and frees TMEM before returning.
 #include <cuda.h>
@@ -45,41 +37,18 @@
 namespace pmcmc {
 namespace tc {
 
-constexpr int BN = 128;  // data rows per block (GEMM1 M)
-constexpr int BT = 32;   // value columns per CTA (plus BT tangent columns)
+constexpr int BN = 128;  // data rows per block of the wide variant
 constexpr int kThreadsTC = 544;  // 16 epilogue warps + 1 producer warp
 constexpr int kEpi = 16;
 constexpr int kProd = 16;  // producer / TMEM-owner warp
 constexpr int kParts = kEpi / 4;  // epilogue warps per TMEM lane quarter
-constexpr uint32_t kTmemCols = 512;  // L at 0, G half h at 128 (h + 1); 96 columns each
+constexpr uint32_t kTmemCols = 512;
 constexpr long long kWaitCycles = 2000000000ll;  // ~1 s at B200 clocks
 constexpr uint32_t kBoxX = BN * 128;       // one 64-wide d box of X: 128 rows x 128 B
-constexpr uint32_t kBoxB = 3 * BT * 128;  // value hi rows | tangent rows | value lo rows
 // R (GEMM2's B operand, N = 96 columns [r hi | s | r lo] by K = BN rows) is
 // MN-major with the 128-byte swizzle, like X^T: two 64-column atoms of BN rows
 // x 128 B; chunk c (8 columns) of row k sits at chunk c ^ (k & 7).
 constexpr uint32_t kRAtom = BN * 128;
-
-struct Layout {
-  uint32_t xh, xl, b, r, bars, total;
-};
-
-__host__ __device__ inline Layout layout(int nkb) {
-  Layout L;
-  uint32_t off = 0;
-  L.xh = off;
-  off += nkb * kBoxX;
-  L.xl = off;
-  off += nkb * kBoxX;
-  L.b = off;
-  off += nkb * kBoxB;
-  L.r = off;
-  off += 2 * kRAtom;
-  L.bars = off;
-  off += 128;
-  L.total = off + 1024;  // slack for 1024-B alignment of the dynamic window
-  return L;
-}
 
 __device__ __forceinline__ uint32_t su32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -102,19 +71,22 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* b, uint32_t bytes) {
 // Bounded wait for the completion of the phase with the given parity: gives up
 // after about a second of SM clock (or at once when another CTA of the launch
 // has already reported an error).
+__device__ __forceinline__ bool mbar_try(uint64_t* b, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(su32(b)), "r"(parity)
+      : "memory");
+  return done != 0;
+}
 __device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity,
                                           const volatile int* err) {
-  const uint32_t a = su32(b);
+  if (mbar_try(b, parity)) return true;
   const long long start = clock64();
   for (long long i = 0;; ++i) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (done) return true;
+    if (mbar_try(b, parity)) return true;
     if ((i & 255) == 255 && (*err || clock64() - start > kWaitCycles)) return false;
   }
 }
@@ -166,59 +138,14 @@ __device__ __forceinline__ void fence_async_smem() {
 // themselves are predicated, so descriptors and addresses stay in uniform
 // registers; a loop inside a lane-0 branch moves every operand there for each
 // MMA, 97 cycles an MMA whatever its size, against the 40 - 56 that these
-// widths take (M = 128: N = 96 in 56, N = 32 in 40).  At N = 10000, D = 256,
-// T = 65536 a pass went from 4.99 to 4.12 ms, the wide one (N = 5000, D = 400,
-// T = 8192) from 1.26 to 0.91 ms.
+// widths take (M = 128: N = 96 in 56, N = 32 in 40).  The wide pass at N = 5000,
+// D = 400, T = 8192 went from 1.26 to 0.91 ms by this alone.
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile(
       "{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(p));
   return p != 0;
-}
-
-// 32 consecutive FP32 TMEM columns of this warp's 32 lanes (one per thread).
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
-  uint32_t r[32];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
-      "%12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, "
-      "%30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
-        "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
-        "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr)
-      : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-// Three 8-column TMEM loads of this warp's 32 lanes, then one wait.  The wait
-// is in the same asm statement as the loads, so no use of the registers can
-// move above it.
-__device__ __forceinline__ void tmem_ld8x3(uint32_t ta, uint32_t tb, uint32_t tc, float (&a)[8],
-                                           float (&b)[8], float (&c)[8]) {
-  uint32_t r[24];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%24];\n\t"
-      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8, %9, %10, %11, %12, %13, %14, %15}, [%25];\n\t"
-      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%16, %17, %18, %19, %20, %21, %22, %23}, [%26];\n\t"
-      "tcgen05.wait::ld.sync.aligned;"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
-        "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23])
-      : "r"(ta), "r"(tb), "r"(tc)
-      : "memory");
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    a[i] = __uint_as_float(r[i]);
-    b[i] = __uint_as_float(r[8 + i]);
-    c[i] = __uint_as_float(r[16 + i]);
-  }
 }
 
 // Shared-memory matrix descriptor (tcgen05): start, leading / stride byte
@@ -271,53 +198,139 @@ __device__ __forceinline__ float split_hi(float x) {
   return __uint_as_float(__float_as_uint(x) & 0xffffe000u);
 }
 
-// G (Dp x 2T column-major: value block then tangent block, FP32) and lp (T,
-// FP64) for the column tile blockIdx.x.  has_tangent = 0: value columns only,
-// no G (the logp pass over a returned trajectory).
-__global__ void __launch_bounds__(kThreadsTC, 1)
-    logistic_pass_tc_kernel(const __grid_constant__ CUtensorMap tmXh,
-                            const __grid_constant__ CUtensorMap tmXl,
-                            const __grid_constant__ CUtensorMap tmBh,
-                            const __grid_constant__ CUtensorMap tmBl,
-                            const __grid_constant__ CUtensorMap tmBt,
-                            const float* __restrict__ ylab, int64_t N, int nkb, int64_t T,
-                            int64_t Dp, float* __restrict__ G, double* __restrict__ lp,
-                            int has_tangent, int* __restrict__ err) {
+// ---------------------------------------------------------------------------
+// The pass for D <= 256: one CTA takes 64 trajectory columns and a run of
+// 64-row blocks of X.  The columns are the MMAs' A operand, resident for the
+// whole run; X streams through shared memory once as the B operand of both GEMMs:
+//   GEMM1  L (128 lanes x 64 rows)  = [Bh | Bt] Xl' + Bl Xh' + [Bh | Bt] Xh'
+//   GEMM2  G (128 lanes x d)       += [Rh | S] Xl + [Rl | 0] Xh + [Rh | S] Xh
+// Lanes: each 32-lane quarter q of TMEM holds value columns 16 q .. 16 q + 15 in
+// its lower half and their tangent columns in its upper half (the lanes an M = 64
+// MMA writes are the lower halves, so Bl needs no padding).  The small products
+// come first, where the accumulator is still small.  TMEM: G in 64 NKB columns,
+// two L buffers of 64, [Bh | Bt] in 32 NKB; R overwrites its L in place.
+//
+// The tensor cores never wait for the epilogue: block b's GEMM1 and block b - 1's
+// GEMM2 run while the epilogue turns L(b - 1) and L(b) into R.  Per block 2 x 24
+// (NKB = 4) products of 32 and 128 cycles = 3072 cycles at D = 256, and 64 KB of X
+// (three stages in flight).  A third of the products' lanes are padding (the lo
+// products of the tangent lanes), which the layout pays for keeping X's traffic
+// at one read for 64 columns.  The form with X as the A operand (32 columns a CTA,
+// one 128 KB block of X, nothing overlapped) took 4.4 us for 128 rows of 32
+// columns at first and 3.5 us with its MMAs issued back to back; this takes 2.15 us for
+// 64 rows of 64 columns (3650 cycles, of which 3072 on the tensor pipe, at the 1.7 GHz
+// the power cap leaves): a pass at N = 10000, D = 256, T = 65536 went from 4.99 and
+// 4.12 ms to 2.34 ms, 574 TFLOP/s algorithmic (8 N D T).
+//
+// A CTA's G is the sum over its rows; `nsplit` CTAs share a tile's rows where the
+// tiles alone leave SMs idle, and lg_mid adds their parts.
+// ---------------------------------------------------------------------------
+constexpr int TB = 64;                        // value columns a CTA
+constexpr int RB = 64;                        // rows of X a block
+constexpr uint32_t kBox = RB * 128;           // 64 rows (or columns) x 64 values of d, FP16
+__host__ __device__ constexpr int stages(int nkb) { return nkb == 4 ? 3 : 4; }
+__host__ __device__ constexpr uint32_t pass_smem(int nkb) {
+  // Bl | stages x (Xh | Xl) | barriers | alignment slack
+  return nkb * kBox + stages(nkb) * 2 * nkb * kBox + 128 + 1024;
+}
+
+constexpr int kThreadsPass = 576;             // 16 epilogue warps, the MMA warp, the load warp
+constexpr int kLoad = 17;
+
+__device__ __forceinline__ void tma_3d(void* dst, const CUtensorMap* tm, int x, int y, int z,
+                                       uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, "
+      "%3, %4}], [%5];" ::"r"(su32(dst)),
+      "l"(reinterpret_cast<uint64_t>(tm)), "r"(x), "r"(y), "r"(z), "r"(su32(bar))
+      : "memory");
+}
+// 1 / x for x in [1, 2] (1 ulp).
+__device__ __forceinline__ float rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// mbar_wait with one answer for the whole warp.
+__device__ __forceinline__ bool warp_wait(uint64_t* b, uint32_t parity, const volatile int* err) {
+  return __all_sync(0xffffffffu, mbar_wait(b, parity, err));
+}
+
+__device__ __forceinline__ void mma_f16_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc,
+                                           uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
+      "r"(a), "l"(b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// 8 consecutive TMEM columns of this warp's 32 lanes.
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() {
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+// 16 consecutive FP32 TMEM columns of this warp's 32 lanes.
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
+  uint32_t r[16];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
+      "%12, %13, %14, %15}, [%16];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// mode 0: value x_bar_t, tangent z_t (probe `probe`); mode 1: value y_t, tangent w_t;
+// mode 2: value S_t, no tangent and no G.  G: nsplit parts of 2T x Dp (value block,
+// then tangent block), lp: nsplit parts of T.
+template <int NKB>
+__global__ void __launch_bounds__(kThreadsPass, 1)
+    logistic_pass_kernel(const __grid_constant__ CUtensorMap tmXh,
+                         const __grid_constant__ CUtensorMap tmXl,
+                         const DevParams* __restrict__ Pg, const DevState* __restrict__ st,
+                         int mode, int probe, const float* __restrict__ ylab, int64_t N,
+                         int64_t T, int64_t Dp, int nsplit, float* __restrict__ G,
+                         double* __restrict__ lp, int* __restrict__ err) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  const Layout Ly = layout(nkb);
-  unsigned char* sXh = base + Ly.xh;
-  unsigned char* sXl = base + Ly.xl;
-  unsigned char* sB = base + Ly.b;
-  unsigned char* sR = base + Ly.r;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(base + Ly.bars);
-  // X moves box by box (64 values of d, hi and lo): GEMM2's d-half h reads
-  // exactly boxes 2h and 2h + 1, so the next block's boxes of half h load
-  // while GEMM2's later half runs, and GEMM1 starts on box 0 as soon as it lands.
-  uint64_t* bar_b = bars + 0;  // B tile loaded
-  uint64_t* bar_x = bars + 1;  // [4] X box kb loaded
-  uint64_t* bar_l = bars + 5;  // GEMM1 done (L ready)
-  uint64_t* bar_r = bars + 6;  // epilogue wrote R (32 kEpi arrivals)
-  uint64_t* bar_g = bars + 7;  // [2] GEMM2 half h done (X boxes of half h free; R free after the last)
-  uint64_t* bar_z = bars + 9;  // teardown drain
+  constexpr int kSt = stages(NKB);
+  constexpr uint32_t kHalf = NKB * kBox;  // one of Xh, Xl of a stage
+  constexpr int DC = 16 * NKB;            // values of d an epilogue warp owns
+  unsigned char* sBl = base;
+  unsigned char* sX = base + kHalf;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sX + kSt * 2 * kHalf);
+  uint64_t* bar_x = bars;       // [kSt] stage loaded
+  uint64_t* bar_f = bars + 4;   // [kSt] the MMAs reading the stage are done
+  uint64_t* bar_l = bars + 8;   // [2] L ready
+  uint64_t* bar_r = bars + 10;  // [2] R written (and G drained, where it was due)
+  uint64_t* bar_g = bars + 12;  // G of two blocks complete
+  uint64_t* bar_b = bars + 13;  // column operands written
+  uint64_t* bar_z = bars + 14;  // teardown drain
   __shared__ uint32_t s_tmem;
-  __shared__ double s_red[kEpi][BT / kParts];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t t0 = static_cast<int64_t>(blockIdx.x) * BT;
-  const int nblocks = static_cast<int>((N + BN - 1) / BN);
-  const int nh = nkb / 2;
-  const bool has_g = has_tangent != 0;
+  const int tile = static_cast<int>(blockIdx.x) / nsplit;
+  const int split = static_cast<int>(blockIdx.x) % nsplit;
+  const int64_t t0 = static_cast<int64_t>(tile) * TB;
+  const int nb_all = static_cast<int>((N + RB - 1) / RB);
+  const int b0 = static_cast<int>(static_cast<int64_t>(nb_all) * split / nsplit);
+  const int nb = static_cast<int>(static_cast<int64_t>(nb_all) * (split + 1) / nsplit) - b0;
+  const bool has_g = mode != 2;
 
   if (threadIdx.x == 0) {
-    mbar_init(bar_b, 1);
-    for (int kb = 0; kb < 4; ++kb) mbar_init(bar_x + kb, 1);
-    mbar_init(bar_l, 1);
-    mbar_init(bar_r, 32 * kEpi);
-    mbar_init(bar_g, 1);
-    mbar_init(bar_g + 1, 1);
-    mbar_init(bar_z, 1);
+    for (int i = 0; i < 15; ++i) mbar_init(bars + i, i == 10 || i == 11 || i == 13 ? 32 * kEpi : 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kProd) tmem_alloc(&s_tmem, kTmemCols);
@@ -325,219 +338,279 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = s_tmem;
-  // L: columns [0, 96) = value (hi*hi + lo*hi) | tangent | value hi*lo.
-  // G half h: columns [128 (h + 1), 128 (h + 1) + 96), the same three parts.
-  const uint32_t tL = tmem;
-  const uint32_t tG = tmem + 128;
+  const uint32_t tG = tmem, tL = tmem + 256, tB = tmem + 384;
 
   if (warp == kProd) {
-    bool ok = true;
     const bool el = elect_one();
-    const uint32_t i1_all = idesc_f16(128, 3 * BT, false, false);
-    const uint32_t i1_v = idesc_f16(128, BT, false, false);
-    const uint32_t i2_all = idesc_f16(128, 3 * BT, true, true);
-    const uint32_t i2_v = idesc_f16(128, BT, true, true);
-    // descriptors of the first box; a step adds its byte offset / 16
-    const uint64_t xh1 = sdesc(su32(sXh), 16, 1024, 2), xl1 = sdesc(su32(sXl), 16, 1024, 2);
-    const uint64_t b1 = sdesc(su32(sB), 16, 1024, 2);
-    const uint64_t xh2 = sdesc(su32(sXh), kBoxX, 1024, 2), xl2 = sdesc(su32(sXl), kBoxX, 1024, 2);
-    const uint64_t r2 = sdesc(su32(sR), kRAtom, 1024, 2);
-    if (el) {
-      mbar_expect_tx(bar_b, nkb * kBoxB);
-      for (int kb = 0; kb < nkb; ++kb) {
-        unsigned char* b = sB + kb * kBoxB;
-        tma_2d(b, &tmBh, kb * 64, static_cast<int>(t0), bar_b);
-        // without tangent columns the middle rows repeat Bh: the MMA reads
-        // them and nothing uses their products
-        tma_2d(b + BT * 128, has_tangent ? &tmBt : &tmBh, kb * 64, static_cast<int>(t0), bar_b);
-        tma_2d(b + 2 * BT * 128, &tmBl, kb * 64, static_cast<int>(t0), bar_b);
-      }
-    }
-    __syncwarp();
-    ok = mbar_wait(bar_b, 0, err);
-    auto load_x = [&](int nb, int kb) {
+    bool ok = true;
+    constexpr uint32_t i1 = idesc_f16(128, RB, false, false), i1h = idesc_f16(64, RB, false, false);
+    constexpr uint32_t i2 = idesc_f16(128, 64 * NKB, false, true);
+    const uint64_t x1 = sdesc(su32(sX), 16, 1024, 2), x2 = sdesc(su32(sX), kBox, 1024, 2);
+    const uint64_t bl = sdesc(su32(sBl), 16, 1024, 2);
+    // GEMM2 of block b (in stage s); G starts afresh every second block
+    auto gemm2 = [&](int b, int s) {
       if (el) {
-        mbar_expect_tx(bar_x + kb, 2 * kBoxX);
-        tma_2d(sXh + kb * kBoxX, &tmXh, kb * 64, nb * BN, bar_x + kb);
-        tma_2d(sXl + kb * kBoxX, &tmXl, kb * 64, nb * BN, bar_x + kb);
+        if (has_g) {
+          const uint32_t a = tL + 64 * (b & 1);
+          const uint64_t xh = x2 + ((s * 2 * kHalf) >> 4), xl = xh + (kHalf >> 4);
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            mma_f16_ts(tG, a + 16 * k, xl + ((k * 2048) >> 4), i2, ((b & 1) | k) != 0);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) mma_f16_ts(tG, a + 16 * k + 8, xh + ((k * 2048) >> 4), i2, 1);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) mma_f16_ts(tG, a + 16 * k, xh + ((k * 2048) >> 4), i2, 1);
+        }
+        mma_commit(bar_f + s);
+        if (has_g && ((b & 1) || b == nb - 1)) mma_commit(bar_g);
       }
       __syncwarp();
     };
-    if (ok)
-      for (int kb = 0; kb < nkb; ++kb) load_x(0, kb);
-    for (int nb = 0; nb < nblocks && ok; ++nb) {
-      // GEMM1: L = Xh [Bh | Bt | Bl] + Xl Bh, box by box as X arrives
-      for (int kb = 0; kb < nkb; ++kb) {
-        if (!(ok = mbar_wait(bar_x + kb, nb & 1, err))) break;
-        tc_fence_after();
-        if (el) {
-#pragma unroll
-          for (int ks = 0; ks < 4; ++ks) {
-            const uint32_t ox = (kb * kBoxX + ks * 32) >> 4, ob = (kb * kBoxB + ks * 32) >> 4;
-            mma_f16(tL, xh1 + ox, b1 + ob, i1_all, (kb | ks) != 0);
-            mma_f16(tL, xl1 + ox, b1 + ob, i1_v, 1);
-          }
-        }
-        __syncwarp();
-      }
-      if (!ok) break;
-      if (el) mma_commit(bar_l);
-      __syncwarp();
-      if (!(ok = mbar_wait(bar_r, nb & 1, err))) break;
+    ok = warp_wait(bar_b, 0, err);
+    tc_fence_after();
+    int s = 0, sp = 0;  // stage of this block and of the one before
+    uint32_t xph = 0;  // phase bit of each stage
+    for (int b = 0; b < nb && ok; ++b) {
+      if (!(ok = warp_wait(bar_x + s, (xph >> s) & 1u, err))) break;
+      xph ^= 1u << s;
       tc_fence_after();
-      // GEMM2: G_h += Xh^T [Rh | S | Rl] + Xl^T Rh  (A MN-major, B MN-major)
-      for (int h = 0; h < nh; ++h) {
-        if (el) {
-          if (has_g) {
+      if (el) {
+        const uint32_t d = tL + 64 * (b & 1);
+        const uint64_t xh = x1 + ((s * 2 * kHalf) >> 4), xl = xh + (kHalf >> 4);
 #pragma unroll
-            for (int kn = 0; kn < BN / 16; ++kn) {
-              const uint32_t ox = (2 * h * kBoxX + kn * 2048) >> 4, orr = (kn * 2048) >> 4;
-              // every row block starts G afresh: the epilogue has added the
-              // previous block's G into its registers before it wrote R
-              mma_f16(tG + 128 * h, xh2 + ox, r2 + orr, i2_all, kn > 0 ? 1u : 0u);
-              mma_f16(tG + 128 * h, xl2 + ox, r2 + orr, i2_v, 1);
-            }
-          }
-          mma_commit(bar_g + h);
-        }
-        __syncwarp();
+        for (int k = 0; k < 4 * NKB; ++k)
+          mma_f16_ts(d, tB + 8 * k, xl + ((k / 4 * kBox + k % 4 * 32) >> 4), i1, k != 0);
+#pragma unroll
+        for (int k = 0; k < 4 * NKB; ++k)
+          mma_f16(d, bl + ((k / 4 * kBox + k % 4 * 32) >> 4),
+                  xh + ((k / 4 * kBox + k % 4 * 32) >> 4), i1h, 1);
+#pragma unroll
+        for (int k = 0; k < 4 * NKB; ++k)
+          mma_f16_ts(d, tB + 8 * k, xh + ((k / 4 * kBox + k % 4 * 32) >> 4), i1, 1);
+        mma_commit(bar_l + (b & 1));
       }
-      // the next block's X, half h as soon as GEMM2's half h has read it
-      if (nb + 1 < nblocks)
-        for (int h = 0; h < nh; ++h) {
-          if (!(ok = mbar_wait(bar_g + h, nb & 1, err))) break;
-          load_x(nb + 1, 2 * h);
-          load_x(nb + 1, 2 * h + 1);
-        }
+      __syncwarp();
+      if (b > 0) {
+        if (!(ok = warp_wait(bar_r + ((b - 1) & 1), ((b - 1) >> 1) & 1, err))) break;
+        tc_fence_after();
+        gemm2(b - 1, sp);
+      }
+      sp = s;
+      s = s + 1 == kSt ? 0 : s + 1;
     }
-    ok = __all_sync(0xffffffffu, ok);
+    if (ok && nb > 0) {
+      ok = warp_wait(bar_r + ((nb - 1) & 1), ((nb - 1) >> 1) & 1, err);
+      if (ok) {
+        tc_fence_after();
+        gemm2(nb - 1, sp);
+      }
+    }
     if (el) {
       if (!ok) atomicExch(err, 1);
       // drain every MMA this warp issued before TMEM is released
       mma_commit(bar_z);
     }
     __syncwarp();
-    if (!mbar_wait(bar_z, 0, err) && el) atomicExch(err, 1);
+    if (!warp_wait(bar_z, 0, err) && el) atomicExch(err, 1);
     __syncwarp();
+  } else if (warp == kLoad) {
+    const bool el = elect_one();
+    int s = 0, use = 0;
+    for (int b = 0; b < nb; ++b) {
+      // the stage's previous block is done with once its GEMM2 has run
+      if (use > 0 && !warp_wait(bar_f + s, (use - 1) & 1, err)) break;
+      if (el) {
+        unsigned char* d = sX + s * 2 * kHalf;
+        mbar_expect_tx(bar_x + s, 2 * kHalf);
+        tma_3d(d + kHalf, &tmXl, 0, (b0 + b) * RB, 0, bar_x + s);
+        tma_3d(d, &tmXh, 0, (b0 + b) * RB, 0, bar_x + s);
+      }
+      __syncwarp();
+      if (++s == kSt) s = 0, ++use;
+    }
+    // no load is in flight when the CTA ends, not even after a wait that gave up
+    for (int i = 0; i < kSt; ++i) {
+      const int n = i < s ? use + 1 : use;  // loads into stage i
+      if (n > 0) warp_wait(bar_x + i, (n - 1) & 1, err);
+    }
   } else {
-    // ---- epilogue: thread = TMEM lane = data row; warp part = column block ----
-    const int quarter = warp & 3, part = warp >> 2;  // columns [8 part, 8 part + 8)
-    const int row = quarter * 32 + lane;
+    // ---- epilogue: lane = (column, value or tangent); warp part = 16 rows, DC values of d ----
+    const int quarter = warp & 3, part = warp >> 2;
     const uint32_t lane_off = static_cast<uint32_t>(quarter * 32) << 16;
-    constexpr int BH = BT / kParts;
-    static_assert(BH == 8, "one 8-column block of R a thread");
-    // log-likelihood sums, compensated (Kahan) in FP32: ls the sum, lc the
-    // running error; the column total is ls - lc, formed in FP64 at the end
-    float ls[BH], lc[BH];
+    const bool tan = lane >= 16;
+    const int m = quarter * 16 + (lane & 15);
+    const int64_t t = t0 + m;
+    const bool in_t = t < T;
+    const int d0 = part * DC;
+    {  // column operands: [Bh | Bt] to TMEM, Bl to shared memory
+      const DevParams& P = *Pg;
+      const float* x0 = static_cast<const float*>(P.x0);
+      const float* S = static_cast<const float*>(P.S[st->cur]);
+      const int iter = st->iter;
+      const float* src = nullptr;
+      if (in_t) {
+        if (mode == 0) src = tan ? nullptr : (iter == 0 || t == 0) ? x0 : S + (t - 1) * Dp;
+        else if (mode == 1) src = static_cast<const float*>(P.lg[tan ? 2 : 1]) + t * Dp;
+        else src = tan ? nullptr : S + t * Dp;
+      }
+      const bool probes = mode == 0 && tan && in_t;
+      const TapeKey key(P.seed, P.block);
 #pragma unroll
-    for (int t = 0; t < BH; ++t) ls[t] = lc[t] = 0.f;
-    bool ok = true;
-    float y_next = row < N ? __ldg(ylab + row) : 0.f;  // label of this row, one block ahead
-    // G accumulates one row block at a time in TMEM; the blocks' partial sums
-    // are added here, in FP32 with round-to-nearest.  Part 2 h + b owns d-half
-    // h of G, the value block (b = 0, hi*lo columns added) or the tangent block.
-    const bool g_owner = has_g && part < 2 * nh;
-    const int gh = part >> 1, gb = part & 1;
-    float gacc[BT];
+      for (int c = 0; c < DC; c += 16) {
+        float v[16];
+        if (probes) {
+          const int d = d0 + c;
+          const U4 pb = probe_bits(key, static_cast<uint32_t>(d >> 7),
+                                   static_cast<uint32_t>(t + P.t_off), probe, iter);
+          const uint32_t w = u4_word(pb, (d >> 5) & 3) >> (d & 31);
 #pragma unroll
-    for (int t = 0; t < BT; ++t) gacc[t] = 0.f;
-    auto add_g = [&]() {
-      const uint32_t ga = tG + 128 * gh + lane_off + BT * gb;
-#pragma unroll
-      for (int c = 0; c < BT; c += 8) {
-        float a[8], b8[8], unused[8];
-        if (gb == 0) {
-          tmem_ld8x3(ga + c, tG + 128 * gh + lane_off + 2 * BT + c, ga + c, a, b8, unused);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) gacc[c + i] += a[i] + b8[i];
+          for (int i = 0; i < 16; ++i) v[i] = d + i < P.D ? (((w >> i) & 1u) ? 1.f : -1.f) : 0.f;
         } else {
-          tmem_ld8x3(ga + c, ga + c, ga + c, a, b8, unused);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) gacc[c + i] += a[i];
+          for (int i = 0; i < 16; i += 4) {
+            float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (src && d0 + c + i < Dp) q = *reinterpret_cast<const float4*>(src + d0 + c + i);
+            v[i] = q.x;
+            v[i + 1] = q.y;
+            v[i + 2] = q.z;
+            v[i + 3] = q.w;
+          }
         }
+        uint32_t hi[8], lo[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const __half2 h = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
+          const float2 f = __half22float2(h);
+          hi[i] = *reinterpret_cast<const uint32_t*>(&h);
+          lo[i] = half2_bits(v[2 * i] - f.x, v[2 * i + 1] - f.y);
+        }
+        tmem_st8(tB + lane_off + (d0 + c) / 2, hi);
+        if (!tan) {
+          const int kb = (d0 + c) >> 6, ch = ((d0 + c) & 63) >> 3;
+          unsigned char* row = sBl + kb * kBox + m * 128;
+          *reinterpret_cast<uint4*>(row + ((ch ^ (m & 7)) << 4)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+          *reinterpret_cast<uint4*>(row + (((ch + 1) ^ (m & 7)) << 4)) = make_uint4(lo[4], lo[5], lo[6], lo[7]);
+        }
+      }
+      tmem_wait_st();
+      fence_async_smem();
+      tc_fence_before();
+      mbar_arrive(bar_b);
+    }
+    float gacc[DC];  // this lane's G over d0 .. d0 + DC - 1, the blocks' partial sums added here
+#pragma unroll
+    for (int i = 0; i < DC; ++i) gacc[i] = 0.f;
+    // log-likelihood sum, compensated (Kahan) in FP32: ls the sum, lc the running error
+    float ls = 0.f, lc = 0.f;
+    bool ok = true;
+    int drained = 0;
+    auto add_g = [&]() {
+      if (!(ok = warp_wait(bar_g, drained & 1, err))) return;
+      ++drained;
+      tc_fence_after();
+#pragma unroll
+      for (int c = 0; c < DC; c += 16) {
+        float a[16];
+        tmem_ld16(tG + lane_off + d0 + c, a);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) gacc[c + i] += a[i];
       }
     };
-    for (int nb = 0; nb < nblocks; ++nb) {
-      const int64_t n = static_cast<int64_t>(nb) * BN + row;
-      const bool valid = n < N;
-      const float yn = y_next;
-      if (n + BN < N) y_next = __ldg(ylab + n + BN);
-      if (g_owner && nb > 0) {
-        // the previous block's G partials are final once its GEMM2 has committed,
-        // and the next GEMM2 restarts G only after this block's R (bar_r): they
-        // are added while this block's X arrives and its GEMM1 runs
-        if (!(ok = mbar_wait(bar_g + (nh - 1), (nb - 1) & 1, err))) break;
-        tc_fence_after();
-        add_g();
-      }
-      if (!(ok = mbar_wait(bar_l, nb & 1, err))) break;
+    // labels (0 or 1) of the warp's 16 rows, one block ahead
+    const float* yp = ylab + static_cast<int64_t>(b0) * RB + 16 * part + (lane & 15);
+    float ynext = nb > 0 ? __ldg(yp) : 0.f;
+    for (int b = 0; b < nb; ++b) {
+      const uint32_t ybits = __ballot_sync(0xffffffffu, ynext != 0.f) >> (tan ? 8 : 0);
+      yp += RB;
+      if (b + 1 < nb) ynext = __ldg(yp);
+      if (!(ok = warp_wait(bar_l + (b & 1), (b >> 1) & 1, err))) break;
       tc_fence_after();
-      float v[BH], vl[BH], w[BH];
-      tmem_ld8x3(tL + lane_off + BH * part, tL + lane_off + 2 * BT + BH * part,
-                 tL + lane_off + BT + BH * part, v, vl, w);
-      float r[BH], s[BH];
+      const uint32_t la = tL + 64 * (b & 1) + 16 * part + lane_off;
+      float v[16];
+      tmem_ld16(la, v);
+      // rows of this lane: the value lane takes the first 8 of the warp's 16, the tangent
+      // lane the last 8; each gets the other's logit or tangent of its rows.
+      // Rows past N have X = 0: whatever R holds there adds nothing to G, and only the
+      // log-likelihood leaves them out.
+      const int nv = static_cast<int>(imin64(
+          RB, N - (static_cast<int64_t>(b0 + b) * RB + 16 * part + (tan ? 8 : 0))));
+      // With z = l for label 0 and -l for label 1: r = y - p = -+ sigmoid(z), and the
+      // log-likelihood term is -softplus(z) = -max(z, 0) - log(1 + e), e = exp(-|l|).  The
+      // block's 1 + e are multiplied (at most 2^8, each product rounded once) and take one log.
+      float r[8], s[8], prod = 1.f;
 #pragma unroll
-      for (int t = 0; t < BH; ++t) {
-        const float l = v[t] + vl[t];
+      for (int j = 0; j < 8; ++j) {
+        const float got = __shfl_xor_sync(0xffffffffu, tan ? v[j] : v[8 + j], 16);
+        const float l = tan ? got : v[j], w = tan ? v[8 + j] : got;
+        const uint32_t flip = (ybits << (31 - j)) & 0x80000000u;
+        const float z = __uint_as_float(__float_as_uint(l) ^ flip);
         const float e = __expf(-fabsf(l));
-        const float inv = __fdividef(1.f, 1.f + e);
-        const float p = l >= 0.f ? inv : e * inv;
-        r[t] = valid ? yn - p : 0.f;
-        s[t] = (valid && has_tangent) ? p * (1.f - p) * w[t] : 0.f;
-        if (valid) {
-          const float y = (yn * l - (fmaxf(l, 0.f) + log1p_unit(e))) - lc[t];
-          const float sum = ls[t] + y;
-          lc[t] = (sum - ls[t]) - y;
-          ls[t] = sum;
+        const float inv = rcp_approx(1.f + e);
+        const float q = e * inv;  // sigmoid(-|l|)
+        const float p = z >= 0.f ? inv : q;
+        r[j] = __uint_as_float(__float_as_uint(p) ^ flip ^ 0x80000000u);
+        s[j] = q * inv * w;
+        if (j < nv) {
+          prod *= 1.f + e;
+          const float y = -fmaxf(z, 0.f) - lc;
+          const float sum = ls + y;
+          lc = (sum - ls) - y;
+          ls = sum;
         }
+      }
+      {
+        const float y = -__logf(prod) - lc;
+        const float sum = ls + y;
+        lc = (sum - ls) - y;
+        ls = sum;
       }
       if (has_g) {
-        // R columns as FP16: r split hi + lo, s one term; two values a conversion
-        uint32_t wh[BH / 2], wl[BH / 2], ws[BH / 2];
+        // R as FP16: r split hi + lo, s one term.  The value lane keeps r of all 16 rows,
+        // the tangent lane s; 8 words of hi (or s) and 8 of lo (or zero), in place of L
+        uint32_t hi[8], lo[8];
 #pragma unroll
-        for (int q = 0; q < BH / 2; ++q) {
-          const float h0 = split_hi(r[2 * q]), h1 = split_hi(r[2 * q + 1]);
-          wh[q] = half2_bits(h0, h1);
-          wl[q] = half2_bits(r[2 * q] - h0, r[2 * q + 1] - h1);
-          ws[q] = half2_bits(s[2 * q], s[2 * q + 1]);
+        for (int i = 0; i < 4; ++i) {
+          const float h0 = split_hi(r[2 * i]), h1 = split_hi(r[2 * i + 1]);
+          const uint32_t wh = half2_bits(h0, h1);
+          const uint32_t wl = half2_bits(r[2 * i] - h0, r[2 * i + 1] - h1);
+          const uint32_t ws = half2_bits(s[2 * i], s[2 * i + 1]);
+          const uint32_t got = __shfl_xor_sync(0xffffffffu, tan ? wh : ws, 16);
+          const uint32_t gotl = __shfl_xor_sync(0xffffffffu, wl, 16);
+          hi[i] = tan ? got : wh;
+          hi[4 + i] = tan ? ws : got;
+          lo[i] = tan ? 0u : wl;
+          lo[4 + i] = tan ? 0u : gotl;
         }
-        // value hi: atom 0 chunk part; s: atom 0 chunk 4 + part; value lo: atom 1 chunk part
-        unsigned char* rrow = sR + row * 128;
-        const int sw = row & 7;
-        *reinterpret_cast<uint4*>(rrow + ((part ^ sw) << 4)) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
-        *reinterpret_cast<uint4*>(rrow + (((4 + part) ^ sw) << 4)) = make_uint4(ws[0], ws[1], ws[2], ws[3]);
-        *reinterpret_cast<uint4*>(rrow + kRAtom + ((part ^ sw) << 4)) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
-        fence_async_smem();
+        tmem_st8(la, hi);
+        tmem_st8(la + 8, lo);
+        // the previous two blocks' G, complete while this block's GEMM1 ran; the next
+        // GEMM2 starts it afresh after bar_r
+        if (b >= 2 && !(b & 1)) add_g();
+        tmem_wait_st();
+        if (!ok) break;
       }
       tc_fence_before();
-      mbar_arrive(bar_r);
+      mbar_arrive(bar_r + (b & 1));
     }
-    if (ok && has_g && mbar_wait(bar_g + (nh - 1), (nblocks - 1) & 1, err)) {
-      tc_fence_after();
-      if (g_owner) {
-        add_g();  // the last row block
-        const int64_t d = 128 * gh + row;
-        if (d < Dp) {
-          const int64_t cbase = gb ? T : 0;
+    if (ok && has_g && nb > 0) add_g();  // the last blocks
+    if (ok && has_g && in_t) {
+      float* g = G + (static_cast<int64_t>(split) * 2 * T + (tan ? T : 0) + t) * Dp + d0;
 #pragma unroll
-          for (int t = 0; t < BT; ++t)
-            if (t0 + t < T) G[(cbase + t0 + t) * Dp + d] = gacc[t];
-        }
-      }
-    } else if (!ok) {
-      atomicExch(err, 1);
+      for (int c = 0; c < DC; c += 4)
+        if (d0 + c < Dp)
+          *reinterpret_cast<float4*>(g + c) = make_float4(gacc[c], gacc[c + 1], gacc[c + 2], gacc[c + 3]);
     }
-#pragma unroll
-    for (int t = 0; t < BH; ++t) {
-      const double sum = warp_sum(static_cast<double>(ls[t]) - static_cast<double>(lc[t]));
-      if (lane == 0) s_red[warp][t] = sum;
-    }
+    if (!ok) atomicExch(err, 1);
+    // log-likelihood of a column: 2 lanes x 4 warps, summed in FP64 in a fixed order.  Bl was
+    // last read by the last block's GEMM1, complete before its L.
+    double* red = reinterpret_cast<double*>(sBl);
+    const double sum = static_cast<double>(ls) - static_cast<double>(lc);
+    red[(part * 2 + (tan ? 1 : 0)) * TB + m] = sum;
     asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpi) : "memory");
-    if (threadIdx.x < BT && t0 + threadIdx.x < T) {
-      const int t = threadIdx.x, hh = t / BH, tt = t % BH;
+    if (threadIdx.x < TB && t0 + threadIdx.x < T) {
       double a = 0.0;
-      for (int q = 0; q < 4; ++q) a += s_red[4 * hh + q][tt];
-      lp[t0 + t] = a;
+      for (int i = 0; i < 8; ++i) a += red[i * TB + threadIdx.x];
+      lp[static_cast<int64_t>(split) * T + t0 + threadIdx.x] = a;
     }
   }
   tc_fence_before();
@@ -962,6 +1035,16 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
   if (warp == kProd) tmem_dealloc(tmem, 512);
 }
 
+// lp[t] = the sum of the nsplit partial sums of column t, in order.
+__global__ void lp_sum_kernel(const double* __restrict__ parts, int nsplit, int64_t T,
+                              double* __restrict__ lp) {
+  const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (t >= T) return;
+  double a = 0.0;
+  for (int p = 0; p < nsplit; ++p) a += parts[static_cast<int64_t>(p) * T + t];
+  lp[t] = a;
+}
+
 // Bound check of the mbarrier wait used by the tensor-core pass: one thread
 // initialises a barrier that expects one arrival, nobody arrives, and the
 // bounded wait on phase 0 gives up after kWaitCycles; err[0] = 1 then.
@@ -1016,35 +1099,86 @@ static bool make_map(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t co
          CUDA_SUCCESS;
 }
 
-bool lg_tc_supported(const LogisticDev& X) { return X.Xh != nullptr && encode_fn() != nullptr; }
-
-size_t lg_tc_ws_bytes(const LogisticDev& X, int64_t T) {
-  return 3 * static_cast<size_t>(T) * X.Dk * 2 + 1024;
+// X (rows x cols FP16, row-major) as 64-column boxes one after another: one load takes
+// box_rows rows of every box.
+static bool make_map_x(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols,
+                       uint32_t box_rows) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return false;
+  const cuuint64_t dims[3] = {64, rows, cols / 64};
+  const cuuint64_t strides[2] = {cols * 2, 128};
+  const cuuint32_t box[3] = {64, box_rows, static_cast<cuuint32_t>(cols / 64)};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(ptr), dims, strides, box,
+            estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) ==
+         CUDA_SUCCESS;
 }
 
-int* lg_tc_err_word(void* ws, const LogisticDev& X, int64_t T) {
-  return reinterpret_cast<int*>(reinterpret_cast<unsigned char*>(ws) + 3 * T * X.Dk * 2);
+bool lg_tc_supported(const LogisticDev& X) { return X.Xh != nullptr && encode_fn() != nullptr; }
+
+// CTAs that share a 64-column tile's rows: the split with the fewest steps, counted in
+// 64-row blocks a CTA (1.6 us each at D = 256) times waves of 148 CTAs, with about 4
+// blocks' time of set-up a CTA and the traffic of the split sums (at 5 TB/s).
+int lg_tc_split(const LogisticDev& X, int64_t T) {
+  if (X.Dk == 512) return 1;
+  const int64_t tiles = (T + tc::TB - 1) / tc::TB, nb = (X.N + tc::RB - 1) / tc::RB;
+  int best = 1;
+  double cost = 1e300;
+  for (int s = 1; s <= 16 && s <= nb; ++s) {
+    const double waves = static_cast<double>((tiles * s + 147) / 148);
+    const double sums = s > 1 ? s * (T * X.Dp * 16.0 / 5e6) / 1.6 : 0.0;
+    const double c = waves * (static_cast<double>((nb + s - 1) / s) + 4.0) + sums;
+    if (c < cost) {
+      cost = c;
+      best = s;
+    }
+  }
+  return best;
+}
+
+// error word | the wide variant's FP16 operands, or the split log-likelihood sums
+size_t lg_tc_ws_bytes(const LogisticDev& X, int64_t T) {
+  if (X.Dk == 512) return 1024 + 3 * static_cast<size_t>(T) * X.Dk * 2;
+  return 1024 + 8 * static_cast<size_t>(T) * lg_tc_split(X, T);
+}
+
+int* lg_tc_err_word(void* ws) { return static_cast<int*>(ws); }
+
+template <int NKB>
+static int launch_pass(cudaStream_t s, const LogisticDev& X, const DevParams* dP,
+                       const DevState* dS, double* lp, int mode, int64_t T, int* err, float* G,
+                       int probe, int nsplit) {
+  CUtensorMap mXh, mXl;
+  if (!make_map_x(&mXh, X.Xh, X.Np, X.Dk, tc::RB) ||
+      !make_map_x(&mXl, X.Xl, X.Np, X.Dk, tc::RB))
+    return 3;
+  const uint32_t smem = tc::pass_smem(NKB);
+  if (raise_smem_limit(reinterpret_cast<const void*>(tc::logistic_pass_kernel<NKB>), smem) !=
+      cudaSuccess)
+    return 3;
+  const int grid = static_cast<int>((T + tc::TB - 1) / tc::TB) * nsplit;
+  tc::logistic_pass_kernel<NKB><<<grid, tc::kThreadsPass, smem, s>>>(
+      mXh, mXl, dP, dS, mode, probe, X.y32, X.N, T, X.Dp, nsplit, G, lp, err);
+  return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }
 
 int lg_tc_pass(cudaStream_t s, const LogisticDev& X, const DevParams* dP, const DevState* dS,
-               double* lp, int mode, int64_t T, void* ws, float* G_out, int probe) {
+               double* lp, int mode, int64_t T, void* ws, float* G, int probe) {
   const int64_t Dk = X.Dk;
-  __half* Bh = static_cast<__half*>(ws);
-  __half* Bl = Bh + T * Dk;
-  __half* Bt = Bl + T * Dk;
-  float* G = G_out;
-  int* err = lg_tc_err_word(ws, X, T);
-  const int g = static_cast<int>((T * Dk + 255) / 256 < 148 * 16 ? (T * Dk + 255) / 256 : 148 * 16);
-  tc::tc_prep_kernel<float><<<g, 256, 0, s>>>(dP, dS, mode, probe, Dk, Bh, Bl, Bt);
-  if (cudaGetLastError() != cudaSuccess) return 3;
-  CUtensorMap mXh, mXl, mBh, mBl, mBt;
-  if (!make_map(&mXh, X.Xh, X.Np, Dk, tc::BN) || !make_map(&mXl, X.Xl, X.Np, Dk, tc::BN) ||
-      !make_map(&mBh, Bh, T, Dk, tc::BT) || !make_map(&mBl, Bl, T, Dk, tc::BT) ||
-      !make_map(&mBt, Bt, T, Dk, tc::BT))
-    return 3;
+  int* err = lg_tc_err_word(ws);
+  unsigned char* buf = static_cast<unsigned char*>(ws) + 1024;
   if (Dk == 512) {  // 256 < D <= 512: the wide variant, 16 value columns a CTA
-    CUtensorMap wBh, wBl, wBt;
-    if (!make_map(&wBh, Bh, T, Dk, tc::BTW) || !make_map(&wBl, Bl, T, Dk, tc::BTW) ||
+    __half* Bh = reinterpret_cast<__half*>(buf);
+    __half* Bl = Bh + T * Dk;
+    __half* Bt = Bl + T * Dk;
+    const int g =
+        static_cast<int>((T * Dk + 255) / 256 < 148 * 16 ? (T * Dk + 255) / 256 : 148 * 16);
+    tc::tc_prep_kernel<float><<<g, 256, 0, s>>>(dP, dS, mode, probe, Dk, Bh, Bl, Bt);
+    if (cudaGetLastError() != cudaSuccess) return 3;
+    CUtensorMap mXh, mXl, wBh, wBl, wBt;
+    if (!make_map(&mXh, X.Xh, X.Np, Dk, tc::BN) || !make_map(&mXl, X.Xl, X.Np, Dk, tc::BN) ||
+        !make_map(&wBh, Bh, T, Dk, tc::BTW) || !make_map(&wBl, Bl, T, Dk, tc::BTW) ||
         !make_map(&wBt, Bt, T, Dk, tc::BTW))
       return 3;
     const uint32_t smem = tc::layout_wide().total;
@@ -1056,12 +1190,14 @@ int lg_tc_pass(cudaStream_t s, const LogisticDev& X, const DevParams* dP, const 
         mXh, mXl, wBh, wBl, wBt, X.y32, X.N, T, X.Dp, G, lp, mode != 2 ? 1 : 0, err);
     return cudaGetLastError() == cudaSuccess ? 0 : 3;
   }
-  const int nkb = static_cast<int>(Dk / 64);
-  const tc::Layout Ly = tc::layout(nkb);
-  raise_smem_limit(reinterpret_cast<const void*>(tc::logistic_pass_tc_kernel), tc::layout(4).total);
-  const int grid = static_cast<int>((T + tc::BT - 1) / tc::BT);
-  tc::logistic_pass_tc_kernel<<<grid, tc::kThreadsTC, Ly.total, s>>>(
-      mXh, mXl, mBh, mBl, mBt, X.y32, X.N, nkb, T, X.Dp, G, lp, mode != 2 ? 1 : 0, err);
+  const int ns = lg_tc_split(X, T);
+  double* lps = ns > 1 ? reinterpret_cast<double*>(buf) : lp;
+  const int rc = Dk == 128
+                     ? launch_pass<2>(s, X, dP, dS, lps, mode, T, err, G, probe, ns)
+                     : launch_pass<4>(s, X, dP, dS, lps, mode, T, err, G, probe, ns);
+  if (rc || ns == 1) return rc;
+  const int g = static_cast<int>((T + 255) / 256);
+  tc::lp_sum_kernel<<<g, 256, 0, s>>>(lps, ns, T, lp);
   return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }
 
