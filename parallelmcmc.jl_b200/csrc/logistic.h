@@ -20,7 +20,7 @@ struct LogisticDev {
   double* y64 = nullptr;
   double tau = 1.0;
   // tensor-core operands: X as FP16 hi + lo, Np x Dk (rows padded to 128,
-  // columns padded to 128); only built when D <= 256
+  // columns padded to 128, 256 or 512); only built when D <= 512
   int64_t Np = 0, Dk = 0;
   __half* Xh = nullptr;
   __half* Xl = nullptr;

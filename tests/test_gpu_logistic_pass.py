@@ -1,5 +1,5 @@
-"""The tensor-core pass at the edges of its tiles (64 columns, 64 rows, 128 / 256 values of d,
-rows split over CTAs): a solve against the FP64 sequential chain on the same tape."""
+"""The tensor-core pass at the edges of its tiles (64 columns, 64 rows, 128 / 256 / 512 values
+of d, rows split over CTAs): a solve against the FP64 sequential chain on the same tape."""
 import numpy as np
 import pytest
 
@@ -19,6 +19,7 @@ def h():
     (128, 128, 129), (129, 129, 128), (300, 250, 40),    # an even and an odd number of blocks
     (1500, 256, 70),                                     # rows split over CTAs, two boxes of d
     (700, 16, 9500),                                     # more tiles than SMs, no split
+    (65, 257, 63), (64, 384, 129), (1000, 512, 65),      # two CTAs a tile, each half of d
 ])
 def test_pass_edges(h, N, D, T):
     rng = np.random.default_rng(N + D + T)
