@@ -62,7 +62,9 @@ struct pmcmc_handle {
   std::string err;
   DevParams* d_params = nullptr;
   DevState* d_state = nullptr;
-  DevState* h_state = nullptr;  // pinned
+  DevState* h_state = nullptr;  // pinned, then the states of two sweeps (h_sweep)
+  DevState* h_sweep = nullptr;
+  cudaEvent_t ev_sweep[2] = {nullptr, nullptr};  // sweep it & 1 of the logistic loop done
   unsigned char* ws = nullptr;
   size_t ws_bytes = 0;
   unsigned char* scan_ws = nullptr;
@@ -375,7 +377,7 @@ struct SolveLayout {
   size_t lg[5], lpx, lpy, acc_col, la_col, Bb, Lb, Gb;  // logistic only
   size_t la_ref, tie, lg_acc;                           // logistic: log alpha, near-tie scratch, probe sum
   size_t xi, logu;
-  size_t tcws, Gtc;  // tensor-core logistic path
+  size_t tcws, Gtc, lgscan;  // tensor-core logistic path
   size_t fU, fV, fR, facc, fPhi, fbeta, fdin, fpart, eS0, eS1, exi, ex0;  // :full mode
   size_t alam, acterm, aarev, adirect, ascr, aout;                 // adjoint
   size_t out2_S, out2_lp, out2_acc;  // second output slot of the host-output pipeline
@@ -386,7 +388,8 @@ struct SolveLayout {
 SolveLayout layout(int64_t D, int64_t Dp, int64_t T, int ntiles, size_t es, bool plain,
                    int64_t N = 0, int64_t Tc = 0, size_t tc_bytes = 0,
                    const FullPlan* fp = nullptr, bool adjoint = false,
-                   bool dual_out = false, size_t tie_bytes = 0, int tc_split = 1) {
+                   bool dual_out = false, size_t tie_bytes = 0, int tc_split = 1,
+                   size_t lgscan_bytes = 0) {
   SolveLayout L{};
   size_t off = 0;
   auto take = [&](size_t bytes) {
@@ -439,6 +442,7 @@ SolveLayout layout(int64_t D, int64_t Dp, int64_t T, int ntiles, size_t es, bool
   if (tc_bytes) {
     L.tcws = take(tc_bytes);
     L.Gtc = take(4 * Dp * 2 * static_cast<size_t>(T) * tc_split);
+    L.lgscan = take(lgscan_bytes);
   }
   if (fp || adjoint) L.facc = take(static_cast<size_t>(T));
   if (fp) {
@@ -744,8 +748,11 @@ int run_logistic(pmcmc_handle* h, const pmcmc_target* tg, const SweepKernels& k,
   CK(cudaMemcpyAsync(h->d_params, &P, sizeof(DevParams), cudaMemcpyHostToDevice, h->stream));
   if (smem_sweep > 0)
     CK(raise_smem_limit(reinterpret_cast<const void*>(coop ? k.sweep_coop : k.sweep), smem_sweep));
-  int rc = ensure_cublas(h);
-  if (rc) return rc;
+  if (!use_tc) {
+    const int rc = ensure_cublas(h);
+    if (rc) return rc;
+  }
+  if (!plain) CK(lg_tie_reset(h->stream, tb));
   void* init_args[] = {&h->d_params, &h->d_state};
   CK(cudaLaunchKernel(k.init, dim3(init_grid), dim3(256), init_args, 0, h->stream));
   cudaGraphConditionalHandle none = 0;
@@ -754,17 +761,26 @@ int run_logistic(pmcmc_handle* h, const pmcmc_target* tg, const SweepKernels& k,
   void *Bb = ws + L.Bb, *Lb = ws + L.Lb, *Gb = ws + L.Gb;
   int* tc_err = use_tc ? lg_tc_err_word(ws + L.tcws) : nullptr;
   if (use_tc) CK(cudaMemsetAsync(tc_err, 0, sizeof(int), h->stream));
+  const bool lg_diag = P.jac == PMCMC_JAC_DIAG;
+  // One probe on the tensor cores: the sweep's kernels after the passes are lg_finish,
+  // lg_tie_solve and lg_scan, which end at once when the solve already has.
+  const bool fast =
+      use_tc && !lg_diag && P.probes == 1 && !h->no_coop && h->tile_override == 0;
+  bool guard = false;  // whether the kernels of `fast` check for the end of the loop
+  float* G = reinterpret_cast<float*>(ws + L.Gtc);
+  const int nsplit = use_tc ? lg_tc_split(tg->lg, P.T) : 1;
+  const double* lp_parts = lg_tc_lp_parts(ws + L.tcws);
+  const int np = use_tc ? lg_tc_lp_count(tg->lg, P.T) : 0;
   auto pass_impl = [&](int mode, double* lp, int probe) -> int {
     if (use_tc) {
-      float* G = reinterpret_cast<float*>(ws + L.Gtc);
-      if (lg_tc_pass(h->stream, tg->lg, h->d_params, h->d_state, lp, mode, P.T, ws + L.tcws, G,
-                     probe))
+      const bool parts = fast && mode != 2;  // the log-likelihood parts are added later
+      if (lg_tc_pass(h->stream, tg->lg, h->d_params, h->d_state, parts ? nullptr : lp, mode, P.T,
+                     ws + L.tcws, G, probe, guard))
         return 1;
-      if (mode != 2 && lg_mid(h->stream, false, h->d_params, h->d_state, mode + 1, 0,
-                              static_cast<int>(P.T), probe, P.Dp, G,
-                              lg_tc_split(tg->lg, P.T)) != cudaSuccess)
-        return 1;
-      return 0;
+      if (mode == 2 || (fast && mode == 1)) return 0;
+      return lg_mid(h->stream, false, h->d_params, h->d_state, mode + 1, 0,
+                    static_cast<int>(P.T), probe, P.Dp, G, nsplit, parts ? lp_parts : nullptr, np,
+                    lp, guard) != cudaSuccess;
     }
     return lg_plain_pass(h->stream, h->cublas, tg->lg, f64, h->d_params, h->d_state, lp, mode,
                          P.T, P.Dp, Bb, Lb, Gb, Tc, probe);
@@ -785,11 +801,15 @@ int run_logistic(pmcmc_handle* h, const pmcmc_target* tg, const SweepKernels& k,
     }
     return pass_impl(mode, lp, probe);
   };
+  // log alpha of every column, and in FP64 near ties (with their affine maps on `fast`)
   auto tie = [&]() -> int {
-    if (lg_tie_refine(h->stream, h->cublas, tg->lg, f64, h->d_params, h->d_state, P.T, la_ref,
-                      tb, kTieBand))
-      return fail(h, PMCMC_ERR_CUDA, "near-tie refinement failed: %s",
-                  cudaGetErrorString(cudaGetLastError()));
+    const cudaError_t e =
+        fast ? lg_finish(h->stream, h->d_params, h->d_state, P.D, P.T, G, nsplit, lp_parts, np,
+                         la_ref, tb, kTieBand, guard)
+             : lg_margin(h->stream, f64, h->d_params, h->d_state, P.T, la_ref, &tb, kTieBand);
+    CK(e);
+    CK(lg_tie_solve(h->stream, tg->lg, h->d_params, h->d_state, la_ref, tb, kTieBand,
+                    fast ? G : nullptr, nsplit, h->num_sms));
     return PMCMC_OK;
   };
   // the tensor-core error word travels with the state in every per-sweep copy
@@ -799,7 +819,6 @@ int run_logistic(pmcmc_handle* h, const pmcmc_target* tg, const SweepKernels& k,
   // last add z_k .* J z_k into lg_acc, the sweep adds the last and divides
   const int grid_acc = static_cast<int>(std::min<int64_t>((P.T + kWarps - 1) / kWarps,
                                                           int64_t(h->num_sms) * 8));
-  const bool lg_diag = P.jac == PMCMC_JAC_DIAG;
   // The launches of one Newton sweep, ending with the finish-and-scan kernel.
   auto issue_sweep = [&]() -> int {
     // exact diagonal: g_x, y, diag H_x | g_y | H_y r | H_x u (logistic.cu, modes 3-6)
@@ -854,10 +873,51 @@ int run_logistic(pmcmc_handle* h, const pmcmc_target* tg, const SweepKernels& k,
     if (*h_err) return fail(h, PMCMC_ERR_TIMEOUT, "tensor-core pass: a bounded wait gave up");
     return PMCMC_OK;
   };
-  for (int it = 0; it < P.maxiter; ++it) {
-    const int rc = eager_sweep();
+  // The same on `fast`, one sweep ahead of the host's check: sweep it + 1 is launched
+  // before the state of sweep it is read, so the device never waits for the host (a
+  // small solve, 256 columns of N = 400, D = 24, spent 60 of 145 us a sweep on that);
+  // after the last sweep one more is launched, whose kernels do nothing.
+  auto ahead_sweep = [&](int it) -> int {
+    if (pass(0, P.lpx) || pass(1, P.lpy))
+      return fail(h, PMCMC_ERR_CUDA, "logistic pass failed: %s",
+                  cudaGetErrorString(cudaGetLastError()));
+    if (h->profiling) CK(cudaEventRecord(h->ev[0], h->stream));
+    const int rc = tie();
     if (rc) return rc;
-    if (h->h_state->converged || h->h_state->status) break;
+    CK(lg_scan(h->stream, h->d_params, h->d_state, P.Dp, P.T, ws + L.lgscan,
+               h->h_sweep + (it & 1), h->num_sms));
+    CK(cudaEventRecord(h->ev_sweep[it & 1], h->stream));
+    if (h->profiling) {
+      float ms = 0;
+      CK(cudaEventRecord(h->ev[1], h->stream));
+      CK(cudaEventSynchronize(h->ev[1]));
+      CK(cudaEventElapsedTime(&ms, h->ev[0], h->ev[1]));
+      h->prof.sweep_launches += 1;
+      h->prof.sweep_ms += ms;
+    }
+    return PMCMC_OK;
+  };
+  if (fast) {
+    for (cudaEvent_t& e : h->ev_sweep)
+      if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    guard = true;
+    for (int it = 0; it <= P.maxiter; ++it) {
+      if (it < P.maxiter) {
+        const int rc = ahead_sweep(it);
+        if (rc) return rc;
+      }
+      if (it == 0) continue;
+      CK(cudaEventSynchronize(h->ev_sweep[(it - 1) & 1]));
+      *h->h_state = h->h_sweep[(it - 1) & 1];
+      if (h->h_state->converged || h->h_state->status) break;
+    }
+    guard = false;
+  } else {
+    for (int it = 0; it < P.maxiter; ++it) {
+      const int rc = eager_sweep();
+      if (rc) return rc;
+      if (h->h_state->converged || h->h_state->status) break;
+    }
   }
   if (!plain && !h->h_state->status) {
     // verification at the returned trajectory: the passes at x_bar_t = S_{t-1},
@@ -869,7 +929,7 @@ int run_logistic(pmcmc_handle* h, const pmcmc_target* tg, const SweepKernels& k,
       const int rc = tie();
       if (rc) return rc;
     } else {
-      CK(lg_margin(h->stream, f64, h->d_params, h->d_state, P.T, la_ref, tb.mg));
+      CK(lg_margin(h->stream, f64, h->d_params, h->d_state, P.T, la_ref, nullptr, 0.f));
     }
     CK(lg_verify(h->stream, f64, h->d_params, h->d_state, P.T, la_ref));
   }
@@ -1311,7 +1371,8 @@ int solve_core(pmcmc_handle* h, const pmcmc_target* tg, const pmcmc_deer_params*
                                use_tc ? lg_tc_ws_bytes(tg->lg, T) : 0, full ? &fplan : nullptr,
                                false, pipe,
                                logistic ? lg_tie_ws_bytes(tg->lg, T, tie_kmax(T)) : 0,
-                               use_tc ? lg_tc_split(tg->lg, T) : 1);
+                               use_tc ? lg_tc_split(tg->lg, T) : 1,
+                               use_tc ? lg_scan_ws_bytes(Dp, T, h->num_sms) : 0);
   rc = ensure_ws(h, L.total);
   if (rc) return rc;
   if (defer) {
@@ -1722,7 +1783,7 @@ int pmcmc_create(int device, void* stream, pmcmc_handle** out) {
   }
   if (cudaMalloc(&h->d_params, sizeof(DevParams)) != cudaSuccess ||
       cudaMalloc(&h->d_state, sizeof(DevState)) != cudaSuccess ||
-      cudaMallocHost(&h->h_state, sizeof(DevState)) != cudaSuccess ||
+      cudaMallocHost(&h->h_state, 3 * sizeof(DevState)) != cudaSuccess ||
       cudaMallocHost(&h->h_red, 4 * sizeof(unsigned long long)) != cudaSuccess ||
       cudaMalloc(&h->d_full, sizeof(FullArgs)) != cudaSuccess ||
       cudaMalloc(&h->d_params_e, sizeof(DevParams)) != cudaSuccess) {
@@ -1730,6 +1791,7 @@ int pmcmc_create(int device, void* stream, pmcmc_handle** out) {
     pmcmc_destroy(h);
     return PMCMC_ERR_NOMEM;
   }
+  h->h_sweep = h->h_state + 1;
   cudaMemset(h->d_state, 0, sizeof(DevState));
   cudaMemset(h->d_params, 0, sizeof(DevParams));
   const char* ev = std::getenv("PMCMC_EAGER");
@@ -1787,6 +1849,8 @@ int pmcmc_destroy(pmcmc_handle* h) {
   if (h->h_state) cudaFreeHost(h->h_state);
   if (h->h_red) cudaFreeHost(h->h_red);
   for (cudaEvent_t e : h->ev)
+    if (e) cudaEventDestroy(e);
+  for (cudaEvent_t e : h->ev_sweep)
     if (e) cudaEventDestroy(e);
   if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
   delete h;

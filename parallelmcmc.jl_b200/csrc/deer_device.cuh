@@ -91,6 +91,14 @@ struct DevState {
   unsigned long long min_margin_bits, max_defect_bits;
 };
 
+// Whether the Newton loop has ended: what a sweep's kernels that were launched ahead of
+// its last test check first.
+__device__ __forceinline__ bool solve_ended(const DevState* st, int maxiter) {
+  return *reinterpret_cast<const volatile int32_t*>(&st->converged) ||
+         *reinterpret_cast<const volatile int32_t*>(&st->iter) >= maxiter ||
+         *reinterpret_cast<const volatile int32_t*>(&st->status) != 0;
+}
+
 __host__ __device__ __forceinline__ int64_t imin64(int64_t a, int64_t b) { return a < b ? a : b; }
 __host__ __device__ __forceinline__ int64_t imax64(int64_t a, int64_t b) { return a > b ? a : b; }
 

@@ -65,6 +65,15 @@ cudaError_t launch_tape(cudaStream_t s, int64_t D, int64_t T, uint64_t seed, uin
 
 // Standalone diagonal affine scan (tape_scan.cu); `scratch` holds
 // scan_scratch_bytes and needs no clearing.
+// A scan's split over T columns and D coordinates (scan_plan).
+constexpr int kScanWindow = 2048;  // most columns composed before a state is applied
+struct ScanPlan {
+  int nchunks, L;       // chunks of L columns
+  int nblk_d, blk_d;    // blocks of blk_d coordinates
+  int nsub, Ls;         // runs of Ls columns inside a chunk
+  int group, threads;   // chunks composed at a time; threads a CTA
+};
+ScanPlan scan_plan(int64_t D, int64_t T, int max_ctas, int min_cols, int max_group);
 int scan_tile_cols(int64_t D, int64_t T);
 size_t scan_scratch_bytes(bool f64, int64_t D, int64_t T);
 cudaError_t launch_affine_scan(cudaStream_t s, bool f64, int64_t D, int64_t T, const void* A,

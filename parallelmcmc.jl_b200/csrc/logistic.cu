@@ -153,8 +153,10 @@ __global__ void lg_epilogue_kernel(const Real* __restrict__ ylab, int64_t N, int
 template <typename Real>
 __global__ void lg_mid_kernel(const DevParams* __restrict__ Pg, const DevState* __restrict__ st,
                               int stage, int64_t t0, int Tc, int probe, const Real* __restrict__ G,
-                              int nsplit) {
+                              int nsplit, const double* __restrict__ lp_parts, int np,
+                              double* __restrict__ lp, int guard) {
   const DevParams& P = *Pg;
+  if (guard && solve_ended(st, P.maxiter)) return;
   const int64_t Dp = P.Dp, D = P.D;
   const int64_t nq = Dp / 4;
   const int iter = st->iter;
@@ -171,6 +173,11 @@ __global__ void lg_mid_kernel(const DevParams* __restrict__ Pg, const DevState* 
     const int64_t q = i % nq;
     const int64_t t = t0 + j;
     if (t >= P.T) continue;
+    if (lp_parts && q == 0) {  // the pass's log-likelihood parts, in order
+      double a = 0.0;
+      for (int p = 0; p < np; ++p) a += lp_parts[p * P.T + t];
+      lp[t] = a;
+    }
     Real gv[4], gt[4];
     {
       const Real* pv = G + static_cast<int64_t>(j) * Dp + 4 * q;
@@ -311,14 +318,17 @@ cudaError_t lg_epilogue(cudaStream_t s, bool f64, const void* ylab, int64_t N, i
 }
 
 cudaError_t lg_mid(cudaStream_t s, bool f64, const DevParams* dP, const DevState* dS, int stage,
-                   int64_t t0, int Tc, int probe, int64_t Dp, const void* G, int nsplit) {
+                   int64_t t0, int Tc, int probe, int64_t Dp, const void* G, int nsplit,
+                   const double* lp_parts, int np, double* lp, bool guard) {
   const int g = grid_for(static_cast<int64_t>(Tc) * (Dp / 4));
   if (f64)
     lg_mid_kernel<double><<<g, 256, 0, s>>>(dP, dS, stage, t0, Tc, probe,
-                                            static_cast<const double*>(G), nsplit);
+                                            static_cast<const double*>(G), nsplit, lp_parts, np,
+                                            lp, guard ? 1 : 0);
   else
     lg_mid_kernel<float><<<g, 256, 0, s>>>(dP, dS, stage, t0, Tc, probe,
-                                           static_cast<const float*>(G), nsplit);
+                                           static_cast<const float*>(G), nsplit, lp_parts, np,
+                                           lp, guard ? 1 : 0);
   return cudaGetLastError();
 }
 

@@ -36,7 +36,9 @@ int lg_plain_pass(cudaStream_t s, cublasHandle_t cb, const LogisticDev& X, bool 
                   int64_t Dp, void* Bbuf, void* Lbuf, void* Gbuf, int64_t Tc, int probe);
 
 cudaError_t lg_mid(cudaStream_t s, bool f64, const DevParams* dP, const DevState* dS, int stage,
-                   int64_t t0, int Tc, int probe, int64_t Dp, const void* G, int nsplit = 1);
+                   int64_t t0, int Tc, int probe, int64_t Dp, const void* G, int nsplit = 1,
+                   const double* lp_parts = nullptr, int np = 0, double* lp = nullptr,
+                   bool guard = false);
 // X2 = X .* X in the state's precision (once; the caller serialises first uses).
 cudaError_t lg_make_square(cudaStream_t s, LogisticDev& X, bool f64);
 
@@ -46,8 +48,12 @@ cudaError_t lg_make_square(cudaStream_t s, LogisticDev& X, bool f64);
 // operand arrays and an error word (lg_tc_ws_bytes).
 bool lg_tc_supported(const LogisticDev& X);
 size_t lg_tc_ws_bytes(const LogisticDev& X, int64_t T);
+// lp = NULL leaves lp as lg_tc_lp_parts partial sums; guard: nothing once the solve has ended.
 int lg_tc_pass(cudaStream_t s, const LogisticDev& X, const DevParams* dP, const DevState* dS,
-               double* lp, int mode, int64_t T, void* ws, float* G, int probe);
+               double* lp, int mode, int64_t T, void* ws, float* G, int probe,
+               bool guard = false);
+int lg_tc_lp_count(const LogisticDev& X, int64_t T);
+const double* lg_tc_lp_parts(void* ws);
 int* lg_tc_err_word(void* ws);
 int lg_tc_split(const LogisticDev& X, int64_t T);  // parts of G that a pass writes
 // One bounded mbarrier wait that nothing completes (bound check); err[0] = 1
@@ -58,24 +64,38 @@ cudaError_t lg_tc_mbar_bound(cudaStream_t s, int* err);
 // Scratch of one refinement over at most kmax columns.
 struct TieBufs {
   int kmax = 0;
-  float* mg = nullptr;      // [T] |log alpha - log u| of the sweep
-  int32_t* list = nullptr;  // [kmax] selected columns, ascending
-  int32_t* info = nullptr;  // [4] selected, inside the widest band, band index
-  double *Bx = nullptr, *By = nullptr, *GX = nullptr, *G = nullptr, *G2 = nullptr;  // [kmax x Dp]
-  double* L = nullptr;                                                            // [kmax x N]
-  double *lpx = nullptr, *lpy = nullptr;                                          // [kmax]
+  float* mg = nullptr;         // [T] |log alpha - log u| of the sweep
+  int32_t* list = nullptr;     // [kmax] columns inside the band
+  uint32_t* count = nullptr;   // [4] columns inside each of the nested bands
+  double *By = nullptr, *GX = nullptr;  // [kmax x Dp]
+  double* R = nullptr;                  // [kmax x N]
+  double *lpP = nullptr, *lpx = nullptr, *GP = nullptr;
 };
 size_t lg_tie_ws_bytes(const LogisticDev& X, int64_t T, int kmax);
 TieBufs lg_tie_carve(void* ws, const LogisticDev& X, int64_t T, int kmax);
-// log alpha of every column as the sweep forms it -> la_ref, |margin| -> mg.
+// Clears the list; once a solve (lg_tie_solve leaves it clear).
+cudaError_t lg_tie_reset(cudaStream_t s, const TieBufs& b);
+// log alpha of every column as the sweep forms it -> la_ref; with b, the columns whose
+// margin is below `band` are listed.
 cudaError_t lg_margin(cudaStream_t s, bool f64, const DevParams* dP, const DevState* dS,
-                      int64_t T, double* la_ref, float* mg);
-// lg_margin, then FP64 log alpha for the columns whose margin is below `band`
-// (or a quarter, sixteenth, sixty-fourth of it, the widest that fits kmax),
-// written over their la_ref entries.  cb must be on stream s.
-int lg_tie_refine(cudaStream_t s, cublasHandle_t cb, const LogisticDev& X, bool f64,
-                  const DevParams* dP, const DevState* dS, int64_t T, double* la_ref,
-                  const TieBufs& b, float band);
+                      int64_t T, double* la_ref, const TieBufs* b, float band);
+// FP64 log alpha of the listed columns (or those below a quarter, sixteenth, sixty-fourth
+// of `band`, the widest that fits kmax) over their la_ref entries; with G (FP32 state, the
+// second pass's parts) their affine maps again by it.
+cudaError_t lg_tie_solve(cudaStream_t s, const LogisticDev& X, const DevParams* dP,
+                         const DevState* dS, double* la_ref, const TieBufs& b, float band,
+                         const float* G, int nsplit, int num_sms);
+// Finish of a sweep on the tensor-core path with one probe (logistic_sweep.cu): every
+// column's log alpha and affine map (lg[3], lg[4]) from the second pass's G, the near-tie
+// columns listed; lp_parts: np parts of loglik(y) (summed into lpy).
+cudaError_t lg_finish(cudaStream_t s, const DevParams* dP, const DevState* dS, int64_t D,
+                      int64_t T, const float* G, int nsplit, const double* lp_parts, int np,
+                      double* la_ref, const TieBufs& b, float band, bool guard);
+// The sweep itself: S <- damped scan of the affine maps, the convergence test; writes the
+// state to *st_host (pinned) as well.  scratch: lg_scan_ws_bytes.
+size_t lg_scan_ws_bytes(int64_t Dp, int64_t T, int num_sms);
+cudaError_t lg_scan(cudaStream_t s, const DevParams* dP, DevState* dS, int64_t Dp, int64_t T,
+                    void* scratch, DevState* st_host, int num_sms);
 // Accept flags, margins and the recursion defect at the returned trajectory from
 // la_ref and the passes' proposals (into acc_col, la_col, max_defect_bits).
 cudaError_t lg_verify(cudaStream_t s, bool f64, const DevParams* dP, DevState* dS, int64_t T,

@@ -372,7 +372,8 @@ __global__ void __launch_bounds__(kThreadsPass, 1)
                          const DevParams* __restrict__ Pg, const DevState* __restrict__ st,
                          int mode, int probe, const float* __restrict__ ylab, int64_t N,
                          int64_t T, int64_t Dp, int nsplit, float* __restrict__ G,
-                         double* __restrict__ lp, int* __restrict__ err) {
+                         double* __restrict__ lp, int guard, int* __restrict__ err) {
+  if (guard && solve_ended(st, Pg->maxiter)) return;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -847,7 +848,7 @@ int* lg_tc_err_word(void* ws) { return static_cast<int*>(ws); }
 template <int NKB, int CL>
 static int launch_pass(cudaStream_t s, const LogisticDev& X, const DevParams* dP,
                        const DevState* dS, double* lp, int mode, int64_t T, int* err, float* G,
-                       int probe, int nsplit) {
+                       int probe, int nsplit, bool guard) {
   CUtensorMap mXh, mXl;
   if (!make_map_x(&mXh, X.Xh, X.Np, X.Dk, tc::RB, NKB) ||
       !make_map_x(&mXl, X.Xl, X.Np, X.Dk, tc::RB, NKB))
@@ -868,22 +869,29 @@ static int launch_pass(cudaStream_t s, const LogisticDev& X, const DevParams* dP
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, fn, mXh, mXl, dP, dS, mode, probe,
                             static_cast<const float*>(X.y32), X.N, T, X.Dp, nsplit, G, lp,
-                            err) == cudaSuccess
+                            guard ? 1 : 0, err) == cudaSuccess
              ? 0
              : 3;
 }
 
+int lg_tc_lp_count(const LogisticDev& X, int64_t T) {
+  return lg_tc_split(X, T) * (X.Dk == 512 ? 2 : 1);
+}
+static double* lp_parts(void* ws) {
+  return reinterpret_cast<double*>(static_cast<unsigned char*>(ws) + 1024);
+}
+const double* lg_tc_lp_parts(void* ws) { return lp_parts(ws); }
+
 int lg_tc_pass(cudaStream_t s, const LogisticDev& X, const DevParams* dP, const DevState* dS,
-               double* lp, int mode, int64_t T, void* ws, float* G, int probe) {
+               double* lp, int mode, int64_t T, void* ws, float* G, int probe, bool guard) {
   int* err = lg_tc_err_word(ws);
-  double* parts = reinterpret_cast<double*>(static_cast<unsigned char*>(ws) + 1024);
-  const int ns = lg_tc_split(X, T), np = X.Dk == 512 ? 2 * ns : ns;
-  double* lps = np > 1 ? parts : lp;
+  const int ns = lg_tc_split(X, T), np = lg_tc_lp_count(X, T);
+  double* lps = lp && np == 1 ? lp : lp_parts(ws);
   const int rc =
-      X.Dk == 128   ? launch_pass<2, 1>(s, X, dP, dS, lps, mode, T, err, G, probe, ns)
-      : X.Dk == 256 ? launch_pass<4, 1>(s, X, dP, dS, lps, mode, T, err, G, probe, ns)
-                    : launch_pass<4, 2>(s, X, dP, dS, lps, mode, T, err, G, probe, ns);
-  if (rc || np == 1) return rc;
+      X.Dk == 128   ? launch_pass<2, 1>(s, X, dP, dS, lps, mode, T, err, G, probe, ns, guard)
+      : X.Dk == 256 ? launch_pass<4, 1>(s, X, dP, dS, lps, mode, T, err, G, probe, ns, guard)
+                    : launch_pass<4, 2>(s, X, dP, dS, lps, mode, T, err, G, probe, ns, guard);
+  if (rc || !lp || np == 1) return rc;
   const int g = static_cast<int>((T + 255) / 256);
   tc::lp_sum_kernel<<<g, 256, 0, s>>>(lps, np, T, lp);
   return cudaGetLastError() == cudaSuccess ? 0 : 3;

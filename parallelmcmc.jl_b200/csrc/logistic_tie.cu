@@ -13,38 +13,39 @@
 // 49, and accept flags that differ from the FP64 sequential chain).
 //
 // The sequential FP64 chain (MALA.jl:377-411, bayes_logreg.jl:37-58) decides
-// such a column by its exact log alpha.  So after the contraction passes of a
+// such a column by its exact log alpha.
+// So after the contraction passes of a
 // sweep:
-//   1. tie_margin_kernel: log alpha_t of every column from the sweep's
-//      quantities (the value the sweep kernel would use) and |margin_t|;
-//   2. tie_select_kernel: the columns whose margin is inside a band, in column
-//      order (deterministic), at most kmax of them: the widest of four nested
-//      bands whose count fits;
-//   3. for those columns, in FP64 from the FP64 design matrix: the gradient at
-//      x_bar_t = S_{t-1}, the proposal y_t = x_bar + eps g + sqrt(2 eps) xi_t,
-//      lp(x_bar), lp(y), the gradient at y and both log proposal densities
-//      (logq_mala, MALA.jl:172-193) -- four DGEMMs over the selected columns
-//      with FP64 elementwise kernels between them;
-//   4. tie_final_kernel: log alpha_t in FP64 replaces the sweep's value.
-// The sweep kernel then reads log alpha from la_ref for every column.
-#include <cublas_v2.h>
+//   1. log alpha_t of every column from the sweep's quantities and |margin_t|; the
+//      columns inside a band are counted and listed (the finish kernel, or
+//      tie_margin_kernel on the paths without it);
+//   2. tie_solve_kernel, one cooperative launch that ends at once when the list is
+//      empty: at most kmax columns (the widest of four nested bands whose count fits),
+//      in FP64 from the FP64 design matrix: the gradient at x_bar_t = S_{t-1}, the
+//      proposal y_t = x_bar + eps g + sqrt(2 eps) xi_t, lp(x_bar), lp(y), the gradient
+//      at y and both log proposal densities (logq_mala, MALA.jl:172-193); log alpha_t
+//      in FP64 replaces the sweep's value, and the column's (A, B) is formed again.
+// The sweep takes log alpha from la_ref for every column.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "deer_device.cuh"
+#include "deer_launch.h"
 #include "logistic.h"
+#include "logistic_column.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace pmcmc {
 namespace tie {
 
-constexpr int kSelThreads = 1024;
-constexpr int kBands = 4;  // band, band / 4, band / 16, band / 64
-
-__device__ __forceinline__ int grid_cap(int64_t n, int per) {
-  const int64_t g = (n + per - 1) / per;
-  return static_cast<int>(g < 148 * 16 ? (g > 0 ? g : 1) : 148 * 16);
-}
+constexpr int kTieThreads = 256;
+constexpr int kTieWarps = kTieThreads / 32;
+constexpr int kTieCtas = 2;    // an SM
+constexpr int kTieParts = 32;  // of the rows, most
 
 // log alpha_t as the sweep computes it (column_logistic in deer_sweep.cu):
 //   sum_d [-tau/2 (y^2 - x^2) + (r1^2 - r2^2) / (4 eps)] + lpy_t - lpx_t,
@@ -53,7 +54,7 @@ __device__ __forceinline__ int grid_cap(int64_t n, int per) {
 template <typename Real>
 __global__ void tie_margin_kernel(const DevParams* __restrict__ Pg,
                                   const DevState* __restrict__ st, double* __restrict__ la_ref,
-                                  float* __restrict__ mg) {
+                                  TieList list) {
   const DevParams& P = *Pg;
   const int lane = threadIdx.x & 31;
   const int64_t D = P.D, Dp = P.Dp;
@@ -77,208 +78,290 @@ __global__ void tie_margin_kernel(const DevParams* __restrict__ Pg,
     la = warp_sum(la) + (P.lpy[t] - P.lpx[t]);
     if (lane == 0) {
       la_ref[t] = la;
-      mg[t] = static_cast<float>(fabs(la - P.logu[t]));
+      if (list.count) tie_note(list, t, la - P.logu[t]);
     }
   }
 }
 
-// Near-tie columns, in column order: the widest of the bands band / 4^i whose
-// count is at most kmax (the narrowest one, truncated to its first kmax
-// columns, if none fits).  One CTA; thread i owns a contiguous run of columns.
-// info[0] = columns selected, info[1] = columns inside the widest band,
-// info[2] = band index used.
-__global__ void __launch_bounds__(kSelThreads)
-    tie_select_kernel(const float* __restrict__ mg, int64_t T, float band, int kmax,
-                      int32_t* __restrict__ list, int32_t* __restrict__ info) {
-  __shared__ int s_cnt[kBands][kSelThreads / 32];
-  __shared__ int s_base[kSelThreads / 32];
-  __shared__ int s_band;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t run = (T + kSelThreads - 1) / kSelThreads;
-  const int64_t c0 = imin64(T, tid * run), c1 = imin64(T, c0 + run);
-  int cnt[kBands] = {0, 0, 0, 0};
-  for (int64_t t = c0; t < c1; ++t) {
-    const float m = mg[t];
-    float b = band;
-#pragma unroll
-    for (int i = 0; i < kBands; ++i, b *= 0.25f) cnt[i] += m < b ? 1 : 0;
-  }
-#pragma unroll
-  for (int i = 0; i < kBands; ++i) {
-    const int s = warp_sum(cnt[i]);
-    if (lane == 0) s_cnt[i][warp] = s;
-  }
-  __syncthreads();
-  if (tid == 0) {
-    int bi = kBands - 1;
-    int tot[kBands];
-    for (int i = 0; i < kBands; ++i) {
-      tot[i] = 0;
-      for (int w = 0; w < kSelThreads / 32; ++w) tot[i] += s_cnt[i][w];
-    }
-    for (int i = 0; i < kBands; ++i)
-      if (tot[i] <= kmax) {
-        bi = i;
-        break;
+// Two FP64 MMAs (8 x 8, k = 4) with the same A: lane l holds A[l / 4][l % 4], B[l % 4][l / 4]
+// and C[l / 4][2 (l % 4) .. + 1].
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(c[0]), "+d"(c[1])
+      : "d"(a), "d"(b));
+}
+
+// Four values another CTA of this launch may have written (FP64), or of the state (FP32,
+// not written here).
+__device__ __forceinline__ void load_cg4(const double* p, double (&v)[4]) {
+  const double2 a = __ldcg(reinterpret_cast<const double2*>(p));
+  const double2 b = __ldcg(reinterpret_cast<const double2*>(p) + 1);
+  v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
+}
+__device__ __forceinline__ void load_cg4(const float* p, double (&v)[4]) {
+  const float4 a = *reinterpret_cast<const float4*>(p);
+  v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
+}
+
+struct TieArgs {
+  TieList list;
+  const double* X;   // N x Dp
+  const double* y;   // N
+  int64_t N;
+  double *By, *GX;   // [kmax x Dp] proposals, gradients at x_bar
+  int64_t Nr;        // N rounded up to 8
+  double* R;         // [kmax x Nr] y - sigmoid
+  double* lpP;       // [ceil(N / 8) x kmax] log-likelihood sums of 8 rows
+  double* lpx;       // [kmax]
+  double* GP;        // parts of the gradients (tie_gp_elems)
+  double* la_ref;
+  PassG G;           // g = NULL: no (A, B) to form again
+  int qpl;
+};
+
+// The work below is bound by L2 (X is read four times, 8 rows or 16 values of d by up to
+// 16 columns a warp), by the five grid barriers where the list is short and by the FP64
+// rate where it is long.  Against the eleven launches around four DGEMMs over all kmax columns
+// that it replaces: 129 us instead of 400 at N = 10000, D = 256 and 65 columns, 45 instead
+// of 80 at N = 3001, D = 101 and 4 columns, 3 instead of 45 with an empty list (N = 400, D = 24).
+__global__ void __launch_bounds__(kTieThreads, kTieCtas)
+    tie_solve_kernel(const DevParams* __restrict__ Pg, const DevState* __restrict__ st, TieArgs a) {
+  __shared__ int s_base[kTieWarps], s_pos;
+  __shared__ double s_sum[kTieWarps];
+  cg::grid_group grid = cg::this_grid();
+  const DevParams& P = *Pg;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int kmax = a.list.kmax;
+  int cnt = static_cast<int>(*reinterpret_cast<const volatile uint32_t*>(a.list.count));
+  if (cnt == 0) return;
+  if (cnt > kmax) {
+    // more columns than fit: the widest band that does, or the first kmax columns of the
+    // narrowest, in column order, from the margins
+    if (blockIdx.x == 0) {
+      if (tid == 0) s_pos = 0;
+      int bi = 1;
+      float b = a.list.band * 0.25f;
+      while (bi < kTieBands - 1 && __ldcg(a.list.count + bi) > static_cast<uint32_t>(kmax)) ++bi, b *= 0.25f;
+      __syncthreads();
+      for (int64_t t0 = 0; t0 < P.T && s_pos < kmax; t0 += kTieThreads) {
+        const bool in = t0 + tid < P.T && a.list.mg[t0 + tid] < b;
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        if (lane == 0) s_base[tid >> 5] = __popc(m);
+        __syncthreads();
+        int pos = s_pos;
+        for (int w = 0; w < (tid >> 5); ++w) pos += s_base[w];
+        pos += __popc(m & ((1u << lane) - 1u));
+        if (in && pos < kmax) a.list.list[pos] = static_cast<int32_t>(t0 + tid);
+        __syncthreads();
+        if (tid == 0)
+          for (int w = 0; w < kTieWarps; ++w) s_pos += s_base[w];
+        __syncthreads();
       }
-    s_band = bi;
-    info[0] = tot[bi] < kmax ? tot[bi] : kmax;
-    info[1] = tot[0];
-    info[2] = bi;
-  }
-  __syncthreads();
-  const int bi = s_band;
-  float b = band;
-  for (int i = 0; i < bi; ++i) b *= 0.25f;
-  // exclusive scan of this thread's count in band bi (warp shuffles, then warps)
-  int mine = 0;
-#pragma unroll
-  for (int i = 0; i < kBands; ++i)
-    if (i == bi) mine = cnt[i];
-  int incl = mine;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += v;
-  }
-  if (tid == 0) {
-    int acc = 0;
-    for (int w = 0; w < kSelThreads / 32; ++w) {
-      s_base[w] = acc;
-      acc += s_cnt[bi][w];
+      if (tid == 0) a.list.count[1] = min(s_pos, kmax);
     }
+    grid.sync();
+    cnt = static_cast<int>(__ldcg(a.list.count + 1));
   }
-  __syncthreads();
-  int pos = s_base[warp] + incl - mine;
-  for (int64_t t = c0; t < c1 && pos < kmax; ++t)
-    if (mg[t] < b) list[pos++] = static_cast<int32_t>(t);
-}
-
-// B[k] (Dp doubles) = x_bar of selected column k; zero beyond the selection.
-template <typename Real>
-__global__ void tie_gather_kernel(const DevParams* __restrict__ Pg,
-                                  const DevState* __restrict__ st,
-                                  const int32_t* __restrict__ list,
-                                  const int32_t* __restrict__ info, int kmax,
-                                  double* __restrict__ B) {
-  const DevParams& P = *Pg;
-  const int64_t Dp = P.Dp;
-  const int cnt = info[0];
+  const int64_t N = a.N, D = P.D, Dp = P.Dp;
+  const int64_t gw = static_cast<int64_t>(blockIdx.x) * kTieWarps + (tid >> 5);
+  const int64_t nw = static_cast<int64_t>(gridDim.x) * kTieWarps;
+  const int ct = (cnt + 15) / 16;              // tiles of 16 columns
+  const int64_t rt = (N + 7) / 8, dt = (Dp + 15) / 16;
+  // parts of the gradients' sums over the rows (each is read again, in order)
+  const int ns = static_cast<int>(imax64(1, imin64(kTieParts, nw / (dt * ct))));
+  const int64_t per = ((N + ns - 1) / ns + 15) / 16 * 16;
   const bool from_x0 = st->iter == 0;
-  const Real* S = static_cast<const Real*>(P.S[st->cur]);
-  const Real* x0 = static_cast<const Real*>(P.x0);
-  const int64_t n = static_cast<int64_t>(kmax) * Dp;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int k = static_cast<int>(i / Dp);
-    const int64_t d = i % Dp;
-    double v = 0.0;
-    if (k < cnt && d < P.D) {
-      const int64_t t = list[k];
-      v = static_cast<double>((from_x0 || t == 0) ? x0[d] : S[(t - 1) * Dp + d]);
+  const float* S = static_cast<const float*>(P.S[st->cur]);
+  const float* x0 = static_cast<const float*>(P.x0);
+  const int r8 = lane >> 2, k4 = lane & 3;
+  auto xbar = [&](int k) {
+    const int64_t t = __ldcg(a.list.list + min(k, cnt - 1));
+    return (from_x0 || t == 0) ? x0 : S + (t - 1) * Dp;
+  };
+  // Logits of 8 rows x 16 columns a warp; R and the rows' log-likelihood terms.  The MMAs'
+  // k runs over the coordinates in an order of its own: lane k4 of a row or column holds
+  // four consecutive ones, loaded 16 bytes at a time (one value a load is bound by the
+  // load unit, 37 us instead of 14 at N = 10000, D = 256, 65 columns).
+  auto logits = [&](auto x_of) {
+    for (int64_t w = gw; w < rt * ct; w += nw) {
+      const int64_t row0 = w / ct * 8;
+      const int c0 = static_cast<int>(w % ct) * 16;
+      const int64_t row = row0 + r8;
+      const double* xr = a.X + (row < N ? row : N - 1) * Dp;
+      const auto* f0 = x_of(min(c0 + r8, cnt - 1));
+      const auto* f1 = x_of(min(c0 + 8 + r8, cnt - 1));
+      const bool two = c0 + 8 < cnt;
+      double c[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+#pragma unroll 2
+      for (int k = 4 * k4; k - 4 * k4 < Dp; k += 16) {
+        double av[4] = {0.0, 0.0, 0.0, 0.0}, b0[4] = {0.0, 0.0, 0.0, 0.0},
+               b1[4] = {0.0, 0.0, 0.0, 0.0};
+        if (k < Dp) {
+          load4(xr + k, av);
+          load_cg4(f0 + k, b0);
+          if (two) load_cg4(f1 + k, b1);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          dmma(c[0], av[i], b0[i]);
+          if (two) dmma(c[1], av[i], b1[i]);
+        }
+      }
+      const double lab = row < N ? a.y[row] : 0.0;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (h && !two) break;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int col = c0 + 8 * h + 2 * k4 + i;
+          const double z = c[h][i];
+          const double e = exp(-fabs(z));
+          const double p = (z >= 0.0 ? 1.0 : e) / (1.0 + e);
+          double term = row < N ? lab * z - (z > 0.0 ? z : 0.0) : 0.0;
+          double prod = row < N ? 1.0 + e : 1.0;  // one log for the 8 rows
+#pragma unroll
+          for (int o = 4; o < 32; o <<= 1) {
+            term += __shfl_xor_sync(0xffffffffu, term, o);
+            prod *= __shfl_xor_sync(0xffffffffu, prod, o);
+          }
+          if (col < cnt) {
+            a.R[static_cast<int64_t>(col) * a.Nr + row] = row < N ? lab - p : 0.0;
+            if (r8 == 0) a.lpP[row0 / 8 * kmax + col] = term - log(prod);
+          }
+        }
+      }
     }
-    B[i] = v;
-  }
-}
-
-// Column k of L (N logits): r = y - sigmoid(l) in place, lp[k] = sum_n
-// y l - softplus(l) (bayes_logreg.jl:37-58 with the stable softplus of
-// docs/src/15-gpu.md:91-97), in FP64, summed in a fixed order.
-__global__ void tie_loglik_kernel(const double* __restrict__ ylab, int64_t N,
-                                  const int32_t* __restrict__ info, double* __restrict__ L,
-                                  double* __restrict__ lp) {
-  __shared__ double red[32];
-  const int k = blockIdx.x;
-  double* l = L + static_cast<int64_t>(k) * N;
-  if (k >= info[0]) {
-    for (int64_t n = threadIdx.x; n < N; n += blockDim.x) l[n] = 0.0;
-    if (threadIdx.x == 0) lp[k] = 0.0;
-    return;
-  }
-  double acc = 0.0;
-  for (int64_t n = threadIdx.x; n < N; n += blockDim.x) {
-    const double z = l[n];
-    const double e = exp(-fabs(z));
-    const double sp = (z > 0.0 ? z : 0.0) + log1p(e);
-    const double p = z >= 0.0 ? 1.0 / (1.0 + e) : e / (1.0 + e);
-    acc += ylab[n] * z - sp;
-    l[n] = ylab[n] - p;
-  }
-  acc = warp_sum(acc);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double a = 0.0;
-    for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) a += red[w];
-    lp[k] = a;
-  }
-}
-
-// gx = X'r - tau x_bar (bayes_logreg.jl:48-58), y = x_bar + eps gx + sqrt(2 eps) xi
-// (MALA.jl:221-222), column by column over the selection.
-__global__ void tie_propose_kernel(const DevParams* __restrict__ Pg,
-                                   const int32_t* __restrict__ list,
-                                   const int32_t* __restrict__ info, int kmax,
-                                   const double* __restrict__ Bx, const double* __restrict__ G,
-                                   double* __restrict__ GX, double* __restrict__ By) {
-  const DevParams& P = *Pg;
-  const int64_t Dp = P.Dp;
-  const int cnt = info[0];
-  const int64_t n = static_cast<int64_t>(kmax) * Dp;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int k = static_cast<int>(i / Dp);
-    const int64_t d = i % Dp;
-    double gx = 0.0, y = 0.0;
-    if (k < cnt && d < P.D) {
-      const int64_t t = list[k];
-      const double x = Bx[i];
-      gx = G[i] - P.tau * x;
-      y = x + P.eps * gx + P.sqrt2eps * static_cast<double>(P.xi[t * Dp + d]);
+  };
+  // Parts of X'R: 16 values of d (lane r8 holds two) x 16 columns a warp, over `per` rows
+  // (lane k4 holds four consecutive ones of 16)
+  auto gradients = [&]() {
+    for (int64_t w = gw; w < dt * ct * ns; w += nw) {
+      const int64_t part = w / (dt * ct), q = w % (dt * ct);
+      const int64_t d = q / ct * 16 + 2 * r8;
+      const int c0 = static_cast<int>(q % ct) * 16;
+      const int64_t n0 = part * per, n1 = imin64(N, n0 + per);
+      const double* xc = a.X + (d < Dp ? d : Dp - 2);
+      const double* q0 = a.R + static_cast<int64_t>(min(c0 + r8, cnt - 1)) * a.Nr;
+      const double* q1 = a.R + static_cast<int64_t>(min(c0 + 8 + r8, cnt - 1)) * a.Nr;
+      const bool two = c0 + 8 < cnt;
+      double c[2][2][2] = {};  // [d][columns]
+#pragma unroll 2
+      for (int64_t n = n0 + 4 * k4; n - 4 * k4 < n1; n += 16) {
+        double2 av[4];
+        double b0[4] = {0.0, 0.0, 0.0, 0.0}, b1[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)  // a row past N is read as the last one, times R = 0
+          av[i] = *reinterpret_cast<const double2*>(xc + imin64(n + i, N - 1) * Dp);
+        if (n < n1) {  // (R is zero from N to its stride)
+          load_cg4(q0 + n, b0);
+          if (two) load_cg4(q1 + n, b1);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          dmma(c[0][0], av[i].x, b0[i]);
+          dmma(c[1][0], av[i].y, b0[i]);
+          if (two) {
+            dmma(c[0][1], av[i].x, b1[i]);
+            dmma(c[1][1], av[i].y, b1[i]);
+          }
+        }
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int col = c0 + 8 * h + 2 * k4 + i;
+          if (col < cnt && d < Dp)
+            *reinterpret_cast<double2*>(a.GP + (part * cnt + col) * Dp + d) =
+                make_double2(c[0][h][i], c[1][h][i]);
+        }
     }
-    GX[i] = gx;
-    By[i] = y;
-  }
-}
+  };
+  auto grad_at = [&](int64_t k, int64_t d) {
+    double g = 0.0;
+#pragma unroll 8
+    for (int p = 0; p < ns; ++p) g += __ldcg(a.GP + (p * cnt + k) * Dp + d);
+    return g;
+  };
+  // sums over the CTA, the same in every thread
+  auto cta_sum = [&](double v) {
+    v = warp_sum(v);
+    __syncthreads();
+    if (lane == 0) s_sum[tid >> 5] = v;
+    __syncthreads();
+    double t = 0.0;
+#pragma unroll
+    for (int w = 0; w < kTieWarps; ++w) t += s_sum[w];
+    return t;
+  };
+  auto loglik = [&](int64_t k) {
+    double l = 0.0;
+#pragma unroll 4
+    for (int64_t r = tid; r < rt; r += kTieThreads) l += __ldcg(a.lpP + r * kmax + k);
+    return cta_sum(l);
+  };
 
-// log alpha_t = [lp(y) + logq(x|y)] - [lp(x) + logq(y|x)] (MALA.jl:172-193,
-// 402) in FP64 for every selected column; one warp a column.
-__global__ void tie_final_kernel(const DevParams* __restrict__ Pg,
-                                 const int32_t* __restrict__ list,
-                                 const int32_t* __restrict__ info, int kmax,
-                                 const double* __restrict__ Bx, const double* __restrict__ By,
-                                 const double* __restrict__ GX, const double* __restrict__ G,
-                                 const double* __restrict__ lpx, const double* __restrict__ lpy,
-                                 double* __restrict__ la_ref) {
-  const DevParams& P = *Pg;
-  const int lane = threadIdx.x & 31;
-  const int64_t Dp = P.Dp;
-  const int cnt = info[0];
-  const int nw = gridDim.x * (blockDim.x >> 5);
-  for (int k = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); k < cnt; k += nw) {
-    const double* x = Bx + static_cast<int64_t>(k) * Dp;
-    const double* y = By + static_cast<int64_t>(k) * Dp;
-    const double* gx = GX + static_cast<int64_t>(k) * Dp;
-    const double* g2 = G + static_cast<int64_t>(k) * Dp;
+  logits([&](int k) { return xbar(k); });
+  grid.sync();
+  gradients();
+  grid.sync();
+  // gx = X'r - tau x_bar (bayes_logreg.jl:48-58), y = x_bar + eps gx + sqrt(2 eps) xi
+  // (MALA.jl:221-222); one CTA a column
+  for (int64_t k = blockIdx.x; k < cnt; k += gridDim.x) {
+    const int64_t t = __ldcg(a.list.list + k);
+    const float* x = xbar(static_cast<int>(k));
+    for (int64_t d = tid; d < Dp; d += kTieThreads) {
+      double gx = 0.0, y = 0.0;
+      if (d < D) {
+        const double xd = static_cast<double>(x[d]);
+        gx = grad_at(k, d) - P.tau * xd;
+        y = xd + P.eps * gx + P.sqrt2eps * static_cast<double>(P.xi[t * Dp + d]);
+      }
+      a.GX[k * Dp + d] = gx;
+      a.By[k * Dp + d] = y;
+    }
+    const double l = loglik(k);
+    if (tid == 0) a.lpx[k] = l;
+  }
+  grid.sync();
+  logits([&](int k) { return static_cast<const double*>(a.By) + static_cast<int64_t>(k) * Dp; });
+  grid.sync();
+  gradients();
+  grid.sync();
+  // log alpha_t = [lp(y) + logq(x|y)] - [lp(x) + logq(y|x)] (MALA.jl:172-193, 402), and
+  // the column's affine map by it; one CTA a column
+  for (int64_t k = blockIdx.x; k < cnt; k += gridDim.x) {
+    const int64_t t = __ldcg(a.list.list + k);
+    const float* x = xbar(static_cast<int>(k));
     double xx = 0.0, yy = 0.0, q1 = 0.0, q2 = 0.0;
-    for (int64_t d = lane; d < P.D; d += 32) {
-      const double gy = g2[d] - P.tau * y[d];
-      const double a = y[d] - (x[d] + P.eps * gx[d]);
-      const double b = x[d] - (y[d] + P.eps * gy);
-      xx += x[d] * x[d];
-      yy += y[d] * y[d];
-      q1 += a * a;
-      q2 += b * b;
+    for (int64_t d = tid; d < D; d += kTieThreads) {
+      const double xd = static_cast<double>(x[d]), yd = __ldcg(a.By + k * Dp + d);
+      const double gx = __ldcg(a.GX + k * Dp + d);
+      const double gy = grad_at(k, d) - P.tau * yd;
+      const double u = yd - (xd + P.eps * gx);
+      const double v = xd - (yd + P.eps * gy);
+      xx += xd * xd;
+      yy += yd * yd;
+      q1 += u * u;
+      q2 += v * v;
     }
-    xx = warp_sum(xx);
-    yy = warp_sum(yy);
-    q1 = warp_sum(q1);
-    q2 = warp_sum(q2);
-    if (lane == 0) {
-      const double lp_x = lpx[k] - 0.5 * P.tau * xx, lp_y = lpy[k] - 0.5 * P.tau * yy;
-      la_ref[list[k]] = (lp_y - q2 * P.inv4eps) - (lp_x - q1 * P.inv4eps);
+    xx = cta_sum(xx);
+    yy = cta_sum(yy);
+    q1 = cta_sum(q1);
+    q2 = cta_sum(q2);
+    const double lp_x = __ldcg(a.lpx + k) - 0.5 * P.tau * xx;
+    const double lp_y = loglik(k) - 0.5 * P.tau * yy;
+    const double la = (lp_y - q2 * P.inv4eps) - (lp_x - q1 * P.inv4eps);
+    if (tid == 0) a.la_ref[t] = la;
+    if (a.G.g && tid < 32) {
+      const TapeKey key(P.seed, P.block);
+      const int iter = st->iter;
+      if (a.qpl == 1) finish_column<1>(P, key, x, t, iter, a.G, 0.0, &la);
+      else if (a.qpl == 2) finish_column<2>(P, key, x, t, iter, a.G, 0.0, &la);
+      else finish_column<4>(P, key, x, t, iter, a.G, 0.0, &la);
     }
   }
+  if (blockIdx.x == 0 && tid < kTieBands) a.list.count[tid] = 0;  // every CTA has read them
 }
 
 // Verification at a returned trajectory S (after the contraction passes at
@@ -330,15 +413,25 @@ namespace {
 size_t up256(size_t b) { return (b + 255) & ~size_t(255); }
 }  // namespace
 
+// Parts of the gradients: more than one only while every part's tile has a warp of its
+// own, so at most 256 entries a warp of the largest grid, or one part of all columns.
+static size_t tie_gp_elems(int64_t Dp, int kmax) {
+  const size_t warps = size_t(256) * tie::kTieCtas * tie::kTieWarps;  // up to 256 SMs
+  return std::max(warps * 256, static_cast<size_t>(Dp) * kmax);
+}
+
 size_t lg_tie_ws_bytes(const LogisticDev& X, int64_t T, int kmax) {
   const size_t K = static_cast<size_t>(kmax), Dp = static_cast<size_t>(X.Dp);
-  return up256(4 * static_cast<size_t>(T)) + up256(4 * K) + up256(16) +
-         5 * up256(8 * Dp * K) + up256(8 * static_cast<size_t>(X.N) * K) + 2 * up256(8 * K);
+  const size_t rt = static_cast<size_t>((X.N + 7) / 8);
+  return up256(4 * static_cast<size_t>(T)) + up256(4 * K) + up256(16) + 2 * up256(8 * Dp * K) +
+         up256(8 * 8 * rt * K) + up256(8 * rt * K) + up256(8 * K) +
+         up256(8 * tie_gp_elems(X.Dp, kmax));
 }
 
 TieBufs lg_tie_carve(void* ws, const LogisticDev& X, int64_t T, int kmax) {
   TieBufs b{};
   const size_t K = static_cast<size_t>(kmax), Dp = static_cast<size_t>(X.Dp);
+  const size_t rt = static_cast<size_t>((X.N + 7) / 8);
   unsigned char* p = static_cast<unsigned char*>(ws);
   auto take = [&](size_t bytes) {
     unsigned char* q = p;
@@ -348,61 +441,55 @@ TieBufs lg_tie_carve(void* ws, const LogisticDev& X, int64_t T, int kmax) {
   b.kmax = kmax;
   b.mg = reinterpret_cast<float*>(take(4 * static_cast<size_t>(T)));
   b.list = reinterpret_cast<int32_t*>(take(4 * K));
-  b.info = reinterpret_cast<int32_t*>(take(16));
-  b.Bx = reinterpret_cast<double*>(take(8 * Dp * K));
+  b.count = reinterpret_cast<uint32_t*>(take(16));
   b.By = reinterpret_cast<double*>(take(8 * Dp * K));
   b.GX = reinterpret_cast<double*>(take(8 * Dp * K));
-  b.G = reinterpret_cast<double*>(take(8 * Dp * K));
-  b.G2 = reinterpret_cast<double*>(take(8 * Dp * K));
-  b.L = reinterpret_cast<double*>(take(8 * static_cast<size_t>(X.N) * K));
+  b.R = reinterpret_cast<double*>(take(8 * 8 * rt * K));
+  b.lpP = reinterpret_cast<double*>(take(8 * rt * K));
   b.lpx = reinterpret_cast<double*>(take(8 * K));
-  b.lpy = reinterpret_cast<double*>(take(8 * K));
+  b.GP = reinterpret_cast<double*>(take(8 * tie_gp_elems(X.Dp, kmax)));
   return b;
 }
 
+cudaError_t lg_tie_reset(cudaStream_t s, const TieBufs& b) {
+  return cudaMemsetAsync(b.count, 0, 16, s);
+}
+
+static TieList tie_list(const TieBufs& b, float band) {
+  return TieList{band, b.kmax, b.mg, b.list, b.count};
+}
+
 cudaError_t lg_margin(cudaStream_t s, bool f64, const DevParams* dP, const DevState* dS,
-                      int64_t T, double* la_ref, float* mg) {
+                      int64_t T, double* la_ref, const TieBufs* b, float band) {
   const int g = static_cast<int>((T + 7) / 8 < 148 * 16 ? (T + 7) / 8 : 148 * 16);
-  if (f64) tie::tie_margin_kernel<double><<<g, 256, 0, s>>>(dP, dS, la_ref, mg);
-  else tie::tie_margin_kernel<float><<<g, 256, 0, s>>>(dP, dS, la_ref, mg);
+  const TieList list = b ? tie_list(*b, band) : TieList{};
+  if (f64) tie::tie_margin_kernel<double><<<g, 256, 0, s>>>(dP, dS, la_ref, list);
+  else tie::tie_margin_kernel<float><<<g, 256, 0, s>>>(dP, dS, la_ref, list);
   return cudaGetLastError();
 }
 
-int lg_tie_refine(cudaStream_t s, cublasHandle_t cb, const LogisticDev& X, bool f64,
-                  const DevParams* dP, const DevState* dS, int64_t T, double* la_ref,
-                  const TieBufs& b, float band) {
-  const int K = b.kmax;
-  const int64_t N = X.N, Dp = X.Dp;
-  if (lg_margin(s, f64, dP, dS, T, la_ref, b.mg) != cudaSuccess) return 3;
-  tie::tie_select_kernel<<<1, tie::kSelThreads, 0, s>>>(b.mg, T, band, K, b.list, b.info);
-  if (cudaGetLastError() != cudaSuccess) return 3;
-  const int64_t nk = static_cast<int64_t>(K) * Dp;
-  const int ge = static_cast<int>((nk + 255) / 256 < 148 * 16 ? (nk + 255) / 256 : 148 * 16);
-  if (f64) tie::tie_gather_kernel<double><<<ge, 256, 0, s>>>(dP, dS, b.list, b.info, K, b.Bx);
-  else tie::tie_gather_kernel<float><<<ge, 256, 0, s>>>(dP, dS, b.list, b.info, K, b.Bx);
-  if (cudaGetLastError() != cudaSuccess) return 3;
-  const double one = 1.0, zero = 0.0;
-  const int n = static_cast<int>(N), dp = static_cast<int>(Dp);
-  // L = X Bx (N x K), X row-major N x Dp = column-major Dp x N
-  if (cublasDgemm(cb, CUBLAS_OP_T, CUBLAS_OP_N, n, K, dp, &one, X.X64, dp, b.Bx, dp, &zero, b.L,
-                  n) != CUBLAS_STATUS_SUCCESS)
-    return 3;
-  tie::tie_loglik_kernel<<<K, 256, 0, s>>>(X.y64, N, b.info, b.L, b.lpx);
-  if (cublasDgemm(cb, CUBLAS_OP_N, CUBLAS_OP_N, dp, K, n, &one, X.X64, dp, b.L, n, &zero, b.G,
-                  dp) != CUBLAS_STATUS_SUCCESS)
-    return 3;
-  tie::tie_propose_kernel<<<ge, 256, 0, s>>>(dP, b.list, b.info, K, b.Bx, b.G, b.GX, b.By);
-  if (cublasDgemm(cb, CUBLAS_OP_T, CUBLAS_OP_N, n, K, dp, &one, X.X64, dp, b.By, dp, &zero, b.L,
-                  n) != CUBLAS_STATUS_SUCCESS)
-    return 3;
-  tie::tie_loglik_kernel<<<K, 256, 0, s>>>(X.y64, N, b.info, b.L, b.lpy);
-  if (cublasDgemm(cb, CUBLAS_OP_N, CUBLAS_OP_N, dp, K, n, &one, X.X64, dp, b.L, n, &zero, b.G2,
-                  dp) != CUBLAS_STATUS_SUCCESS)
-    return 3;
-  const int gf = (K + 7) / 8;
-  tie::tie_final_kernel<<<gf, 256, 0, s>>>(dP, b.list, b.info, K, b.Bx, b.By, b.GX, b.G2, b.lpx,
-                                           b.lpy, la_ref);
-  return cudaGetLastError() == cudaSuccess ? 0 : 3;
+cudaError_t lg_tie_solve(cudaStream_t s, const LogisticDev& X, const DevParams* dP,
+                         const DevState* dS, double* la_ref, const TieBufs& b, float band,
+                         const float* G, int nsplit, int num_sms) {
+  tie::TieArgs a{};
+  a.list = tie_list(b, band);
+  a.X = X.X64;
+  a.y = X.y64;
+  a.N = X.N;
+  a.Nr = (X.N + 7) / 8 * 8;
+  a.By = b.By;
+  a.GX = b.GX;
+  a.R = b.R;
+  a.lpP = b.lpP;
+  a.lpx = b.lpx;
+  a.GP = b.GP;
+  a.la_ref = la_ref;
+  a.G = PassG{G, nsplit};
+  a.qpl = X.D <= 128 ? 1 : X.D <= 256 ? 2 : 4;
+  void* args[] = {&dP, &dS, &a};
+  return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(tie::tie_solve_kernel),
+                                     dim3(std::min(num_sms, 256) * tie::kTieCtas),
+                                     dim3(tie::kTieThreads), args, 0, s);
 }
 
 cudaError_t lg_verify(cudaStream_t s, bool f64, const DevParams* dP, DevState* dS, int64_t T,

@@ -13,17 +13,6 @@ namespace cg = cooperative_groups;
 
 namespace pmcmc {
 
-namespace {
-constexpr int kScanWindow = 2048;  // most columns composed before a state is applied
-
-struct ScanPlan {
-  int nchunks, L;       // chunks of L columns
-  int nblk_d, blk_d;    // blocks of blk_d coordinates
-  int nsub, Ls;         // runs of Ls columns inside a chunk
-  int group, threads;   // chunks composed at a time; threads a CTA
-};
-}  // namespace
-
 // Tape block of (seed, block): Xi (D x T, column-major) and u (T)
 // (counterpart of _make_mala_tape_block, interface.jl:334-358).
 __global__ void tape_kernel(int64_t D, int64_t T, uint64_t seed, uint64_t block, float* Xi,
@@ -209,7 +198,7 @@ __global__ void __launch_bounds__(kThreads, kScanCtas)
 // Up to 3 CTAs an SM, 96 KB of loads in flight an SM; chunks of
 // min_cols columns at least (scan_tile_cols of the whole scan), so that the chunks
 // fit the scratch.
-static ScanPlan scan_plan(int64_t D, int64_t T, int max_ctas, int min_cols,
+ScanPlan scan_plan(int64_t D, int64_t T, int max_ctas, int min_cols,
                           int max_group) {
   ScanPlan p{};
   p.nblk_d = static_cast<int>((D + kThreads - 1) / kThreads);
