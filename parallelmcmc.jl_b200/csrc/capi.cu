@@ -64,6 +64,8 @@ struct pmcmc_handle {
   DevState* d_state = nullptr;
   DevState* h_state = nullptr;  // pinned, then the states of two sweeps (h_sweep)
   DevState* h_sweep = nullptr;
+  uint32_t* d_bar = nullptr;   // grid_barrier's word of this handle's launches
+  int* h_scan_err = nullptr;   // pinned: a scan's barrier wait gave up
   cudaEvent_t ev_sweep[2] = {nullptr, nullptr};  // sweep it & 1 of the logistic loop done
   unsigned char* ws = nullptr;
   size_t ws_bytes = 0;
@@ -351,6 +353,16 @@ int choose_persist_tile(pmcmc_handle* h, const void* fn, bool f64, int64_t Dp, i
     const int TT = persist_tile_for(fn, f64, Dp, T, dense, tuned, h->num_sms);
     if (TT > 0) return TT;
   }
+  // A block that one CTA evaluates in two rounds at most (8 warps, 32 lanes a warp over the
+  // lanes of a column) is solved by one: its sweeps need no grid barrier and no carry over
+  // CTAs (about 6 us of a 2-D block's 10.6 us a sweep; a round costs about 2).
+  int lanes = 32;
+  if (key.kind == kDiagGauss)
+    for (lanes = 1; lanes < 16 && 4 * lanes < key.D;) lanes *= 2;
+  if (T <= std::min<int64_t>(256, 2 * kWarps * (32 / lanes))) {
+    const size_t smem = persist_smem(f64, Dp, static_cast<int>(T), dense).total;
+    if (smem <= 200 * 1024 && max_active_blocks(fn, smem) > 0) return static_cast<int>(T);
+  }
   for (int per_sm = 8; per_sm >= 1; --per_sm) {
     const int64_t TT = (T + int64_t(per_sm) * h->num_sms - 1) / (int64_t(per_sm) * h->num_sms);
     if (TT > 256) break;
@@ -389,7 +401,7 @@ SolveLayout layout(int64_t D, int64_t Dp, int64_t T, int ntiles, size_t es, bool
                    int64_t N = 0, int64_t Tc = 0, size_t tc_bytes = 0,
                    const FullPlan* fp = nullptr, bool adjoint = false,
                    bool dual_out = false, size_t tie_bytes = 0, int tc_split = 1,
-                   size_t lgscan_bytes = 0) {
+                   size_t lgscan_bytes = 0, int64_t out_cols = 0) {
   SolveLayout L{};
   size_t off = 0;
   auto take = [&](size_t bytes) {
@@ -407,9 +419,10 @@ SolveLayout layout(int64_t D, int64_t Dp, int64_t T, int ntiles, size_t es, bool
   L.incl = take(es * (ntiles + 1) * Dp);  // + the persistent solve's S_0
   L.colmax = take(4 * static_cast<size_t>(T));
   L.part = take(8 * 8 * static_cast<size_t>(ntiles));
-  L.out_S = take(es * T * D);
-  L.out_lp = take(es * T);
-  L.out_acc = take(static_cast<size_t>(T));
+  out_cols = std::max(out_cols, T);  // columns of one output slot
+  L.out_S = take(es * out_cols * D);
+  L.out_lp = take(es * out_cols);
+  L.out_acc = take(static_cast<size_t>(out_cols));
   if (dual_out) {
     L.out2_S = take(es * T * D);
     L.out2_lp = take(es * T);
@@ -1277,8 +1290,10 @@ void fill_info(const DevState& s, pmcmc_info* info) {
 }
 
 int status_error(pmcmc_handle* h, int status) {
-  if (status == kStTimeout)
-    return fail(h, PMCMC_ERR_TIMEOUT, "device look-back wait exceeded its bound");
+  if (status == kStTimeout) {
+    cudaMemsetAsync(h->d_bar, 0, sizeof(uint32_t), h->stream);  // a barrier given up mid-phase
+    return fail(h, PMCMC_ERR_TIMEOUT, "a device wait (look-back or grid barrier) exceeded its bound");
+  }
   if (status == kStNonfinite)
     return fail(h, PMCMC_ERR_NONFINITE, "non-finite value in the DEER trajectory");
   return PMCMC_OK;
@@ -1358,21 +1373,26 @@ int solve_core(pmcmc_handle* h, const pmcmc_target* tg, const pmcmc_deer_params*
   }
   const int64_t Tc = logistic && !use_tc ? std::min<int64_t>(T, lg_chunk_cols(tg->N, T)) : 0;
   const int64_t nblocks = (N + T - 1) / T;
-  // Host outputs of several blocks: block b's copy-out overlaps block b + 1's solve.
-  const bool pipe = mem == PMCMC_MEM_HOST && nblocks > 1;
+  // Small host outputs of a persistent solve: all blocks in one launch, staged on the device
+  // and copied out once (4 MB take about 80 us; a launch and three copies a block cost
+  // more than the sweeps of a small block).
+  const bool stage = persist && mem == PMCMC_MEM_HOST && nblocks > 1 &&
+                     N * (es * (D + 1) + 1) <= size_t(4) << 20;
+  // Other host outputs of several blocks: block b's copy-out overlaps block b + 1's solve.
+  const bool pipe = mem == PMCMC_MEM_HOST && nblocks > 1 && !stage;
   // Several blocks: each block's state goes to a pinned ring, read after the last
   // block, so the blocks run back to back with no host round trip between them.
   const bool defer = nblocks > 1;
-  // Device outputs of several blocks on the persistent path: one launch solves
+  // Device or staged outputs of several blocks on the persistent path: one launch solves
   // them all, the kernel looping over the blocks (a grid barrier between blocks
   // instead of a kernel boundary).
-  const bool batch = persist && mem == PMCMC_MEM_DEVICE && nblocks > 1;
+  const bool batch = persist && (mem == PMCMC_MEM_DEVICE || stage) && nblocks > 1;
   const SolveLayout L = layout(D, Dp, T, ntiles, es, plain, logistic ? tg->N : 0, Tc,
                                use_tc ? lg_tc_ws_bytes(tg->lg, T) : 0, full ? &fplan : nullptr,
                                false, pipe,
                                logistic ? lg_tie_ws_bytes(tg->lg, T, tie_kmax(T)) : 0,
                                use_tc ? lg_tc_split(tg->lg, T) : 1,
-                               use_tc ? lg_scan_ws_bytes(Dp, T, h->num_sms) : 0);
+                               use_tc ? lg_scan_ws_bytes(Dp, T, h->num_sms) : 0, stage ? N : 0);
   rc = ensure_ws(h, L.total);
   if (rc) return rc;
   if (defer) {
@@ -1430,6 +1450,7 @@ int solve_core(pmcmc_handle* h, const pmcmc_target* tg, const pmcmc_deer_params*
   P.incl = ws + L.incl;
   P.colmax = reinterpret_cast<float*>(ws + L.colmax);
   P.part = reinterpret_cast<double*>(ws + L.part);
+  P.grid_bar = h->d_bar;
   P.xi = reinterpret_cast<float*>(ws + L.xi);
   P.logu = reinterpret_cast<double*>(ws + L.logu);
   if (logistic) {
@@ -1508,6 +1529,7 @@ int solve_core(pmcmc_handle* h, const pmcmc_target* tg, const pmcmc_deer_params*
                                init_grid);
     if (rc) return rc;
     if (mem == PMCMC_MEM_HOST) {
+      const int64_t ncopy = batch ? N : nkeep;
       cudaStream_t cs = h->stream;
       if (pipe) {
         CK(cudaEventRecord(h->ev_fin[slot], h->stream));
@@ -1515,12 +1537,12 @@ int solve_core(pmcmc_handle* h, const pmcmc_target* tg, const pmcmc_deer_params*
         cs = h->copy_stream;
       }
       CK(cudaMemcpyAsync(static_cast<unsigned char*>(S_out) + es * nsteps * D, ws + oS,
-                         es * nkeep * D, cudaMemcpyDeviceToHost, cs));
+                         es * ncopy * D, cudaMemcpyDeviceToHost, cs));
       if (logp_out)
         CK(cudaMemcpyAsync(static_cast<unsigned char*>(logp_out) + es * nsteps, ws + olp,
-                           es * nkeep, cudaMemcpyDeviceToHost, cs));
+                           es * ncopy, cudaMemcpyDeviceToHost, cs));
       if (accept_out)
-        CK(cudaMemcpyAsync(accept_out + nsteps, ws + oacc, nkeep, cudaMemcpyDeviceToHost, cs));
+        CK(cudaMemcpyAsync(accept_out + nsteps, ws + oacc, ncopy, cudaMemcpyDeviceToHost, cs));
       if (pipe) CK(cudaEventRecord(h->ev_copy[slot], cs));
     }
     nsteps += nkeep;
@@ -1784,6 +1806,8 @@ int pmcmc_create(int device, void* stream, pmcmc_handle** out) {
   if (cudaMalloc(&h->d_params, sizeof(DevParams)) != cudaSuccess ||
       cudaMalloc(&h->d_state, sizeof(DevState)) != cudaSuccess ||
       cudaMallocHost(&h->h_state, 3 * sizeof(DevState)) != cudaSuccess ||
+      cudaMallocHost(&h->h_scan_err, 64) != cudaSuccess ||
+      cudaMalloc(&h->d_bar, 256) != cudaSuccess ||
       cudaMallocHost(&h->h_red, 4 * sizeof(unsigned long long)) != cudaSuccess ||
       cudaMalloc(&h->d_full, sizeof(FullArgs)) != cudaSuccess ||
       cudaMalloc(&h->d_params_e, sizeof(DevParams)) != cudaSuccess) {
@@ -1792,6 +1816,8 @@ int pmcmc_create(int device, void* stream, pmcmc_handle** out) {
     return PMCMC_ERR_NOMEM;
   }
   h->h_sweep = h->h_state + 1;
+  *h->h_scan_err = 0;
+  cudaMemset(h->d_bar, 0, 256);
   cudaMemset(h->d_state, 0, sizeof(DevState));
   cudaMemset(h->d_params, 0, sizeof(DevParams));
   const char* ev = std::getenv("PMCMC_EAGER");
@@ -1847,6 +1873,8 @@ int pmcmc_destroy(pmcmc_handle* h) {
   cudaFree(h->d_params);
   cudaFree(h->d_state);
   if (h->h_state) cudaFreeHost(h->h_state);
+  if (h->h_scan_err) cudaFreeHost(h->h_scan_err);
+  cudaFree(h->d_bar);
   if (h->h_red) cudaFreeHost(h->h_red);
   for (cudaEvent_t e : h->ev)
     if (e) cudaEventDestroy(e);
@@ -2303,6 +2331,7 @@ int pmcmc_affine_scan_diag(pmcmc_handle* h, int32_t dtype, int64_t D, int64_t T,
       cudaGetLastError();
       return fail(h, PMCMC_ERR_NOMEM, "scan scratch allocation failed");
     }
+    CK(cudaMemsetAsync(h->scan_ws, 0, kScanBarBytes, h->stream));
     h->scan_ws_bytes = need;
   }
   unsigned char* base = h->scan_ws;
@@ -2318,10 +2347,15 @@ int pmcmc_affine_scan_diag(pmcmc_handle* h, int32_t dtype, int64_t D, int64_t T,
     CK(cudaMemcpyAsync(const_cast<void*>(dB), B, es * D * T, cudaMemcpyHostToDevice, h->stream));
     CK(cudaMemcpyAsync(const_cast<void*>(ds0), s0, es * D, cudaMemcpyHostToDevice, h->stream));
   }
-  CK(launch_affine_scan(h->stream, f64, D, T, dA, dB, ds0, dS, base));
+  *h->h_scan_err = 0;
+  CK(launch_affine_scan(h->stream, f64, D, T, dA, dB, ds0, dS, base, h->h_scan_err));
   if (mem == PMCMC_MEM_HOST)
     CK(cudaMemcpyAsync(S, dS, es * D * T, cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
+  if (*h->h_scan_err) {
+    cudaMemsetAsync(h->scan_ws, 0, kScanBarBytes, h->stream);
+    return fail(h, PMCMC_ERR_TIMEOUT, "scan barrier wait exceeded its bound");
+  }
   return PMCMC_OK;
 }
 
@@ -2593,10 +2627,14 @@ int pmcmc_deer_adjoint(pmcmc_handle* h, const pmcmc_target* tg, const pmcmc_deer
   void* init_args[] = {&h->d_params, &h->d_state};
   CK(cudaLaunchKernel(k.init, dim3(init_grid), dim3(256), init_args, 0, h->stream));
   double* out = reinterpret_cast<double*>(ws + L.aout);
+  *h->h_scan_err = 0;
   CK(full_adjoint(h->stream, h->d_params, h->d_full, F, D, Dp, T, tg->kind, h->num_sms,
-                  objective, reinterpret_cast<const float*>(ws + L.S0), out, ws + L.ascr));
+                  objective, reinterpret_cast<const float*>(ws + L.S0), out, ws + L.ascr,
+                  h->h_scan_err));
   CK(cudaMemcpyAsync(grad, out, sizeof(double) * (1 + D), cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
+  if (*h->h_scan_err)
+    return fail(h, PMCMC_ERR_TIMEOUT, "adjoint scan barrier wait exceeded its bound");
   return PMCMC_OK;
 }
 
@@ -2625,7 +2663,7 @@ int slice_copy_out(pmcmc_handle* h, void* dst, const void* src, size_t bytes, in
 int slice_scan(pmcmc_handle* h, const void* B, const void* s0, void* out) {
   SliceState& sl = h->slice;
   CK(launch_affine_scan(h->stream, sl.es == 8, sl.P.Dp, sl.P.T, h->ws + sl.A, B, s0, out,
-                        h->ws + sl.scr));
+                        h->ws + sl.scr, h->h_scan_err));
   return PMCMC_OK;
 }
 
@@ -2759,6 +2797,7 @@ int pmcmc_slice_local(pmcmc_handle* h, const void* xbar0, void* agg, int32_t mem
   void* eval_args[] = {&h->d_params, const_cast<void**>(&Sold), &it, &from_x0, &A, &B};
   CK(cudaLaunchKernel(k.eval, dim3(grid), dim3(kThreads), eval_args, smem, h->stream));
   // slice map: b = scan(A, B) from 0, prod A = scan(A, 0) from 1 (last columns)
+  *h->h_scan_err = 0;
   rc = slice_scan(h, ws + sl.B, ws + sl.Zb, ws + sl.Sloc);
   if (rc) return rc;
   unsigned char* out = static_cast<unsigned char*>(agg);
@@ -2769,6 +2808,8 @@ int pmcmc_slice_local(pmcmc_handle* h, const void* xbar0, void* agg, int32_t mem
   rc = slice_copy_out(h, out, ws + sl.Sloc + es * (W - 1) * Dp, es * D, mem);
   if (rc) return rc;
   CK(cudaStreamSynchronize(h->stream));
+  if (*h->h_scan_err)
+    return fail(h, PMCMC_ERR_TIMEOUT, "slice scan barrier wait exceeded its bound");
   return PMCMC_OK;
 }
 
@@ -2785,6 +2826,7 @@ int pmcmc_slice_finish(pmcmc_handle* h, const void* carry_in, void* last_out, do
   int rc = slice_copy_in(h, ws + sl.carry, carry_in, es * D, mem);
   if (rc) return rc;
   void* Snew = ws + sl.S[sl.cur ^ 1];
+  *h->h_scan_err = 0;
   rc = slice_scan(h, ws + sl.B, ws + sl.carry, Snew);
   if (rc) return rc;
   auto* r = reinterpret_cast<unsigned long long*>(ws + sl.red);
@@ -2797,6 +2839,8 @@ int pmcmc_slice_finish(pmcmc_handle* h, const void* carry_in, void* last_out, do
   unsigned long long hr[3] = {0, 0, 0};
   CK(cudaMemcpyAsync(hr, r, sizeof hr, cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
+  if (*h->h_scan_err)
+    return fail(h, PMCMC_ERR_TIMEOUT, "slice scan barrier wait exceeded its bound");
   std::memcpy(&red[0], &hr[0], 8);
   std::memcpy(&red[1], &hr[1], 8);
   sl.cur ^= 1;

@@ -94,6 +94,7 @@ struct Smem {
   Real* Bs;     // TT x Dp
   Real* carry;  // Dp
   const double* Pd;  // dense precision in double (smem copy or global)
+  int split;         // Pd holds rows 4j, 4j + 1 of every quad, then 4j + 2, 4j + 3
   const Real* Pf;    // dense precision in Real
   double* Vd;        // kWarps x Dp warp-private vectors
   Real* Vf;          // kWarps x Dp
@@ -130,7 +131,8 @@ __host__ __device__ inline SmemPlan plan_sweep_smem(int64_t Dp, int TT, bool den
 }
 
 template <typename Real>
-__device__ Smem<Real> carve(unsigned char* base, const DevParams& P, int TT, bool dense) {
+__device__ Smem<Real> carve(unsigned char* base, const DevParams& P, int TT, bool dense,
+                            bool split = false) {
   const SmemPlan pl = plan_sweep_smem<Real>(P.Dp, TT, dense);
   Smem<Real> s;
   s.Xs = reinterpret_cast<Real*>(base + pl.xs);
@@ -141,6 +143,7 @@ __device__ Smem<Real> carve(unsigned char* base, const DevParams& P, int TT, boo
   s.Vf = nullptr;
   s.Pd = P.prec_d;
   s.Pf = prec_of<Real>(P);
+  s.split = 0;
   if (dense) {
     s.Vd = reinterpret_cast<double*>(base + pl.vd);
     s.Vf = reinterpret_cast<Real*>(base + pl.vf);
@@ -153,10 +156,14 @@ __device__ Smem<Real> carve(unsigned char* base, const DevParams& P, int TT, boo
       double* pd = reinterpret_cast<double*>(base + pl.pd);
       Real* pf = reinterpret_cast<Real*>(base + pl.pf);
       const int n = static_cast<int>(P.Dp * P.Dp);
+      const int dp = static_cast<int>(P.Dp);
       for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        pd[i] = P.prec_d[i];
+        const int k = i / dp, r = i - k * dp;
+        const int to = split ? k * dp + (r & 2 ? dp / 2 : 0) + 2 * (r >> 2) + (r & 1) : i;
+        pd[to] = P.prec_d[i];
         pf[i] = prec_of<Real>(P)[i];
       }
+      s.split = split;
       s.Pd = pd;
       s.Pf = pf;
     }

@@ -65,6 +65,7 @@ struct DevParams {
   void* lg_acc;
   // error word of the tensor-core pass (a bounded wait gave up), or nullptr
   const int* tc_err;
+  uint32_t* grid_bar;  // grid_barrier's word of the handle
   double tau;  // prior precision
   // tape of the block, written once by the init kernel: xi (T x Dp, FP32,
   // padded rows zero) and log(u_t) in FP64
@@ -144,6 +145,32 @@ __device__ __forceinline__ unsigned long long dbits(double v) {
 }
 __device__ __forceinline__ double bitsd(unsigned long long b) {
   return __longlong_as_double(static_cast<long long>(b));
+}
+
+// Barrier over the n CTAs of a cooperative launch.  *bar holds a phase in its top bit and
+// zeros below it between launches (any n), so it is cleared once, when it is allocated.
+// All of warp 0 polls: where thread 0 polls alone (cooperative_groups), it does not rejoin its
+// warp by itself, and what follows runs twice in warp 0, 6 us for an apply phase of 2.6.
+// The wait is bounded (the CTAs are co-resident, so it ends far earlier); false: it gave up.
+constexpr int kBarrierSpins = 1 << 22;
+__device__ __forceinline__ bool grid_barrier(uint32_t* bar, unsigned n) {
+  __shared__ int s_gave_up;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    uint32_t old = 0;
+    if (threadIdx.x == 0) {
+      __threadfence();
+      old = atomicAdd(bar, blockIdx.x == 0 ? 0x80000000u - (n - 1) : 1u);
+    }
+    old = __shfl_sync(0xffffffffu, old, 0);
+    int spins = 0;
+    while (((ld_acquire(bar) ^ old) & 0x80000000u) == 0 && ++spins < kBarrierSpins) {
+    }
+    __syncwarp();
+    if (threadIdx.x == 0) s_gave_up = spins >= kBarrierSpins;
+  }
+  __syncthreads();
+  return s_gave_up == 0;
 }
 
 // Inclusive scan of the affine maps x -> A[c][d] x + B[c][d] along c (columns

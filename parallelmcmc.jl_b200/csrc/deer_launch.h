@@ -27,7 +27,7 @@ struct SweepKernels {
 // plan at TT columns plus the CTA's tape (TT + 1 columns of xi and log u).
 struct PersistPlan {
   SmemPlan sweep;
-  size_t xi, lu, x0, total;
+  size_t xi, lu, x0, tab, total;
 };
 PersistPlan persist_smem(bool f64, int64_t Dp, int TT, bool dense);
 const void* persist_kernel(bool f64, int tk, int jac, int64_t D);
@@ -63,8 +63,10 @@ cudaError_t launch_mala_chains(cudaStream_t s, bool f64, int tk, const DevParams
 cudaError_t launch_tape(cudaStream_t s, int64_t D, int64_t T, uint64_t seed, uint64_t block,
                         float* Xi, float* u);
 
-// Standalone diagonal affine scan (tape_scan.cu); `scratch` holds
-// scan_scratch_bytes and needs no clearing.
+// Standalone diagonal affine scan (tape_scan.cu); `scratch` holds scan_scratch_bytes, of
+// which the first kScanBarBytes (the grid barrier's word) are cleared once, when allocated;
+// *err (device-visible, 0 before) becomes 1 if a barrier's bounded wait gave up.
+constexpr size_t kScanBarBytes = 64;
 // A scan's split over T columns and D coordinates (scan_plan).
 constexpr int kScanWindow = 2048;  // most columns composed before a state is applied
 struct ScanPlan {
@@ -77,7 +79,7 @@ ScanPlan scan_plan(int64_t D, int64_t T, int max_ctas, int min_cols, int max_gro
 int scan_tile_cols(int64_t D, int64_t T);
 size_t scan_scratch_bytes(bool f64, int64_t D, int64_t T);
 cudaError_t launch_affine_scan(cudaStream_t s, bool f64, int64_t D, int64_t T, const void* A,
-                               const void* B, const void* s0, void* S, void* scratch);
+                               const void* B, const void* s0, void* S, void* scratch, int* err);
 
 // Plain path (tape_scan.cu): the reference's Hillis-Steele doubling scan
 // (DEERScan.jl:102-173) as one launch per level over buffers of T x Dp

@@ -12,10 +12,10 @@
 //    maps S_{t0} to S_{t0 + ncols}, the first column of the next CTA.
 //  - Column 0 depends on x0 alone: S_0 = f(x0) in every sweep; CTA 0 forms it
 //    once and it seeds the scan over the group aggregates.
-//  - Per sweep: evaluate + tile scan, grid barrier, the previous sweep's
+//  - Per sweep: evaluate and compose the group, grid barrier, the previous sweep's
 //    convergence test (DEER.jl:567-578) read by every CTA alike, per-coordinate
 //    scan of the group aggregates (state entering every CTA), grid barrier,
-//    apply with damping in shared memory, max|dS| / max|S| atomics.  Testing a
+//    replay with damping in shared memory, max|dS| / max|S| atomics.  Testing a
 //    sweep after the next sweep's first barrier saves a barrier a sweep; the
 //    evaluation after the last sweep is discarded.  Sweep 0 is tested at once
 //    after a third barrier, so a one-sweep solve evaluates once.
@@ -26,7 +26,6 @@
 // block has no sliding window and the target is a diagonal or dense Gaussian.
 // Its parameters come by value in the launch, so a solve is one launch and
 // the state readback.
-#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -34,8 +33,7 @@
 #include "deer_column.cuh"
 #include "deer_device.cuh"
 #include "deer_launch.h"
-
-namespace cg = cooperative_groups;
+#include "persist_column.cuh"
 
 namespace pmcmc {
 
@@ -53,6 +51,9 @@ __host__ __device__ inline PersistPlan plan_persist_smem(int64_t Dp, int TT, boo
   off = al(off + sizeof(double) * (TT + 1));
   p.x0 = off;
   off = al(off + sizeof(Real) * Dp);
+  p.tab = off;
+  if (dense) off = al(off + sizeof(double) * Dp);
+  else if (Dp <= 256) off = al(off + diag_tab_bytes<Real>(Dp));
   p.total = off;
   return p;
 }
@@ -61,34 +62,75 @@ PersistPlan persist_smem(bool f64, int64_t Dp, int TT, bool dense) {
   return f64 ? plan_persist_smem<double>(Dp, TT, dense) : plan_persist_smem<float>(Dp, TT, dense);
 }
 
-namespace {
-
-template <int QPL, int LPC>
-__device__ __forceinline__ void xi_from_smem(const float* col, int D, float (&n)[QPL][4]) {
-  const int lane = threadIdx.x & (LPC - 1);
+// State entering every CTA (column t0 of CTA j), from the group aggregates: one warp a
+// coordinate.  Each lane composes kCarryGroup groups, the lanes' maps are applied to the state in
+// turn, and each lane replays its groups (the same association in every run).  One
+// warp instead of a CTA needs no CTA barrier, and its first maps are loaded ahead of the
+// convergence test: 3.3 -> 2.7 us a sweep with the test at 293 CTAs.
+constexpr int kCarryGroup = 10;
+template <typename Real>
+struct CarryMaps {
+  Real a[kCarryGroup], b[kCarryGroup];
+  // this lane's groups j0 .. j0 + grp - 1 (identity past the last)
+  __device__ __forceinline__ void load(int n, int grp, int j0, int d, int Dp, const Real* agg_a,
+                                       const Real* agg_b) {
 #pragma unroll
-  for (int q = 0; q < QPL; ++q) {
-    const int j = lane + LPC * q;
-    if (4 * j < D) {
-      load4(col + 4 * j, n[q]);
-    } else {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) n[q][e] = 0.f;
+    for (int k = 0; k < kCarryGroup; ++k) {
+      const bool in = k < grp && j0 + k < n;
+      a[k] = in ? __ldcg(agg_a + static_cast<size_t>(j0 + k) * Dp + d) : Real(1);
+      b[k] = in ? __ldcg(agg_b + static_cast<size_t>(j0 + k) * Dp + d) : Real(0);
     }
+  }
+};
+__device__ __forceinline__ int carry_group(int n) { return min(kCarryGroup, (n + 31) / 32); }
+// m holds the maps of the first 32 grp groups, loaded ahead.
+template <typename Real>
+__device__ __forceinline__ void carry_warp(int n, int d, int Dp, const Real* agg_a,
+                                           const Real* agg_b, Real s, Real* incl, Real* wa,
+                                           Real* wb, CarryMaps<Real>& m) {
+  const int lane = threadIdx.x & 31;
+  const int grp = carry_group(n);
+  for (int base = 0; base < n; base += 32 * grp) {
+    const int j0 = base + lane * grp;
+    if (base > 0) m.load(n, grp, j0, d, Dp, agg_a, agg_b);
+    Real a = 1, b = 0;
+#pragma unroll
+    for (int k = 0; k < kCarryGroup; ++k)
+      if (k < grp && j0 + k < n) {
+        b = m.a[k] * b + m.b[k];
+        a = m.a[k] * a;
+      }
+    __syncwarp();
+    wa[lane] = a;
+    wb[lane] = b;
+    __syncwarp();
+    Real mine = s;  // state entering this lane's groups
+#pragma unroll 8
+    for (int l = 0; l < 32; ++l) {
+      const Real al = wa[l], bl = wb[l];
+      s = al * s + bl;
+      if (l < lane) mine = s;
+    }
+#pragma unroll
+    for (int k = 0; k < kCarryGroup; ++k)
+      if (k < grp && j0 + k < n) {
+        incl[static_cast<size_t>(j0 + k) * Dp + d] = mine;
+        mine = m.a[k] * mine + m.b[k];
+      }
   }
 }
 
-}  // namespace
+// Two CTAs per SM (at most 128 registers a thread) where that costs few spills:
+// FP32 state with up to two quads a lane, FP64 with one on a diagonal target.
+template <typename Real, int TK, int QPL>
+constexpr int kPersistMinBlocks =
+    sizeof(Real) * QPL <= 8 && !(TK == kDenseGauss && sizeof(Real) == 8) ? 2 : 1;
 
-// Two CTAs per SM (at most 128 registers a thread) where that costs no spills:
-// FP32 state with up to two quads a lane, FP64 with one.
-template <typename Real, int QPL>
-constexpr int kPersistMinBlocks = sizeof(Real) * QPL <= 8 ? 2 : 1;
-
-// Columns are evaluated by LPC lanes each (32 / LPC columns per warp); QPL
-// quads per lane cover Dp / 4 <= LPC * QPL.
+// Columns of a diagonal target are evaluated by LPC lanes each (32 / LPC columns per
+// warp), those of a dense one by a warp, LPC lanes for its quads and the rest for shares of
+// the sums over the coordinates; QPL quads per lane cover Dp / 4 <= LPC * QPL.
 template <typename Real, int TK, int JAC, int QPL, int LPC>
-__global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, QPL>)
+__global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL>)
     deer_persist_kernel(const DevParams Pv, DevState* __restrict__ st) {
   __shared__ DevParams P;
   __shared__ Real s_sa[kThreads], s_sb[kThreads];
@@ -97,14 +139,22 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, QPL>)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   if (threadIdx.x == 0) P = Pv;  // parameters by value: no upload before the launch
   __syncthreads();
-  cg::grid_group grid = cg::this_grid();
+  // one CTA (small blocks): its own barrier
+  bool gave_up = false;
+  auto all_sync = [&]() {
+    if (gridDim.x == 1) __syncthreads();
+    else if (!grid_barrier(P.grid_bar, gridDim.x)) gave_up = true;
+  };
   // this sweep's maxima max|dS|, max|S| and the non-finite flag, as ordered
   // bits of non-negative doubles, in two slots by sweep parity (P.part[0..5])
   unsigned long long* red = reinterpret_cast<unsigned long long*>(P.part);
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int CPW = 32 / LPC;                  // columns per warp
-  const int lq = lane & (LPC - 1), half = lane / LPC;  // quad lane, column slot
+  constexpr bool kDense = TK == kDenseGauss;
+  constexpr int CPW = kDense ? 1 : 32 / LPC;          // columns per warp
+  const int lq = lane & (LPC - 1);                    // quad lane
+  const int half = kDense ? 0 : lane / LPC;           // column slot
+  const bool stores = !kDense || lane < LPC;          // of several lanes with the same quad
   const int cta = static_cast<int>(blockIdx.x), nctas = static_cast<int>(gridDim.x);
   const int TT = P.tile_cols;
   const int D = static_cast<int>(P.D), Dp = static_cast<int>(P.Dp);
@@ -113,8 +163,7 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, QPL>)
   const int ncols = static_cast<int>(imin64(TT, T - t0));  // >= 1: one CTA per tile
   const bool has_next = t0 + ncols < T;
   const int ng = has_next ? ncols : ncols - 1;  // columns of the scan group
-  constexpr bool kDense = TK == kDenseGauss;
-  Smem<Real> sm = carve<Real>(smem_raw, P, TT, kDense);
+  Smem<Real> sm = carve<Real>(smem_raw, P, TT, kDense, true);
   const PersistPlan pp = plan_persist_smem<Real>(Dp, TT, kDense);
   float* xis = reinterpret_cast<float*>(smem_raw + pp.xi);
   double* lus = reinterpret_cast<double*>(smem_raw + pp.lu);
@@ -125,6 +174,11 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, QPL>)
   Real* Sb = static_cast<Real*>(P.S[0]);                   // last column of every CTA
 
   Real* x0s = reinterpret_cast<Real*>(smem_raw + pp.x0);
+  DiagTab<Real> tab{};
+  [[maybe_unused]] double* mud = reinterpret_cast<double*>(smem_raw + pp.tab);
+  if constexpr (kDense)
+    for (int d = tid; d < Dp; d += kThreads) mud[d] = d < D ? P.mean_d[d] : 0.0;
+  if constexpr (!kDense && QPL <= 2) tab = fill_diag_tab<Real>(smem_raw + pp.tab, P);
   const int nblk = P.nblk > 1 ? static_cast<int>(P.nblk) : 1;
   for (int bi = 0; bi < nblk; ++bi) {  // blocks of one call, back to back
     const int64_t ncols_out = bi + 1 < nblk ? T : P.ncols_out;
@@ -164,13 +218,24 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, QPL>)
         store4(xis + c * Dp + 4 * q, n);
       }
     }
-    // log u of the columns t0 .. t0 + ng (the CTA's own and its scan group's), in
-    // FP64, one column a thread: the evaluation reads them from shared memory
-    for (int c = tid; c <= ng; c += kThreads)
-      lus[c] = log(static_cast<double>(tape_u(key, static_cast<uint32_t>(t0 + c + P.t_off))));
     for (int d = tid; d < Dp; d += kThreads)
       x0s[d] = d == tid ? x0r : d < D ? x0src[d] : Real(0);
     __syncthreads();
+    // log u - 0.5 |xi|^2 of the columns t0 .. t0 + ng (the CTA's own and its scan
+    // group's), in FP64, one column a thread: what the evaluation compares its part of
+    // log alpha with
+    for (int c = tid; c <= ng; c += kThreads) {
+      double h = 0.0;
+      const float* n = xis + c * Dp;
+#pragma unroll 4
+      for (int d = 0; d < Dp; d += 4) {
+        float v[4];
+        load4(n + d, v);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) h = fma(static_cast<double>(v[e]), static_cast<double>(v[e]), h);
+      }
+      lus[c] = log(static_cast<double>(tape_u(key, static_cast<uint32_t>(t0 + c + P.t_off)))) - 0.5 * h;
+    }
     for (int i = tid; i < ncols * (Dp / 4); i += kThreads) {
       const int nq = Dp / 4, c = i / nq, k = 4 * (i - c * nq);
       Real v[4];
@@ -178,17 +243,22 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, QPL>)
       store4(sm.Xs + c * Dp + k, v);
     }
 
+    __syncthreads();
+
     // ---- S_0 = f(x0): the same in every sweep ----
     if (cta == 0 && warp == 0) {  // every column slot of warp 0 forms it; slot 0 stores
-      float xic[QPL][4];
-      xi_from_smem<QPL, LPC>(xis, D, xic);
       Col<Real, QPL> col;
-      column_forward<Real, TK, QPL, LPC>(P, sm, key, x0s, 0, col, xic);
-      const bool acc = lus[0] < col.la;
+      if constexpr (kDense) {
+        Real z[QPL][4], w[QPL][4], hv[QPL][4];
+        persist_forward_dense<Real, JAC, QPL, LPC, false>(P, sm, mud, key, x0s, xis, 0, 0, col, z, w, hv);
+      } else {
+        persist_forward_diag<Real, QPL, LPC, JAC == kJacDiag>(P, tab, x0s, xis, col);
+      }
+      const bool acc = lus[0] < seg_sum<LPC>(col.la);
 #pragma unroll
       for (int q = 0; q < QPL; ++q) {
         const int j = lq + LPC * q;
-        if (half == 0 && 4 * j < D) {
+        if (lane < LPC && 4 * j < D) {
           Real f[4];
 #pragma unroll
           for (int e = 0; e < 4; ++e)
@@ -199,7 +269,16 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, QPL>)
     }
 
     const Real dmp = static_cast<Real>(P.damping), omd = static_cast<Real>(1.0 - P.damping);
-    const bool undamped = P.damping == 1.0;
+    const Real big = sizeof(Real) == 4 ? Real(3.402823466e+38f) : Real(1.7976931348623157e308);
+    // runs of the scan: nsub runs of Ls columns a coordinate (above 256 coordinates: one run,
+    // several coordinates a thread)
+    constexpr bool kRuns = 4 * QPL * LPC <= kThreads;
+    int nsub = 1, Ls = ng;
+    if constexpr (kRuns) {
+      nsub = max(1, min(min(kThreads / Dp, 8), ng));
+      Ls = (ng + nsub - 1) / nsub;
+      nsub = Ls > 0 ? max(1, (ng + Ls - 1) / Ls) : 1;
+    }
     int iter = 0, converged = 0, status = 0;
     Real sprev = 0;
     double metric = 0.0;
@@ -213,7 +292,8 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, QPL>)
       const bool nonfinite = __ldcg(sl + 2) != 0ull;
       metric = dmax / (P.tol_abs + P.tol_rel * smax);
       converged = metric <= 1.0;
-      status = nonfinite ? static_cast<int>(kStNonfinite) : 0;
+      status = gave_up ? static_cast<int>(kStTimeout)
+               : nonfinite ? static_cast<int>(kStNonfinite) : 0;
       const bool stop = converged || iter >= P.maxiter || status != 0;
       if (stop && cta > 0 && tid < Dp) sprev = __ldcg(Sb + (t0 - 1) * Dp + tid);
       return stop;
@@ -232,45 +312,116 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, QPL>)
         const bool valid = cb + half < ng;
         const int c = valid ? cb + half : cb;
         const int t = static_cast<int>(t0 + c + 1);
-        float xic[QPL][4];
-        xi_from_smem<QPL, LPC>(xis + (c + 1) * Dp, D, xic);
         const double logu = lus[c + 1];
+        const float* xic = xis + (c + 1) * Dp;
+        const Real* xcol = sm.Xs + c * Dp;
         Col<Real, QPL> col;
-        column_forward<Real, TK, QPL, LPC>(P, sm, key, sm.Xs + c * Dp, t, col, xic);
-        const bool acc = logu < col.la;
-        const Real gp = sigmoid_slope<Real>(col.la - logu);
         Real A[QPL][4];
-        column_jacobian<Real, TK, JAC, QPL, LPC>(P, sm, key, t + P.t_off, iter, acc, gp, col, A);
+        bool acc;
+        if constexpr (kDense) {
+          Real z[QPL][4], w[QPL][4], hv[QPL][4];
+          persist_forward_dense<Real, JAC, QPL, LPC, true>(P, sm, mud, key, xcol, xic,
+                                                           t + P.t_off, iter, col, z, w, hv);
+          col.la = seg_sum<LPC>(col.la);
+          acc = logu < col.la;
+          persist_jacobian_dense<Real, JAC, QPL, LPC>(P, sm, key, t + P.t_off, iter, acc,
+                                                      sigmoid_slope<Real>(col.la - logu), col, z,
+                                                      w, hv, A);
+        } else {
+          persist_forward_diag<Real, QPL, LPC, JAC == kJacDiag>(P, tab, xcol, xic, col);
+          col.la = seg_sum<LPC>(col.la);
+          acc = logu < col.la;
+          const Real gp = sigmoid_slope<Real>(col.la - logu);
+          if constexpr (JAC == kJacDiag) {
+#pragma unroll
+            for (int q = 0; q < QPL; ++q)
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+                A[q][e] = fma(gp, col.gx[q][e], acc ? Real(1) - col.gy[q][e] : Real(1));
+          } else {
+            column_jacobian<Real, TK, JAC, QPL, LPC>(P, sm, key, t + P.t_off, iter, acc, gp, col,
+                                                     A);
+          }
+        }
 #pragma unroll
         for (int q = 0; q < QPL; ++q) {
           const int j = lq + LPC * q;
-          if (valid && 4 * j < D) {
+          if (valid && stores && 4 * j < D) {
             Real a4[4], b4[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
+              // (past D the state is zero, and stays zero under any A)
               const Real f = acc ? col.y[q][e] : col.x[q][e];
-              a4[e] = (4 * j + e < D) ? A[q][e] : Real(0);
-              b4[e] = (4 * j + e < D) ? f - A[q][e] * col.x[q][e] : Real(0);
+              a4[e] = A[q][e];
+              b4[e] = f - A[q][e] * col.x[q][e];
             }
             store4(sm.As + c * Dp + 4 * j, a4);
             store4(sm.Bs + c * Dp + 4 * j, b4);
           }
         }
       }
+      // ---- the group's map of every coordinate: runs of consecutive columns, one a
+      // thread, composed and joined (the maps stay as they are for the replay below) ----
+      Real ea = 1, eb = 0;  // this thread's earlier runs
       if (sweep) {
-        __syncthreads();
-        tile_scan_inplace<Real>(sm.As, sm.Bs, ng, D, Dp);
-        __syncthreads();
-        for (int d = tid; d < D; d += kThreads) {
-          agg_a[static_cast<size_t>(cta) * Dp + d] = ng > 0 ? sm.As[(ng - 1) * Dp + d] : Real(1);
-          agg_b[static_cast<size_t>(cta) * Dp + d] = ng > 0 ? sm.Bs[(ng - 1) * Dp + d] : Real(0);
+        __syncthreads();  // evaluated
+        if constexpr (kRuns) {
+          const int d = tid % Dp, sub = tid / Dp;
+          // (the same trip count in every lane: runs of two lengths would diverge)
+          const int g0 = sub * Ls, n = sub < nsub ? min(Ls, ng - g0) : 0;
+          const Real *pa = sm.As + g0 * Dp + d, *pb = sm.Bs + g0 * Dp + d;
+          Real a = 1, b = 0;
+          for (int i = 0; i < Ls; i += 4, pa += 4 * Dp, pb += 4 * Dp) {
+            Real va[4], vb[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              va[k] = i + k < n ? pa[k * Dp] : Real(1);
+              vb[k] = i + k < n ? pb[k * Dp] : Real(0);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              b = va[k] * b + vb[k];
+              a = va[k] * a;
+            }
+          }
+          s_sa[tid] = a;
+          s_sb[tid] = b;
+          __syncthreads();
+          for (int j = 0; j < sub; ++j) {
+            const Real aj = s_sa[j * Dp + d], bj = s_sb[j * Dp + d];
+            eb = aj * eb + bj;
+            ea = aj * ea;
+          }
+          if (sub == nsub - 1 && nctas > 1) {
+            agg_a[static_cast<size_t>(cta) * Dp + d] = a * ea;
+            agg_b[static_cast<size_t>(cta) * Dp + d] = a * eb + b;
+          }
+        } else {  // more coordinates than threads: one run each
+          for (int d = tid; d < Dp; d += kThreads) {
+            Real a = 1, b = 0;
+            for (int g = 0; g < ng; ++g) {
+              const Real ag = sm.As[g * Dp + d], bg = sm.Bs[g * Dp + d];
+              b = ag * b + bg;
+              a = ag * a;
+            }
+            agg_a[static_cast<size_t>(cta) * Dp + d] = a;
+            agg_b[static_cast<size_t>(cta) * Dp + d] = b;
+          }
         }
       }
-      grid.sync();
+      all_sync();
 
       // ---- convergence test of the previous sweep (DEER.jl:567-578), the same in
       // every CTA: its maxima are complete, every CTA having applied it.  Sweep 0
       // was tested at once, after a barrier of its own (below) ----
+      // (the maps of this warp's first coordinate are fetched beside the maxima)
+      const int dw = warp * nctas + cta;
+      Real s0w = 0;
+      CarryMaps<Real> maps;
+      if (nctas > 1 && dw < D) {
+        maps.load(nctas, carry_group(nctas), lane * carry_group(nctas), dw, Dp, agg_a, agg_b);
+        s0w = __ldcg(carry0 + dw);
+      }
       if (iter >= 2 && stop_test(iter - 1)) break;
       // this sweep's slot was last read in the test of sweep iter - 2, which
       // every CTA finished before the previous sweep's second barrier: clear it
@@ -278,49 +429,66 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, QPL>)
       if (cta == 0 && tid == 0)
         for (int i = 0; i < 3; ++i) red[3 * (iter & 1) + i] = 0ull;
 
-      // ---- state entering every CTA: scan of the group aggregates per coordinate ----
-      for (int d = cta; d < D; d += nctas)
-        carry_scan_tiles<Real>(nctas, d, Dp, agg_a, agg_b, __ldcg(carry0 + d), incl, s_sa, s_sb);
-      grid.sync();
-
-      // ---- apply: Newton state of every column, damping, maxima ----
-      Real my_dmax = 0, my_smax = 0;  // maxima are exact in the state's precision
-      bool bad = false;
-      Real cr[QPL][4];
-#pragma unroll
-      for (int q = 0; q < QPL; ++q) {
-        const int j = lane + 32 * q;
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          cr[q][e] = 4 * j + e < D ? __ldcg(incl + static_cast<size_t>(cta) * Dp + 4 * j + e)
-                                   : Real(0);
-      }
-      for (int c = warp; c < ncols; c += kWarps) {
-#pragma unroll
-        for (int q = 0; q < QPL; ++q) {
-          const int j = lane + 32 * q;
-          if (4 * j < D) {
-            Real a4[4] = {1, 1, 1, 1}, b4[4] = {0, 0, 0, 0}, o4[4], n4[4];
-            if (c > 0) {
-              load4(sm.As + (c - 1) * Dp + 4 * j, a4);
-              load4(sm.Bs + (c - 1) * Dp + 4 * j, b4);
-            }
-            load4(sm.Xs + c * Dp + 4 * j, o4);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const Real s = a4[e] * cr[q][e] + b4[e];
-              n4[e] = undamped ? s : omd * o4[e] + dmp * s;
-              if (4 * j + e < D) {
-                my_dmax = max(my_dmax, fabs(n4[e] - o4[e]));
-                my_smax = max(my_smax, fabs(n4[e]));
-                bad |= !isfinite(n4[e]);
-              } else {
-                n4[e] = Real(0);
-              }
-            }
-            store4(sm.Xs + c * Dp + 4 * j, n4);
-            if (c == ncols - 1 && has_next) store4(Sb + (t0 + c) * Dp + 4 * j, n4);
+      // ---- state entering every CTA: the group aggregates per coordinate ----
+      if (nctas > 1) {
+        for (int d = dw; d < D; d += kWarps * nctas) {
+          if (d != dw) {
+            maps.load(nctas, carry_group(nctas), lane * carry_group(nctas), d, Dp, agg_a, agg_b);
+            s0w = __ldcg(carry0 + d);
           }
+          carry_warp<Real>(nctas, d, Dp, agg_a, agg_b, s0w, incl, s_sa + 32 * warp,
+                           s_sb + 32 * warp, maps);
+        }
+        all_sync();
+      }
+
+      // ---- apply: every thread replays its run from the state entering it; damping and
+      // maxima (exact in the state's precision) ----
+      Real my_dmax = 0, my_smax = 0;
+      bool bad = false;
+      const Real* in = nctas > 1 ? incl + static_cast<size_t>(cta) * Dp : carry0;
+      // column c's value v from its Newton state s and its old value o
+      auto damp = [&](Real s, Real o) {
+        const Real v = omd * o + dmp * s;
+        my_dmax = max(my_dmax, fabs(v - o));
+        my_smax = max(my_smax, fabs(v));
+        bad |= !(fabs(v) <= big);
+        return v;
+      };
+      // n columns of coordinate d after column c0, from its state s; four columns' loads go
+      // ahead of their stores
+      auto replay = [&](int d, int c0, int n, Real s) {
+        const Real *pa = sm.As + c0 * Dp + d, *pb = sm.Bs + c0 * Dp + d;
+        Real* px = sm.Xs + (c0 + 1) * Dp + d;
+        int i = 0;
+        for (; i + 4 <= n; i += 4, pa += 4 * Dp, pb += 4 * Dp, px += 4 * Dp) {
+          Real va[4], vb[4], vo[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) va[k] = pa[k * Dp], vb[k] = pb[k * Dp], vo[k] = px[k * Dp];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            s = va[k] * s + vb[k];
+            px[k * Dp] = damp(s, vo[k]);
+          }
+        }
+        for (; i < n; ++i, pa += Dp, pb += Dp, px += Dp) {
+          s = *pa * s + *pb;
+          *px = damp(s, *px);
+        }
+      };
+      if constexpr (kRuns) {
+        const int d = tid % Dp, sub = tid / Dp;
+        const bool on = sub < nsub && d < D;
+        const int c0 = sub * Ls, n = on ? min(Ls, ncols - 1 - c0) : 0;
+        const Real cr = on ? __ldcg(in + d) : Real(0);
+        if (on && sub == 0) sm.Xs[d] = damp(cr, sm.Xs[d]);
+        __syncwarp();
+        replay(d, c0, n, ea * cr + eb);
+      } else {
+        for (int d = tid; d < D; d += kThreads) {
+          const Real cr = __ldcg(in + d);
+          sm.Xs[d] = damp(cr, sm.Xs[d]);
+          replay(d, 0, ncols - 1, cr);
         }
       }
       // this CTA's maxima into the sweep's slot (max is exact in any order; the
@@ -334,6 +502,9 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, QPL>)
         s_red[2][warp] = bad ? 1.0 : 0.0;
       }
       __syncthreads();
+      if (has_next)  // the next CTA's verification starts from this column
+        for (int d = tid; d < Dp; d += kThreads)
+          Sb[(t0 + ncols - 1) * Dp + d] = sm.Xs[(ncols - 1) * Dp + d];
       unsigned long long* slot = red + 3 * (iter & 1);
       if (tid == 0) {
         double a = 0, b = 0, c = 0;
@@ -343,11 +514,12 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, QPL>)
         atomicMax(slot + 1, dbits(b));
         if (c != 0.0) atomicMax(slot + 2, 1ull);
       }
+      __syncwarp();  // warp 0 evaluates together again
       ++iter;
       // the first sweep is tested at once: a block that converges in one sweep
       // (no accepted move) then evaluates nothing more
       if (iter == 1) {
-        grid.sync();
+        all_sync();
         if (stop_test(0)) break;
       }
     }
@@ -385,11 +557,15 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, QPL>)
       const int64_t t = t0 + c;
       const Real* xcol = c == 0 ? sm.carry : sm.Xs + (c - 1) * Dp;
       const Real* scol = sm.Xs + c * Dp;
-      float xic[QPL][4];
-      xi_from_smem<QPL, LPC>(xis + c * Dp, D, xic);
       Col<Real, QPL> col;
       // log alpha reduced below with the log density and the defect (one pass)
-      column_forward<Real, TK, QPL, LPC, false>(P, sm, key, xcol, static_cast<int>(t), col, xic);
+      if constexpr (kDense) {
+        Real z[QPL][4], w[QPL][4], hv[QPL][4];
+        persist_forward_dense<Real, JAC, QPL, LPC, false>(P, sm, mud, key, xcol, xis + c * Dp,
+                                                          static_cast<int>(t), 0, col, z, w, hv);
+      } else {
+        persist_forward_diag<Real, QPL, LPC, JAC == kJacDiag>(P, tab, xcol, xis + c * Dp, col);
+      }
       const double logu = lus[c];
       const bool out = valid && t < ncols_out;
       // the recursion defect max|S_t - f_t| for both outcomes, selected after the
@@ -408,25 +584,24 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, QPL>)
             if (4 * j + e >= D) continue;
             dx = max(dx, fabs(s4[e] - col.x[q][e]));
             dy = max(dy, fabs(s4[e] - col.y[q][e]));
-            const double sd = static_cast<double>(s4[e]) - P.mean_d[4 * j + e];
+            const double sd = static_cast<double>(s4[e]) - (kDense ? mud[4 * j + e] : P.mean_d[4 * j + e]);
             if constexpr (TK == kDiagGauss) lp += -0.5 * P.prec_d[4 * j + e] * sd * sd;
-            else vd[4 * j + e] = sd;
-            if (out && t == ncols_out - 1) static_cast<Real*>(P.x_next)[4 * j + e] = s4[e];
+            else if (stores) vd[4 * j + e] = sd;
+            if (out && stores && t == ncols_out - 1) static_cast<Real*>(P.x_next)[4 * j + e] = s4[e];
           }
         }
       }
       if constexpr (kDense) {
         __syncwarp();
+        double o[QPL][4];
+        Real none[QPL][4];
+        dense_products<Real, QPL, LPC, true, false>(sm, D, Dp, o, none);
 #pragma unroll
         for (int q = 0; q < QPL; ++q) {
           const int j = lq + LPC * q;
-          if (4 * j < D) {
-            double o[4];
-            matvec4<double, double, double>(sm.Pd, vd, D, Dp, j, o);
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-              if (4 * j + e < D) lp += -0.5 * vd[4 * j + e] * o[e];
-          }
+          for (int e = 0; e < 4; ++e)
+            if (4 * j + e < D) lp += -0.5 * vd[4 * j + e] * o[q][e];
         }
         __syncwarp();
       }
@@ -438,7 +613,7 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, QPL>)
         dy = max(dy, __shfl_xor_sync(0xffffffffu, dy, o));
       }
       const bool acc = logu < col.la;
-      if (valid && lq == 0) {
+      if (valid && stores && lq == 0) {
         if (out) {
           if (logp_out) logp_out[t] = static_cast<Real>(lp);
           if (accept_out) accept_out[t] = acc ? 1 : 0;
@@ -501,23 +676,34 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, QPL>)
     }
     // the next block starts from this block's last column (x_next) once every
     // CTA has finished this one
-    if (bi + 1 < nblk) grid.sync();
+    if (bi + 1 < nblk) all_sync();
   }  // blocks
 }
 
 namespace {
 
+template <typename Real, int TK, int JAC, int QPL, int LPC>
+const void* persist_fn() {
+  return reinterpret_cast<const void*>(&deer_persist_kernel<Real, TK, JAC, QPL, LPC>);
+}
+
+// Lanes a column: as many as it has quads, rounded up to a power of two, so that a small
+// state fills the warp with columns (diagonal) or shares of its products (dense).
 template <typename Real, int TK, int JAC>
 const void* pick_persist(int64_t D) {
-  const void* k = nullptr;
-  if constexpr (TK == kDiagGauss) {  // two columns per warp while D <= 128
-    if (D <= 64) return reinterpret_cast<const void*>(&deer_persist_kernel<Real, TK, JAC, 1, 16>);
-    if (D <= 128) return reinterpret_cast<const void*>(&deer_persist_kernel<Real, TK, JAC, 2, 16>);
+  if constexpr (TK == kDiagGauss) {
+    if (D <= 4) return persist_fn<Real, TK, JAC, 1, 1>();
+    if (D <= 8) return persist_fn<Real, TK, JAC, 1, 2>();
+    if (D <= 16) return persist_fn<Real, TK, JAC, 1, 4>();
+    if (D <= 32) return persist_fn<Real, TK, JAC, 1, 8>();
+    if (D <= 64) return persist_fn<Real, TK, JAC, 1, 16>();
+    if (D <= 128) return persist_fn<Real, TK, JAC, 2, 16>();
+  } else {
+    if (D <= 32) return persist_fn<Real, TK, JAC, 1, 8>();
+    if (D <= 64) return persist_fn<Real, TK, JAC, 1, 16>();
+    if (D <= 128) return persist_fn<Real, TK, JAC, 1, 32>();
   }
-  if (D <= 128) k = reinterpret_cast<const void*>(&deer_persist_kernel<Real, TK, JAC, 1, 32>);
-  else if (D <= 256) k = reinterpret_cast<const void*>(&deer_persist_kernel<Real, TK, JAC, 2, 32>);
-  else k = reinterpret_cast<const void*>(&deer_persist_kernel<Real, TK, JAC, 4, 32>);
-  return k;
+  return D <= 256 ? persist_fn<Real, TK, JAC, 2, 32>() : persist_fn<Real, TK, JAC, 4, 32>();
 }
 
 template <typename Real>

@@ -957,7 +957,7 @@ size_t full_adjoint_scratch_bytes(int64_t Dp, int64_t T) {
 
 cudaError_t full_adjoint(cudaStream_t s, const DevParams* Pg, const FullArgs* Fg,
                          const FullArgs& Fh, int64_t D, int64_t Dp, int64_t T, int tkind,
-                         int num_sms, int objective, const float* S, double* out, void* scratch) {
+                         int num_sms, int objective, const float* S, double* out, void* scratch, int* err) {
   const bool dense = tkind == kDenseGauss;
   cudaError_t e = cudaMemsetAsync(out, 0, sizeof(double) * (1 + D), s);
   if (e == cudaSuccess) e = cudaMemsetAsync(Fh.direct, 0, sizeof(double), s);
@@ -981,9 +981,10 @@ cudaError_t full_adjoint(cudaStream_t s, const DevParams* Pg, const FullArgs* Fg
   // reverse scan in reversed time: Lrev_tau = Arev_tau * Lrev_{tau-1} + Brev_tau, Lrev_{-1} = 0
   unsigned char* w = static_cast<unsigned char*>(scratch);
   float* zero = reinterpret_cast<float*>(w);
-  e = cudaMemsetAsync(zero, 0, sizeof(float) * Dp, s);
+  // the zero vector, and the barrier's word at the start of the scan's scratch
+  e = cudaMemsetAsync(zero, 0, al256(4 * Dp) + kScanBarBytes, s);
   if (e != cudaSuccess) return e;
-  e = launch_affine_scan(s, false, Dp, T, Arev, Brev, zero, Fh.lam_adj, w + al256(4 * Dp));
+  e = launch_affine_scan(s, false, Dp, T, Arev, Brev, zero, Fh.lam_adj, w + al256(4 * Dp), err);
   if (e != cudaSuccess) return e;
   e = cudaMemcpyAsync(out, Fh.direct, sizeof(double), cudaMemcpyDeviceToDevice, s);
   if (e != cudaSuccess) return e;

@@ -80,7 +80,7 @@ cudaError_t full_sweep(cudaStream_t s, const FullPlan& fp, const DevParams* Pg, 
 cudaError_t full_adjoint(cudaStream_t s, const DevParams* Pg, const FullArgs* Fg,
                          const FullArgs& Fh, int64_t D, int64_t Dp, int64_t T, int tkind,
                          int num_sms, int objective, const float* S, double* out,
-                         void* scratch);
+                         void* scratch, int* err);
 
 size_t full_adjoint_scratch_bytes(int64_t Dp, int64_t T);
 

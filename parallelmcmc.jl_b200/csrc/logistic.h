@@ -83,7 +83,7 @@ cudaError_t lg_margin(cudaStream_t s, bool f64, const DevParams* dP, const DevSt
 // of `band`, the widest that fits kmax) over their la_ref entries; with G (FP32 state, the
 // second pass's parts) their affine maps again by it.
 cudaError_t lg_tie_solve(cudaStream_t s, const LogisticDev& X, const DevParams* dP,
-                         const DevState* dS, double* la_ref, const TieBufs& b, float band,
+                         DevState* dS, double* la_ref, const TieBufs& b, float band,
                          const float* G, int nsplit, int num_sms);
 // Finish of a sweep on the tensor-core path with one probe (logistic_sweep.cu): every
 // column's log alpha and affine map (lg[3], lg[4]) from the second pass's G, the near-tie

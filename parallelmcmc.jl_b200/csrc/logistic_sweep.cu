@@ -7,7 +7,6 @@
 // so the sweep is bound by HBM, and each quantity is formed where it costs no array of
 // its own: g_y and H(y) w go straight from the pass's G into A and B, log alpha and the
 // near-tie list come from the same read.
-#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -16,8 +15,6 @@
 #include "deer_launch.h"
 #include "logistic.h"
 #include "logistic_column.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace pmcmc {
 
@@ -64,7 +61,6 @@ __global__ void __launch_bounds__(kThreads, 3)
   // (a launch after the sweep's first goes on whatever status that one set)
   if (c_lo == 0 && solve_ended(st, P.maxiter)) return;
   if (c_lo > 0 && (st->converged || st->iter >= P.maxiter)) return;
-  cg::grid_group grid = cg::this_grid();
   constexpr int kLoads = 16, kG = 8;
   const int tid = threadIdx.x, lane = tid & 31;
   const int iter = st->iter, cur = st->cur;
@@ -120,7 +116,8 @@ __global__ void __launch_bounds__(kThreads, 3)
       agg_b[ch * Dp + d] = a * eb + b;
     }
   }
-  grid.sync();
+  if (!grid_barrier(P.grid_bar, gridDim.x))
+    atomicCAS(&st->status, 0, static_cast<int>(kStTimeout));
   for (int dd = (tid >> 5) * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x); dd < Dp;
        dd += static_cast<int>(blockDim.x >> 5) * static_cast<int>(gridDim.x)) {
     float s = c_lo ? __ldcg(entry + dd) : x0[dd];
@@ -160,7 +157,8 @@ __global__ void __launch_bounds__(kThreads, 3)
     }
     if (lane == 0) entry[dd] = s;
   }
-  grid.sync();
+  if (!grid_barrier(P.grid_bar, gridDim.x))
+    atomicCAS(&st->status, 0, static_cast<int>(kStTimeout));
   const float dmp = static_cast<float>(P.damping), omd = static_cast<float>(1.0 - P.damping);
   const bool undamped = P.damping == 1.0;
   float dmax = 0.f, smax = 0.f;  // exact in the state's precision

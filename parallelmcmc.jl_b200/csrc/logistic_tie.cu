@@ -26,7 +26,6 @@
 //      at y and both log proposal densities (logq_mala, MALA.jl:172-193); log alpha_t
 //      in FP64 replaces the sweep's value, and the column's (A, B) is formed again.
 // The sweep takes log alpha from la_ref for every column.
-#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -36,8 +35,6 @@
 #include "deer_launch.h"
 #include "logistic.h"
 #include "logistic_column.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace pmcmc {
 namespace tie {
@@ -125,11 +122,14 @@ struct TieArgs {
 // that it replaces: 129 us instead of 400 at N = 10000, D = 256 and 65 columns, 45 instead
 // of 80 at N = 3001, D = 101 and 4 columns, 3 instead of 45 with an empty list (N = 400, D = 24).
 __global__ void __launch_bounds__(kTieThreads, kTieCtas)
-    tie_solve_kernel(const DevParams* __restrict__ Pg, const DevState* __restrict__ st, TieArgs a) {
+    tie_solve_kernel(const DevParams* __restrict__ Pg, DevState* __restrict__ st, TieArgs a) {
   __shared__ int s_base[kTieWarps], s_pos;
   __shared__ double s_sum[kTieWarps];
-  cg::grid_group grid = cg::this_grid();
   const DevParams& P = *Pg;
+  auto all_sync = [&]() {
+    if (!grid_barrier(P.grid_bar, gridDim.x))
+      atomicCAS(&st->status, 0, static_cast<int>(kStTimeout));
+  };
   const int tid = threadIdx.x, lane = tid & 31;
   const int kmax = a.list.kmax;
   int cnt = static_cast<int>(*reinterpret_cast<const volatile uint32_t*>(a.list.count));
@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(kTieThreads, kTieCtas)
       }
       if (tid == 0) a.list.count[1] = min(s_pos, kmax);
     }
-    grid.sync();
+    all_sync();
     cnt = static_cast<int>(__ldcg(a.list.count + 1));
   }
   const int64_t N = a.N, D = P.D, Dp = P.Dp;
@@ -302,9 +302,9 @@ __global__ void __launch_bounds__(kTieThreads, kTieCtas)
   };
 
   logits([&](int k) { return xbar(k); });
-  grid.sync();
+  all_sync();
   gradients();
-  grid.sync();
+  all_sync();
   // gx = X'r - tau x_bar (bayes_logreg.jl:48-58), y = x_bar + eps gx + sqrt(2 eps) xi
   // (MALA.jl:221-222); one CTA a column
   for (int64_t k = blockIdx.x; k < cnt; k += gridDim.x) {
@@ -323,11 +323,11 @@ __global__ void __launch_bounds__(kTieThreads, kTieCtas)
     const double l = loglik(k);
     if (tid == 0) a.lpx[k] = l;
   }
-  grid.sync();
+  all_sync();
   logits([&](int k) { return static_cast<const double*>(a.By) + static_cast<int64_t>(k) * Dp; });
-  grid.sync();
+  all_sync();
   gradients();
-  grid.sync();
+  all_sync();
   // log alpha_t = [lp(y) + logq(x|y)] - [lp(x) + logq(y|x)] (MALA.jl:172-193, 402), and
   // the column's affine map by it; one CTA a column
   for (int64_t k = blockIdx.x; k < cnt; k += gridDim.x) {
@@ -469,7 +469,7 @@ cudaError_t lg_margin(cudaStream_t s, bool f64, const DevParams* dP, const DevSt
 }
 
 cudaError_t lg_tie_solve(cudaStream_t s, const LogisticDev& X, const DevParams* dP,
-                         const DevState* dS, double* la_ref, const TieBufs& b, float band,
+                         DevState* dS, double* la_ref, const TieBufs& b, float band,
                          const float* G, int nsplit, int num_sms) {
   tie::TieArgs a{};
   a.list = tie_list(b, band);

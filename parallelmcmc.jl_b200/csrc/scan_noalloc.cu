@@ -81,10 +81,15 @@ extern "C" int pmcmc_affine_scan_diag_noalloc(int32_t dtype, int64_t D, int64_t 
   const int rc = scratch_for_current_device(&base);
   if (rc) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (pmcmc::launch_affine_scan(s, f64, D, T, A, B, s0, S, base) != cudaSuccess ||
+  // the barrier's word is the array's first, the error flag follows it
+  int* err = static_cast<int*>(base) + 1;
+  int flag = 0;
+  if (cudaMemsetAsync(err, 0, sizeof flag, s) != cudaSuccess ||
+      pmcmc::launch_affine_scan(s, f64, D, T, A, B, s0, S, base, err) != cudaSuccess ||
+      cudaMemcpyAsync(&flag, err, sizeof flag, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess) {
     cudaGetLastError();
     return PMCMC_ERR_CUDA;
   }
-  return PMCMC_OK;
+  return flag ? PMCMC_ERR_TIMEOUT : PMCMC_OK;
 }

@@ -1,5 +1,4 @@
 // tape_scan.cu -- tape materialisation and the standalone diagonal affine scan.
-#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -8,8 +7,6 @@
 
 #include "deer_device.cuh"
 #include "deer_launch.h"
-
-namespace cg = cooperative_groups;
 
 namespace pmcmc {
 
@@ -63,7 +60,7 @@ cudaError_t launch_tape(cudaStream_t s, int64_t D, int64_t T, uint64_t seed, uin
 // ---------------------------------------------------------------------------
 // CTAs an SM and chunks a lane composes at a time, without spills: a spilled value in
 // phase 2 is read from L2 each time, because the CTAs that already wait at the barrier
-// invalidate the SM's L1 with every poll (17 us of a 28 us scan at D = 64, T = 2048)
+// invalidate the SM's L1 with every poll
 constexpr int kScanCtas = 3;
 template <typename Real>
 constexpr int kScanLoads = 64 / sizeof(Real);  // columns of loads in flight a thread
@@ -75,9 +72,8 @@ __global__ void __launch_bounds__(kThreads, kScanCtas)
     affine_scan_kernel(int64_t D, int64_t T, ScanPlan pl, const Real* __restrict__ A,
                        const Real* __restrict__ B, const Real* s0, Real* __restrict__ S,
                        Real* __restrict__ agg_a, Real* __restrict__ agg_b,
-                       Real* __restrict__ carry) {
+                       Real* __restrict__ carry, uint32_t* bar, int* err) {
   __shared__ Real s_a[kThreads], s_b[kThreads];
-  cg::grid_group grid = cg::this_grid();
   constexpr int kScanUnroll = kScanLoads<Real>;
   const int tid = threadIdx.x;
   const int nch = pl.nchunks;
@@ -130,7 +126,7 @@ __global__ void __launch_bounds__(kThreads, kScanCtas)
       agg_b[ch * D + d] = a * eb + b;
     }
   }
-  grid.sync();
+  if (!grid_barrier(bar, gridDim.x)) atomicExch(err, 1);
   {
     const int lane = tid & 31, nw = static_cast<int>(blockDim.x) >> 5;
     constexpr int kG = kScanGroup<Real>;
@@ -174,7 +170,7 @@ __global__ void __launch_bounds__(kThreads, kScanCtas)
       }
     }
   }
-  grid.sync();
+  if (!grid_barrier(bar, gridDim.x)) atomicExch(err, 1);
   if (active && u0 < u1) {
     Real st = __ldcg(carry + d * nch + ch);
     if (sub > 0) st = ea * st + eb;
@@ -241,12 +237,13 @@ int scan_tile_cols(int64_t D, int64_t T) {
 size_t scan_scratch_bytes(bool f64, int64_t D, int64_t T) {
   const int TT = scan_tile_cols(D, T);
   const int64_t nt = (T + TT - 1) / TT;
-  return 3 * (f64 ? 8 : 4) * static_cast<size_t>(nt * D);
+  return kScanBarBytes + 3 * (f64 ? 8 : 4) * static_cast<size_t>(nt * D);
 }
 
 template <typename Real>
 static cudaError_t scan_launches(cudaStream_t s, int64_t D, int64_t T, const Real* A,
-                                 const Real* B, const Real* s0, Real* S, Real* scratch) {
+                                 const Real* B, const Real* s0, Real* S, void* scratch,
+                                 int* err) {
   int dev = 0, sms = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -265,9 +262,11 @@ static cudaError_t scan_launches(cudaStream_t s, int64_t D, int64_t T, const Rea
     int64_t Tn = imin64(Tseg, T - t0), Dn = D;
     ScanPlan pl = scan_plan(D, Tn, max_ctas, scan_tile_cols(D, T), kScanGroup<Real>);
     const Real *An = A + t0 * D, *Bn = B + t0 * D, *sn = t0 ? S + (t0 - 1) * D : s0;
-    Real *Sn = S + t0 * D, *aa = scratch, *ab = aa + static_cast<size_t>(pl.nchunks) * D,
+    uint32_t* bar = static_cast<uint32_t*>(scratch);
+    Real *Sn = S + t0 * D,
+         *aa = reinterpret_cast<Real*>(static_cast<unsigned char*>(scratch) + kScanBarBytes), *ab = aa + static_cast<size_t>(pl.nchunks) * D,
          *ca = ab + static_cast<size_t>(pl.nchunks) * D;
-    void* args[] = {&Dn, &Tn, &pl, &An, &Bn, &sn, &Sn, &aa, &ab, &ca};
+    void* args[] = {&Dn, &Tn, &pl, &An, &Bn, &sn, &Sn, &aa, &ab, &ca, &bar, &err};
     e = cudaLaunchCooperativeKernel(fn, dim3(pl.nchunks * pl.nblk_d), dim3(pl.threads), args, 0,
                                     s);
     if (e != cudaSuccess) return e;
@@ -276,14 +275,12 @@ static cudaError_t scan_launches(cudaStream_t s, int64_t D, int64_t T, const Rea
 }
 
 cudaError_t launch_affine_scan(cudaStream_t s, bool f64, int64_t D, int64_t T, const void* A,
-                               const void* B, const void* s0, void* S, void* scratch) {
+                               const void* B, const void* s0, void* S, void* scratch, int* err) {
   if (T == 0 || D == 0) return cudaSuccess;
   return f64 ? scan_launches(s, D, T, static_cast<const double*>(A), static_cast<const double*>(B),
-                             static_cast<const double*>(s0), static_cast<double*>(S),
-                             static_cast<double*>(scratch))
+                             static_cast<const double*>(s0), static_cast<double*>(S), scratch, err)
              : scan_launches(s, D, T, static_cast<const float*>(A), static_cast<const float*>(B),
-                             static_cast<const float*>(s0), static_cast<float*>(S),
-                             static_cast<float*>(scratch));
+                             static_cast<const float*>(s0), static_cast<float*>(S), scratch, err);
 }
 
 // ---------------------------------------------------------------------------
