@@ -88,7 +88,7 @@ struct pmcmc_handle {
   DevParams* d_params_e = nullptr;  // eigenbasis view of the :full solve
   cudaGraphExec_t gexec_full = nullptr;
   cudaGraphConditionalHandle cond_full = 0;
-  unsigned char gkey_full[192] = {};
+  unsigned char gkey_full[512] = {};
   int full_chunks_override = 0;
   // candidate shapes while pmcmc_autotune times them (0: none)
   int tune_per_sm = 0;
@@ -390,7 +390,7 @@ struct SolveLayout {
   size_t la_ref, tie, lg_acc;                           // logistic: log alpha, near-tie scratch, probe sum
   size_t xi, logu;
   size_t tcws, Gtc, lgscan;  // tensor-core logistic path
-  size_t fU, fV, fR, facc, fPhi, fbeta, fdin, fpart, eS0, eS1, exi, ex0;  // :full mode
+  size_t fU, fV, fR, facc, fPhi, fbeta, fdin, fpart, fGPhi, fgbeta, fPPhi, fpbeta, eS0, eS1, exi, ex0;  // :full mode
   size_t alam, acterm, aarev, adirect, ascr, aout;                 // adjoint
   size_t out2_S, out2_lp, out2_acc;  // second output slot of the host-output pipeline
   size_t part;                       // per-CTA partial reductions of the persistent solve
@@ -469,7 +469,13 @@ SolveLayout layout(int64_t D, int64_t Dp, int64_t T, int ntiles, size_t es, bool
     L.fR = take(4 * T * Dq);
     L.fPhi = take(4 * static_cast<size_t>(fp->nchunks) * Dq * Dq);
     L.fbeta = take(4 * static_cast<size_t>(fp->nchunks) * Dq);
-    L.fdin = take(4 * static_cast<size_t>(fp->nchunks) * Dq);
+    if (fp->G > 1) {
+      L.fGPhi = take(4 * static_cast<size_t>(fp->ngroups) * Dq * Dq);
+      L.fgbeta = take(4 * static_cast<size_t>(fp->ngroups) * Dq);
+      L.fPPhi = take(4 * static_cast<size_t>(fp->nchunks) * Dq * Dq);
+      L.fpbeta = take(4 * static_cast<size_t>(fp->nchunks) * Dq);
+    }
+    L.fdin = take(4 * static_cast<size_t>(fp->ngroups + 1) * Dq);
     L.fpart = take(16 * static_cast<size_t>(fp->nchunks));
   }
   if (adjoint) {
@@ -1163,18 +1169,14 @@ int build_graph_full(pmcmc_handle* h, const FullGraphKey& key) {
   }
   if (e == cudaSuccess) {
     cudaGraph_t body = cp.conditional.phGraph_out[0];
-    const void* fns[4] = {key.fp.eval, key.fp.chunk, key.fp.carry, key.fp.apply};
-    const size_t sm[4] = {key.fp.smem_eval, key.fp.smem_chunk, key.fp.smem_carry,
-                          key.fp.smem_apply};
-    const int grid[4] = {key.fp.eval_grid, key.fp.nchunks, 1, key.fp.nchunks};
-    const int thr[4] = {kThreads, key.fp.threads_chunk, 256, kThreads};
     cudaGraphNode_t prev = nullptr;
-    for (int i = 0; i < 4 && e == cudaSuccess; ++i) {
+    for (int i = 0; i < key.fp.nnodes && e == cudaSuccess; ++i) {
+      const FullNode& nd = key.fp.nodes[i];
       cudaKernelNodeParams sp{};
-      sp.func = const_cast<void*>(fns[i]);
-      sp.gridDim = dim3(grid[i]);
-      sp.blockDim = dim3(thr[i]);
-      sp.sharedMemBytes = static_cast<unsigned>(sm[i]);
+      sp.func = const_cast<void*>(nd.fn);
+      sp.gridDim = dim3(nd.grid);
+      sp.blockDim = dim3(nd.threads);
+      sp.sharedMemBytes = static_cast<unsigned>(nd.smem);
       sp.kernelParams = sweep_args;
       cudaGraphNode_t n;
       e = cudaGraphAddKernelNode(&n, body, prev ? &prev : nullptr, prev ? 1 : 0, &sp);
@@ -1208,12 +1210,10 @@ int run_full(pmcmc_handle* h, const SweepKernels& k, const FullPlan& fp, const D
   CK(cudaMemcpyAsync(h->d_params_e, &Pe, sizeof(DevParams), cudaMemcpyHostToDevice, h->stream));
   CK(cudaMemcpyAsync(h->d_full, &F, sizeof(FullArgs), cudaMemcpyHostToDevice, h->stream));
   {
-    const void* fns[6] = {fp.eval, fp.chunk, fp.carry, fp.apply, k.finalize, fp.rotate};
-    const size_t sm[6] = {fp.smem_eval, fp.smem_chunk, fp.smem_carry, fp.smem_apply, smem_fin,
-                          fp.smem_rotate};
-    for (int i = 0; i < 6; ++i)
-      if (sm[i] > 0)
-        CK(raise_smem_limit(reinterpret_cast<const void*>(fns[i]), sm[i]));
+    for (int i = 0; i < fp.nnodes; ++i)
+      if (fp.nodes[i].smem > 0) CK(raise_smem_limit(fp.nodes[i].fn, fp.nodes[i].smem));
+    if (smem_fin > 0) CK(raise_smem_limit(k.finalize, smem_fin));
+    if (fp.smem_rotate > 0) CK(raise_smem_limit(fp.rotate, fp.smem_rotate));
   }
   if (!h->force_eager && !h->profiling) {
     FullGraphKey key{};
@@ -1464,6 +1464,13 @@ int solve_core(pmcmc_handle* h, const pmcmc_target* tg, const pmcmc_deer_params*
   FullArgs F{};
   if (full) {
     F.Pe = h->d_params_e;
+    F.eS[0] = reinterpret_cast<float*>(ws + L.eS0);
+    F.eS[1] = reinterpret_cast<float*>(ws + L.eS1);
+    F.ex0 = reinterpret_cast<const float*>(ws + L.ex0);
+    F.T = T;
+    F.eps = static_cast<float>(p->epsilon);
+    F.D = static_cast<int32_t>(D);
+    F.maxiter = p->maxiter;
     F.lam = tg->lam_f;
     F.Qrm = tg->qrm_f;
     F.Qcm = tg->qcm_f;
@@ -1477,6 +1484,12 @@ int solve_core(pmcmc_handle* h, const pmcmc_target* tg, const pmcmc_deer_params*
     F.Phi = reinterpret_cast<float*>(ws + L.fPhi);
     F.beta = reinterpret_cast<float*>(ws + L.fbeta);
     F.din = reinterpret_cast<float*>(ws + L.fdin);
+    F.GPhi = reinterpret_cast<float*>(ws + L.fGPhi);
+    F.gbeta = reinterpret_cast<float*>(ws + L.fgbeta);
+    F.PPhi = reinterpret_cast<float*>(ws + L.fPPhi);
+    F.pbeta = reinterpret_cast<float*>(ws + L.fpbeta);
+    F.G = fplan.G;
+    F.ngroups = fplan.ngroups;
     F.part = reinterpret_cast<double*>(ws + L.fpart);
     F.L = fplan.L;
     F.nchunks = fplan.nchunks;

@@ -20,14 +20,14 @@
 // so rounding in the chunk products slows convergence at worst and never
 // moves the fixed point.  All sweep buffers use the stride DQ (16, 32, 64 or
 // 128, zero-padded) so that the per-step loops have compile-time trip counts.
-// Per solve, `rotate` forms xi' and x0'.  A sweep is four launches:
+// Per solve, `rotate` forms xi' and x0'.  A sweep is five launches (four with few chunks):
 //   eval   one warp per column: the diagonal-target forward step in the
 //          eigenbasis, u', v', r' = f'_t - S'_t and the accept flag
 //   chunk  one CTA per chunk of L columns: the chunk's map [Phi'|beta'] as an
-//          augmented DQ x (DQ+1) matrix in registers; four or eight lanes own a
-//          column, whose recursion needs no barrier (column sums by shuffles)
-//   carry  one CTA: updates entering each chunk, chunk maps streamed through
-//          a cp.async ring
+//          augmented DQ x (DQ+1) matrix in registers; four or eight lanes own a few
+//          columns, whose recursions need no barrier (column sums by shuffles)
+//   group  a few CTAs per group of chunks: the group's map, and each chunk's prefix
+//   carry  one CTA: updates entering each group, the maps read two steps ahead
 //   apply  one CTA per chunk: exact replay of the chunk from its entering
 //          update (the old iterates arrive by cp.async meanwhile), the
 //          rotation Q delta' as a warp-tiled product, damping, max|dS| and
@@ -71,6 +71,34 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// Two single-precision operations an instruction, each rounded as its scalar form.
+struct F2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ F2 pack2(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(F2 p, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p.v));
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
 }
 
 // out = rows 4*lane .. 4*lane+3 of M v for one warp (M in shared memory in
@@ -245,141 +273,278 @@ __global__ void __launch_bounds__(kThreads)
 
 // ---------------------------------------------------------------------------
 // chunk: the augmented map [Phi' | beta'] of each chunk.  TPC consecutive
-// lanes own column j (j == DQ is beta'), lane q of them rows [q*NR, (q+1)*NR)
-// in registers (NR = DQ / TPC).  Per step: w_j = v'^T [Phi'|beta']_{:,j}
-// (log2 TPC shuffles), then
+// lanes own NCOL columns (column DQ is beta'), lane q of them the row quads
+// q, q + TPC, ... in registers (NR = DQ / TPC rows).  Per step: w_j = v'^T
+// [Phi'|beta']_{:,j} (log2 TPC shuffles a column), then
 // [Phi'|beta'] <- diag(c_t) [Phi'|beta'] + u' w^T + r' e_DQ^T.
 // Padded rows and columns stay zero.
+// Shared memory returns 128 B a cycle whether lanes share an address or not, so
+// the loads of u' and v' bound a step at one column a thread (22 us at D = 64,
+// T = 8192; at D = 128, where a lane's rows lay 128 B apart, 150): NCOL = 4 columns
+// use each load, and neighbouring lanes read neighbouring quads.
 // ---------------------------------------------------------------------------
-template <int NR, int TPC>
-__global__ void __launch_bounds__(544)
+constexpr int chunk_tpc(int DQ) { return DQ == 16 ? 4 : 8; }
+constexpr int chunk_ncol(int DQ) { return DQ <= 32 ? 2 : 4; }
+constexpr int chunk_threads(int DQ) {
+  return (chunk_tpc(DQ) * (DQ / chunk_ncol(DQ) + 1) + 31) / 32 * 32;
+}
+template <int DQ>
+__global__ void __launch_bounds__(chunk_threads(DQ))
     full_chunk_kernel(const DevParams* __restrict__, const FullArgs* __restrict__ Fg,
                       DevState* __restrict__ st, cudaGraphConditionalHandle, int use_cond) {
-  constexpr int DQ = TPC * NR;
-  static_assert(NR % 4 == 0 && (TPC == 4 || TPC == 8), "chunk tiling");
-  __shared__ DevParams P;
+  constexpr int TPC = chunk_tpc(DQ), NCOL = chunk_ncol(DQ), NR = DQ / TPC, NQ = NR / 4;
+  static_assert(NR % 4 == 0 && (TPC == 4 || TPC == 8) && DQ % NCOL == 0, "chunk tiling");
   __shared__ FullArgs F;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   load_struct(Fg, F);
   __syncthreads();
-  load_params(F.Pe, P);
-  if (sweep_done(st, use_cond, P.maxiter)) return;
+  if (sweep_done(st, use_cond, F.maxiter)) return;
   const int tid = threadIdx.x;
-  const int D = static_cast<int>(P.D);
+  const int D = F.D;
   const int L = F.L;
   const int64_t t0 = static_cast<int64_t>(blockIdx.x) * L;
-  const int nt = static_cast<int>(imin64(L, P.T - t0));
+  const int nt = static_cast<int>(imin64(L, F.T - t0));
   float* Us = reinterpret_cast<float*>(smem_raw);
   float* Vs = Us + L * DQ;
   float* Rs = Vs + L * DQ;
   uint8_t* as = reinterpret_cast<uint8_t*>(Rs + L * DQ);
   {
     const int n4 = nt * DQ / 4;
-    const float4* gu = reinterpret_cast<const float4*>(F.U + t0 * DQ);
-    const float4* gv = reinterpret_cast<const float4*>(F.V + t0 * DQ);
-    const float4* gr = reinterpret_cast<const float4*>(F.R + t0 * DQ);
+    const float* gu = F.U + t0 * DQ;
+    const float* gv = F.V + t0 * DQ;
+    const float* gr = F.R + t0 * DQ;
     for (int i = tid; i < n4; i += blockDim.x) {
-      reinterpret_cast<float4*>(Us)[i] = gu[i];
-      reinterpret_cast<float4*>(Vs)[i] = gv[i];
-      reinterpret_cast<float4*>(Rs)[i] = gr[i];
+      cp_async16(Us + 4 * i, gu + 4 * i);
+      cp_async16(Vs + 4 * i, gv + 4 * i);
+      cp_async16(Rs + 4 * i, gr + 4 * i);
     }
+    cp_async_commit();
     for (int i = tid; i < nt; i += blockDim.x) as[i] = F.acc[t0 + i];
   }
-  const int j = tid / TPC, q = tid % TPC;
-  const bool active = j <= DQ;
-  const bool bcol = j == DQ;
-  const int r0 = q * NR;
-  const float eps = static_cast<float>(P.eps);
-  float phi[NR], ml[NR];
+  const int j0 = tid / TPC * NCOL, q = tid % TPC;
+  const bool bcol = j0 == DQ;  // the offset's thread: its column is the first
+  F2 phi[NCOL][NR / 2], ml[NR / 2];
 #pragma unroll
-  for (int k = 0; k < NR; ++k) {
-    const int i = r0 + k;
-    phi[k] = (active && i == j && i < D) ? 1.f : 0.f;
-    ml[k] = i < D ? 1.f - eps * F.lamQ[i] : 0.f;
+  for (int k = 0; k < NR; k += 2) {
+    const int i = 4 * (q + TPC * (k / 4)) + k % 4;
+#pragma unroll
+    for (int c = 0; c < NCOL; ++c)
+      phi[c][k / 2] = pack2(i == j0 + c && i < D ? 1.f : 0.f, i + 1 == j0 + c && i + 1 < D ? 1.f : 0.f);
+    ml[k / 2] = pack2(i < D ? 1.f - F.eps * F.lamQ[i] : 0.f,
+                      i + 1 < D ? 1.f - F.eps * F.lamQ[i + 1] : 0.f);
   }
+  cp_async_wait<0>();
   __syncthreads();
   for (int s = 0; s < nt; ++s) {
-    const float4* v4 = reinterpret_cast<const float4*>(Vs + s * DQ + r0);
-    const float4* u4 = reinterpret_cast<const float4*>(Us + s * DQ + r0);
-    float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+    const ulonglong2* v4 = reinterpret_cast<const ulonglong2*>(Vs + s * DQ) + q;
+    const ulonglong2* u4 = reinterpret_cast<const ulonglong2*>(Us + s * DQ) + q;
+    F2 a01[NCOL], a23[NCOL];
 #pragma unroll
-    for (int k = 0; k < NR / 4; ++k) {
-      const float4 v = v4[k];
-      a0 = fmaf(v.x, phi[4 * k], a0);
-      a1 = fmaf(v.y, phi[4 * k + 1], a1);
-      a2 = fmaf(v.z, phi[4 * k + 2], a2);
-      a3 = fmaf(v.w, phi[4 * k + 3], a3);
+    for (int c = 0; c < NCOL; ++c) a01[c] = a23[c] = F2{0ull};
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) {
+      const ulonglong2 v = v4[k * TPC];
+#pragma unroll
+      for (int c = 0; c < NCOL; ++c) {
+        a01[c] = fma2(F2{v.x}, phi[c][2 * k], a01[c]);
+        a23[c] = fma2(F2{v.y}, phi[c][2 * k + 1], a23[c]);
+      }
     }
-    float w = (a0 + a1) + (a2 + a3);
-    w += __shfl_xor_sync(0xffffffffu, w, 1);
-    w += __shfl_xor_sync(0xffffffffu, w, 2);
-    if (TPC == 8) w += __shfl_xor_sync(0xffffffffu, w, 4);
+    float w[NCOL];
+#pragma unroll
+    for (int c = 0; c < NCOL; ++c) {
+      float a0, a1, a2, a3;
+      unpack2(a01[c], a0, a1);
+      unpack2(a23[c], a2, a3);
+      w[c] = (a0 + a1) + (a2 + a3);
+    }
+#pragma unroll
+    for (int o = 1; o < TPC; o *= 2)
+#pragma unroll
+      for (int c = 0; c < NCOL; ++c) w[c] += __shfl_xor_sync(0xffffffffu, w[c], o);
     if (as[s]) {  // uniform across the CTA
 #pragma unroll
-      for (int k = 0; k < NR / 4; ++k) {
-        const float4 u = u4[k];
-        phi[4 * k] = fmaf(u.x, w, ml[4 * k] * phi[4 * k]);
-        phi[4 * k + 1] = fmaf(u.y, w, ml[4 * k + 1] * phi[4 * k + 1]);
-        phi[4 * k + 2] = fmaf(u.z, w, ml[4 * k + 2] * phi[4 * k + 2]);
-        phi[4 * k + 3] = fmaf(u.w, w, ml[4 * k + 3] * phi[4 * k + 3]);
-      }
-    } else {
+      for (int c = 0; c < NCOL; ++c)
 #pragma unroll
-      for (int k = 0; k < NR / 4; ++k) {
-        const float4 u = u4[k];
-        phi[4 * k] = fmaf(u.x, w, phi[4 * k]);
-        phi[4 * k + 1] = fmaf(u.y, w, phi[4 * k + 1]);
-        phi[4 * k + 2] = fmaf(u.z, w, phi[4 * k + 2]);
-        phi[4 * k + 3] = fmaf(u.w, w, phi[4 * k + 3]);
+        for (int k = 0; k < NR / 2; ++k) phi[c][k] = mul2(ml[k], phi[c][k]);
+    }
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) {
+      const ulonglong2 u = u4[k * TPC];
+#pragma unroll
+      for (int c = 0; c < NCOL; ++c) {
+        const F2 ww = pack2(w[c], w[c]);
+        phi[c][2 * k] = fma2(F2{u.x}, ww, phi[c][2 * k]);
+        phi[c][2 * k + 1] = fma2(F2{u.y}, ww, phi[c][2 * k + 1]);
       }
     }
     if (bcol) {
-      const float4* r4 = reinterpret_cast<const float4*>(Rs + s * DQ + r0);
+      const ulonglong2* r4 = reinterpret_cast<const ulonglong2*>(Rs + s * DQ) + q;
 #pragma unroll
-      for (int k = 0; k < NR / 4; ++k) {
-        const float4 r = r4[k];
-        phi[4 * k] += r.x;
-        phi[4 * k + 1] += r.y;
-        phi[4 * k + 2] += r.z;
-        phi[4 * k + 3] += r.w;
+      for (int k = 0; k < NQ; ++k) {
+        const ulonglong2 r = r4[k * TPC];
+        phi[0][2 * k] = add2(phi[0][2 * k], F2{r.x});
+        phi[0][2 * k + 1] = add2(phi[0][2 * k + 1], F2{r.y});
       }
     }
   }
-  if (active) {
-    float* dst = bcol ? F.beta + static_cast<size_t>(blockIdx.x) * DQ + r0
-                      : F.Phi + (static_cast<size_t>(blockIdx.x) * DQ + j) * DQ + r0;  // column-major
 #pragma unroll
-    for (int k = 0; k < NR / 4; ++k)
-      reinterpret_cast<float4*>(dst)[k] =
-          make_float4(phi[4 * k], phi[4 * k + 1], phi[4 * k + 2], phi[4 * k + 3]);
+  for (int c = 0; c < NCOL; ++c) {
+    const int j = j0 + c;
+    if (j > DQ) break;
+    float* dst = j == DQ ? F.beta + static_cast<size_t>(blockIdx.x) * DQ
+                         : F.Phi + (static_cast<size_t>(blockIdx.x) * DQ + j) * DQ;  // column-major
+#pragma unroll
+    for (int k = 0; k < NQ; ++k)
+      reinterpret_cast<ulonglong2*>(dst)[q + k * TPC] =
+          make_ulonglong2(phi[c][2 * k].v, phi[c][2 * k + 1].v);
   }
 }
 
 // ---------------------------------------------------------------------------
-// carry: din_0 = 0, din_{c+1} = Phi'_c din_c + beta'_c (one CTA).  Thread
+// group: the maps of a group of G consecutive chunks, [Phi'|beta']_{c+G-1} ... composed
+// in order, and before each chunk the composition of those ahead of it in the group.
+// A column of the augmented product depends on that column alone, so the DQ + 1 columns
+// are split over gridDim.x / ngroups CTAs of NC columns.  A warp forms 4 * RG rows of
+// four columns: a lane adds a 4 x 4 tile over every KS-th k, and the KS partial tiles
+// are summed by exchanging halves (32 B of shared memory a 16 products; with one row a
+// lane it was 20 B a 4, and a step took twice as long).  The maps pass through a ring of three
+// slots, copied two steps ahead.  With it the carry runs over the groups and an apply CTA forms its
+// entering update by one product with its prefix: the serial chain of a sweep is
+// G + nchunks / G steps instead of nchunks (45 of 103 us a sweep at D = 64, T = 8192).
+// ---------------------------------------------------------------------------
+template <int DQ>
+struct GroupTile {
+  static constexpr int RG = DQ >= 32 ? 8 : 4, KS = 32 / RG, RB = DQ / (4 * RG), NC = 4 * (8 / RB);
+  static constexpr int SX = NC + 4;
+  static constexpr size_t smem = sizeof(float) * (3 * (DQ * DQ + DQ) + 2 * DQ * SX);
+};
+template <int DQ>
+__global__ void __launch_bounds__(256)
+    full_group_kernel(const DevParams* __restrict__, const FullArgs* __restrict__ Fg,
+                      DevState* __restrict__ st, cudaGraphConditionalHandle, int use_cond) {
+  using Tile = GroupTile<DQ>;
+  constexpr int RG = Tile::RG, KS = Tile::KS, RB = Tile::RB, NC = Tile::NC, SX = Tile::SX;
+  __shared__ FullArgs F;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  load_struct(Fg, F);
+  __syncthreads();
+  if (sweep_done(st, use_cond, F.maxiter)) return;
+  float* Ms = reinterpret_cast<float*>(smem_raw);  // three maps, DQ x DQ column-major
+  float* bs = Ms + 3 * DQ * DQ;                    // their offsets
+  float* xs = bs + 3 * DQ;                         // DQ x SX, the columns, two turns
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int row = warp % RB * 4 * RG + lane % RG * 4, cg = 4 * (warp / RB), kq = lane / RG;
+  constexpr int slices = (DQ + NC) / NC;
+  const int grp = static_cast<int>(blockIdx.x) / slices, slice = static_cast<int>(blockIdx.x) % slices;
+  const int ch0 = grp * F.G, n = min(F.G, F.nchunks - ch0);
+  auto fetch = [&](int i) {
+    if (i < n) {
+      const int slot = i % 3;
+      const float* src = F.Phi + static_cast<size_t>(ch0 + i) * DQ * DQ;
+      float* dst = Ms + slot * DQ * DQ;
+      for (int k = tid; k < DQ * DQ / 4; k += 256) cp_async16(dst + 4 * k, src + 4 * k);
+      if (tid < DQ / 4)
+        cp_async16(bs + slot * DQ + 4 * tid, F.beta + static_cast<size_t>(ch0 + i) * DQ + 4 * tid);
+    }
+    cp_async_commit();
+  };
+  fetch(0);
+  fetch(1);
+  for (int i = tid; i < DQ * NC; i += 256) {
+    const int r = i / NC, c = slice * NC + i % NC;
+    xs[r * SX + i % NC] = r == c ? 1.f : 0.f;
+  }
+  // the lane's column once the partial tiles are summed (column DQ is the offset's; past
+  // it, unused)
+  const int own = cg + 2 * (lane >> 4) + (lane >> 3 & 1), col = slice * NC + own;
+  for (int i = 0; i < n; ++i) {
+    cp_async_wait<1>();
+    __syncthreads();  // map i and the columns are in place, map i - 1's slot is free
+    fetch(i + 2);
+    const int slot = i % 3;
+    const float* M = Ms + slot * DQ * DQ + row;
+    const float* x = xs + (i & 1) * DQ * SX + cg;
+    F2 a[4][2];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) a[c][0] = a[c][1] = F2{0ull};
+#pragma unroll 4
+    for (int k = kq; k < DQ; k += KS) {
+      const ulonglong2 m = *reinterpret_cast<const ulonglong2*>(M + k * DQ);
+      float v[4];
+      load4(x + k * SX, v);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const F2 vv = pack2(v[c], v[c]);
+        a[c][0] = fma2(F2{m.x}, vv, a[c][0]);
+        a[c][1] = fma2(F2{m.y}, vv, a[c][1]);
+      }
+    }
+    float t[4][4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      unpack2(a[c][0], t[c][0], t[c][1]);
+      unpack2(a[c][1], t[c][2], t[c][3]);
+    }
+    const bool hi16 = lane & 16, hi8 = lane & 8;
+    float h[2][4], acc[4];
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        h[c][e] = (hi16 ? t[c + 2][e] : t[c][e]) +
+                  __shfl_xor_sync(0xffffffffu, hi16 ? t[c][e] : t[c + 2][e], 16);
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      acc[e] = (hi8 ? h[1][e] : h[0][e]) + __shfl_xor_sync(0xffffffffu, hi8 ? h[0][e] : h[1][e], 8);
+    if (KS == 8)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], 4);
+    if (col == DQ) {
+      float b[4];
+      load4(bs + slot * DQ + row, b);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[e] += b[e];
+    }
+    float* xn = xs + ((i + 1) & 1) * DQ * SX;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) xn[(row + e) * SX + own] = acc[e];
+    // after chunk i: the prefix of chunk i + 1, or the group's map
+    float* phi = i + 1 < n ? F.PPhi + static_cast<size_t>(ch0 + i + 1) * DQ * DQ
+                           : F.GPhi + static_cast<size_t>(grp) * DQ * DQ;
+    float* beta = i + 1 < n ? F.pbeta + static_cast<size_t>(ch0 + i + 1) * DQ
+                            : F.gbeta + static_cast<size_t>(grp) * DQ;
+    if (col <= DQ && (KS == 4 || !(lane & 4)))
+      store4(col < DQ ? phi + static_cast<size_t>(col) * DQ + row : beta + row, acc);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// carry, over the groups: din_0 = 0, din_{g+1} = Phi'_g din_g + beta'_g (one CTA).  Thread
 // (part, row) sums KC terms of row `row` (the map is column-major, so the
 // threads of a part read consecutive rows: coalesced), partial sums combined
 // through shared memory.  Each thread keeps its KC map entries for the next
 // two chunks in registers, loaded from L2 two steps ahead (a three-slot ring),
 // so a step waits on no copy.
 // ---------------------------------------------------------------------------
-template <int DQ, int NST>
+template <int DQ>
 __global__ void __launch_bounds__(256)
     full_carry_kernel(const DevParams* __restrict__, const FullArgs* __restrict__ Fg,
                       DevState* __restrict__ st, cudaGraphConditionalHandle, int use_cond) {
   constexpr int PARTS = DQ >= 128 ? 2 : 4;
   constexpr int KC = DQ / PARTS;
   static_assert(PARTS * DQ <= 256, "one thread a (part, row)");
-  __shared__ DevParams P;
   __shared__ FullArgs F;
   __shared__ float vec[2][DQ];
   __shared__ float pbuf[PARTS][DQ];
   load_struct(Fg, F);
   __syncthreads();
-  load_params(F.Pe, P);
-  if (sweep_done(st, use_cond, P.maxiter)) return;
+  if (sweep_done(st, use_cond, F.maxiter)) return;
   const int tid = threadIdx.x;
-  const int nch = F.nchunks;
+  // the groups' maps, or with one chunk a group the chunks'
+  const int nch = F.ngroups;
+  const float* __restrict__ maps = F.G > 1 ? F.GPhi : F.Phi;
+  const float* __restrict__ offs = F.G > 1 ? F.gbeta : F.beta;
   const int row = tid % DQ, part = tid / DQ;
   const bool worker = part < PARTS;
   const int k0 = part * KC;
@@ -390,11 +555,11 @@ __global__ void __launch_bounds__(256)
   auto fetch = [&](int c, float (&dst)[KC], float& b) {
     if (c < nch - 1) {
       if (worker) {
-        const float* Ph = F.Phi + static_cast<size_t>(c) * DQ * DQ + static_cast<size_t>(k0) * DQ + row;
+        const float* Ph = maps + static_cast<size_t>(c) * DQ * DQ + static_cast<size_t>(k0) * DQ + row;
 #pragma unroll
         for (int k = 0; k < KC; ++k) dst[k] = __ldcg(Ph + static_cast<size_t>(k) * DQ);
       }
-      if (tid < DQ) b = __ldcg(F.beta + static_cast<size_t>(c) * DQ + tid);
+      if (tid < DQ) b = __ldcg(offs + static_cast<size_t>(c) * DQ + tid);
     }
   };
   auto step = [&](int c, const float (&cur)[KC], float b) {
@@ -444,15 +609,16 @@ __global__ void __launch_bounds__(kThreads)
     full_apply_kernel(const DevParams* __restrict__ Pg, const FullArgs* __restrict__ Fg,
                       DevState* __restrict__ st, cudaGraphConditionalHandle cond, int use_cond) {
   __shared__ DevParams P;   // original basis
-  __shared__ DevParams Pe;  // eigenbasis
   __shared__ FullArgs F;
   __shared__ double r_dm[kWarps], r_sm[kWarps];
   __shared__ int s_bad, s_last;
+  __shared__ __align__(16) float s_din[kThreads / DQ][DQ];
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int cur = st->cur;
+  const bool first = st->iter == 0;
   load_struct(Fg, F);
   load_struct(Pg, P);
   __syncthreads();
-  load_params(F.Pe, Pe);
   if (sweep_done(st, use_cond, P.maxiter)) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int D = static_cast<int>(P.D), Dp = static_cast<int>(P.Dp);
@@ -466,8 +632,6 @@ __global__ void __launch_bounds__(kThreads)
   float* Eo = Qs + DQ * DQ;  // L x DQ old eigenbasis iterate
   float* So = Eo + L * DQ;   // L x Dp old iterate
   uint8_t* as = reinterpret_cast<uint8_t*>(So + L * Dp);
-  const int cur = st->cur;
-  const bool first = st->iter == 0;
   {
     const int n4 = nt * DQ / 4;
     const float* gu = F.U + t0 * DQ;
@@ -482,13 +646,32 @@ __global__ void __launch_bounds__(kThreads)
     cp_async_commit();
     if (!first) {
       const float* go = static_cast<const float*>(P.S[cur]) + t0 * Dp;
-      const float* ge = static_cast<const float*>(Pe.S[cur]) + t0 * DQ;
+      const float* ge = F.eS[cur] + t0 * DQ;
       for (int i = tid; i < nt * Dp / 4; i += blockDim.x) cp_async16(So + 4 * i, go + 4 * i);
       for (int i = tid; i < n4; i += blockDim.x) cp_async16(Eo + 4 * i, ge + 4 * i);
     }
     cp_async_commit();
     for (int i = tid; i < nt; i += blockDim.x) as[i] = F.acc[t0 + i];
     if (tid == 0) s_bad = 0;
+  }
+  // the update entering the chunk: its group's, through the prefix of the group's
+  // earlier chunks (the group's first chunk has none)
+  const int ch = static_cast<int>(blockIdx.x), grp = ch / F.G;
+  {
+    constexpr int PARTS = kThreads / DQ, KC = DQ / PARTS;
+    const float* gin = F.din + static_cast<size_t>(grp) * DQ;
+    const int row = tid % DQ, part = tid / DQ;
+    if (ch > grp * F.G) {
+      float a = 0.f;
+      const float* Ph = F.PPhi + static_cast<size_t>(ch) * DQ * DQ + static_cast<size_t>(part * KC) * DQ + row;
+#pragma unroll
+      for (int k = 0; k < KC; ++k)
+        a = fmaf(__ldcg(Ph + static_cast<size_t>(k) * DQ), __ldcg(gin + part * KC + k), a);
+      s_din[part][row] = a;
+      if (part == 0) s_din[0][row] += __ldcg(F.pbeta + static_cast<size_t>(ch) * DQ + row);
+    } else {
+      s_din[part][row] = part == 0 ? __ldcg(gin + row) : 0.f;
+    }
   }
   cp_async_wait<1>();
   __syncthreads();
@@ -498,7 +681,13 @@ __global__ void __launch_bounds__(kThreads)
     const float eps = static_cast<float>(P.eps);
     float d[4] = {0.f, 0.f, 0.f, 0.f}, lc[4] = {0.f, 0.f, 0.f, 0.f};
     if (in) {
-      load4(F.din + static_cast<size_t>(blockIdx.x) * DQ + 4 * lane, d);
+#pragma unroll
+      for (int p = 0; p < kThreads / DQ; ++p) {
+        float v[4];
+        load4(&s_din[p][4 * lane], v);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) d[e] += v[e];
+      }
       float l4[4];
       load4(F.lamQ + 4 * lane, l4);
 #pragma unroll
@@ -542,9 +731,9 @@ __global__ void __launch_bounds__(kThreads)
   cp_async_wait<0>();
   __syncthreads();
   float* Snew = static_cast<float*>(P.S[cur ^ 1]);
-  float* Enew = static_cast<float*>(Pe.S[cur ^ 1]);
+  float* Enew = F.eS[cur ^ 1];
   const float* x0 = static_cast<const float*>(P.x0);
-  const float* x0e = static_cast<const float*>(Pe.x0);
+  const float* x0e = F.ex0;
   const float dmp = static_cast<float>(P.damping);
   float dm = 0.f, smx = 0.f;  // maxima are exact in FP32
   bool bad = false;
@@ -864,20 +1053,20 @@ size_t apply_smem(int Dq, int64_t Dp, int L) {
   return sizeof(float) * (4 * static_cast<size_t>(L) * Dq + static_cast<size_t>(Dq) * Dq + L * Dp) +
          L + 16;
 }
-int carry_stages(int Dq) { return Dq <= 64 ? 8 : 2; }
 
 size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // lanes per column of the chunk kernel: 8 where NR stays a multiple of 4 and
 // the CTA within 544 threads
-constexpr int chunk_tpc(int DQ) { return (DQ == 32 || DQ == 64) ? 8 : 4; }
 
 template <int DQ>
 void pick_kernels(FullPlan* fp) {
-  constexpr int NST = DQ <= 64 ? 8 : 2;
-  constexpr int TPC = chunk_tpc(DQ);
-  fp->chunk = reinterpret_cast<const void*>(&full_chunk_kernel<DQ / TPC, TPC>);
-  fp->carry = reinterpret_cast<const void*>(&full_carry_kernel<DQ, NST>);
+  fp->chunk = reinterpret_cast<const void*>(&full_chunk_kernel<DQ>);
+  fp->threads_chunk = chunk_threads(DQ);
+  fp->carry = reinterpret_cast<const void*>(&full_carry_kernel<DQ>);
+  fp->group = reinterpret_cast<const void*>(&full_group_kernel<DQ>);
+  fp->group_slices = (DQ + GroupTile<DQ>::NC) / GroupTile<DQ>::NC;
+  fp->smem_group = GroupTile<DQ>::smem;
   fp->apply = reinterpret_cast<const void*>(&full_apply_kernel<DQ>);
   fp->rotate = reinterpret_cast<const void*>(&full_rotate_kernel<DQ>);
 }
@@ -895,40 +1084,72 @@ bool full_plan(int64_t Dp, int64_t T, int tkind, int num_sms, int chunks_overrid
   const int Dq = full_stride(Dp);
   if (Dq == 0 || T < 1) return false;
   fp->Dq = Dq;
-  const size_t budget = 200 * 1024;
-  int Lmax = 1;
-  while (Lmax < 4096 && chunk_smem(Dq, Lmax + 1) <= budget && apply_smem(Dq, Dp, Lmax + 1) <= budget)
-    ++Lmax;
-  // the sequential depth of a sweep is ~L chunk steps + L replay steps +
-  // nchunks carry steps, a carry step about a quarter of the cost of the other
-  // two together: about sqrt(2 T) chunks balances them (128 at T = 8192:
-  // 121 us a sweep against 139 us at 64 chunks, D = 64)
-  int nch = chunks_override > 0
-                ? chunks_override
-                : std::min(num_sms, static_cast<int>(std::sqrt(2.0 * static_cast<double>(T)) + 0.5));
-  nch = std::max(1, nch);
-  int64_t L = (T + nch - 1) / nch;
-  if (L > Lmax) L = Lmax;
-  fp->L = static_cast<int>(L);
-  fp->nchunks = static_cast<int>((T + L - 1) / L);
-  fp->smem_chunk = chunk_smem(Dq, fp->L);
-  fp->smem_apply = apply_smem(Dq, Dp, fp->L);
-  const int nst = carry_stages(Dq);
-  const int parts = Dq >= 128 ? 2 : 4;
-  fp->smem_carry = 0;  // static shared memory only
-  (void)nst;
-  (void)parts;
-  fp->smem_eval = plan_sweep_smem<float>(Dq, 1, false).total;
-  fp->eval_grid =
-      static_cast<int>(std::min<int64_t>((T + kWarps - 1) / kWarps, int64_t(num_sms) * 4));
-  fp->threads_chunk = ((chunk_tpc(Dq) * (Dq + 1) + 31) / 32) * 32;
-  fp->eval = reinterpret_cast<const void*>(&full_eval_kernel);
   switch (Dq) {
     case 16: pick_kernels<16>(fp); break;
     case 32: pick_kernels<32>(fp); break;
     case 64: pick_kernels<64>(fp); break;
     default: pick_kernels<128>(fp); break;
   }
+  const size_t budget = 200 * 1024;
+  int Lmax = 1;
+  while (Lmax < 4096 && chunk_smem(Dq, Lmax + 1) <= budget && apply_smem(Dq, Dp, Lmax + 1) <= budget)
+    ++Lmax;
+  // The serial chain of a sweep: L steps of the chunk maps and of the replay, G steps of
+  // the groups' composition, nchunks / G steps of the carry.  us a step, fitted to sweeps
+  // timed over 64 .. 592 chunks: a chunk step takes c_lat, or c_iss for each chunk its SM
+  // holds; a group step c_g for each CTA (group_slices a group) its SM holds; a carry step c_c.
+  // At D = 64, T = 8192: 56 + 7 + 22 steps or 28 + 14 + 21, 67 to 70 us a sweep, against 64 + 128 steps and
+  // 103 us with the carry over the chunks; 64 chunks take 100 us, 592 take 89.  D = 128: 171 us (start 428), 592 chunks 264.
+  const int w = Dq == 16 ? 0 : Dq == 32 ? 1 : Dq == 64 ? 2 : 3;
+  static constexpr double kStep[4][4] = {{0.30, 0.10, 0.30, 0.30},
+                                         {0.30, 0.10, 0.40, 0.30},
+                                         {0.35, 0.17, 0.70, 0.30},
+                                         {0.60, 0.45, 1.30, 0.60}};
+  const double c_lat = kStep[w][0], c_iss = kStep[w][1], c_g = kStep[w][2], c_c = kStep[w][3];
+  auto per_sm = [&](int64_t n) { return static_cast<double>((n + num_sms - 1) / num_sms); };
+  auto groups = [&](int64_t n, double* cost) {  // chunks a group
+    int best = 1;
+    *cost = c_c * static_cast<double>(n);
+    for (int g = 2; g <= 64 && g <= n; g += 1 + g / 8) {
+      const int64_t ng = (n + g - 1) / g;
+      const double c = 4.0 + c_g * g * per_sm(ng * fp->group_slices) + c_c * static_cast<double>(ng);
+      if (c < *cost) *cost = c, best = g;
+    }
+    return best;
+  };
+  int64_t L = 0;
+  double best = 0.0, c = 0.0;
+  if (chunks_override > 0) {
+    L = std::min<int64_t>((T + chunks_override - 1) / chunks_override, Lmax);
+  } else {
+    const int64_t l0 = std::min<int64_t>(Lmax, (T + 4 * num_sms - 1) / (4 * num_sms));
+    for (int64_t l = l0; l <= Lmax && (L == 0 || l <= T); l += 1 + l / 16) {
+      const int64_t n = (T + l - 1) / l;
+      groups(n, &c);
+      c += static_cast<double>(l) * std::max(c_lat, c_iss * per_sm(n));
+      if (L == 0 || c < best) best = c, L = l;
+    }
+  }
+  fp->L = static_cast<int>(L);
+  fp->nchunks = static_cast<int>((T + L - 1) / L);
+  fp->G = groups(fp->nchunks, &c);
+  fp->ngroups = (fp->nchunks + fp->G - 1) / fp->G;
+  fp->smem_chunk = chunk_smem(Dq, fp->L);
+  fp->smem_apply = apply_smem(Dq, Dp, fp->L);
+  fp->smem_carry = 0;  // static shared memory only
+  fp->smem_eval = plan_sweep_smem<float>(Dq, 1, false).total;
+  fp->eval_grid =
+      static_cast<int>(std::min<int64_t>((T + kWarps - 1) / kWarps, int64_t(num_sms) * 4));
+  fp->eval = reinterpret_cast<const void*>(&full_eval_kernel);
+  fp->nnodes = 0;
+  auto node = [&](const void* fn, int grid, int threads, size_t smem) {
+    fp->nodes[fp->nnodes++] = FullNode{fn, smem, grid, threads};
+  };
+  node(fp->eval, fp->eval_grid, kThreads, fp->smem_eval);
+  node(fp->chunk, fp->nchunks, fp->threads_chunk, fp->smem_chunk);
+  if (fp->G > 1) node(fp->group, fp->ngroups * fp->group_slices, 256, fp->smem_group);
+  node(fp->carry, 1, 256, fp->smem_carry);
+  node(fp->apply, fp->nchunks, kThreads, fp->smem_apply);
   fp->smem_rotate = sizeof(float) * (static_cast<size_t>(Dq) * Dq + kWarps * 8 * Dp);
   fp->rotate_grid = static_cast<int>(
       std::max<int64_t>(1, std::min<int64_t>((T + 8 * kWarps - 1) / (8 * kWarps), num_sms)));
@@ -939,12 +1160,9 @@ cudaError_t full_sweep(cudaStream_t s, const FullPlan& fp, const DevParams* Pg, 
                        DevState* st, cudaGraphConditionalHandle cond, int use_cond) {
   void* args[] = {const_cast<DevParams**>(&Pg), const_cast<FullArgs**>(&Fg), &st, &cond,
                   &use_cond};
-  const void* fns[4] = {fp.eval, fp.chunk, fp.carry, fp.apply};
-  const size_t sm[4] = {fp.smem_eval, fp.smem_chunk, fp.smem_carry, fp.smem_apply};
-  const int grid[4] = {fp.eval_grid, fp.nchunks, 1, fp.nchunks};
-  const int thr[4] = {kThreads, fp.threads_chunk, 256, kThreads};
-  for (int i = 0; i < 4; ++i) {
-    const cudaError_t e = cudaLaunchKernel(fns[i], dim3(grid[i]), dim3(thr[i]), args, sm[i], s);
+  for (int i = 0; i < fp.nnodes; ++i) {
+    const FullNode& n = fp.nodes[i];
+    const cudaError_t e = cudaLaunchKernel(n.fn, dim3(n.grid), dim3(n.threads), args, n.smem, s);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;

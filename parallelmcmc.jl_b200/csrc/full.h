@@ -23,15 +23,23 @@ struct FullArgs {
   const float* lamQ;    // the same three padded to the sweep stride Dq (16, 32, 64 or 128)
   const float* QrmQ;
   const float* QcmQ;
+  float* eS[2];         // S' of the eigenbasis view, and x0'
+  const float* ex0;
+  int64_t T;            // of the solve, beside the parameters for one load at a kernel's start
+  float eps;
+  int32_t D, maxiter, pad;
   float* U;             // T x Dq  u'_t = Q^T g(1-g)(y_t - x_t)
   float* V;             // T x Dq  v'_t = Q^T grad log alpha_t
   float* R;             // T x Dq  r'_t = f'_t - S'_t   (Newton residual)
   uint8_t* acc;         // T       accept flags of the current sweep
   float* Phi;           // nchunks x Dq x Dq chunk maps (column-major)
   float* beta;          // nchunks x Dq      chunk offsets
-  float* din;           // nchunks x Dq      primed update entering each chunk
+  float* din;           // ngroups x Dq      primed update entering each group
+  float *GPhi, *gbeta;  // ngroups x ...     the groups' maps and offsets (G > 1)
+  float *PPhi, *pbeta;  // nchunks x ...     the prefix of each chunk in its group (G > 1)
   double* part;         // nchunks x 2       each apply CTA's max|dS|, max|S|
   int32_t L, nchunks;
+  int32_t G, ngroups;   // chunks a group
   int32_t rot, Dq;
   // adjoint
   float* lam_adj;       // T x Dp  reversed primed adjoint
@@ -44,9 +52,20 @@ struct FullArgs {
 // (0 when Dp > 128).
 int full_stride(int64_t Dp);
 
+// One launch of a sweep.
+struct FullNode {
+  const void* fn;
+  size_t smem;
+  int grid, threads;
+};
+
 struct FullPlan {
   int Dq = 0;
-  int L = 0, nchunks = 0;
+  int L = 0, nchunks = 0, G = 1, ngroups = 0, group_slices = 0;
+  int nnodes = 0;
+  FullNode nodes[5] = {};
+  const void* group = nullptr;
+  size_t smem_group = 0;
   int eval_grid = 0;
   size_t smem_eval = 0, smem_chunk = 0, smem_carry = 0, smem_apply = 0;
   int threads_chunk = 0;
@@ -63,7 +82,7 @@ struct FullPlan {
 // returns false when the dimension is outside the built range.
 bool full_plan(int64_t Dp, int64_t T, int tkind, int num_sms, int chunks_override, FullPlan* fp);
 
-// One sweep = eval, chunk maps, carry, replay + damping + convergence test.
+// One sweep = eval, chunk maps, group maps, carry, replay + damping + convergence test.
 // Kernel signatures: (const DevParams*, const FullArgs*, DevState*, cudaGraphConditionalHandle, int use_cond).
 // `rotate` (same signature, grid rotate_grid) fills the eigenbasis tape xi' and
 // x0' once per solve, after the tape kernel.
