@@ -2463,7 +2463,7 @@ int chains_impl(pmcmc_handle* h, const pmcmc_target* tg, const pmcmc_deer_params
     dx0 = h->ws;
   }
   CK(launch_mala_chains(h->stream, f64, tg->kind, P, cad, n, dx0, dseeds, dS, dlp, dacc, deps,
-                        dst));
+                        dst, h->num_sms));
   if (mass) CK(mass_map(h->stream, tg->mass_Ld, D, n * T, dS, f64, h->num_sms));
   if (mem == PMCMC_MEM_HOST) {
     CK(cudaMemcpyAsync(S_out, dS, bS, cudaMemcpyDeviceToHost, h->stream));

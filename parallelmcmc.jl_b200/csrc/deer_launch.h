@@ -57,7 +57,7 @@ size_t mala_chains_smem(bool f64, int64_t Dp, bool dense);
 cudaError_t launch_mala_chains(cudaStream_t s, bool f64, int tk, const DevParams& P,
                                const ChainAdapt& ad, int64_t nchains, const void* x0,
                                const uint64_t* seeds, void* S, void* logp, uint8_t* acc,
-                               double* eps_out, double* state_out);
+                               double* eps_out, double* state_out, int num_sms);
 
 // Tape materialisation (tape.cu).
 cudaError_t launch_tape(cudaStream_t s, int64_t D, int64_t T, uint64_t seed, uint64_t block,
