@@ -11,28 +11,29 @@
 //   dL/deps  = direct + sum_{t accepted} lambda_t . (g(x_{t-1}) + xi_t / sqrt(2 eps)),
 // where c_t (the objective's gradient in x_t) and `direct` (its partial in eps)
 // come from per-step terms.  Those need Hessian-vector products at x_{t-1} and
-// y_t for every t, batched as GEMMs:
+// y_t for every t, batched over the columns (hvp_kernel, GEMMs above 128 coordinates):
 //   H(z) V = -X^T (p(1 - p) .* (X V)) - tau V,  p = sigmoid(X z).
 // J_{t+1} is dense and changes with t, so the recurrence is not one affine scan
 // of diagonal maps.  It is solved by Jacobi iterations on its diagonal part:
 //   lambda^{k+1}_t = D_{t+1} lambda^{k+1}_{t+1} + c_t + (J_{t+1} - D_{t+1}) lambda^k_{t+1},
 // D_{t+1} = 1 + eps diag H(x_t) = 1 - eps (X.*X)^T p(1 - p) - eps tau; each
 // iteration is one batched HVP and one diagonal affine scan (the standalone
-// look-back scan, run on the time-reversed arrays).  The fixed point is the
+// scan, run on the time-reversed arrays).  The fixed point is the
 // exact recurrence; the iterations stop when max|lambda^{k+1} - lambda^k| <=
 // 1e-12 max|lambda^{k+1}|.
 //
-// Everything runs in FP64 (cuBLAS DGEMM, pedantic math) whatever the state's
-// type.  Layouts: D-vectors of column t at t * Dp (zero-padded to Dp); N x T
+// Everything runs in FP64 (FP64 MMAs, and cuBLAS DGEMM with pedantic math) whatever the
+// state's type.  Layouts: D-vectors of column t at t * Dp (zero-padded to Dp); N x T
 // matrices column-major (column t at t * N).
 #include <cublas_v2.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
-#include <vector>
 
 #include "deer_device.cuh"
+#include "deer_launch.h"
 #include "logistic.h"
 #include "pmcmc_rng.cuh"
 
@@ -100,6 +101,163 @@ __global__ void lik_kernel(double* __restrict__ L, const double* __restrict__ yl
   }
   s = block_sum(s, sh);
   if (threadIdx.x == 0) ll[t] = s;
+}
+
+// An FP64 MMA (16 x 8, k = 8): with r = l / 4 and q = l % 4, lane l holds A[r + 8 (i % 2)]
+// [q + 4 (i / 2)], B[q + 4 i][r] and C[r + 8 (i / 2)][2 q + i % 2].
+__device__ __forceinline__ void dmma(double (&c)[4], const double (&a)[4], const double (&b)[2]) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+      "{%8, %9}, {%0, %1, %2, %3};"
+      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
+}
+
+// 16 bytes into shared memory, zeros unless `in`.
+__device__ __forceinline__ void cp16(double* dst, const double* src, bool in) {
+  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src),
+               "r"(in ? 16 : 0)
+               : "memory");
+}
+
+// X^T (W .* (X V)) over the rows of split blockIdx.y, 32 columns a CTA, into P + split *
+// Dp * n.  Per chunk of 64 rows: the logits' derivative tile L = (X V) .* W (a warp: 16
+// rows, 16 columns), then acc += X^T L (a warp: every fourth tile of 16 coordinates) -- X
+// is read once, L stays in shared memory and the sums over the rows in registers.  The FP64
+// tensor rate bounds it (2 N Dp n products; a warp loads 1 byte of shared memory a product,
+// half of what an MMA's time allows).  Row strides of 4 mod 16 doubles keep the fragments
+// conflict-free.  N = 2000, D = 64, n = 2048: 52 us (20 TFLOP/s; 55 with 8 x 8 x 4 MMAs),
+// against 62 for two DGEMMs, their split-k reduction, the product with W between them
+// and the axpby after.
+constexpr int kHvRows = 64, kHvCols = 32, kHvMaxDp = 128, kHvSL = kHvRows + 4;
+__host__ __device__ inline int hv_stride(int Dp) { return ((Dp + 15) / 16 * 16 + 11) / 16 * 16 + 4; }
+inline size_t hv_smem(int Dp) {
+  return 8 * (static_cast<size_t>(2 * kHvRows + kHvCols) * hv_stride(Dp) + kHvCols * kHvSL);
+}
+template <int ND>  // tiles of 16 coordinates a warp
+__global__ void __launch_bounds__(kTh)
+    hvp_kernel(const double* __restrict__ X, const double* __restrict__ W,
+               const double* __restrict__ V, int64_t N, int Dp, int64_t n,
+               double* __restrict__ P) {
+  extern __shared__ __align__(16) double sh[];
+  const int SX = hv_stride(Dp);
+  double* Xs = sh;                         // two chunks of rows
+  double* Vs = Xs + 2 * kHvRows * SX;      // the columns
+  double* Ls = Vs + kHvCols * SX;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r8 = lane >> 2, k4 = lane & 3;
+  const int64_t c0 = static_cast<int64_t>(blockIdx.x) * kHvCols;
+  const int64_t chunks = (N + kHvRows - 1) / kHvRows;
+  const int64_t ch0 = chunks * blockIdx.y / gridDim.y, ch1 = chunks * (blockIdx.y + 1) / gridDim.y;
+  const int h = Dp / 2;  // pairs a row
+  auto fetch = [&](int64_t ch) {
+    if (ch < ch1)
+      for (int i = tid; i < kHvRows * h; i += kTh) {
+        const int r = i / h, k = 2 * (i - r * h);
+        const int64_t row = ch * kHvRows + r;
+        cp16(Xs + ((ch & 1) * kHvRows + r) * SX + k, X + (row < N ? row : 0) * Dp + k, row < N);
+      }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int i = tid; i < kHvCols * h; i += kTh) {
+    const int c = i / h, k = 2 * (i - c * h);
+    cp16(Vs + c * SX + k, V + (c0 + c < n ? c0 + c : 0) * Dp + k, c0 + c < n);
+  }
+  fetch(ch0);
+  fetch(ch0 + 1);
+  const int m = warp % 4, cw = 16 * (warp / 4);  // the warp's 16 rows (and coordinates), 16 columns
+  double acc[ND][2][4] = {};
+  for (int64_t ch = ch0; ch < ch1; ++ch) {
+    double w[2][4];
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int64_t row = ch * kHvRows + 16 * m + 8 * (e / 2) + r8;
+        const int64_t c = c0 + cw + 8 * j + 2 * k4 + e % 2;
+        w[j][e] = row < N && c < n ? __ldg(W + c * N + row) : 0.0;
+      }
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();  // the chunk has arrived, the last one's L is read
+    const double* Xc = Xs + (ch & 1) * kHvRows * SX;
+    double l[2][4] = {};
+    {
+      const double* a = Xc + (16 * m + r8) * SX + k4;
+      const double* b = Vs + (cw + r8) * SX + k4;
+#pragma unroll 2
+      for (int k = 0; k < Dp; k += 8) {  // (Dp a multiple of 4: the last half step multiplies zeros)
+        const bool two = k + 4 < Dp;
+        double av[4], bv[2][2];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) av[i] = i < 2 || two ? a[8 * (i % 2) * SX + k + 4 * (i / 2)] : 0.0;
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int i = 0; i < 2; ++i) bv[j][i] = i == 0 || two ? b[8 * j * SX + k + 4 * i] : 0.0;
+        dmma(l[0], av, bv[0]);
+        dmma(l[1], av, bv[1]);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        Ls[(cw + 8 * j + 2 * k4 + e % 2) * kHvSL + 16 * m + 8 * (e / 2) + r8] = l[j][e] * w[j][e];
+    __syncthreads();
+    {
+      const double* a = Xc + k4 * SX + 16 * m + r8;
+      const double* b = Ls + (cw + r8) * kHvSL + k4;
+#pragma unroll 2
+      for (int k = 0; k < kHvRows; k += 8) {
+        double bv[2][2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int i = 0; i < 2; ++i) bv[j][i] = b[8 * j * kHvSL + k + 4 * i];
+#pragma unroll
+        for (int t = 0; t < ND; ++t)
+          if (16 * (m + 4 * t) < Dp) {
+            double av[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) av[i] = a[(k + 4 * (i / 2)) * SX + 64 * t + 8 * (i % 2)];
+            dmma(acc[t][0], av, bv[0]);
+            dmma(acc[t][1], av, bv[1]);
+          }
+      }
+    }
+    __syncthreads();  // this chunk's slot is free
+    fetch(ch + 2);
+  }
+  double* out = P + static_cast<size_t>(blockIdx.y) * Dp * n;
+#pragma unroll
+  for (int t = 0; t < ND; ++t)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int d = 16 * (m + 4 * t) + 8 * (e / 2) + r8;
+        const int64_t c = c0 + cw + 8 * j + 2 * k4 + e % 2;
+        if (d < Dp && c < n) out[c * Dp + d] = acc[t][j][e];
+      }
+}
+
+// A Hessian-vector product whose sum over the rows is in ns parts, `stride` apart:
+// -(P_0 + ... ) - tau v (ns = 0: the product itself).
+struct HvSum {
+  const double* P;
+  int ns;
+  size_t stride;
+  double tau;
+  __device__ __forceinline__ double at(size_t i, double v) const {
+    if (ns == 0) return P[i];
+    double s = P[i];
+    for (int k = 1; k < ns; ++k) s += P[k * stride + i];
+    return -s - tau * v;
+  }
+};
+__global__ void hvsum_kernel(HvSum h, const double* V, double* out, int64_t n) {
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x)
+    out[i] = h.at(i, V[i]);
 }
 
 // L .* W elementwise (N x T).
@@ -265,9 +423,9 @@ __global__ void diagj_kernel(double* __restrict__ DJ, int D, int Dp, int64_t T, 
 
 // The diagonal affine maps of one Jacobi iteration, time-reversed (row s holds
 // step t = T - 1 - s): lambda_t = a_t lambda_{t+1} + b_t.  HL column t is
-// H(x_t) lambda^k_{t+1} (t < T - 1).
+// H(x_t) lambda^k_{t+1} (t < T - 1), its parts summed here.
 __global__ void revmaps_kernel(const double* __restrict__ C, const double* __restrict__ LAM,
-                               const double* __restrict__ HL, const double* __restrict__ DJ,
+                               const HvSum HL, const double* __restrict__ DJ,
                                const double* __restrict__ sc, int Dp, int64_t T, double eps,
                                double* __restrict__ Ar, double* __restrict__ Br) {
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < T * Dp;
@@ -279,7 +437,7 @@ __global__ void revmaps_kernel(const double* __restrict__ C, const double* __res
       if (sc[8 * (t + 1) + 1] != 0.0) {
         const double dj = DJ[i + Dp], lk = LAM[i + Dp];
         a = dj;
-        b += lk + eps * HL[i] - dj * lk;
+        b += lk + eps * HL.at(i, lk) - dj * lk;
       } else {
         a = 1.0;
       }
@@ -290,10 +448,13 @@ __global__ void revmaps_kernel(const double* __restrict__ C, const double* __res
 }
 
 // LAM_new column t = Sr row T - 1 - t; per-block maxima of |new - old| and
-// |new| into part[2 * block .. ].
+// |new| into part[2 * block .. ], and over the blocks (in the last one to end, `left`
+// counts them and is 0 again after) into out.
 __global__ void revgather_kernel(const double* __restrict__ Sr, double* __restrict__ LAM,
-                                 int Dp, int64_t T, double* __restrict__ part) {
+                                 int Dp, int64_t T, double* __restrict__ part,
+                                 unsigned* __restrict__ left, double* __restrict__ out) {
   __shared__ double sd[kTh], sm[kTh];
+  __shared__ bool last;
   double md = 0.0, mx = 0.0;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < T * Dp;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -316,24 +477,59 @@ __global__ void revgather_kernel(const double* __restrict__ Sr, double* __restri
   if (threadIdx.x == 0) {
     part[2 * blockIdx.x] = sd[0];
     part[2 * blockIdx.x + 1] = sm[0];
+    __threadfence();
+    last = atomicAdd(left, 1u) == gridDim.x - 1;
   }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  md = mx = 0.0;
+  for (int b = threadIdx.x; b < static_cast<int>(gridDim.x); b += kTh) {
+    const double d = __ldcg(part + 2 * b), m = __ldcg(part + 2 * b + 1);
+    md = fmax(md, d);
+    mx = fmax(mx, m);
+  }
+  sd[threadIdx.x] = md;
+  sm[threadIdx.x] = mx;
+  __syncthreads();
+  for (int o = kTh / 2; o > 0; o >>= 1) {
+    if (threadIdx.x < o) {
+      sd[threadIdx.x] = fmax(sd[threadIdx.x], sd[threadIdx.x + o]);
+      sm[threadIdx.x] = fmax(sm[threadIdx.x], sm[threadIdx.x + o]);
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    out[0] = sd[0];
+    out[1] = sm[0];
+    *left = 0;
+  }
+}
+
+// sc[8 t + 7] = LAM_t . DY_t of the accepted columns (one warp a column; in the one block
+// that sums them, a thread a column, the uncoalesced reads took 130 us at T = 2048, D = 64).
+__global__ void lamdy_kernel(const double* __restrict__ LAM, const double* __restrict__ DY,
+                             double* __restrict__ sc, int Dp, int64_t T) {
+  const int lane = threadIdx.x & 31;
+  const int64_t t = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  if (t >= T) return;
+  double v = 0.0;
+  if (sc[8 * t + 1] != 0.0)
+    for (int d = lane; d < Dp; d += 32) v += LAM[t * Dp + d] * DY[t * Dp + d];
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (lane == 0) sc[8 * t + 7] = v;
 }
 
 // out[0] = sum_t direct_t / T (esjd) + sum_{t accepted} LAM_t . DY_t, in a
 // fixed order (one block).
-__global__ void final_kernel(const double* __restrict__ LAM, const double* __restrict__ DY,
-                             const double* __restrict__ sc, int Dp, int64_t T, int esjd,
+__global__ void final_kernel(const double* __restrict__ sc, int64_t T, int esjd,
                              double* __restrict__ out) {
   __shared__ double sh[kTh / 32];
   double s = 0.0;
   for (int64_t t = threadIdx.x; t < T; t += blockDim.x) {
     const double* st = sc + 8 * t;
     if (esjd) s += st[6] / static_cast<double>(T);
-    if (st[1] != 0.0) {
-      double v = 0.0;
-      for (int d = 0; d < Dp; ++d) v += LAM[t * Dp + d] * DY[t * Dp + d];
-      s += v;
-    }
+    s += st[7];
   }
   s = block_sum(s, sh);
   if (threadIdx.x == 0) out[0] = s;
@@ -362,7 +558,7 @@ AdjLayout adj_layout(int64_t N, int64_t Dp, int64_t T) {
   AdjLayout a{};
   a.v = static_cast<size_t>(Dp) * T;
   a.m = static_cast<size_t>(N) * T;
-  a.gpart = lga::grid_for(Dp * T);
+  a.gpart = std::min(148, lga::grid_for(Dp * T));  // (each ends with an atomic)
   const size_t t = static_cast<size_t>(T);
   a.total = 16 * r32(a.v) + 3 * r32(a.m) + 3 * r32(t) + r32(8 * t) +
             r32(2 * static_cast<size_t>(a.gpart)) + r32(8) + r32(static_cast<size_t>(Dp));
@@ -377,12 +573,28 @@ size_t lg_adjoint_ws_bytes(const LogisticDev& X, int64_t T) {
 
 namespace {
 
-// H(z) V for the columns [c0, c0 + n) of V against the W columns [w0, w0 + n):
-// out = -X^T (W .* (X V)) - tau V.
-int hvp(cudaStream_t s, cublasHandle_t cb, const LogisticDev& X, const double* W, const double* V,
-        int64_t n, double* L, double* out) {
+// -X^T (W .* (X V)) - tau V for n columns, `sum` its parts: up to kHvMaxDp coordinates by
+// hvp_kernel, the rows in as many splits as fill the chip and fit L (N x n), or in one into
+// `out`; above, where the products dominate, by two DGEMMs over L into `out`.
+int hvp_parts(cudaStream_t s, cublasHandle_t cb, const LogisticDev& X, const double* W,
+              const double* V, int64_t n, double* L, double* out, lga::HvSum* sum) {
   const double one = 1.0, zero = 0.0, mone = -1.0;
   const int N = static_cast<int>(X.N), dp = static_cast<int>(X.Dp), nc = static_cast<int>(n);
+  if (dp <= lga::kHvMaxDp) {
+    const int64_t tiles = (n + lga::kHvCols - 1) / lga::kHvCols;
+    const int64_t chunks = (X.N + lga::kHvRows - 1) / lga::kHvRows;
+    const int64_t slots = 148 * (dp <= 64 ? 2 : 1);
+    const int64_t ns =
+        std::max<int64_t>(1, std::min({slots / tiles, chunks, X.N / X.Dp, int64_t(16)}));
+    double* P = ns > 1 ? L : out;
+    const size_t smem = lga::hv_smem(dp);
+    auto k = dp <= 64 ? lga::hvp_kernel<1> : lga::hvp_kernel<2>;
+    if (raise_smem_limit(reinterpret_cast<const void*>(k), smem) != cudaSuccess) return 3;
+    k<<<dim3(static_cast<unsigned>(tiles), static_cast<unsigned>(ns)), lga::kTh, smem, s>>>(
+        X.X64, W, V, X.N, dp, n, P);
+    *sum = lga::HvSum{P, static_cast<int>(ns), static_cast<size_t>(X.Dp) * n, X.tau};
+    return cudaGetLastError() == cudaSuccess ? 0 : 3;
+  }
   if (cublasDgemm(cb, CUBLAS_OP_T, CUBLAS_OP_N, N, nc, dp, &one, X.X64, dp, V, dp, &zero, L, N) !=
       CUBLAS_STATUS_SUCCESS)
     return 3;
@@ -391,6 +603,17 @@ int hvp(cudaStream_t s, cublasHandle_t cb, const LogisticDev& X, const double* W
                   dp) != CUBLAS_STATUS_SUCCESS)
     return 3;
   lga::axpby_kernel<<<lga::grid_for(X.Dp * n), lga::kTh, 0, s>>>(out, 1.0, V, -X.tau, X.Dp * n);
+  *sum = lga::HvSum{out, 0, 0, 0.0};
+  return cudaGetLastError() == cudaSuccess ? 0 : 3;
+}
+
+// H(z) V in one array.
+int hvp(cudaStream_t s, cublasHandle_t cb, const LogisticDev& X, const double* W, const double* V,
+        int64_t n, double* L, double* out) {
+  lga::HvSum h{};
+  const int rc = hvp_parts(s, cb, X, W, V, n, L, out, &h);
+  if (rc || h.ns == 0) return rc;
+  lga::hvsum_kernel<<<lga::grid_for(X.Dp * n), lga::kTh, 0, s>>>(h, V, out, X.Dp * n);
   return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }
 
@@ -482,27 +705,27 @@ int lg_adjoint(cudaStream_t s, cublasHandle_t cb, const LogisticDev& X, bool f64
   double* Sr = V3;
   int k = 0;
   bool done = false;
-  std::vector<double> hp(2 * static_cast<size_t>(gpart));
+  unsigned* left = reinterpret_cast<unsigned*>(out + 4);
+  if (cudaMemsetAsync(left, 0, 8, s) != cudaSuccess) return 3;
   for (; k < max_iter && !done; ++k) {
     // HL column t = H(x_t) lambda^k_{t+1}: W column t + 1 (x_t = XB column t + 1)
-    if (T > 1 && hvp(s, cb, X, Wx + N, LAM + Dp, T - 1, Lb, HL)) return 3;
-    revmaps_kernel<<<gv, kTh, 0, s>>>(C, LAM, HL, DJ, sc, dp, T, eps, Ar, Br);
+    HvSum hl{HL, 0, 0, 0.0};
+    if (T > 1 && hvp_parts(s, cb, X, Wx + N, LAM + Dp, T - 1, Lb, HL, &hl)) return 3;
+    revmaps_kernel<<<gv, kTh, 0, s>>>(C, LAM, hl, DJ, sc, dp, T, eps, Ar, Br);
     if (cudaGetLastError() != cudaSuccess) return 3;
     const int rc = scan(scan_ctx, Dp, T, Ar, Br, s0, Sr);
     if (rc) return rc;
-    revgather_kernel<<<gpart, kTh, 0, s>>>(Sr, LAM, dp, T, part);
-    if (cudaMemcpyAsync(hp.data(), part, 8 * hp.size(), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+    revgather_kernel<<<gpart, kTh, 0, s>>>(Sr, LAM, dp, T, part, left, out);
+    double mm[2];
+    if (cudaMemcpyAsync(mm, out, sizeof mm, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess)
       return 3;
-    double md = 0.0, mx = 0.0;
-    for (int b = 0; b < gpart; ++b) {
-      md = std::fmax(md, hp[2 * b]);
-      mx = std::fmax(mx, hp[2 * b + 1]);
-    }
+    const double md = mm[0], mx = mm[1];
     if (!std::isfinite(md) || !std::isfinite(mx)) return 4;
     done = md <= 1e-12 * mx || mx == 0.0;
   }
-  final_kernel<<<1, kTh, 0, s>>>(LAM, DY, sc, dp, T, esjd, out);
+  lamdy_kernel<<<gw, kTh, 0, s>>>(LAM, DY, sc, dp, T);
+  final_kernel<<<1, kTh, 0, s>>>(sc, T, esjd, out);
   if (cudaMemcpyAsync(grad_eps, out, 8, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess)
     return 3;
