@@ -54,6 +54,8 @@ struct SliceState {
 
 constexpr size_t kCublasWsBytes = size_t(32) << 20;
 
+constexpr size_t kStateBytes = (sizeof(DevState) + 255) & ~size_t(255);
+
 struct pmcmc_handle {
   int device = 0;
   int num_sms = 148;
@@ -62,10 +64,10 @@ struct pmcmc_handle {
   std::string err;
   DevParams* d_params = nullptr;
   DevState* d_state = nullptr;
-  DevState* h_state = nullptr;  // pinned, then the states of two sweeps (h_sweep)
+  DevState* h_state = nullptr;  // pinned, then the states of two sweeps (h_sweep), h_scan_err
   DevState* h_sweep = nullptr;
-  uint32_t* d_bar = nullptr;   // grid_barrier's word of this handle's launches
-  int* h_scan_err = nullptr;   // pinned: a scan's barrier wait gave up
+  uint32_t* d_bar = nullptr;   // grid_barrier's word of this handle's launches, behind d_state
+  int* h_scan_err = nullptr;   // a scan's barrier wait gave up
   cudaEvent_t ev_sweep[2] = {nullptr, nullptr};  // sweep it & 1 of the logistic loop done
   unsigned char* ws = nullptr;
   size_t ws_bytes = 0;
@@ -1817,10 +1819,8 @@ int pmcmc_create(int device, void* stream, pmcmc_handle** out) {
     h->own_stream = true;
   }
   if (cudaMalloc(&h->d_params, sizeof(DevParams)) != cudaSuccess ||
-      cudaMalloc(&h->d_state, sizeof(DevState)) != cudaSuccess ||
-      cudaMallocHost(&h->h_state, 3 * sizeof(DevState)) != cudaSuccess ||
-      cudaMallocHost(&h->h_scan_err, 64) != cudaSuccess ||
-      cudaMalloc(&h->d_bar, 256) != cudaSuccess ||
+      cudaMalloc(&h->d_state, kStateBytes + 256) != cudaSuccess ||
+      cudaMallocHost(&h->h_state, 3 * sizeof(DevState) + 64) != cudaSuccess ||
       cudaMallocHost(&h->h_red, 4 * sizeof(unsigned long long)) != cudaSuccess ||
       cudaMalloc(&h->d_full, sizeof(FullArgs)) != cudaSuccess ||
       cudaMalloc(&h->d_params_e, sizeof(DevParams)) != cudaSuccess) {
@@ -1829,7 +1829,9 @@ int pmcmc_create(int device, void* stream, pmcmc_handle** out) {
     return PMCMC_ERR_NOMEM;
   }
   h->h_sweep = h->h_state + 1;
+  h->h_scan_err = reinterpret_cast<int*>(h->h_state + 3);
   *h->h_scan_err = 0;
+  h->d_bar = reinterpret_cast<uint32_t*>(reinterpret_cast<unsigned char*>(h->d_state) + kStateBytes);
   cudaMemset(h->d_bar, 0, 256);
   cudaMemset(h->d_state, 0, sizeof(DevState));
   cudaMemset(h->d_params, 0, sizeof(DevParams));
@@ -1886,8 +1888,6 @@ int pmcmc_destroy(pmcmc_handle* h) {
   cudaFree(h->d_params);
   cudaFree(h->d_state);
   if (h->h_state) cudaFreeHost(h->h_state);
-  if (h->h_scan_err) cudaFreeHost(h->h_scan_err);
-  cudaFree(h->d_bar);
   if (h->h_red) cudaFreeHost(h->h_red);
   for (cudaEvent_t e : h->ev)
     if (e) cudaEventDestroy(e);
