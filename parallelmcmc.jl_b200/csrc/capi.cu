@@ -830,7 +830,7 @@ int run_logistic(pmcmc_handle* h, const pmcmc_target* tg, const SweepKernels& k,
              : lg_margin(h->stream, f64, h->d_params, h->d_state, P.T, la_ref, &tb, kTieBand);
     CK(e);
     CK(lg_tie_solve(h->stream, tg->lg, h->d_params, h->d_state, la_ref, tb, kTieBand,
-                    fast ? G : nullptr, nsplit, h->num_sms));
+                    fast ? G : nullptr, nsplit, P.T, h->num_sms));
     return PMCMC_OK;
   };
   // the tensor-core error word travels with the state in every per-sweep copy

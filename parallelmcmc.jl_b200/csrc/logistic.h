@@ -84,7 +84,7 @@ cudaError_t lg_margin(cudaStream_t s, bool f64, const DevParams* dP, const DevSt
 // second pass's parts) their affine maps again by it.
 cudaError_t lg_tie_solve(cudaStream_t s, const LogisticDev& X, const DevParams* dP,
                          DevState* dS, double* la_ref, const TieBufs& b, float band,
-                         const float* G, int nsplit, int num_sms);
+                         const float* G, int nsplit, int64_t T, int num_sms);
 // Finish of a sweep on the tensor-core path with one probe (logistic_sweep.cu): every
 // column's log alpha and affine map (lg[3], lg[4]) from the second pass's G, the near-tie
 // columns listed; lp_parts: np parts of loglik(y) (summed into lpy).
