@@ -314,13 +314,12 @@ def run_ours(args):
         total_ms = float(t.item())
     value = world * args.steps * T / (total_ms / 1e3)
     iters = [i.iters for i in infos]
-    # kernels of ours a block: init; a sweep = 2 passes x (operand split, tensor-core
-    # pass, mid) + near-tie selection (margin, select, gather, 2 x loglik, propose,
-    # final) + the finish-and-scan sweep kernel; the verification the same without the
-    # sweep kernel plus the verify kernel; the logp pass (split, tensor-core pass);
-    # finalize.  cuBLAS DGEMMs of the near-tie columns are not counted.
-    per_sweep = 6 + 7 + 1
-    launches = sum(1 + per_sweep * i.iters + (6 + 7 + 1) + 2 + 1 for i in infos)
+    # kernels of ours a block: init; a sweep = tensor-core pass, mid, tensor-core pass,
+    # finish, near-tie solve, scan; the sweep launched ahead of the last one's check,
+    # whose kernels end at once; the verification = the first five and the verify kernel;
+    # the logp pass; finalize.
+    per_sweep = 6
+    launches = sum(1 + per_sweep * (i.iters + 1) + 6 + 1 + 1 for i in infos)
 
     # ---- end to end through the public API with host buffers: pmcmc.sample of one
     # block per step (x0 from pinned memory in, the chain's values, logp and accept
@@ -408,7 +407,7 @@ def run_ours(args):
     flops = 8.0 * N * D * T  # two GEMMs of 2 N D (2T) per contraction pass
     tpk = float(pk.get("bf16_tflops_sustained", pk["bf16_tflops"]))
     achieved = flops / (pass_ms / 1e3) / 1e12
-    kname = "logistic_pass_tc_kernel"
+    kname = "logistic_pass_kernel"
     roofline = {"bound": "tensor", "kernel": kname, "achieved": achieved, "peak": tpk,
                 "unit": "TFLOP/s", "frac": achieved / tpk, "traffic": traffic_of(kname, workload_name()),
                 "peak_source": f"{src}: bf16 dense, sustained (the pass runs inside a "
@@ -624,7 +623,7 @@ def run_secondary(args):
         flops = 8.0 * N * D * T  # two GEMMs of 2 N D (2T) per contraction pass
         tpk = float(pk.get("bf16_tflops_sustained", pk["bf16_tflops"]))
         achieved = flops / (pass_ms / 1e3) / 1e12
-        kname = "logistic_pass_tc_wide_kernel" if D > 256 else "logistic_pass_tc_kernel"
+        kname = "logistic_pass_kernel"
         line["roofline"] = {"bound": "tensor", "kernel": f"{kname} (+ mid kernel)",
                             "achieved": achieved, "peak": tpk, "unit": "TFLOP/s",
                             "frac": achieved / tpk, "peak_source": f"{src}, sustained",
@@ -638,11 +637,11 @@ def run_secondary(args):
         alg_bytes = 4 * T * (13 * Dq + 2 * D) + 9 * T
         achieved = alg_bytes / (sweep_ms / 1e3) / 1e9
         hbm = float(pk["hbm_gbs"])
-        line["roofline"] = {"bound": "hbm", "kernel": "full sweep (eval+chunk+carry+apply)",
+        line["roofline"] = {"bound": "hbm", "kernel": "full sweep (eval+chunk+group+carry+apply)",
                             "achieved": achieved, "peak": hbm, "unit": "GB/s",
                             "frac": achieved / hbm, "peak_source": src, "avg_sweep_ms": sweep_ms,
                             "alg_bytes_per_sweep": alg_bytes,
-                            "note": "latency-bound: the chunk, carry and replay recursions are sequential"}
+                            "note": "latency-bound: the chunk, group, carry and replay recursions are sequential"}
         sys.path.insert(0, os.path.join(ROOT, "oracle"))
         import oracle as O
         solve_dev(sampler, 1000)

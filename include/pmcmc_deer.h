@@ -59,8 +59,9 @@ typedef enum { PMCMC_MEM_HOST = 0, PMCMC_MEM_DEVICE = 1 } pmcmc_mem;
  * PMCMC_EXEC_FUSED: the product path.  Gaussian targets: a whole solve in one
  *   persistent launch, or one fused kernel per Newton sweep with the loop in a
  *   CUDA graph and a device-side convergence test.  Logistic targets: the
- *   tensor-core contraction passes and one fused finish-and-scan kernel per
- *   sweep, the state read by the host after each sweep.
+ *   tensor-core contraction passes, the FP64 decisions of near ties and the
+ *   scan of every sweep, launched one sweep ahead of the host's reading of
+ *   the state.
  * PMCMC_EXEC_PLAIN: the reference's structure on the GPU -- separate
  *   broadcast-style kernels, Hillis-Steele doubling scan, host-synchronised
  *   convergence check every iteration, FP32 SIMT only (the "plain GPU DEER"
@@ -375,7 +376,8 @@ int pmcmc_autotune(pmcmc_handle* h, const pmcmc_target* t, const pmcmc_deer_para
 /* ---- bound check of the device waits (no counterpart in the reference, whose
  * device code never waits on another block) ------------------------------------
  * Runs one of the library's bounded waits on a flag that nothing sets: the
- * look-back spin of the scans and sweeps (PMCMC_WAIT_LOOKBACK), or the
+ * look-back spin of the per-sweep kernel (PMCMC_WAIT_LOOKBACK; the grid barriers have the same
+ * bound), or the
  * mbarrier wait of the tensor-core pass (PMCMC_WAIT_MBARRIER).  The wait
  * gives up at its bound, the kernel returns normally and the call returns
  * PMCMC_ERR_TIMEOUT with the device time in *wait_ms; the handle and its

@@ -94,8 +94,8 @@ cudaError_t full_sweep(cudaStream_t s, const FullPlan& fp, const DevParams* Pg, 
 // Rao-Blackwellised squared jump (ESJD), 1 = mean |x_t|^2.  out[0] = dL/deps,
 // out[1 + i] = dL/dlog s_i for the covariance eigenvalues s_i = 1/lam_i
 // (objective 1 only; zeros for objective 0).
-// `scratch` holds full_adjoint_scratch_bytes(Dp, T) bytes; `epoch` must differ
-// from every earlier call on it.
+// `scratch` holds full_adjoint_scratch_bytes(Dp, T) bytes; `err` (pinned) is set when a wait of
+// the scan gives up.
 cudaError_t full_adjoint(cudaStream_t s, const DevParams* Pg, const FullArgs* Fg,
                          const FullArgs& Fh, int64_t D, int64_t Dp, int64_t T, int tkind,
                          int num_sms, int objective, const float* S, double* out,

@@ -1,6 +1,7 @@
 // tape_scan.cu -- tape materialisation and the standalone diagonal affine scan.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <mutex>
 #include <unordered_map>
@@ -52,8 +53,8 @@ cudaError_t launch_tape(cudaStream_t s, int64_t D, int64_t T, uint64_t seed, uin
 // Bound: HBM, one read of A and B and one write of S; phase 3's second read of A
 // and B comes from L2, which a launch's columns fit (scan_plan).  The look-back over
 // 64-column tiles that this replaces was a serial chain of T / 2048 hops: 471 us at
-// D = 100, T = 65536 in FP32 (78.6 MB), against 29 us here (2.7 TB/s; the floor is
-// 12 us, phase 2 and the barriers take 9).
+// D = 100, T = 65536 in FP32 (78.6 MB), against 21 us here (3.7 TB/s; the floor is
+// 12 us, phase 2 and the barriers take most of the rest).
 // States are carried by composition over at most 2048 columns at a time, as the
 // look-back did, so a coordinate that stays at zero under growing maps stays at
 // zero.  A cooperative launch's CTAs are co-resident, so the barriers end.
@@ -62,6 +63,9 @@ cudaError_t launch_tape(cudaStream_t s, int64_t D, int64_t T, uint64_t seed, uin
 // phase 2 is read from L2 each time, because the CTAs that already wait at the barrier
 // invalidate the SM's L1 with every poll
 constexpr int kScanCtas = 3;
+// Columns of a chunk, at least (us with 8, 16, 32, 64: D = 64, T = 2048 in FP64 8.8, 6.9, 7.1,
+// 7.9; D = 100, T = 8192 in FP32 10.6, 10.5, 8.5, 8.7; D = 256, T = 8192 13.2, 13.3, 10.6, 11.8).
+constexpr int kScanMinCols = 32;
 template <typename Real>
 constexpr int kScanLoads = 64 / sizeof(Real);  // columns of loads in flight a thread
 template <typename Real>
@@ -260,7 +264,7 @@ static cudaError_t scan_launches(cudaStream_t s, int64_t D, int64_t T, const Rea
   const int64_t nseg = (T + seg - 1) / seg, Tseg = (T + nseg - 1) / nseg;
   for (int64_t t0 = 0; t0 < T; t0 += Tseg) {
     int64_t Tn = imin64(Tseg, T - t0), Dn = D;
-    ScanPlan pl = scan_plan(D, Tn, max_ctas, scan_tile_cols(D, T), kScanGroup<Real>);
+    ScanPlan pl = scan_plan(D, Tn, max_ctas, std::max(kScanMinCols, scan_tile_cols(D, T)), kScanGroup<Real>);
     const Real *An = A + t0 * D, *Bn = B + t0 * D, *sn = t0 ? S + (t0 - 1) * D : s0;
     uint32_t* bar = static_cast<uint32_t*>(scratch);
     Real *Sn = S + t0 * D,
