@@ -15,6 +15,7 @@
 #include "deer_launch.h"
 #include "logistic.h"
 #include "logistic_column.cuh"
+#include "scan_phases.cuh"
 
 namespace pmcmc {
 
@@ -84,36 +85,18 @@ __global__ void __launch_bounds__(kThreads, 3)
   const int64_t u1 = imin64(c1, u0 + pl.Ls);
   if (tid == 0) s_bad = 0;
   float a = 1.f, b = 0.f;
-  if (active) {
-    const float *pa = A + u0 * Dp + d, *pb = B + u0 * Dp + d;
-    for (int n = static_cast<int>(u1 - u0); n > 0; n -= kLoads, pa += kLoads * Dp, pb += kLoads * Dp) {
-      float va[kLoads], vb[kLoads];
-#pragma unroll
-      for (int k = 0; k < kLoads; ++k) {
-        va[k] = k < n ? pa[k * Dp] : 1.f;
-        vb[k] = k < n ? pb[k * Dp] : 0.f;
-      }
-#pragma unroll
-      for (int k = 0; k < kLoads; ++k)
-        if (k < n) {
-          b = va[k] * b + vb[k];
-          a = va[k] * a;
-        }
-    }
-  }
+  if (active)
+    scan_compose_run<float, kLoads>(A + u0 * Dp + d, B + u0 * Dp + d, static_cast<int>(u1 - u0),
+                                    Dp, a, b);
   s_a[tid] = a;
   s_b[tid] = b;
   __syncthreads();
   float ea = 1.f, eb = 0.f;  // the chunk's earlier runs, composed
   if (active) {
-    for (int j = 0; j < sub; ++j) {
-      const float aj = s_a[j * pl.blk_d + dl], bj = s_b[j * pl.blk_d + dl];
-      eb = aj * eb + bj;
-      ea = aj * ea;
-    }
+    if (sub > 0) scan_earlier_runs<float>(s_a, s_b, pl.blk_d, dl, sub, ea, eb);
     if (sub == pl.nsub - 1) {
-      agg_a[ch * Dp + d] = a * ea;
-      agg_b[ch * Dp + d] = a * eb + b;
+      agg_a[ch * Dp + d] = sub > 0 ? a * ea : a;
+      agg_b[ch * Dp + d] = sub > 0 ? a * eb + b : b;
     }
   }
   const bool one = gridDim.x == 1;  // one chunk: its state is the entering one, no barrier
@@ -121,41 +104,9 @@ __global__ void __launch_bounds__(kThreads, 3)
     atomicCAS(&st->status, 0, static_cast<int>(kStTimeout));
   for (int dd = one ? Dp : (tid >> 5) * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x); dd < Dp;
        dd += static_cast<int>(blockDim.x >> 5) * static_cast<int>(gridDim.x)) {
-    float s = c_lo ? __ldcg(entry + dd) : x0[dd];
-    for (int base = 0; base < nch; base += 32 * pl.group) {
-      const int j0 = base + lane * pl.group;
-      float ra[kG], rb[kG];
-      float ga = 1.f, gb = 0.f;
-#pragma unroll
-      for (int k = 0; k < kG; ++k) {
-        const bool in = k < pl.group && j0 + k < nch;
-        ra[k] = in ? __ldcg(agg_a + (j0 + k) * Dp + dd) : 1.f;
-        rb[k] = in ? __ldcg(agg_b + (j0 + k) * Dp + dd) : 0.f;
-      }
-#pragma unroll
-      for (int k = 0; k < kG; ++k)
-        if (k < pl.group && j0 + k < nch) {
-          gb = ra[k] * gb + rb[k];
-          ga = ra[k] * ga;
-        }
-      __syncwarp();
-      s_a[tid] = ga;
-      s_b[tid] = gb;
-      __syncwarp();
-      float mine = s;
-      const int w0 = tid - lane;
-#pragma unroll 8
-      for (int l = 0; l < 32; ++l) {
-        s = s_a[w0 + l] * s + s_b[w0 + l];
-        if (l < lane) mine = s;
-      }
-#pragma unroll
-      for (int k = 0; k < kG; ++k)
-        if (k < pl.group && j0 + k < nch) {
-          carry[dd * nch + j0 + k] = mine;
-          mine = ra[k] * mine + rb[k];
-        }
-    }
+    const float s = scan_carry<float, kG>(nch, pl.group, agg_a, agg_b, Dp, dd,
+                                          c_lo ? __ldcg(entry + dd) : x0[dd], carry,
+                                          s_a + (tid & ~31), s_b + (tid & ~31));
     if (lane == 0) entry[dd] = s;
   }
   if (!one && !grid_barrier(P.grid_bar, gridDim.x))

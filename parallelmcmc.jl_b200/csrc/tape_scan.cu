@@ -8,6 +8,7 @@
 
 #include "deer_device.cuh"
 #include "deer_launch.h"
+#include "scan_phases.cuh"
 
 namespace pmcmc {
 
@@ -100,79 +101,28 @@ __global__ void __launch_bounds__(kThreads, kScanCtas)
     }
   };
   Real a = 1, b = 0;
-  if (active) {
-    const Real *pa = A + u0 * D + d, *pb = B + u0 * D + d;
-    for (int n = static_cast<int>(u1 - u0); n > 0;
-         n -= kScanUnroll, pa += kScanUnroll * Di, pb += kScanUnroll * Di) {
-      Real va[kScanUnroll], vb[kScanUnroll];
-      load(pa, pb, n, va, vb);
-#pragma unroll
-      for (int k = 0; k < kScanUnroll; ++k)
-        if (k < n) {
-          b = va[k] * b + vb[k];
-          a = va[k] * a;
-        }
-    }
-  }
+  if (active)
+    scan_compose_run<Real, kScanUnroll>(A + u0 * D + d, B + u0 * D + d,
+                                        static_cast<int>(u1 - u0), Di, a, b);
   s_a[tid] = a;
   s_b[tid] = b;
   __syncthreads();
-  // the maps of the chunk's earlier runs, composed
-  Real ea = 1, eb = 0;
+  Real ea = 1, eb = 0;  // the maps of the chunk's earlier runs, composed
   if (active) {
-    for (int j = 0; j < sub; ++j) {
-      const Real aj = s_a[j * pl.blk_d + dl], bj = s_b[j * pl.blk_d + dl];
-      eb = aj * eb + bj;
-      ea = aj * ea;
-    }
+    if (sub > 0) scan_earlier_runs<Real>(s_a, s_b, pl.blk_d, dl, sub, ea, eb);
     if (sub == pl.nsub - 1) {
-      agg_a[ch * D + d] = a * ea;
-      agg_b[ch * D + d] = a * eb + b;
+      agg_a[ch * D + d] = sub > 0 ? a * ea : a;
+      agg_b[ch * D + d] = sub > 0 ? a * eb + b : b;
     }
   }
   if (!grid_barrier(bar, gridDim.x)) atomicExch(err, 1);
   {
-    const int lane = tid & 31, nw = static_cast<int>(blockDim.x) >> 5;
-    constexpr int kG = kScanGroup<Real>;
+    // (the runs' maps in s_a and s_b were last read before the barrier)
+    const int w0 = tid & ~31, nw = static_cast<int>(blockDim.x) >> 5;
     for (int64_t dd = static_cast<int64_t>(tid >> 5) * gridDim.x + blockIdx.x; dd < D;
-         dd += static_cast<int64_t>(nw) * gridDim.x) {
-      Real st = s0[dd];
-      for (int base = 0; base < nch; base += 32 * pl.group) {
-        const int j0 = base + lane * pl.group;
-        Real ra[kG], rb[kG];
-        Real ga = 1, gb = 0;
-#pragma unroll
-        for (int k = 0; k < kG; ++k) {
-          const bool in = k < pl.group && j0 + k < nch;
-          ra[k] = in ? __ldcg(agg_a + (j0 + k) * D + dd) : Real(1);
-          rb[k] = in ? __ldcg(agg_b + (j0 + k) * D + dd) : Real(0);
-        }
-#pragma unroll
-        for (int k = 0; k < kG; ++k)
-          if (k < pl.group && j0 + k < nch) {
-            gb = ra[k] * gb + rb[k];
-            ga = ra[k] * ga;
-          }
-        __syncwarp();
-        s_a[tid] = ga;  // (the runs' maps were last read before the barrier)
-        s_b[tid] = gb;
-        __syncwarp();
-        Real mine = st;  // state entering this lane's group
-        const int w0 = tid - lane;
-#pragma unroll 8
-        for (int l = 0; l < 32; ++l) {  // identity maps past the last group
-          const Real al = s_a[w0 + l], bl = s_b[w0 + l];
-          st = al * st + bl;
-          if (l < lane) mine = st;
-        }
-#pragma unroll
-        for (int k = 0; k < kG; ++k)
-          if (k < pl.group && j0 + k < nch) {
-            carry[dd * nch + j0 + k] = mine;
-            mine = ra[k] * mine + rb[k];
-          }
-      }
-    }
+         dd += static_cast<int64_t>(nw) * gridDim.x)
+      scan_carry<Real, kScanGroup<Real>>(nch, pl.group, agg_a, agg_b, D, dd, s0[dd], carry,
+                                         s_a + w0, s_b + w0);
   }
   if (!grid_barrier(bar, gridDim.x)) atomicExch(err, 1);
   if (active && u0 < u1) {
