@@ -217,16 +217,14 @@ __global__ void __launch_bounds__(kTieThreads, kTieCtas)
           const double z = c[h][i];
           const double e = exp(-fabs(z));
           const double p = (z >= 0.0 ? 1.0 : e) / (1.0 + e);
-          double term = row < N ? lab * z - (z > 0.0 ? z : 0.0) : 0.0;
-          double prod = row < N ? 1.0 + e : 1.0;  // one log for the 8 rows
+          // lab z - softplus(z), without the cancellation where lab = 1 and z > 0
+          const double zn = lab != 0.0 ? -z : z;
+          double term = row < N ? -((zn > 0.0 ? zn : 0.0) + log1p(e)) : 0.0;
 #pragma unroll
-          for (int o = 4; o < 32; o <<= 1) {
-            term += __shfl_xor_sync(0xffffffffu, term, o);
-            prod *= __shfl_xor_sync(0xffffffffu, prod, o);
-          }
+          for (int o = 4; o < 32; o <<= 1) term += __shfl_xor_sync(0xffffffffu, term, o);
           if (col < cnt) {
             a.R[static_cast<int64_t>(col) * a.Nr + row] = row < N ? lab - p : 0.0;
-            if (r8 == 0) a.lpP[row0 / 8 * kmax + col] = term - log(prod);
+            if (r8 == 0) a.lpP[row0 / 8 * kmax + col] = term;
           }
         }
       }
