@@ -174,6 +174,20 @@ struct DeviceGuard {
   }
 };
 
+// What a pinned state holds until the kernel that is to write it has: a kernel that does not
+// run to its end (a bounded wait gave up ahead of it) must not leave the state of an earlier
+// solve there.
+DevState unwritten_state() {
+  DevState s{};
+  s.status = kStTimeout;
+  return s;
+}
+
+// Clears the grid barrier's word, which a wait that gave up leaves mid-phase.
+void reset_barrier(pmcmc_handle* h) {
+  cudaMemsetAsync(h->d_bar, 0, sizeof(uint32_t), h->stream);
+}
+
 int ensure_ws(pmcmc_handle* h, size_t bytes) {
   if (bytes <= h->ws_bytes) return PMCMC_OK;
   if (h->ws) {
@@ -1292,10 +1306,9 @@ void fill_info(const DevState& s, pmcmc_info* info) {
 }
 
 int status_error(pmcmc_handle* h, int status) {
-  if (status == kStTimeout) {
-    cudaMemsetAsync(h->d_bar, 0, sizeof(uint32_t), h->stream);  // a barrier given up mid-phase
+  if (status) reset_barrier(h);  // (a block after the failed one may have timed out)
+  if (status == kStTimeout)
     return fail(h, PMCMC_ERR_TIMEOUT, "a device wait (look-back or grid barrier) exceeded its bound");
-  }
   if (status == kStNonfinite)
     return fail(h, PMCMC_ERR_NONFINITE, "non-finite value in the DEER trajectory");
   return PMCMC_OK;
@@ -1521,6 +1534,8 @@ int solve_core(pmcmc_handle* h, const pmcmc_target* tg, const pmcmc_deer_params*
     if (persist) {
       P.x0_src = (b == 0 && mem == PMCMC_MEM_DEVICE) ? x0 : P.x0;
       P.st_host = defer ? h->h_states + b : h->h_state;  // written by the kernel
+      // (all that a block which a barrier wait that gave up kept from running leaves there)
+      for (int64_t i = 0; i < (batch ? nblocks : 1); ++i) P.st_host[i] = unwritten_state();
     }
     if (mem == PMCMC_MEM_DEVICE) {
       P.S_out = static_cast<unsigned char*>(S_out) + es * nsteps * D;

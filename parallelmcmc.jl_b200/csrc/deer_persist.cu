@@ -139,15 +139,22 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL>)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   if (threadIdx.x == 0) P = Pv;  // parameters by value: no upload before the launch
   __syncthreads();
-  // one CTA (small blocks): its own barrier
+  // this sweep's maxima max|dS|, max|S| and the non-finite flag, as ordered bits of
+  // non-negative doubles, in two slots by sweep parity (P.part[0..5]), and whether a CTA's
+  // barrier wait gave up (P.part[6])
+  unsigned long long* red = reinterpret_cast<unsigned long long*>(P.part);
+  // One CTA (small blocks): its own barrier.  A CTA whose wait gives up publishes it and
+  // arrives at no further barrier (its phases would pair wrongly with the others'), so the
+  // others' next waits end at their bound too and every CTA leaves with the timeout status.
   bool gave_up = false;
   auto all_sync = [&]() {
-    if (gridDim.x == 1) __syncthreads();
-    else if (!grid_barrier(P.grid_bar, gridDim.x)) gave_up = true;
+    if (gridDim.x == 1 || gave_up) {
+      __syncthreads();
+    } else if (!grid_barrier(P.grid_bar, gridDim.x)) {
+      gave_up = true;
+      if (threadIdx.x == 0) atomicExch(red + 6, 1ull);
+    }
   };
-  // this sweep's maxima max|dS|, max|S| and the non-finite flag, as ordered
-  // bits of non-negative doubles, in two slots by sweep parity (P.part[0..5])
-  unsigned long long* red = reinterpret_cast<unsigned long long*>(P.part);
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr bool kDense = TK == kDenseGauss;
@@ -191,7 +198,7 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL>)
     // the arrival counter and the sweep maxima (the grid barriers in between
     // order these resets before every update, and after the previous block's reads)
     if (cta == 0 && tid == 0) {
-      for (int i = 0; i < 6; ++i) red[i] = 0ull;
+      for (int i = 0; i < 7; ++i) red[i] = 0ull;
       st->fin_counter = 0;
       st->n_accept = 0;
       st->min_margin_bits = dbits(INFINITY);
@@ -292,8 +299,9 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL>)
       const bool nonfinite = __ldcg(sl + 2) != 0ull;
       metric = dmax / (P.tol_abs + P.tol_rel * smax);
       converged = metric <= 1.0;
-      status = gave_up ? static_cast<int>(kStTimeout)
-               : nonfinite ? static_cast<int>(kStNonfinite) : 0;
+      status = gave_up || __ldcg(red + 6) != 0ull ? static_cast<int>(kStTimeout)
+               : nonfinite                        ? static_cast<int>(kStNonfinite)
+                                                  : 0;
       const bool stop = converged || iter >= P.maxiter || status != 0;
       if (stop && cta > 0 && tid < Dp) sprev = __ldcg(Sb + (t0 - 1) * Dp + tid);
       return stop;
@@ -662,7 +670,7 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL>)
         f.epoch = st->epoch;  // look-back epochs of the per-sweep path continue
         f.iter = iter;
         f.converged = converged;
-        f.status = status;
+        f.status = __ldcg(red + 6) != 0ull ? static_cast<int>(kStTimeout) : status;
         f.metric = metric;
         f.n_accept = __ldcg(tot);
         f.min_margin_bits = __ldcg(&st->min_margin_bits);
@@ -675,8 +683,12 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL>)
       }
     }
     // the next block starts from this block's last column (x_next) once every
-    // CTA has finished this one
-    if (bi + 1 < nblk) all_sync();
+    // CTA has finished this one (after a wait that gave up none does: the states of the
+    // blocks that never ran keep the timeout status that the host put there)
+    if (bi + 1 < nblk) {
+      all_sync();
+      if (nctas > 1 && (gave_up || __ldcg(red + 6) != 0ull)) break;
+    }
   }  // blocks
 }
 
