@@ -376,13 +376,20 @@ int pmcmc_autotune(pmcmc_handle* h, const pmcmc_target* t, const pmcmc_deer_para
 /* ---- bound check of the device waits (no counterpart in the reference, whose
  * device code never waits on another block) ------------------------------------
  * Runs one of the library's bounded waits on a flag that nothing sets: the
- * look-back spin of the per-sweep kernel (PMCMC_WAIT_LOOKBACK; the grid barriers have the same
- * bound), or the
- * mbarrier wait of the tensor-core pass (PMCMC_WAIT_MBARRIER).  The wait
+ * look-back spin of the per-sweep kernel (PMCMC_WAIT_LOOKBACK), the mbarrier
+ * wait of the tensor-core pass (PMCMC_WAIT_MBARRIER), the grid barrier of the
+ * persistent solve, the scans and the near ties (PMCMC_WAIT_GRID_BARRIER, on
+ * the handle's own barrier word), or the two-CTA pass's wait for its peer's
+ * message (PMCMC_WAIT_MAILBOX).  The wait
  * gives up at its bound, the kernel returns normally and the call returns
  * PMCMC_ERR_TIMEOUT with the device time in *wait_ms; the handle and its
  * context stay usable.  PMCMC_OK would mean the wait ended without its flag. */
-typedef enum { PMCMC_WAIT_LOOKBACK = 0, PMCMC_WAIT_MBARRIER = 1 } pmcmc_wait_kind;
+typedef enum {
+  PMCMC_WAIT_LOOKBACK = 0,
+  PMCMC_WAIT_MBARRIER = 1,
+  PMCMC_WAIT_GRID_BARRIER = 2,
+  PMCMC_WAIT_MAILBOX = 3
+} pmcmc_wait_kind;
 int pmcmc_check_wait_bound(pmcmc_handle* h, int32_t kind, double* wait_ms);
 
 #ifdef __cplusplus

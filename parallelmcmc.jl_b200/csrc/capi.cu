@@ -1935,8 +1935,8 @@ int pmcmc_get_profile(pmcmc_handle* h, pmcmc_profile* out, int32_t reset) {
 
 int pmcmc_check_wait_bound(pmcmc_handle* h, int32_t kind, double* wait_ms) {
   if (!h) return PMCMC_ERR_ARGUMENT;
-  if (kind != PMCMC_WAIT_LOOKBACK && kind != PMCMC_WAIT_MBARRIER)
-    return fail(h, PMCMC_ERR_ARGUMENT, "kind must be PMCMC_WAIT_LOOKBACK or PMCMC_WAIT_MBARRIER");
+  if (kind < PMCMC_WAIT_LOOKBACK || kind > PMCMC_WAIT_MAILBOX)
+    return fail(h, PMCMC_ERR_ARGUMENT, "kind must be a pmcmc_wait_kind");
   DeviceGuard guard(h->device);
   struct Scratch {
     void* buf = nullptr;
@@ -1954,11 +1954,21 @@ int pmcmc_check_wait_bound(pmcmc_handle* h, int32_t kind, double* wait_ms) {
   int* err = reinterpret_cast<int*>(static_cast<char*>(sc.buf) + 128);  // out
   CK(cudaMemsetAsync(sc.buf, 0, 256, h->stream));
   CK(cudaEventRecord(sc.ev[0], h->stream));
-  if (kind == PMCMC_WAIT_LOOKBACK)
+  const char* name = "look-back";
+  if (kind == PMCMC_WAIT_LOOKBACK) {
     CK(launch_lookback_bound(h->stream, flags, err));
-  else
+  } else if (kind == PMCMC_WAIT_MBARRIER) {
+    name = "mbarrier";
     CK(lg_tc_mbar_bound(h->stream, err));
+  } else if (kind == PMCMC_WAIT_GRID_BARRIER) {
+    name = "grid barrier";
+    CK(launch_barrier_bound(h->stream, h->d_bar, err));
+  } else {
+    name = "mailbox";
+    CK(lg_tc_mail_bound(h->stream, err));
+  }
   CK(cudaEventRecord(sc.ev[1], h->stream));
+  if (kind == PMCMC_WAIT_GRID_BARRIER) reset_barrier(h);  // as after a solve that timed out
   int gave_up = 0;
   CK(cudaMemcpyAsync(&gave_up, err, sizeof gave_up, cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
@@ -1966,8 +1976,7 @@ int pmcmc_check_wait_bound(pmcmc_handle* h, int32_t kind, double* wait_ms) {
   CK(cudaEventElapsedTime(&ms, sc.ev[0], sc.ev[1]));
   if (wait_ms) *wait_ms = ms;
   if (!gave_up) return PMCMC_OK;
-  return fail(h, PMCMC_ERR_TIMEOUT, "%s wait reached its bound after %.1f ms",
-              kind == PMCMC_WAIT_LOOKBACK ? "look-back" : "mbarrier", ms);
+  return fail(h, PMCMC_ERR_TIMEOUT, "%s wait reached its bound after %.1f ms", name, ms);
 }
 
 int pmcmc_target_diag_gauss(pmcmc_handle* h, int64_t D, const double* mean, const double* prec,

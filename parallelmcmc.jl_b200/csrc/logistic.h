@@ -59,6 +59,8 @@ int lg_tc_split(const LogisticDev& X, int64_t T);  // parts of G that a pass wri
 // One bounded mbarrier wait that nothing completes (bound check); err[0] = 1
 // when it gave up.
 cudaError_t lg_tc_mbar_bound(cudaStream_t s, int* err);
+// The same for the wait of the two-CTA pass on a message of its peer.
+cudaError_t lg_tc_mail_bound(cudaStream_t s, int* err);
 
 // Near-tie decisions in FP64 and the verification pass (logistic_tie.cu).
 // Scratch of one refinement over at most kmax columns.

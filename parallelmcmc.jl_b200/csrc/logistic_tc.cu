@@ -786,6 +786,22 @@ __global__ void mbar_bound_kernel(int* err) {
   if (threadIdx.x == 0) err[0] = mbar_wait(&bar, 0, &s_err) ? 0 : 1;
 }
 
+// The same for Mail::wait: a warp waits for a message that its peer never sends.
+__global__ void mail_bound_kernel(int* err) {
+  __shared__ __align__(8) uint64_t bar[2];
+  __shared__ __align__(16) unsigned char box[kMail];
+  __shared__ int s_err;
+  if (threadIdx.x == 0) {
+    s_err = 0;
+    mbar_init(bar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  const Mail mail(box, bar, 0);
+  const bool got = mail.wait(0, 0, 1024, &s_err);
+  if (threadIdx.x == 0) err[0] = got ? 0 : 1;
+}
+
 }  // namespace tc
 
 
@@ -910,6 +926,11 @@ int lg_tc_pass(cudaStream_t s, const LogisticDev& X, const DevParams* dP, const 
 
 cudaError_t lg_tc_mbar_bound(cudaStream_t s, int* err) {
   tc::mbar_bound_kernel<<<1, 32, 0, s>>>(err);
+  return cudaGetLastError();
+}
+
+cudaError_t lg_tc_mail_bound(cudaStream_t s, int* err) {
+  tc::mail_bound_kernel<<<1, 32, 0, s>>>(err);
   return cudaGetLastError();
 }
 

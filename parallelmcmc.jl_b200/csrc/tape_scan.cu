@@ -374,7 +374,7 @@ cudaError_t launch_broadcast(cudaStream_t s, bool f64, int64_t Dp, int64_t T, co
 // Bound check of the look-back wait: one warp looks back from tile 1 over a
 // flag array that nothing publishes (all zeros: no epoch, no state), so lane 0
 // spins on tile 0 until kMaxSpins and the warp reports the give-up in err[0].  The same
-// routine guards every scan and sweep launch.
+// routine guards the per-sweep kernel.
 __global__ void lookback_bound_kernel(const uint32_t* flags, int* err) {
   int e = 0;
   lookback_fixed(1, 1u, flags, &e);
@@ -383,6 +383,18 @@ __global__ void lookback_bound_kernel(const uint32_t* flags, int* err) {
 
 cudaError_t launch_lookback_bound(cudaStream_t s, const uint32_t* flags, int* err) {
   lookback_bound_kernel<<<1, 32, 0, s>>>(flags, err);
+  return cudaGetLastError();
+}
+
+// Bound check of the grid barrier (the persistent solve, the scans, the near ties): one CTA
+// arrives at a barrier of two.
+__global__ void barrier_bound_kernel(uint32_t* bar, int* err) {
+  const bool met = grid_barrier(bar, 2);
+  if (threadIdx.x == 0) err[0] = met ? 0 : 1;
+}
+
+cudaError_t launch_barrier_bound(cudaStream_t s, uint32_t* bar, int* err) {
+  barrier_bound_kernel<<<1, kThreads, 0, s>>>(bar, err);
   return cudaGetLastError();
 }
 

@@ -31,7 +31,7 @@ SYMBOLS = [
     "pmcmc_mala_chains_adaptive",
 ]
 OBJECTIVE = {"esjd": 0, "mean_sq": 1}
-WAIT_KIND = {"lookback": 0, "mbarrier": 1}
+WAIT_KIND = {"lookback": 0, "mbarrier": 1, "grid_barrier": 2, "mailbox": 3}
 
 
 class ArgumentError(ValueError):
@@ -199,8 +199,8 @@ class Handle:
         return {k: getattr(p, k) for k, _ in p._fields_}
 
     def check_wait_bound(self, kind: str = "lookback") -> dict:
-        """Run one of the library's bounded device waits ("lookback" or
-        "mbarrier") on a flag that nothing sets.  A working bound returns
+        """Run one of the library's bounded device waits ("lookback", "mbarrier",
+        "grid_barrier" or "mailbox") on a flag that nothing sets.  A working bound returns
         status ERR_TIMEOUT with the device time the wait took; the handle
         stays usable afterwards."""
         if kind not in WAIT_KIND:
