@@ -919,6 +919,8 @@ int run_logistic(pmcmc_handle* h, const pmcmc_target* tg, const SweepKernels& k,
     if (h->profiling) CK(cudaEventRecord(h->ev[0], h->stream));
     const int rc = tie();
     if (rc) return rc;
+    // (lg_scan writes no state where a wait of the near ties gave up ahead of it)
+    h->h_sweep[it & 1] = unwritten_state();
     CK(lg_scan(h->stream, h->d_params, h->d_state, P.Dp, P.T, ws + L.lgscan,
                h->h_sweep + (it & 1), h->num_sms));
     CK(cudaEventRecord(h->ev_sweep[it & 1], h->stream));
