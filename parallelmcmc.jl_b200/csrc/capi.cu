@@ -2706,6 +2706,13 @@ int slice_scan(pmcmc_handle* h, const void* B, const void* s0, void* out) {
   return PMCMC_OK;
 }
 
+// After a synchronisation: whether a slice's scan gave up a barrier wait.
+int slice_scan_error(pmcmc_handle* h) {
+  if (!*h->h_scan_err) return PMCMC_OK;
+  cudaMemsetAsync(h->ws + h->slice.scr, 0, kScanBarBytes, h->stream);  // left mid-phase
+  return fail(h, PMCMC_ERR_TIMEOUT, "slice scan barrier wait exceeded its bound");
+}
+
 }  // namespace
 
 int pmcmc_slice_begin(pmcmc_handle* h, const pmcmc_target* tg, const pmcmc_deer_params* p,
@@ -2847,9 +2854,7 @@ int pmcmc_slice_local(pmcmc_handle* h, const void* xbar0, void* agg, int32_t mem
   rc = slice_copy_out(h, out, ws + sl.Sloc + es * (W - 1) * Dp, es * D, mem);
   if (rc) return rc;
   CK(cudaStreamSynchronize(h->stream));
-  if (*h->h_scan_err)
-    return fail(h, PMCMC_ERR_TIMEOUT, "slice scan barrier wait exceeded its bound");
-  return PMCMC_OK;
+  return slice_scan_error(h);
 }
 
 int pmcmc_slice_finish(pmcmc_handle* h, const void* carry_in, void* last_out, double* red,
@@ -2878,8 +2883,8 @@ int pmcmc_slice_finish(pmcmc_handle* h, const void* carry_in, void* last_out, do
   unsigned long long hr[3] = {0, 0, 0};
   CK(cudaMemcpyAsync(hr, r, sizeof hr, cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
-  if (*h->h_scan_err)
-    return fail(h, PMCMC_ERR_TIMEOUT, "slice scan barrier wait exceeded its bound");
+  rc = slice_scan_error(h);
+  if (rc) return rc;
   std::memcpy(&red[0], &hr[0], 8);
   std::memcpy(&red[1], &hr[1], 8);
   sl.cur ^= 1;

@@ -7,13 +7,15 @@
 // memory budget), or a latency-critical loop that cannot afford the implicit
 // device synchronisation of an allocation.  pmcmc_affine_scan_diag_noalloc
 // serves them: the caller passes device inputs and outputs, and the scan's
-// scratch (the chunks' maps and states) lives in the file-scope array below instead of a handle's workspace.  No cudaMalloc,
+// scratch (the barrier's word, the chunks' maps and states) lives in the
+// file-scope array below instead of a handle's workspace.  No cudaMalloc,
 // cudaFree or allocating library routine is called.
 //
 // The array is kPmcmcNoallocScratchBytes (4 MiB) on every GPU that loads the
 // library, held until the process exits.  It is shared by all calls on a
-// device, and each call writes what it reads there; calls that overlap on the GPU (different streams, or several host threads)
-// race on the array and must be serialised by the caller.  The array's memory
+// device; each call clears the barrier's word and writes what else it reads
+// there.  Calls that overlap on the GPU (different streams, or several host
+// threads) race on the array and must be serialised by the caller.  The array's memory
 // is taken when the module is loaded on a device, which under lazy loading is
 // the first call there: callers that give every free byte to their own pool
 // make one small call first.
@@ -81,10 +83,11 @@ extern "C" int pmcmc_affine_scan_diag_noalloc(int32_t dtype, int64_t D, int64_t 
   const int rc = scratch_for_current_device(&base);
   if (rc) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // the barrier's word is the array's first, the error flag follows it
+  // the barrier's word is the array's first, the error flag follows it; both are cleared, so
+  // that a wait that gave up, or calls that overlapped, leave nothing to the next call
   int* err = static_cast<int*>(base) + 1;
   int flag = 0;
-  if (cudaMemsetAsync(err, 0, sizeof flag, s) != cudaSuccess ||
+  if (cudaMemsetAsync(base, 0, pmcmc::kScanBarBytes, s) != cudaSuccess ||
       pmcmc::launch_affine_scan(s, f64, D, T, A, B, s0, S, base, err) != cudaSuccess ||
       cudaMemcpyAsync(&flag, err, sizeof flag, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess) {
