@@ -274,8 +274,8 @@ int pmcmc_slice_result(pmcmc_handle* h, const void* xbar0, void* S_out, void* lo
 
 /* ---- diagonal affine scan ----------------------------------------------------
  * Replaces DEERScan.solve_affine_scan_diag! (src/DEER/DEERScan.jl:102-173):
- * S[:,t] = A[:,t] .* S[:,t-1] + B[:,t], S[:,0-1] = s0.  One
- * cooperative launch (a few for long scans).  S may not alias A or B (DEERScan.jl:124-125). */
+ * S[:,t] = A[:,t] .* S[:,t-1] + B[:,t], S[:,0-1] = s0.  One launch
+ * (a few for long scans).  S may not alias A or B (DEERScan.jl:124-125). */
 int pmcmc_affine_scan_diag(pmcmc_handle* h, int32_t dtype, int64_t D, int64_t T, const void* A,
                            const void* B, const void* s0, void* S, int32_t mem);
 

@@ -100,6 +100,10 @@ __global__ void __launch_bounds__(kThreads, kScanCtas)
       vb[k] = k < n ? pb[k * Di] : Real(0);
     }
   };
+  // One chunk: its entering state is s0, nothing to carry and no other CTA to wait for (one
+  // warp a coordinate carried 256 of them in turn: 62 us a call at D = 256, T = 8, 35 so).
+  const bool one = nch == 1;
+  const Real st0 = one && active ? s0[d] : Real(0);
   Real a = 1, b = 0;
   if (active)
     scan_compose_run<Real, kScanUnroll>(A + u0 * D + d, B + u0 * D + d,
@@ -110,23 +114,23 @@ __global__ void __launch_bounds__(kThreads, kScanCtas)
   Real ea = 1, eb = 0;  // the maps of the chunk's earlier runs, composed
   if (active) {
     if (sub > 0) scan_earlier_runs<Real>(s_a, s_b, pl.blk_d, dl, sub, ea, eb);
-    if (sub == pl.nsub - 1) {
+    if (sub == pl.nsub - 1 && !one) {
       agg_a[ch * D + d] = sub > 0 ? a * ea : a;
       agg_b[ch * D + d] = sub > 0 ? a * eb + b : b;
     }
   }
-  if (!grid_barrier(bar, gridDim.x)) atomicExch(err, 1);
-  {
+  if (!one) {
+    if (!grid_barrier(bar, gridDim.x)) atomicExch(err, 1);
     // (the runs' maps in s_a and s_b were last read before the barrier)
     const int w0 = tid & ~31, nw = static_cast<int>(blockDim.x) >> 5;
     for (int64_t dd = static_cast<int64_t>(tid >> 5) * gridDim.x + blockIdx.x; dd < D;
          dd += static_cast<int64_t>(nw) * gridDim.x)
       scan_carry<Real, kScanGroup<Real>>(nch, pl.group, agg_a, agg_b, D, dd, s0[dd], carry,
                                          s_a + w0, s_b + w0);
+    if (!grid_barrier(bar, gridDim.x)) atomicExch(err, 1);
   }
-  if (!grid_barrier(bar, gridDim.x)) atomicExch(err, 1);
   if (active && u0 < u1) {
-    Real st = __ldcg(carry + d * nch + ch);
+    Real st = one ? st0 : __ldcg(carry + d * nch + ch);
     if (sub > 0) st = ea * st + eb;
     const Real *pa = A + u0 * D + d, *pb = B + u0 * D + d;
     Real* ps = S + u0 * D + d;
@@ -214,15 +218,18 @@ static cudaError_t scan_launches(cudaStream_t s, int64_t D, int64_t T, const Rea
   const int64_t nseg = (T + seg - 1) / seg, Tseg = (T + nseg - 1) / nseg;
   for (int64_t t0 = 0; t0 < T; t0 += Tseg) {
     int64_t Tn = imin64(Tseg, T - t0), Dn = D;
-    ScanPlan pl = scan_plan(D, Tn, max_ctas, std::max(kScanMinCols, scan_tile_cols(D, T)), kScanGroup<Real>);
+    ScanPlan pl = scan_plan(D, Tn, max_ctas, std::max(kScanMinCols, scan_tile_cols(D, T)),
+                            kScanGroup<Real>);
     const Real *An = A + t0 * D, *Bn = B + t0 * D, *sn = t0 ? S + (t0 - 1) * D : s0;
     uint32_t* bar = static_cast<uint32_t*>(scratch);
-    Real *Sn = S + t0 * D,
-         *aa = reinterpret_cast<Real*>(static_cast<unsigned char*>(scratch) + kScanBarBytes), *ab = aa + static_cast<size_t>(pl.nchunks) * D,
+    Real* Sn = S + t0 * D;
+    Real* aa = reinterpret_cast<Real*>(static_cast<unsigned char*>(scratch) + kScanBarBytes);
+    Real *ab = aa + static_cast<size_t>(pl.nchunks) * D,
          *ca = ab + static_cast<size_t>(pl.nchunks) * D;
     void* args[] = {&Dn, &Tn, &pl, &An, &Bn, &sn, &Sn, &aa, &ab, &ca, &bar, &err};
-    e = cudaLaunchCooperativeKernel(fn, dim3(pl.nchunks * pl.nblk_d), dim3(pl.threads), args, 0,
-                                    s);
+    const dim3 grid(pl.nchunks * pl.nblk_d), threads(pl.threads);
+    e = pl.nchunks == 1 ? cudaLaunchKernel(fn, grid, threads, args, 0, s)
+                        : cudaLaunchCooperativeKernel(fn, grid, threads, args, 0, s);
     if (e != cudaSuccess) return e;
   }
   return cudaGetLastError();
