@@ -66,7 +66,7 @@ struct pmcmc_handle {
   DevState* d_state = nullptr;
   DevState* h_state = nullptr;  // pinned, then the states of two sweeps (h_sweep), h_scan_err
   DevState* h_sweep = nullptr;
-  uint32_t* d_bar = nullptr;   // grid_barrier's word of this handle's launches, behind d_state
+  uint32_t* d_bar = nullptr;   // grid barrier's two words of this handle's launches, behind d_state
   int* h_scan_err = nullptr;   // a scan's barrier wait gave up
   cudaEvent_t ev_sweep[2] = {nullptr, nullptr};  // sweep it & 1 of the logistic loop done
   unsigned char* ws = nullptr;
@@ -183,9 +183,10 @@ DevState unwritten_state() {
   return s;
 }
 
-// Clears the grid barrier's word, which a wait that gave up leaves mid-phase.
+// Clears the grid barrier's word, which a wait that gave up leaves mid-phase, and the note of
+// that beside it.
 void reset_barrier(pmcmc_handle* h) {
-  cudaMemsetAsync(h->d_bar, 0, sizeof(uint32_t), h->stream);
+  cudaMemsetAsync(h->d_bar, 0, 2 * sizeof(uint32_t), h->stream);
 }
 
 int ensure_ws(pmcmc_handle* h, size_t bytes) {

@@ -153,24 +153,36 @@ __device__ __forceinline__ double bitsd(unsigned long long b) {
 // warp by itself, and what follows runs twice in warp 0, 6 us for an apply phase of 2.6.
 // The wait is bounded (the CTAs are co-resident, so it ends far earlier); false: it gave up.
 constexpr int kBarrierSpins = 1 << 22;
+// Warp 0's part; its CTA is synchronised before and after.
+__device__ __forceinline__ bool barrier_warp(uint32_t* bar, unsigned n) {
+  uint32_t old = 0;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    old = atomicAdd(bar, blockIdx.x == 0 ? 0x80000000u - (n - 1) : 1u);
+  }
+  old = __shfl_sync(0xffffffffu, old, 0);
+  int spins = 0;
+  while (((ld_acquire(bar) ^ old) & 0x80000000u) == 0 && ++spins < kBarrierSpins) {
+  }
+  __syncwarp();
+  return spins < kBarrierSpins;
+}
 __device__ __forceinline__ bool grid_barrier(uint32_t* bar, unsigned n) {
-  __shared__ int s_gave_up;
+  __shared__ int s_met;
   __syncthreads();
   if (threadIdx.x < 32) {
-    uint32_t old = 0;
-    if (threadIdx.x == 0) {
-      __threadfence();
-      old = atomicAdd(bar, blockIdx.x == 0 ? 0x80000000u - (n - 1) : 1u);
-    }
-    old = __shfl_sync(0xffffffffu, old, 0);
-    int spins = 0;
-    while (((ld_acquire(bar) ^ old) & 0x80000000u) == 0 && ++spins < kBarrierSpins) {
-    }
-    __syncwarp();
-    if (threadIdx.x == 0) s_gave_up = spins >= kBarrierSpins;
+    const bool met = barrier_warp(bar, n);
+    if (threadIdx.x == 0) s_met = met;
   }
   __syncthreads();
-  return s_gave_up == 0;
+  return s_met != 0;
+}
+// The same for a loop over many of them: a wait that gives up sets bar[1], which the loop's
+// test reads with what else it loads.  Nothing but the host clears it.
+__device__ __forceinline__ void grid_barrier_noted(uint32_t* bar, unsigned n) {
+  __syncthreads();
+  if (threadIdx.x < 32 && !barrier_warp(bar, n) && threadIdx.x == 0) atomicExch(bar + 1, 1u);
+  __syncthreads();
 }
 
 // Inclusive scan of the affine maps x -> A[c][d] x + B[c][d] along c (columns

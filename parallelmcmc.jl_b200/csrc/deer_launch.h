@@ -94,7 +94,7 @@ cudaError_t launch_damp_metric(cudaStream_t s, bool f64, int64_t D, int64_t Dp, 
 // One look-back over `flags` (>= 1 zero word) that nothing publishes; err[0] =
 // 1 when the wait reached its bound (bound check of the scans' waits).
 cudaError_t launch_lookback_bound(cudaStream_t s, const uint32_t* flags, int* err);
-cudaError_t launch_barrier_bound(cudaStream_t s, uint32_t* bar, int* err);  // leaves *bar mid-phase
+cudaError_t launch_barrier_bound(cudaStream_t s, uint32_t* bar, int* err);  // leaves it mid-phase
 
 cudaError_t launch_broadcast(cudaStream_t s, bool f64, int64_t Dp, int64_t T, const void* x0,
                              void* S);

@@ -139,22 +139,18 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL>)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   if (threadIdx.x == 0) P = Pv;  // parameters by value: no upload before the launch
   __syncthreads();
-  // this sweep's maxima max|dS|, max|S| and the non-finite flag, as ordered bits of
-  // non-negative doubles, in two slots by sweep parity (P.part[0..5]), and whether a CTA's
-  // barrier wait gave up (P.part[6])
-  unsigned long long* red = reinterpret_cast<unsigned long long*>(P.part);
-  // One CTA (small blocks): its own barrier.  A CTA whose wait gives up publishes it and
-  // arrives at no further barrier (its phases would pair wrongly with the others'), so the
-  // others' next waits end at their bound too and every CTA leaves with the timeout status.
-  bool gave_up = false;
+  // One CTA (small blocks): its own barrier.  A wait that gives up is noted in grid_bar[1],
+  // which every CTA's stop test and the final state read: the phases pair wrongly from there
+  // on, but each wait ends at its bound and no result leaves without the timeout status.
   auto all_sync = [&]() {
-    if (gridDim.x == 1 || gave_up) {
-      __syncthreads();
-    } else if (!grid_barrier(P.grid_bar, gridDim.x)) {
-      gave_up = true;
-      if (threadIdx.x == 0) atomicExch(red + 6, 1ull);
-    }
+    if (gridDim.x == 1) __syncthreads();
+    else grid_barrier_noted(P.grid_bar, gridDim.x);
   };
+  const uint32_t* const note = P.grid_bar + 1;
+  auto timed_out = [&]() { return __ldcg(note) != 0u; };
+  // this sweep's maxima max|dS|, max|S| and the non-finite flag, as ordered
+  // bits of non-negative doubles, in two slots by sweep parity (P.part[0..5])
+  unsigned long long* red = reinterpret_cast<unsigned long long*>(P.part);
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr bool kDense = TK == kDenseGauss;
@@ -198,7 +194,7 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL>)
     // the arrival counter and the sweep maxima (the grid barriers in between
     // order these resets before every update, and after the previous block's reads)
     if (cta == 0 && tid == 0) {
-      for (int i = 0; i < 7; ++i) red[i] = 0ull;
+      for (int i = 0; i < 6; ++i) red[i] = 0ull;
       st->fin_counter = 0;
       st->n_accept = 0;
       st->min_margin_bits = dbits(INFINITY);
@@ -294,14 +290,16 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL>)
     // column) is read for the verification
     auto stop_test = [&](int k) {
       const unsigned long long* sl = red + 3 * (k & 1);
-      const double dmax = __longlong_as_double(static_cast<long long>(__ldcg(sl)));
-      const double smax = __longlong_as_double(static_cast<long long>(__ldcg(sl + 1)));
-      const bool nonfinite = __ldcg(sl + 2) != 0ull;
+      const unsigned long long b0 = __ldcg(sl), b1 = __ldcg(sl + 1), b2 = __ldcg(sl + 2);
+      const bool late = timed_out();
+      const double dmax = __longlong_as_double(static_cast<long long>(b0));
+      const double smax = __longlong_as_double(static_cast<long long>(b1));
+      const bool nonfinite = b2 != 0ull;
       metric = dmax / (P.tol_abs + P.tol_rel * smax);
       converged = metric <= 1.0;
-      status = gave_up || __ldcg(red + 6) != 0ull ? static_cast<int>(kStTimeout)
-               : nonfinite                        ? static_cast<int>(kStNonfinite)
-                                                  : 0;
+      status = late        ? static_cast<int>(kStTimeout)
+               : nonfinite ? static_cast<int>(kStNonfinite)
+                           : 0;
       const bool stop = converged || iter >= P.maxiter || status != 0;
       if (stop && cta > 0 && tid < Dp) sprev = __ldcg(Sb + (t0 - 1) * Dp + tid);
       return stop;
@@ -670,7 +668,7 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL>)
         f.epoch = st->epoch;  // look-back epochs of the per-sweep path continue
         f.iter = iter;
         f.converged = converged;
-        f.status = __ldcg(red + 6) != 0ull ? static_cast<int>(kStTimeout) : status;
+        f.status = timed_out() ? static_cast<int>(kStTimeout) : status;
         f.metric = metric;
         f.n_accept = __ldcg(tot);
         f.min_margin_bits = __ldcg(&st->min_margin_bits);
@@ -686,8 +684,9 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL>)
     // CTA has finished this one (after a wait that gave up none does: the states of the
     // blocks that never ran keep the timeout status that the host put there)
     if (bi + 1 < nblk) {
+      if (status == static_cast<int>(kStTimeout)) break;
       all_sync();
-      if (nctas > 1 && (gave_up || __ldcg(red + 6) != 0ull)) break;
+      if (nctas > 1 && timed_out()) break;
     }
   }  // blocks
 }

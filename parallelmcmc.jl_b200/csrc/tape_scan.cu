@@ -396,8 +396,8 @@ cudaError_t launch_lookback_bound(cudaStream_t s, const uint32_t* flags, int* er
 // Bound check of the grid barrier (the persistent solve, the scans, the near ties): one CTA
 // arrives at a barrier of two.
 __global__ void barrier_bound_kernel(uint32_t* bar, int* err) {
-  const bool met = grid_barrier(bar, 2);
-  if (threadIdx.x == 0) err[0] = met ? 0 : 1;
+  grid_barrier_noted(bar, 2);
+  if (threadIdx.x == 0) err[0] = __ldcg(bar + 1) != 0u ? 1 : 0;
 }
 
 cudaError_t launch_barrier_bound(cudaStream_t s, uint32_t* bar, int* err) {
