@@ -372,11 +372,14 @@ int choose_persist_tile(pmcmc_handle* h, const void* fn, bool f64, int64_t Dp, i
   }
   // A block that one CTA evaluates in two rounds at most (8 warps, 32 lanes a warp over the
   // lanes of a column) is solved by one: its sweeps need no grid barrier and no carry over
-  // CTAs (about 6 us of a 2-D block's 10.6 us a sweep; a round costs about 2).
+  // CTAs (about 6 us of a 2-D block's 10.6 us a sweep; a round costs about 2).  Dense targets
+  // up to 64 coordinates: above, a round of columns on one SM costs more than the barriers
+  // (D = 100, T = 16: 40 us a sweep, 23 on 16 CTAs; D = 256: 427 and 105).
   int lanes = 32;
   if (key.kind == kDiagGauss)
     for (lanes = 1; lanes < 16 && 4 * lanes < key.D;) lanes *= 2;
-  if (T <= std::min<int64_t>(256, 2 * kWarps * (32 / lanes))) {
+  if (T <= std::min<int64_t>(256, 2 * kWarps * (32 / lanes)) &&
+      (key.kind == kDiagGauss || key.D <= 64)) {
     const size_t smem = persist_smem(f64, Dp, static_cast<int>(T), dense).total;
     if (smem <= 200 * 1024 && max_active_blocks(fn, smem) > 0) return static_cast<int>(T);
   }
