@@ -120,17 +120,21 @@ __device__ __forceinline__ void carry_warp(int n, int d, int Dp, const Real* agg
   }
 }
 
-// Two CTAs per SM (at most 128 registers a thread) where that costs few spills:
-// FP32 state with up to two quads a lane, FP64 with one on a diagonal target.
-template <typename Real, int TK, int QPL>
+// Two CTAs per SM (at most 128 registers a thread) where that costs few spills: FP32 state
+// with up to two quads a lane, FP64 with one on a diagonal target.  Dense targets above 64
+// coordinates take one CTA an SM whatever the precision: the loads of P that their products
+// keep in flight spill under 128 registers (FP32, D = 128, T = 1024: 76 us a sweep, 46 without;
+// D = 256: 234 and 132), and their columns and P leave no more room for a second CTA's columns
+// than one has.
+template <typename Real, int TK, int QPL, int LPC>
 constexpr int kPersistMinBlocks =
-    sizeof(Real) * QPL <= 8 && !(TK == kDenseGauss && sizeof(Real) == 8) ? 2 : 1;
+    sizeof(Real) * QPL <= 8 && !(TK == kDenseGauss && (sizeof(Real) == 8 || LPC == 32)) ? 2 : 1;
 
 // Columns of a diagonal target are evaluated by LPC lanes each (32 / LPC columns per
 // warp), those of a dense one by a warp, LPC lanes for its quads and the rest for shares of
 // the sums over the coordinates; QPL quads per lane cover Dp / 4 <= LPC * QPL.
 template <typename Real, int TK, int JAC, int QPL, int LPC>
-__global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL>)
+__global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL, LPC>)
     deer_persist_kernel(const DevParams Pv, DevState* __restrict__ st) {
   __shared__ DevParams P;
   __shared__ Real s_sa[kThreads], s_sb[kThreads];
@@ -154,6 +158,7 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL>)
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr bool kDense = TK == kDenseGauss;
+  constexpr bool kWhole = kWholeColumn<Real, TK, JAC, QPL>;
   constexpr int CPW = kDense ? 1 : 32 / LPC;          // columns per warp
   const int lq = lane & (LPC - 1);                    // quad lane
   const int half = kDense ? 0 : lane / LPC;           // column slot
@@ -166,7 +171,7 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL>)
   const int ncols = static_cast<int>(imin64(TT, T - t0));  // >= 1: one CTA per tile
   const bool has_next = t0 + ncols < T;
   const int ng = has_next ? ncols : ncols - 1;  // columns of the scan group
-  Smem<Real> sm = carve<Real>(smem_raw, P, TT, kDense, true);
+  Smem<Real> sm = carve<Real>(smem_raw, P, TT, kDense, !kWhole);
   const PersistPlan pp = plan_persist_smem<Real>(Dp, TT, kDense);
   float* xis = reinterpret_cast<float*>(smem_raw + pp.xi);
   double* lus = reinterpret_cast<double*>(smem_raw + pp.lu);
@@ -228,10 +233,10 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL>)
     // group's), in FP64, one column a thread: what the evaluation compares its part of
     // log alpha with
     for (int c = tid; c <= ng; c += kThreads) {
-      double h = 0.0;
+      double h = 0.0;  // (kWhole: log alpha has the tape term itself)
       const float* n = xis + c * Dp;
 #pragma unroll 4
-      for (int d = 0; d < Dp; d += 4) {
+      for (int d = 0; d < (kWhole ? 0 : Dp); d += 4) {
         float v[4];
         load4(n + d, v);
 #pragma unroll
@@ -251,7 +256,9 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL>)
     // ---- S_0 = f(x0): the same in every sweep ----
     if (cta == 0 && warp == 0) {  // every column slot of warp 0 forms it; slot 0 stores
       Col<Real, QPL> col;
-      if constexpr (kDense) {
+      if constexpr (kWhole) {
+        persist_forward_whole<Real, QPL>(P, sm, key, x0s, xis, col);
+      } else if constexpr (kDense) {
         Real z[QPL][4], w[QPL][4], hv[QPL][4];
         persist_forward_dense<Real, JAC, QPL, LPC, false>(P, sm, mud, key, x0s, xis, 0, 0, col, z, w, hv);
       } else {
@@ -324,7 +331,13 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL>)
         Col<Real, QPL> col;
         Real A[QPL][4];
         bool acc;
-        if constexpr (kDense) {
+        if constexpr (kWhole) {
+          persist_forward_whole<Real, QPL>(P, sm, key, xcol, xic, col);
+          col.la = seg_sum<LPC>(col.la);
+          acc = logu < col.la;
+          column_jacobian<Real, TK, JAC, QPL, LPC>(P, sm, key, t + P.t_off, iter, acc,
+                                                   sigmoid_slope<Real>(col.la - logu), col, A);
+        } else if constexpr (kDense) {
           Real z[QPL][4], w[QPL][4], hv[QPL][4];
           persist_forward_dense<Real, JAC, QPL, LPC, true>(P, sm, mud, key, xcol, xic,
                                                            t + P.t_off, iter, col, z, w, hv);
@@ -565,7 +578,9 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL>)
       const Real* scol = sm.Xs + c * Dp;
       Col<Real, QPL> col;
       // log alpha reduced below with the log density and the defect (one pass)
-      if constexpr (kDense) {
+      if constexpr (kWhole) {
+        persist_forward_whole<Real, QPL>(P, sm, key, xcol, xis + c * Dp, col);
+      } else if constexpr (kDense) {
         Real z[QPL][4], w[QPL][4], hv[QPL][4];
         persist_forward_dense<Real, JAC, QPL, LPC, false>(P, sm, mud, key, xcol, xis + c * Dp,
                                                           static_cast<int>(t), 0, col, z, w, hv);
