@@ -395,6 +395,28 @@ int choose_persist_tile(pmcmc_handle* h, const void* fn, bool f64, int64_t Dp, i
   return 0;
 }
 
+// Dense targets above 64 coordinates: columns a CTA with two CTAs an SM in half the registers
+// (persist_kernel_two), 0 where the other form is no slower.  What counts is the rounds of
+// columns a warp takes, one and a half to two times fewer over 16 warps; a round then takes
+// about 1.6 times as long, and the other form is ahead where P fits beside its columns.  FP32,
+// us a sweep, one CTA an SM and two: D = 128, T = 4000 171, 122; T = 3000 115, 121; D = 200,
+// T = 4000 371, 364; T = 3000 278, 323.  FP64 (exact diagonal only: the probe's products read P
+// once for both there): D = 128, T = 6500 367, 321; T = 3000 150, 172; up to 104 coordinates
+// only where the columns leave the L1 too small for P's rows (D = 80, T = 12000 376, 301;
+// T = 10000 202, 259).
+int persist_two_tile(pmcmc_handle* h, const void* fn, bool f64, int64_t Dp, int64_t T, int TT,
+                     const TuneKey& key) {
+  if (!fn || TT <= 0 || h->tune_per_sm > 0 || tune_get(key)) return 0;
+  const PersistPlan pp = persist_smem(f64, Dp, TT, true);
+  if (pp.sweep.p_in_smem) return 0;
+  const int two = persist_tile_for(fn, f64, Dp, T, true, 2, h->num_sms);
+  auto rounds = [](int cols) { return (cols + kWarps - 1) / kWarps; };
+  const bool fewer = 10 * rounds(TT) > (f64 ? 17 : 16) * rounds(two);
+  return !f64        ? (fewer ? two : 0)
+         : Dp <= 104 ? (pp.total > 170 * 1024 ? two : 0)
+                     : (fewer && rounds(TT) >= 4 ? two : 0);
+}
+
 cudaError_t launch_sweep(const void* fn, bool coop, int grid, size_t smem, void** args,
                          cudaStream_t s) {
   if (coop)
@@ -1364,13 +1386,17 @@ int solve_core(pmcmc_handle* h, const pmcmc_target* tg, const pmcmc_deer_params*
     rc = ensure_eigen(h, const_cast<pmcmc_target*>(tg));
     if (rc) return rc;
   }
-  const SweepKernels k = logistic ? logistic_sweep_kernels(f64, D, p->jacobian)
-                                  : gauss_sweep_kernels(f64, tg->kind, p->jacobian, D);
+  SweepKernels k = logistic ? logistic_sweep_kernels(f64, D, p->jacobian)
+                            : gauss_sweep_kernels(f64, tg->kind, p->jacobian, D);
   // whole solve in one cooperative launch when every tile is co-resident
-  const int TTp = (!plain && !logistic && !full && W == T && !h->force_eager && !h->no_persist)
-                      ? choose_persist_tile(h, k.persist, f64, Dp, T, dense,
-                                            TuneKey{0, tg->kind, p->jacobian, f64, D, T})
-                      : 0;
+  const TuneKey tkey{0, tg->kind, p->jacobian, f64, D, T};
+  int TTp = (!plain && !logistic && !full && W == T && !h->force_eager && !h->no_persist)
+                ? choose_persist_tile(h, k.persist, f64, Dp, T, dense, tkey)
+                : 0;
+  if (const int two = persist_two_tile(h, k.persist_two, f64, Dp, T, TTp, tkey)) {
+    TTp = two;
+    k.persist = k.persist_two;
+  }
   const bool persist = TTp > 0;
   const TilePlan tp = full      ? TilePlan{}
                       : persist ? TilePlan{TTp, true}

@@ -20,6 +20,7 @@ struct SweepKernels {
   const void* eval = nullptr;      // (const DevParams*, const Real* Sold, int iter, int from_x0, Real* A, Real* B);
                                    // logistic: the probe accumulation (const DevParams*, const DevState*, int probe)
   const void* persist = nullptr;   // (const DevParams*, DevState*): whole solve, cooperative
+  const void* persist_two = nullptr;  // the same in half the registers, where it has its use
   int qpl = 1;
 };
 
@@ -31,6 +32,7 @@ struct PersistPlan {
 };
 PersistPlan persist_smem(bool f64, int64_t Dp, int TT, bool dense);
 const void* persist_kernel(bool f64, int tk, int jac, int64_t D);
+const void* persist_kernel_two(bool f64, int tk, int jac, int64_t D);  // nullptr: not built
 
 // Raises a kernel's dynamic shared-memory limit to at least `bytes`, never
 // lowering it: the attribute is global per function, and handles on other

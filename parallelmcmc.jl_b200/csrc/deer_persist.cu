@@ -125,16 +125,19 @@ __device__ __forceinline__ void carry_warp(int n, int d, int Dp, const Real* agg
 // coordinates take one CTA an SM whatever the precision: the loads of P that their products
 // keep in flight spill under 128 registers (FP32, D = 128, T = 1024: 76 us a sweep, 46 without;
 // D = 256: 234 and 132), and their columns and P leave no more room for a second CTA's columns
-// than one has.
-template <typename Real, int TK, int QPL, int LPC>
+// than one has.  kTwo asks for two all the
+// same (persist_two_tile in capi.cu says where).
+template <typename Real, int TK, int QPL, int LPC, bool kTwo>
 constexpr int kPersistMinBlocks =
-    sizeof(Real) * QPL <= 8 && !(TK == kDenseGauss && (sizeof(Real) == 8 || LPC == 32)) ? 2 : 1;
+    kTwo || (sizeof(Real) * QPL <= 8 && !(TK == kDenseGauss && (sizeof(Real) == 8 || LPC == 32)))
+        ? 2
+        : 1;
 
 // Columns of a diagonal target are evaluated by LPC lanes each (32 / LPC columns per
 // warp), those of a dense one by a warp, LPC lanes for its quads and the rest for shares of
 // the sums over the coordinates; QPL quads per lane cover Dp / 4 <= LPC * QPL.
-template <typename Real, int TK, int JAC, int QPL, int LPC>
-__global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL, LPC>)
+template <typename Real, int TK, int JAC, int QPL, int LPC, bool kTwo>
+__global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL, LPC, kTwo>)
     deer_persist_kernel(const DevParams Pv, DevState* __restrict__ st) {
   __shared__ DevParams P;
   __shared__ Real s_sa[kThreads], s_sb[kThreads];
@@ -158,7 +161,7 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL, LPC
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr bool kDense = TK == kDenseGauss;
-  constexpr bool kWhole = kWholeColumn<Real, TK, JAC, QPL>;
+  constexpr bool kWhole = kTwo || kWholeColumn<Real, TK, JAC, QPL>;
   constexpr int CPW = kDense ? 1 : 32 / LPC;          // columns per warp
   const int lq = lane & (LPC - 1);                    // quad lane
   const int half = kDense ? 0 : lane / LPC;           // column slot
@@ -708,9 +711,9 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL, LPC
 
 namespace {
 
-template <typename Real, int TK, int JAC, int QPL, int LPC>
+template <typename Real, int TK, int JAC, int QPL, int LPC, bool kTwo = false>
 const void* persist_fn() {
-  return reinterpret_cast<const void*>(&deer_persist_kernel<Real, TK, JAC, QPL, LPC>);
+  return reinterpret_cast<const void*>(&deer_persist_kernel<Real, TK, JAC, QPL, LPC, kTwo>);
 }
 
 // Lanes a column: as many as it has quads, rounded up to a power of two, so that a small
@@ -742,6 +745,19 @@ const void* pick_persist_t(int tk, int jac, int64_t D) {
 }
 
 }  // namespace
+
+const void* persist_kernel_two(bool f64, int tk, int jac, int64_t D) {
+  if (tk != kDenseGauss || D <= 64) return nullptr;
+  if (f64)
+    return jac == kJacStoch || D > 128 ? nullptr
+                                       : persist_fn<double, kDenseGauss, kJacDiag, 1, 32, true>();
+  if (D > 256) return nullptr;
+  if (jac == kJacStoch)
+    return D <= 128 ? persist_fn<float, kDenseGauss, kJacStoch, 1, 32, true>()
+                    : persist_fn<float, kDenseGauss, kJacStoch, 2, 32, true>();
+  return D <= 128 ? persist_fn<float, kDenseGauss, kJacDiag, 1, 32, true>()
+                  : persist_fn<float, kDenseGauss, kJacDiag, 2, 32, true>();
+}
 
 const void* persist_kernel(bool f64, int tk, int jac, int64_t D) {
   if (tk != kDiagGauss && tk != kDenseGauss) return nullptr;
