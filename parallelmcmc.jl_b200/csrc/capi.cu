@@ -347,15 +347,23 @@ void tune_put(const TuneKey& k, int v) {
   g_tune[k] = v;
 }
 
+// Shared memory of a persistent CTA whose columns, P and tape fit 200 KB, with the target's
+// tables where `per_sm` CTAs an SM leave room for them and without them else (they must cost
+// no block its CTAs an SM or its path: FP32, D = 100, T = 19828 .. 20420 went from two CTAs an
+// SM to the per-sweep graph, 1650 us for 20 sweeps instead of 575).  0: per_sm do not fit.
+size_t persist_bytes(const void* fn, const PersistPlan& p, int per_sm) {
+  if (p.tab > 200 * 1024) return 0;
+  if (max_active_blocks(fn, p.total) >= per_sm) return p.total;
+  return max_active_blocks(fn, p.tab) >= per_sm ? p.tab : 0;
+}
+
 // TT for `per_sm` co-resident CTAs a SM of the persistent solve, 0 if they do not fit.
 int persist_tile_for(const void* fn, bool f64, int64_t Dp, int64_t T, bool dense, int per_sm,
                      int num_sms) {
   const int64_t TT = (T + int64_t(per_sm) * num_sms - 1) / (int64_t(per_sm) * num_sms);
   if (TT > 256) return 0;
-  const size_t smem = persist_smem(f64, Dp, static_cast<int>(TT), dense).total;
-  if (smem > 200 * 1024) return 0;
-  const int nb = max_active_blocks(fn, smem);
-  return nb >= per_sm ? static_cast<int>(TT) : 0;
+  const PersistPlan pp = persist_smem(f64, Dp, static_cast<int>(TT), dense);
+  return persist_bytes(fn, pp, per_sm) ? static_cast<int>(TT) : 0;
 }
 
 // Columns per CTA of the persistent solve: the autotuned CTAs a SM for this
@@ -380,17 +388,14 @@ int choose_persist_tile(pmcmc_handle* h, const void* fn, bool f64, int64_t Dp, i
     for (lanes = 1; lanes < 16 && 4 * lanes < key.D;) lanes *= 2;
   if (T <= std::min<int64_t>(256, 2 * kWarps * (32 / lanes)) &&
       (key.kind == kDiagGauss || key.D <= 64)) {
-    const size_t smem = persist_smem(f64, Dp, static_cast<int>(T), dense).total;
-    if (smem <= 200 * 1024 && max_active_blocks(fn, smem) > 0) return static_cast<int>(T);
+    const PersistPlan pp = persist_smem(f64, Dp, static_cast<int>(T), dense);
+    if (persist_bytes(fn, pp, 1)) return static_cast<int>(T);
   }
   for (int per_sm = 8; per_sm >= 1; --per_sm) {
     const int64_t TT = (T + int64_t(per_sm) * h->num_sms - 1) / (int64_t(per_sm) * h->num_sms);
     if (TT > 256) break;
-    const size_t smem = persist_smem(f64, Dp, static_cast<int>(TT), dense).total;
-    if (smem > 200 * 1024) continue;
-    const int nb = max_active_blocks(fn, smem);
-    if (nb < 0) return 0;
-    if (nb >= per_sm) return static_cast<int>(TT);
+    const PersistPlan pp = persist_smem(f64, Dp, static_cast<int>(TT), dense);
+    if (persist_bytes(fn, pp, per_sm)) return static_cast<int>(TT);
   }
   return 0;
 }
@@ -1585,7 +1590,9 @@ int solve_core(pmcmc_handle* h, const pmcmc_target* tg, const pmcmc_deer_params*
          : full   ? run_full(h, k, fplan, P, eigen_view(P, tg, ws, L), F, sp_fin.total,
                              fin_grid, init_grid)
          : plain   ? run_plain(h, k, P, L, es, sp_fin.total, fin_grid, init_grid)
-         : persist ? run_persist(h, k, P, persist_smem(f64, Dp, TT, dense).total,
+         : persist ? run_persist(h, k, P,
+                                 persist_bytes(k.persist, persist_smem(f64, Dp, TT, dense),
+                                               (ntiles + h->num_sms - 1) / h->num_sms),
                                  batch ? nblocks : 1)
                    : run_fused(h, k, tp.coop, P, sp_sweep.total, sp_fin.total, fin_grid,
                                init_grid);

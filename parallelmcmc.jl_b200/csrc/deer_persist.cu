@@ -185,11 +185,19 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL, LPC
   Real* Sb = static_cast<Real*>(P.S[0]);                   // last column of every CTA
 
   Real* x0s = reinterpret_cast<Real*>(smem_raw + pp.x0);
+  // the target's tables, where the launch has shared memory for them
+  uint32_t smem_bytes;
+  asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(smem_bytes));
+  const bool has_tab = smem_bytes >= pp.total;
   DiagTab<Real> tab{};
-  [[maybe_unused]] double* mud = reinterpret_cast<double*>(smem_raw + pp.tab);
-  if constexpr (kDense)
-    for (int d = tid; d < Dp; d += kThreads) mud[d] = d < D ? P.mean_d[d] : 0.0;
-  if constexpr (!kDense && QPL <= 2) tab = fill_diag_tab<Real>(smem_raw + pp.tab, P);
+  [[maybe_unused]] const double* mud = P.mean_d;
+  if (kDense && has_tab) {
+    double* m = reinterpret_cast<double*>(smem_raw + pp.tab);
+    for (int d = tid; d < Dp; d += kThreads) m[d] = d < D ? P.mean_d[d] : 0.0;
+    mud = m;
+  }
+  if constexpr (!kDense && QPL <= 2)
+    if (has_tab) tab = fill_diag_tab<Real>(smem_raw + pp.tab, P);
   const int nblk = P.nblk > 1 ? static_cast<int>(P.nblk) : 1;
   for (int bi = 0; bi < nblk; ++bi) {  // blocks of one call, back to back
     const int64_t ncols_out = bi + 1 < nblk ? T : P.ncols_out;

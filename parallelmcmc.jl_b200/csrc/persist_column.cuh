@@ -19,7 +19,7 @@
 namespace pmcmc {
 
 // Diagonal target.  Per-coordinate constants, in shared memory (zero-padded to Dp) for
-// D <= 256; above, formed where they are used.
+// D <= 256 where they fit beside the columns (nq > 0); else, formed where they are used.
 template <typename Real>
 struct DiagTab {
   const Real *lam, *mu, *el, *k2;      // precision, mean, eps lam, eps lam^2 / 2
@@ -87,7 +87,7 @@ __device__ __forceinline__ void persist_forward_diag(const DevParams& P, const D
     float n[4];
     load4(xcol + 4 * j, c.x[q]);
     load4(xic + 4 * j, n);
-    if constexpr (kTab) {
+    if (kTab && tab.nq > 0) {
       load4(tab.lam + 4 * j, lam);
       load4(tab.mu + 4 * j, mu);
       if constexpr (sizeof(Real) == 4) {
