@@ -365,10 +365,13 @@ int pmcmc_mala_chains_adaptive(pmcmc_handle* h, const pmcmc_target* t,
  * shapes of the kernels that would solve (t, p) on x0 and keeps the fastest
  * for every later solve of the same shape (target kind, Jacobian, precision, D,
  * T), process-wide.  Candidates: CTAs a SM of the persistent solve (1..4, as
- * fit), or the :full chunk count (about sqrt(f T), f = 1/2, 1, 2, 4).  Each
- * candidate solves tape block 0 of `seed` three times (the first warms up).
- * *choice gets the kept value (0 when the path has nothing to tune) and
- * *best_ms its time.  Allocates and frees its own scratch. */
+ * fit), or the :full chunk count (about sqrt(f T), f = 1/2, 1, 2, 4); and the
+ * shape that an untuned solve takes (one CTA for a small block, the chunk count
+ * of the cost model), which later solves keep unless a candidate is faster.
+ * Each solves tape block 0 of `seed` three times (the first warms up).
+ * *choice gets the fastest candidate (0 when the path has nothing to tune) and
+ * *best_ms the time of the shape that is kept.  Allocates and frees its own
+ * scratch. */
 int pmcmc_autotune(pmcmc_handle* h, const pmcmc_target* t, const pmcmc_deer_params* p,
                    const void* x0, uint64_t seed, int32_t mem, int32_t* choice,
                    double* best_ms);

@@ -92,7 +92,7 @@ struct pmcmc_handle {
   cudaGraphConditionalHandle cond_full = 0;
   unsigned char gkey_full[512] = {};
   int full_chunks_override = 0;
-  // candidate shapes while pmcmc_autotune times them (0: none)
+  // candidate shapes while pmcmc_autotune times them (0: none, -1: the untuned shape)
   int tune_per_sm = 0;
   int tune_full_chunks = 0;
   SliceState slice;
@@ -374,7 +374,7 @@ int choose_persist_tile(pmcmc_handle* h, const void* fn, bool f64, int64_t Dp, i
                         bool dense, const TuneKey& key) {
   if (!fn || h->no_coop || h->tile_override > 0) return 0;
   if (h->tune_per_sm > 0) return persist_tile_for(fn, f64, Dp, T, dense, h->tune_per_sm, h->num_sms);
-  if (const int tuned = tune_get(key)) {
+  if (const int tuned = h->tune_per_sm < 0 ? 0 : tune_get(key)) {
     const int TT = persist_tile_for(fn, f64, Dp, T, dense, tuned, h->num_sms);
     if (TT > 0) return TT;
   }
@@ -411,7 +411,7 @@ int choose_persist_tile(pmcmc_handle* h, const void* fn, bool f64, int64_t Dp, i
 // T = 10000 202, 259).
 int persist_two_tile(pmcmc_handle* h, const void* fn, bool f64, int64_t Dp, int64_t T, int TT,
                      const TuneKey& key) {
-  if (!fn || TT <= 0 || h->tune_per_sm > 0 || tune_get(key)) return 0;
+  if (!fn || TT <= 0 || h->tune_per_sm > 0 || (h->tune_per_sm == 0 && tune_get(key))) return 0;
   const PersistPlan pp = persist_smem(f64, Dp, TT, true);
   if (pp.sweep.p_in_smem) return 0;
   const int two = persist_tile_for(fn, f64, Dp, T, true, 2, h->num_sms);
@@ -1384,6 +1384,7 @@ int solve_core(pmcmc_handle* h, const pmcmc_target* tg, const pmcmc_deer_params*
     if (W < T) return fail(h, PMCMC_ERR_UNSUPPORTED, ":full has no sliding window");
     const int nch = h->full_chunks_override > 0 ? h->full_chunks_override
                     : h->tune_full_chunks > 0   ? h->tune_full_chunks
+                    : h->tune_full_chunks < 0   ? 0
                                                 : tune_get(TuneKey{1, tg->kind, p->jacobian, 0, D, T});
     if (!full_plan(Dp, T, tg->kind, h->num_sms, nch, &fplan))
       return fail(h, PMCMC_ERR_UNSUPPORTED, ":full is built for D <= 128, got %lld",
@@ -2240,7 +2241,7 @@ int pmcmc_autotune(pmcmc_handle* h, const pmcmc_target* tg, const pmcmc_deer_par
   const int64_t D = tg->D, T = p->T;
   const bool full = p->jacobian == PMCMC_JAC_FULL;
   const bool windowed = p->window > 0 && p->window < T;
-  std::vector<int> cands;
+  std::vector<int> cands;  // and the untuned shape, -1
   TuneKey key{};
   if (full) {
     key = TuneKey{1, tg->kind, p->jacobian, 0, D, T};
@@ -2252,14 +2253,18 @@ int pmcmc_autotune(pmcmc_handle* h, const pmcmc_target* tg, const pmcmc_deer_par
              !h->force_eager && !h->no_persist && !h->no_coop && h->tile_override == 0) {
     key = TuneKey{0, tg->kind, p->jacobian, f64, D, T};
     const SweepKernels k = gauss_sweep_kernels(f64, tg->kind, p->jacobian, D);
-    for (int per_sm = 1; per_sm <= 4; ++per_sm)
-      if (persist_tile_for(k.persist, f64, tg->Dp, T, tg->kind == kDenseGauss, per_sm,
-                           h->num_sms) > 0)
-        cands.push_back(per_sm);
+    int last = 0;
+    for (int per_sm = 1; per_sm <= 4; ++per_sm) {
+      const int TT = persist_tile_for(k.persist, f64, tg->Dp, T, tg->kind == kDenseGauss, per_sm,
+                                      h->num_sms);
+      if (TT > 0 && TT != last) cands.push_back(per_sm);
+      last = TT;
+    }
   }
-  if (choice) *choice = cands.empty() ? 0 : cands.front();
+  if (choice) *choice = 0;
   if (best_ms) *best_ms = 0.0;
-  if (cands.size() < 2) return PMCMC_OK;  // nothing to choose between
+  if (cands.empty()) return PMCMC_OK;  // nothing to choose between
+  cands.insert(cands.begin(), -1);
 
   struct Scratch {
     void* buf = nullptr;
@@ -2282,8 +2287,8 @@ int pmcmc_autotune(pmcmc_handle* h, const pmcmc_target* tg, const pmcmc_deer_par
   CK(cudaMemcpyAsync(b, x0, es * D,
                      mem == PMCMC_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
                      h->stream));
-  int best = cands.front();
-  double best_t = INFINITY;
+  int best = 0;  // of the listed candidates
+  double best_t = INFINITY, untuned_t = INFINITY;
   for (const int c : cands) {
     if (full) h->tune_full_chunks = c;
     else h->tune_per_sm = c;
@@ -2300,14 +2305,16 @@ int pmcmc_autotune(pmcmc_handle* h, const pmcmc_target* tg, const pmcmc_deer_par
       CK(cudaEventElapsedTime(&ms, sc.ev[0], sc.ev[1]));
       if (rep > 0) t_min = std::min(t_min, static_cast<double>(ms));
     }
-    if (t_min < best_t) {
+    if (c < 0) {
+      untuned_t = t_min;
+    } else if (t_min < best_t) {
       best_t = t_min;
       best = c;
     }
   }
-  tune_put(key, best);
+  tune_put(key, best_t < untuned_t ? best : 0);  // 0: later solves keep the untuned shape
   if (choice) *choice = best;
-  if (best_ms) *best_ms = best_t;
+  if (best_ms) *best_ms = std::min(best_t, untuned_t);
   return PMCMC_OK;
 }
 

@@ -539,9 +539,10 @@ def solve(model: DensityModel, sampler: ParallelMALASampler, s0, *, seed: int = 
 def autotune(model: DensityModel, sampler: ParallelMALASampler, x0, *, seed: int = 0,
              handle: Optional[L.Handle] = None, device: int = 0) -> dict:
     """Time the candidate kernel shapes for this problem on the device and keep
-    the fastest for later solves of the same shape (pmcmc_autotune).  Returns
-    {"choice": kept value (CTAs a SM, or :full chunk count; 0 if nothing to
-    tune), "ms": its time a solve}."""
+    the fastest for later solves of the same shape, the untuned shape among
+    them (pmcmc_autotune).  Returns {"choice": the fastest candidate (CTAs a SM,
+    or :full chunk count; 0 if nothing to tune), kept unless the untuned shape
+    is faster, "ms": the time a solve of the kept shape}."""
     h = handle or L.default_handle(device)
     tgt = sampler.target(model, h)
     keep, x0p, mem = _input_vector(x0, model.dim, sampler.dtype, None)
