@@ -871,7 +871,7 @@ int run_logistic(pmcmc_handle* h, const pmcmc_target* tg, const SweepKernels& k,
   auto tie = [&]() -> int {
     const cudaError_t e =
         fast ? lg_finish(h->stream, h->d_params, h->d_state, P.D, P.T, G, nsplit, lp_parts, np,
-                         la_ref, tb, kTieBand, guard)
+                         la_ref, tb, kTieBand, guard, h->num_sms)
              : lg_margin(h->stream, f64, h->d_params, h->d_state, P.T, la_ref, &tb, kTieBand);
     CK(e);
     CK(lg_tie_solve(h->stream, tg->lg, h->d_params, h->d_state, la_ref, tb, kTieBand,
@@ -2124,6 +2124,7 @@ int pmcmc_target_logistic(pmcmc_handle* h, int64_t N, int64_t D, const double* X
   t->lg.D = D;
   t->lg.Dp = Dp;
   t->lg.tau = prior_prec;
+  t->lg.num_sms = h->num_sms;
   std::vector<double> x64(static_cast<size_t>(N * Dp), 0.0);
   for (int64_t i = 0; i < D; ++i)
     for (int64_t n = 0; n < N; ++n) x64[n * Dp + i] = X[i * N + n];

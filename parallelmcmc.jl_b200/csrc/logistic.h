@@ -19,6 +19,7 @@ struct LogisticDev {
   float* y32 = nullptr;
   double* y64 = nullptr;
   double tau = 1.0;
+  int num_sms = 148;  // of the target's device
   // tensor-core operands: X as FP16 hi + lo, Np x Dk (rows padded to 128,
   // columns padded to 128, 256 or 512); only built when D <= 512
   int64_t Np = 0, Dk = 0;
@@ -92,7 +93,7 @@ cudaError_t lg_tie_solve(cudaStream_t s, const LogisticDev& X, const DevParams* 
 // columns listed; lp_parts: np parts of loglik(y) (summed into lpy).
 cudaError_t lg_finish(cudaStream_t s, const DevParams* dP, const DevState* dS, int64_t D,
                       int64_t T, const float* G, int nsplit, const double* lp_parts, int np,
-                      double* la_ref, const TieBufs& b, float band, bool guard);
+                      double* la_ref, const TieBufs& b, float band, bool guard, int num_sms);
 // The sweep itself: S <- damped scan of the affine maps, the convergence test; writes the
 // state to *st_host (pinned) as well.  scratch: lg_scan_ws_bytes.
 size_t lg_scan_ws_bytes(int64_t Dp, int64_t T, int num_sms);

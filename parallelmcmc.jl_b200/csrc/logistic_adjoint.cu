@@ -554,11 +554,12 @@ struct AdjLayout {
 
 inline size_t r32(size_t n) { return (n + 31) & ~size_t(31); }
 
-AdjLayout adj_layout(int64_t N, int64_t Dp, int64_t T) {
+AdjLayout adj_layout(const LogisticDev& X, int64_t T) {
+  const int64_t N = X.N, Dp = X.Dp;
   AdjLayout a{};
   a.v = static_cast<size_t>(Dp) * T;
   a.m = static_cast<size_t>(N) * T;
-  a.gpart = std::min(148, lga::grid_for(Dp * T));  // (each ends with an atomic)
+  a.gpart = std::min(X.num_sms, lga::grid_for(Dp * T));  // (each ends with an atomic)
   const size_t t = static_cast<size_t>(T);
   a.total = 16 * r32(a.v) + 3 * r32(a.m) + 3 * r32(t) + r32(8 * t) +
             r32(2 * static_cast<size_t>(a.gpart)) + r32(8) + r32(static_cast<size_t>(Dp));
@@ -568,7 +569,7 @@ AdjLayout adj_layout(int64_t N, int64_t Dp, int64_t T) {
 }  // namespace
 
 size_t lg_adjoint_ws_bytes(const LogisticDev& X, int64_t T) {
-  return 8 * adj_layout(X.N, X.Dp, T).total;
+  return 8 * adj_layout(X, T).total;
 }
 
 namespace {
@@ -583,7 +584,7 @@ int hvp_parts(cudaStream_t s, cublasHandle_t cb, const LogisticDev& X, const dou
   if (dp <= lga::kHvMaxDp) {
     const int64_t tiles = (n + lga::kHvCols - 1) / lga::kHvCols;
     const int64_t chunks = (X.N + lga::kHvRows - 1) / lga::kHvRows;
-    const int64_t slots = 148 * (dp <= 64 ? 2 : 1);
+    const int64_t slots = X.num_sms * (dp <= 64 ? 2 : 1);
     const int64_t ns =
         std::max<int64_t>(1, std::min({slots / tiles, chunks, X.N / X.Dp, int64_t(16)}));
     double* P = ns > 1 ? L : out;
@@ -626,7 +627,7 @@ int lg_adjoint(cudaStream_t s, cublasHandle_t cb, const LogisticDev& X, bool f64
   using namespace lga;
   const int64_t Dp = X.Dp, N = X.N;
   const int D = static_cast<int>(X.D);
-  const AdjLayout Ly = adj_layout(N, Dp, T);
+  const AdjLayout Ly = adj_layout(X, T);
   const size_t v = Ly.v, m = Ly.m;
   double* p = static_cast<double*>(ws);
   double* const end = p + Ly.total;

@@ -191,10 +191,10 @@ __global__ void __launch_bounds__(kThreads, 3)
 
 cudaError_t lg_finish(cudaStream_t s, const DevParams* dP, const DevState* dS, int64_t D,
                       int64_t T, const float* G, int nsplit, const double* lp_parts, int np,
-                      double* la_ref, const TieBufs& b, float band, bool guard) {
+                      double* la_ref, const TieBufs& b, float band, bool guard, int num_sms) {
   const PassG g{G, nsplit};
   const TieList list{band, b.kmax, b.mg, b.list, b.count};
-  const int grid = static_cast<int>(imin64((T + kWarps - 1) / kWarps, 148 * 8));
+  const int grid = static_cast<int>(imin64((T + kWarps - 1) / kWarps, int64_t(num_sms) * 8));
   const auto fn = D <= 128 ? lg_finish_kernel<1> : D <= 256 ? lg_finish_kernel<2>
                                                             : lg_finish_kernel<4>;
   fn<<<grid, kThreads, 0, s>>>(dP, dS, g, lp_parts, np, la_ref, list, guard ? 1 : 0);

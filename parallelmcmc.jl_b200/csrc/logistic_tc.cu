@@ -846,11 +846,11 @@ bool lg_tc_supported(const LogisticDev& X) { return X.Xh != nullptr && encode_fn
 
 // CTAs (pairs of CTAs for D > 256) that share a 64-column tile's rows: the split with
 // the fewest steps, counted in 64-row blocks a CTA (1.6 us each at D = 256) times waves
-// of 148 CTAs (74 pairs), with about 4 blocks' time of set-up a CTA and the traffic of
+// of a CTA an SM (a pair two), with about 4 blocks' time of set-up a CTA and the traffic of
 // the split sums (at 5 TB/s).
 int lg_tc_split(const LogisticDev& X, int64_t T) {
   const int64_t tiles = (T + tc::TB - 1) / tc::TB, nb = (X.N + tc::RB - 1) / tc::RB;
-  const int64_t slots = X.Dk == 512 ? 74 : 148;
+  const int64_t slots = X.Dk == 512 ? X.num_sms / 2 : X.num_sms;
   int best = 1;
   double cost = 1e300;
   for (int s = 1; s <= 16 && s <= nb; ++s) {
