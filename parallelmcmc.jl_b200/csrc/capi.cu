@@ -778,12 +778,6 @@ constexpr float kTieBand = 1e-3f;
 constexpr int kTieMax = 256;
 int tie_kmax(int64_t T) { return static_cast<int>(std::min<int64_t>(kTieMax, T)); }
 
-// One DEER block for the logistic target: per Newton iteration two GEMM
-// passes (pass 1 at [x_bar | z], pass 2 at [y | w]) feed the fused
-// finish + scan sweep kernel.  On the fused FP32 path the columns near a tie
-// are decided in FP64 before the sweep (`refine`).  Then, on the fused path, a
-// verification pass at the returned trajectory (its passes at x_bar_t =
-// S_{t-1}: accept flags, margins, defect) and a logp pass over it.
 // The handle's cuBLAS (pedantic math, a workspace of its own so that cuBLAS
 // allocates nothing during a solve), on the handle's stream.
 int ensure_cublas(pmcmc_handle* h) {
@@ -799,6 +793,14 @@ int ensure_cublas(pmcmc_handle* h) {
   return PMCMC_OK;
 }
 
+// One DEER block for the logistic target: per Newton iteration two contraction
+// passes (pass 1 at [x_bar | z], pass 2 at [y | w]) feed the sweep: on the
+// tensor-core path with one probe the finish kernel, the near-tie decisions and
+// the chunked scan (`fast`), else the fused finish + scan sweep kernel.  On the
+// fused FP32 path the columns near a tie are decided in FP64 before the sweep
+// (`refine`).  Then, on the fused path, a verification pass at the returned
+// trajectory (its passes at x_bar_t = S_{t-1}: accept flags, margins, defect)
+// and a logp pass over it.
 int run_logistic(pmcmc_handle* h, const pmcmc_target* tg, const SweepKernels& k, bool coop,
                  DevParams P, const SolveLayout& L, size_t es, size_t smem_sweep,
                  int fin_grid, int init_grid, int64_t Tc, bool use_tc, bool plain) {
@@ -1170,7 +1172,7 @@ struct FullGraphKey {
 };
 static_assert(sizeof(FullGraphKey) <= sizeof(pmcmc_handle::gkey_full), "graph key size");
 
-// init -> rotate -> while(eval, chunk, carry, apply) -> finalize, the loop
+// init -> rotate -> while(eval, chunk, group, carry, apply) -> finalize, the loop
 // condition set by the last CTA of the apply kernel.
 int build_graph_full(pmcmc_handle* h, const FullGraphKey& key) {
   unsigned char kb[sizeof(pmcmc_handle::gkey_full)] = {};

@@ -1029,9 +1029,6 @@ size_t apply_smem(int Dq, int64_t Dp, int L) {
 
 size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 
-// lanes per column of the chunk kernel: 8 where NR stays a multiple of 4 and
-// the CTA within 544 threads
-
 template <int DQ>
 void pick_kernels(FullPlan* fp) {
   fp->chunk = reinterpret_cast<const void*>(&full_chunk_kernel<DQ>);

@@ -701,7 +701,6 @@ int lg_adjoint(cudaStream_t s, cublasHandle_t cb, const LogisticDev& X, bool f64
   // ---- Jacobi iterations on lambda_t = c_t + J_{t+1} lambda_{t+1} ----
   if (cudaMemcpyAsync(LAM, C, 8 * v, cudaMemcpyDeviceToDevice, s) != cudaSuccess) return 3;
   if (cudaMemsetAsync(s0, 0, 8 * Dp, s) != cudaSuccess) return 3;
-  if (cudaMemsetAsync(V1, 0, 8 * v, s) != cudaSuccess) return 3;
   double* HL = V1;
   double* Sr = V3;
   int k = 0;
