@@ -347,35 +347,43 @@ void tune_put(const TuneKey& k, int v) {
   g_tune[k] = v;
 }
 
-// Shared memory of a persistent CTA whose columns, P and tape fit 200 KB, with the target's
-// tables where `per_sm` CTAs an SM leave room for them and without them else (they must cost
-// no block its CTAs an SM or its path: FP32, D = 100, T = 19828 .. 20420 went from two CTAs an
-// SM to the per-sweep graph, 1650 us for 20 sweeps instead of 575).  0: per_sm do not fit.
-size_t persist_bytes(const void* fn, const PersistPlan& p, int per_sm) {
-  if (p.tab > 200 * 1024) return 0;
-  if (max_active_blocks(fn, p.total) >= per_sm) return p.total;
-  return max_active_blocks(fn, p.tab) >= per_sm ? p.tab : 0;
+// A form of the persistent solve and its shared memory.
+struct PersistForm {
+  const void* fn = nullptr;
+  size_t smem = 0;
+};
+
+// The form for `per_sm` CTAs an SM whose columns, P and tape fit 200 KB: with the diagonal
+// target's tables where they fit beside those, and without them else (they must cost no block
+// its CTAs an SM or its path: FP32, D = 100, T = 19828 .. 20420 went from two CTAs an SM to the
+// per-sweep graph, 1650 us for 20 sweeps instead of 575).  fn = NULL: per_sm do not fit.
+PersistForm persist_form(const SweepKernels& k, const PersistPlan& p, int per_sm) {
+  if (!k.persist || p.tab > 200 * 1024) return {};
+  if (max_active_blocks(k.persist, p.total) >= per_sm) return {k.persist, p.total};
+  if (k.persist_bare && max_active_blocks(k.persist_bare, p.tab) >= per_sm)
+    return {k.persist_bare, p.tab};
+  return {};
 }
 
 // TT for `per_sm` co-resident CTAs a SM of the persistent solve, 0 if they do not fit.
-int persist_tile_for(const void* fn, bool f64, int64_t Dp, int64_t T, bool dense, int per_sm,
-                     int num_sms) {
+int persist_tile_for(const SweepKernels& k, bool f64, int64_t Dp, int64_t T, bool dense,
+                     int per_sm, int num_sms) {
   const int64_t TT = (T + int64_t(per_sm) * num_sms - 1) / (int64_t(per_sm) * num_sms);
   if (TT > 256) return 0;
   const PersistPlan pp = persist_smem(f64, Dp, static_cast<int>(TT), dense);
-  return persist_bytes(fn, pp, per_sm) ? static_cast<int>(TT) : 0;
+  return persist_form(k, pp, per_sm).fn ? static_cast<int>(TT) : 0;
 }
 
 // Columns per CTA of the persistent solve: the autotuned CTAs a SM for this
 // shape when there is one, else the most CTAs a SM whose tiles all fit
 // co-resident (one cooperative launch), TT = ceil(T / (CTAs a SM x SMs)); 0
 // when none fits.
-int choose_persist_tile(pmcmc_handle* h, const void* fn, bool f64, int64_t Dp, int64_t T,
+int choose_persist_tile(pmcmc_handle* h, const SweepKernels& k, bool f64, int64_t Dp, int64_t T,
                         bool dense, const TuneKey& key) {
-  if (!fn || h->no_coop || h->tile_override > 0) return 0;
-  if (h->tune_per_sm > 0) return persist_tile_for(fn, f64, Dp, T, dense, h->tune_per_sm, h->num_sms);
+  if (!k.persist || h->no_coop || h->tile_override > 0) return 0;
+  if (h->tune_per_sm > 0) return persist_tile_for(k, f64, Dp, T, dense, h->tune_per_sm, h->num_sms);
   if (const int tuned = h->tune_per_sm < 0 ? 0 : tune_get(key)) {
-    const int TT = persist_tile_for(fn, f64, Dp, T, dense, tuned, h->num_sms);
+    const int TT = persist_tile_for(k, f64, Dp, T, dense, tuned, h->num_sms);
     if (TT > 0) return TT;
   }
   // A block that one CTA evaluates in two rounds at most (8 warps, 32 lanes a warp over the
@@ -389,13 +397,13 @@ int choose_persist_tile(pmcmc_handle* h, const void* fn, bool f64, int64_t Dp, i
   if (T <= std::min<int64_t>(256, 2 * kWarps * (32 / lanes)) &&
       (key.kind == kDiagGauss || key.D <= 64)) {
     const PersistPlan pp = persist_smem(f64, Dp, static_cast<int>(T), dense);
-    if (persist_bytes(fn, pp, 1)) return static_cast<int>(T);
+    if (persist_form(k, pp, 1).fn) return static_cast<int>(T);
   }
   for (int per_sm = 8; per_sm >= 1; --per_sm) {
     const int64_t TT = (T + int64_t(per_sm) * h->num_sms - 1) / (int64_t(per_sm) * h->num_sms);
     if (TT > 256) break;
     const PersistPlan pp = persist_smem(f64, Dp, static_cast<int>(TT), dense);
-    if (persist_bytes(fn, pp, per_sm)) return static_cast<int>(TT);
+    if (persist_form(k, pp, per_sm).fn) return static_cast<int>(TT);
   }
   return 0;
 }
@@ -409,12 +417,14 @@ int choose_persist_tile(pmcmc_handle* h, const void* fn, bool f64, int64_t Dp, i
 // once for both there): D = 128, T = 6500 367, 321; T = 3000 150, 172; up to 104 coordinates
 // only where the columns leave the L1 too small for P's rows (D = 80, T = 12000 376, 301;
 // T = 10000 202, 259).
-int persist_two_tile(pmcmc_handle* h, const void* fn, bool f64, int64_t Dp, int64_t T, int TT,
-                     const TuneKey& key) {
-  if (!fn || TT <= 0 || h->tune_per_sm > 0 || (h->tune_per_sm == 0 && tune_get(key))) return 0;
+int persist_two_tile(pmcmc_handle* h, const SweepKernels& k, bool f64, int64_t Dp, int64_t T,
+                     int TT, const TuneKey& key) {
+  if (!k.persist_two || TT <= 0 || h->tune_per_sm > 0 || (h->tune_per_sm == 0 && tune_get(key))) return 0;
   const PersistPlan pp = persist_smem(f64, Dp, TT, true);
   if (pp.sweep.p_in_smem) return 0;
-  const int two = persist_tile_for(fn, f64, Dp, T, true, 2, h->num_sms);
+  SweepKernels kt;
+  kt.persist = k.persist_two;
+  const int two = persist_tile_for(kt, f64, Dp, T, true, 2, h->num_sms);
   auto rounds = [](int cols) { return (cols + kWarps - 1) / kWarps; };
   const bool fewer = 10 * rounds(TT) > (f64 ? 17 : 16) * rounds(two);
   return !f64        ? (fewer ? two : 0)
@@ -679,13 +689,13 @@ int run_fused(pmcmc_handle* h, const SweepKernels& k, bool coop, const DevParams
 
 // One DEER block as one cooperative launch of the persistent solve kernel
 // (tape, every sweep and the verification pass; deer_persist.cu).
-int run_persist(pmcmc_handle* h, const SweepKernels& k, const DevParams& P, size_t smem,
+int run_persist(pmcmc_handle* h, const DevParams& P, const PersistForm& form,
                 int64_t nblk) {
-  CK(raise_smem_limit(k.persist, smem));
+  CK(raise_smem_limit(form.fn, form.smem));
   DevParams Pv = P;  // by value in the launch
   void* args[] = {&Pv, &h->d_state};
   if (h->profiling) CK(cudaEventRecord(h->ev[0], h->stream));
-  CK(cudaLaunchCooperativeKernel(k.persist, dim3(P.ntiles), dim3(kThreads), args, smem,
+  CK(cudaLaunchCooperativeKernel(form.fn, dim3(P.ntiles), dim3(kThreads), args, form.smem,
                                  h->stream));
   if (h->profiling) {
     CK(cudaEventRecord(h->ev[1], h->stream));
@@ -1399,9 +1409,9 @@ int solve_core(pmcmc_handle* h, const pmcmc_target* tg, const pmcmc_deer_params*
   // whole solve in one cooperative launch when every tile is co-resident
   const TuneKey tkey{0, tg->kind, p->jacobian, f64, D, T};
   int TTp = (!plain && !logistic && !full && W == T && !h->force_eager && !h->no_persist)
-                ? choose_persist_tile(h, k.persist, f64, Dp, T, dense, tkey)
+                ? choose_persist_tile(h, k, f64, Dp, T, dense, tkey)
                 : 0;
-  if (const int two = persist_two_tile(h, k.persist_two, f64, Dp, T, TTp, tkey)) {
+  if (const int two = persist_two_tile(h, k, f64, Dp, T, TTp, tkey)) {
     TTp = two;
     k.persist = k.persist_two;
   }
@@ -1593,9 +1603,9 @@ int solve_core(pmcmc_handle* h, const pmcmc_target* tg, const pmcmc_deer_params*
          : full   ? run_full(h, k, fplan, P, eigen_view(P, tg, ws, L), F, sp_fin.total,
                              fin_grid, init_grid)
          : plain   ? run_plain(h, k, P, L, es, sp_fin.total, fin_grid, init_grid)
-         : persist ? run_persist(h, k, P,
-                                 persist_bytes(k.persist, persist_smem(f64, Dp, TT, dense),
-                                               (ntiles + h->num_sms - 1) / h->num_sms),
+         : persist ? run_persist(h, P,
+                                 persist_form(k, persist_smem(f64, Dp, TT, dense),
+                                              (ntiles + h->num_sms - 1) / h->num_sms),
                                  batch ? nblocks : 1)
                    : run_fused(h, k, tp.coop, P, sp_sweep.total, sp_fin.total, fin_grid,
                                init_grid);
@@ -2258,7 +2268,7 @@ int pmcmc_autotune(pmcmc_handle* h, const pmcmc_target* tg, const pmcmc_deer_par
     const SweepKernels k = gauss_sweep_kernels(f64, tg->kind, p->jacobian, D);
     int last = 0;
     for (int per_sm = 1; per_sm <= 4; ++per_sm) {
-      const int TT = persist_tile_for(k.persist, f64, tg->Dp, T, tg->kind == kDenseGauss, per_sm,
+      const int TT = persist_tile_for(k, f64, tg->Dp, T, tg->kind == kDenseGauss, per_sm,
                                       h->num_sms);
       if (TT > 0 && TT != last) cands.push_back(per_sm);
       last = TT;

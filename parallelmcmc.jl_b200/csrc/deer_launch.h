@@ -20,7 +20,8 @@ struct SweepKernels {
   const void* eval = nullptr;      // (const DevParams*, const Real* Sold, int iter, int from_x0, Real* A, Real* B);
                                    // logistic: the probe accumulation (const DevParams*, const DevState*, int probe)
   const void* persist = nullptr;   // (const DevParams*, DevState*): whole solve, cooperative
-  const void* persist_two = nullptr;  // the same in half the registers, where it has its use
+  const void* persist_bare = nullptr;  // the same without the target's tables
+  const void* persist_two = nullptr;   // the same in half the registers, where it has its use
   int qpl = 1;
 };
 
@@ -31,7 +32,8 @@ struct PersistPlan {
   size_t xi, lu, x0, tab, total;
 };
 PersistPlan persist_smem(bool f64, int64_t Dp, int TT, bool dense);
-const void* persist_kernel(bool f64, int tk, int jac, int64_t D);
+// tables: the diagonal target's constants in shared memory (PersistPlan::total; tab without)
+const void* persist_kernel(bool f64, int tk, int jac, int64_t D, bool tables);
 const void* persist_kernel_two(bool f64, int tk, int jac, int64_t D);  // nullptr: not built
 
 // Raises a kernel's dynamic shared-memory limit to at least `bytes`, never

@@ -136,7 +136,7 @@ constexpr int kPersistMinBlocks =
 // Columns of a diagonal target are evaluated by LPC lanes each (32 / LPC columns per
 // warp), those of a dense one by a warp, LPC lanes for its quads and the rest for shares of
 // the sums over the coordinates; QPL quads per lane cover Dp / 4 <= LPC * QPL.
-template <typename Real, int TK, int JAC, int QPL, int LPC, bool kTwo>
+template <typename Real, int TK, int JAC, int QPL, int LPC, bool kTwo, bool kTables>
 __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL, LPC, kTwo>)
     deer_persist_kernel(const DevParams Pv, DevState* __restrict__ st) {
   __shared__ DevParams P;
@@ -185,19 +185,12 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL, LPC
   Real* Sb = static_cast<Real*>(P.S[0]);                   // last column of every CTA
 
   Real* x0s = reinterpret_cast<Real*>(smem_raw + pp.x0);
-  // the target's tables, where the launch has shared memory for them
-  uint32_t smem_bytes;
-  asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(smem_bytes));
-  const bool has_tab = smem_bytes >= pp.total;
   DiagTab<Real> tab{};
-  [[maybe_unused]] const double* mud = P.mean_d;
-  if (kDense && has_tab) {
-    double* m = reinterpret_cast<double*>(smem_raw + pp.tab);
-    for (int d = tid; d < Dp; d += kThreads) m[d] = d < D ? P.mean_d[d] : 0.0;
-    mud = m;
-  }
-  if constexpr (!kDense && QPL <= 2)
-    if (has_tab) tab = fill_diag_tab<Real>(smem_raw + pp.tab, P);
+  [[maybe_unused]] double* mud = reinterpret_cast<double*>(smem_raw + pp.tab);
+  constexpr bool kTab = kTables && QPL <= 2;
+  if constexpr (kDense)
+    for (int d = tid; d < Dp; d += kThreads) mud[d] = d < D ? P.mean_d[d] : 0.0;
+  if constexpr (!kDense && kTab) tab = fill_diag_tab<Real>(smem_raw + pp.tab, P);
   const int nblk = P.nblk > 1 ? static_cast<int>(P.nblk) : 1;
   for (int bi = 0; bi < nblk; ++bi) {  // blocks of one call, back to back
     const int64_t ncols_out = bi + 1 < nblk ? T : P.ncols_out;
@@ -273,7 +266,7 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL, LPC
         Real z[QPL][4], w[QPL][4], hv[QPL][4];
         persist_forward_dense<Real, JAC, QPL, LPC, false>(P, sm, mud, key, x0s, xis, 0, 0, col, z, w, hv);
       } else {
-        persist_forward_diag<Real, QPL, LPC, JAC == kJacDiag>(P, tab, x0s, xis, col);
+        persist_forward_diag<Real, QPL, LPC, JAC == kJacDiag, kTab>(P, tab, x0s, xis, col);
       }
       const bool acc = lus[0] < seg_sum<LPC>(col.la);
 #pragma unroll
@@ -358,7 +351,7 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL, LPC
                                                       sigmoid_slope<Real>(col.la - logu), col, z,
                                                       w, hv, A);
         } else {
-          persist_forward_diag<Real, QPL, LPC, JAC == kJacDiag>(P, tab, xcol, xic, col);
+          persist_forward_diag<Real, QPL, LPC, JAC == kJacDiag, kTab>(P, tab, xcol, xic, col);
           col.la = seg_sum<LPC>(col.la);
           acc = logu < col.la;
           const Real gp = sigmoid_slope<Real>(col.la - logu);
@@ -596,7 +589,7 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL, LPC
         persist_forward_dense<Real, JAC, QPL, LPC, false>(P, sm, mud, key, xcol, xis + c * Dp,
                                                           static_cast<int>(t), 0, col, z, w, hv);
       } else {
-        persist_forward_diag<Real, QPL, LPC, JAC == kJacDiag>(P, tab, xcol, xis + c * Dp, col);
+        persist_forward_diag<Real, QPL, LPC, JAC == kJacDiag, kTab>(P, tab, xcol, xis + c * Dp, col);
       }
       const double logu = lus[c];
       const bool out = valid && t < ncols_out;
@@ -707,49 +700,52 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL, LPC
       }
     }
     // the next block starts from this block's last column (x_next) once every
-    // CTA has finished this one (after a wait that gave up none does: the states of the
-    // blocks that never ran keep the timeout status that the host put there)
+    // CTA has finished this one.  After a wait that gave up, the note stops every CTA at a
+    // stop test and here, and the states of the blocks that never ran keep the timeout status
+    // that the host put there.
     if (bi + 1 < nblk) {
       if (status == static_cast<int>(kStTimeout)) break;
       all_sync();
-      if (nctas > 1 && timed_out()) break;
     }
   }  // blocks
 }
 
 namespace {
 
-template <typename Real, int TK, int JAC, int QPL, int LPC, bool kTwo = false>
+template <typename Real, int TK, int JAC, int QPL, int LPC, bool kTwo = false, bool kTables = true>
 const void* persist_fn() {
-  return reinterpret_cast<const void*>(&deer_persist_kernel<Real, TK, JAC, QPL, LPC, kTwo>);
+  return reinterpret_cast<const void*>(
+      &deer_persist_kernel<Real, TK, JAC, QPL, LPC, kTwo, kTables>);
 }
 
 // Lanes a column: as many as it has quads, rounded up to a power of two, so that a small
 // state fills the warp with columns (diagonal) or shares of its products (dense).
-template <typename Real, int TK, int JAC>
+template <typename Real, int TK, int JAC, bool kTables>
 const void* pick_persist(int64_t D) {
   if constexpr (TK == kDiagGauss) {
-    if (D <= 4) return persist_fn<Real, TK, JAC, 1, 1>();
-    if (D <= 8) return persist_fn<Real, TK, JAC, 1, 2>();
-    if (D <= 16) return persist_fn<Real, TK, JAC, 1, 4>();
-    if (D <= 32) return persist_fn<Real, TK, JAC, 1, 8>();
-    if (D <= 64) return persist_fn<Real, TK, JAC, 1, 16>();
-    if (D <= 128) return persist_fn<Real, TK, JAC, 2, 16>();
+    if (D <= 4) return persist_fn<Real, TK, JAC, 1, 1, false, kTables>();
+    if (D <= 8) return persist_fn<Real, TK, JAC, 1, 2, false, kTables>();
+    if (D <= 16) return persist_fn<Real, TK, JAC, 1, 4, false, kTables>();
+    if (D <= 32) return persist_fn<Real, TK, JAC, 1, 8, false, kTables>();
+    if (D <= 64) return persist_fn<Real, TK, JAC, 1, 16, false, kTables>();
+    if (D <= 128) return persist_fn<Real, TK, JAC, 2, 16, false, kTables>();
+    if (D <= 256) return persist_fn<Real, TK, JAC, 2, 32, false, kTables>();
+    return persist_fn<Real, TK, JAC, 4, 32>();
   } else {
     if (D <= 32) return persist_fn<Real, TK, JAC, 1, 8>();
     if (D <= 64) return persist_fn<Real, TK, JAC, 1, 16>();
     if (D <= 128) return persist_fn<Real, TK, JAC, 1, 32>();
+    return D <= 256 ? persist_fn<Real, TK, JAC, 2, 32>() : persist_fn<Real, TK, JAC, 4, 32>();
   }
-  return D <= 256 ? persist_fn<Real, TK, JAC, 2, 32>() : persist_fn<Real, TK, JAC, 4, 32>();
 }
 
-template <typename Real>
+template <typename Real, bool kTables>
 const void* pick_persist_t(int tk, int jac, int64_t D) {
   if (tk == kDiagGauss)
-    return jac == kJacStoch ? pick_persist<Real, kDiagGauss, kJacStoch>(D)
-                            : pick_persist<Real, kDiagGauss, kJacDiag>(D);
-  return jac == kJacStoch ? pick_persist<Real, kDenseGauss, kJacStoch>(D)
-                          : pick_persist<Real, kDenseGauss, kJacDiag>(D);
+    return jac == kJacStoch ? pick_persist<Real, kDiagGauss, kJacStoch, kTables>(D)
+                            : pick_persist<Real, kDiagGauss, kJacDiag, kTables>(D);
+  return jac == kJacStoch ? pick_persist<Real, kDenseGauss, kJacStoch, kTables>(D)
+                          : pick_persist<Real, kDenseGauss, kJacDiag, kTables>(D);
 }
 
 }  // namespace
@@ -767,9 +763,12 @@ const void* persist_kernel_two(bool f64, int tk, int jac, int64_t D) {
                   : persist_fn<float, kDenseGauss, kJacDiag, 2, 32, true>();
 }
 
-const void* persist_kernel(bool f64, int tk, int jac, int64_t D) {
+const void* persist_kernel(bool f64, int tk, int jac, int64_t D, bool tables) {
   if (tk != kDiagGauss && tk != kDenseGauss) return nullptr;
-  return f64 ? pick_persist_t<double>(tk, jac, D) : pick_persist_t<float>(tk, jac, D);
+  if (tables)
+    return f64 ? pick_persist_t<double, true>(tk, jac, D) : pick_persist_t<float, true>(tk, jac, D);
+  return f64 ? pick_persist_t<double, false>(tk, jac, D)
+             : pick_persist_t<float, false>(tk, jac, D);
 }
 
 }  // namespace pmcmc

@@ -873,7 +873,8 @@ SweepKernels logistic_sweep_kernels(bool f64, int64_t D, int jac) {
 SweepKernels gauss_sweep_kernels(bool f64, int tk, int jac, int64_t D) {
   const int qpl = D <= 128 ? 1 : (D <= 256 ? 2 : 4);
   SweepKernels k = f64 ? pick1<double>(tk, jac, qpl) : pick1<float>(tk, jac, qpl);
-  k.persist = persist_kernel(f64, tk, jac, D);
+  k.persist = persist_kernel(f64, tk, jac, D, true);
+  k.persist_bare = tk == kDiagGauss ? persist_kernel(f64, tk, jac, D, false) : nullptr;
   k.persist_two = persist_kernel_two(f64, tk, jac, D);
   k.qpl = qpl;
   return k;

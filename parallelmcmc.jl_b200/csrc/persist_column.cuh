@@ -19,7 +19,7 @@
 namespace pmcmc {
 
 // Diagonal target.  Per-coordinate constants, in shared memory (zero-padded to Dp) for
-// D <= 256 where they fit beside the columns (nq > 0); else, formed where they are used.
+// D <= 256 where they fit beside the columns; else, formed where they are used.
 template <typename Real>
 struct DiagTab {
   const Real *lam, *mu, *el, *k2;      // precision, mean, eps lam, eps lam^2 / 2
@@ -65,11 +65,10 @@ __device__ __forceinline__ DiagTab<Real> fill_diag_tab(unsigned char* base, cons
 // a diagonal Gaussian the gradient of log alpha in coordinate i (column_jacobian) is
 // (1 - eps lam) g_y - g_x - lam r (1 - eps lam / 2) = eps lam^2 r / 2, because
 // (1 - eps lam)(y - mu) - (x - mu) = -r; and c.gy holds eps lam.
-template <typename Real, int QPL, int LPC, bool kExact>
+template <typename Real, int QPL, int LPC, bool kExact, bool kTab>
 __device__ __forceinline__ void persist_forward_diag(const DevParams& P, const DiagTab<Real>& tab,
                                                      const Real* xcol, const float* xic,
                                                      Col<Real, QPL>& c) {
-  constexpr bool kTab = QPL <= 2;
   const int lane = threadIdx.x & (LPC - 1);
   const int D = static_cast<int>(P.D);
   const Real eps = static_cast<Real>(P.eps), c2 = static_cast<Real>(P.sqrt2eps);
@@ -87,7 +86,7 @@ __device__ __forceinline__ void persist_forward_diag(const DevParams& P, const D
     float n[4];
     load4(xcol + 4 * j, c.x[q]);
     load4(xic + 4 * j, n);
-    if (kTab && tab.nq > 0) {
+    if constexpr (kTab) {
       load4(tab.lam + 4 * j, lam);
       load4(tab.mu + 4 * j, mu);
       if constexpr (sizeof(Real) == 4) {
