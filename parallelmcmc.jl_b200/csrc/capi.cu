@@ -782,8 +782,9 @@ int run_plain(pmcmc_handle* h, const SweepKernels& k, const DevParams& P, const 
 
 // Near-tie band of the FP64 decisions of the logistic target and the most
 // columns one refinement recomputes (logistic_tie.cu).  The tensor-core
-// log alpha is off by up to ~1e-4; columns inside 1e-3 (about 60 of 65536 at
-// N = 10000, D = 256) are decided in FP64.
+// log alpha is off from FP64 by up to 4e-5 at N = 10000, D = 256 (rms 9e-6) and
+// 7e-5 at N = 20000, D = 300 (rms 1.5e-5); columns inside 1e-3 (about 60 of
+// 65536 at N = 10000, D = 256) are decided in FP64.
 constexpr float kTieBand = 1e-3f;
 constexpr int kTieMax = 256;
 int tie_kmax(int64_t T) { return static_cast<int>(std::min<int64_t>(kTieMax, T)); }

@@ -209,8 +209,10 @@ __device__ __forceinline__ float split_hi(float x) {
 // columns at first and 3.5 us with its MMAs issued back to back; this takes 2.15 us for
 // 64 rows of 64 columns (3650 cycles, of which 3072 on the tensor pipe, at the 1.7 GHz
 // the power cap leaves): a pass at N = 10000, D = 256, T = 65536 went from 4.99 and
-// 4.12 ms to 2.34 ms, 574 TFLOP/s algorithmic (8 N D T).  The TMEM datapath (A operand,
-// accumulators, the epilogue's loads) is active 88 % of the cycles of a full wave.
+// 4.12 ms to 2.34 ms, 574 TFLOP/s algorithmic (8 N D T); each row's log(1 + e) by itself in
+// the epilogue adds 1.3 % to that (3 % with NKB = 2, whose MMAs hide less of it).  The TMEM
+// datapath (A operand, accumulators, the epilogue's loads) is active 88 % of the cycles of a
+// full wave.
 //
 // Two CTAs (CL = 2): each forms the logits' sum over its half of d.  Of a warp's 16
 // rows each CTA finishes 8: it sends its part of the other 8 to the same warp of the
