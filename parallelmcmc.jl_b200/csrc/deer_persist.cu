@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(kThreads, kPersistMinBlocks<Real, TK, QPL, LPC
     auto stop_test = [&](int k) {
       const unsigned long long* sl = red + 3 * (k & 1);
       const unsigned long long b0 = __ldcg(sl), b1 = __ldcg(sl + 1), b2 = __ldcg(sl + 2);
-      const bool late = timed_out();
+      const bool late = nctas > 1 && timed_out();
       const double dmax = __longlong_as_double(static_cast<long long>(b0));
       const double smax = __longlong_as_double(static_cast<long long>(b1));
       const bool nonfinite = b2 != 0ull;
